@@ -74,9 +74,10 @@ int  ODPX_Batch_info(const ODPX_Batch *batch, int graph, int *njobs, int *nslots
  * chunk of at least 128 sources fit in one CTA's shared memory beside its
  * share of the row table, and the plan's CTAs fit on the SMs in one wave, so
  * each job runs in the small-graph kernel, on the CTAs
- * of one thread-block cluster; 0 for the persistent engine (larger or mixed
- * plans, explicit schedule settings, change tracking).  Results are the same
- * either way. */
+ * of one thread-block cluster; 0 otherwise: larger single graphs run on every
+ * SM in lockstep (ODP_GB300_SWEEP=0 turns that off), batches and plans with
+ * explicit schedule settings or change tracking in the persistent engine.
+ * Results are the same either way. */
 int  ODPX_Batch_kernel(const ODPX_Batch *batch);
 /* For a plan on the small-graph kernel: the CTAs of the thread-block cluster
  * that runs each job (1, 2, 4 or 8; each CTA computes its share of the

@@ -42,6 +42,7 @@
 #include <stdint.h>
 #include <string.h>
 #include "odp_engine.h"
+#include "odp_device.cuh"
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
@@ -53,91 +54,6 @@ namespace cg = cooperative_groups;
 #endif
 
 namespace {
-
-__device__ __forceinline__ unsigned popc4(const uint4 &v)
-{
-  return __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
-}
-
-__device__ __forceinline__ void or_into(uint4 &a, const uint4 &b)
-{
-  a.x |= b.x; a.y |= b.y; a.z |= b.z; a.w |= b.w;
-}
-
-template <typename T>
-__device__ __forceinline__ T vload(const T *p) { return *(const volatile T *)p; }
-
-__device__ __forceinline__ unsigned long long globaltimer()
-{
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-
-/* ---------------------------------------------------------------------- */
-/* Neighbour-table expansion.                                              */
-/* ---------------------------------------------------------------------- */
-
-/* ODP_ROTATE for the grid symmetries (reference utils_cuda.cu:3-14). */
-__device__ __forceinline__ int grid_rotate(int v, int width, int height, int s, int deg)
-{
-  int x = v / height, y = v % height;
-  if(s == 2) return (width - x - 1) * height + (height - y - 1);
-  if(deg == 90)  return y * height + (height - x - 1);
-  if(deg == 180) return (height - x - 1) * height + (height - y - 1);
-  return (height - y - 1) * height + x;
-}
-
-/* Row of a base-quadrant vertex (utils_cuda.cu:16-23). */
-__device__ __forceinline__ int grid_base_row(int x, int height, int s)
-{
-  if(s == 2) return x;
-  return (x / height) * (height / 2) + x % height;
-}
-
-/* Neighbour j of global vertex v of a rotation-symmetric grid
- * (utils_cuda.cu:25-59), read from the compact adjacency `adj`; -1 when the
- * stored entry is out of range. */
-__device__ __forceinline__ int grid_source_row(const gbx_expand_desc &e, int v, int &back)
-{
-  const int w = e.width, h = e.height, s = e.s;
-  int x = v / h, y = v % h, bw = w / 2, bh = h / 2;
-  if(s == 2){
-    if(x < bw){ back = 0; return v; }
-    back = 180;
-    return grid_rotate(v, w, h, s, 180);
-  }
-  if(x < bw && y < bh){ back = 0; return grid_base_row(v, h, s); }
-  if(x < bw)          { back = 90; return grid_base_row(grid_rotate(v, w, h, s, 270), h, s); }
-  if(y >= bh)         { back = 180; return grid_base_row(grid_rotate(v, w, h, s, 180), h, s); }
-  back = 270;
-  return grid_base_row(grid_rotate(v, w, h, s, 90), h, s);
-}
-
-/* Compact-adjacency position of entry j of global vertex v, and the
- * rotation that maps the stored value back (grid symmetry) or the shift
- * that does (general symmetry). */
-__device__ __forceinline__ size_t entry_source(const gbx_expand_desc &e, int v, int j, int &back)
-{
-  if(e.grid_s) return (size_t)grid_source_row(e, v, back) * e.d + j;
-  const int base = e.n / e.s;
-  back = (v / base) * base;
-  return (size_t)(v % base) * e.d + j;
-}
-
-/* Row-table entry from the stored value `a` of entry (v, j) (entries at or
- * past the vertex's degree hold the row itself, and so does an out-of-range
- * value, which also sets `bad`): the rotated vertex's row for symmetric
- * grids, the shifted vertex (mod n) for general symmetry. */
-__device__ __forceinline__ int expand_value(const gbx_expand_desc &e, int a, int back, int j, int deg, int row,
-                                            bool &bad)
-{
-  if(j >= deg) return row;
-  if(a < 0 || a >= e.n){ bad = true; return row; }
-  if(e.grid_s) return e.itable[back ? grid_rotate(a, e.width, e.height, e.s, back) : a];
-  const int nb = a + back;
-  return nb >= e.n ? nb - e.n : nb;
-}
 
 /* One descriptor per blockIdx.y: its compact adjacency, read from host
  * memory by consecutive threads in 16-byte pieces when both ends are 16-byte
@@ -1219,6 +1135,11 @@ int gbx_l2_read_probe(size_t bytes, int reps, double *gbs)
 }
 
 int gbx_malloc(void **p, size_t bytes) { return (int)cudaMalloc(p, bytes ? bytes : 256); }
+int gbx_mem_free(size_t *bytes)
+{
+  size_t total = 0;
+  return (int)cudaMemGetInfo(bytes, &total);
+}
 int gbx_free(void *p) { return p ? (int)cudaFree(p) : 0; }
 int gbx_host_alloc(void **p, size_t bytes) { return (int)cudaMallocHost(p, bytes ? bytes : 64); }
 int gbx_host_free(void *p) { return p ? (int)cudaFreeHost(p) : 0; }

@@ -104,6 +104,7 @@ int ODPX_Anneal_create(const ODPX_Chain *chains, int count, ODPX_Anneal **out)
    * SMs that hold other groups' engine CTAs: with four groups on four
    * streams, 1024-vertex chains ran at 52k instead of 121k evals/s. */
   t.small_n = 0;
+  t.sweep = 0;                        /* a step's evaluation is enqueued between its other kernels */
   if((rc = odp_plan_create(shapes, count, &t, &a->p))) goto fail;
   odp_plan *p = a->p;
   /* the starting graphs' evaluation; it also uploads and expands them */

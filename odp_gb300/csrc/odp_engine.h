@@ -120,6 +120,7 @@ typedef struct {
 /* Device / memory / stream plumbing. */
 int  gbx_device_init(int *sm_count);
 int  gbx_malloc(void **p, size_t bytes);
+int  gbx_mem_free(size_t *bytes);      /* device memory free now */
 int  gbx_free(void *p);
 int  gbx_host_alloc(void **p, size_t bytes);
 int  gbx_host_free(void *p);
@@ -189,6 +190,45 @@ int  gbx_host_device_ptr(void *host, void **dev);
 /* Allows the small-graph kernel GBX_SMALL_SMEM_MAX bytes of shared memory
  * (once per process; call before the first launch or capture). */
 int  gbx_small_prepare(void);
+
+/* One graph evaluated by all SMs in lockstep (sweep.cu): a single
+ * cooperative launch per call.  Sources are the rows below B, in row order;
+ * column chunks of 2^wc_log2 words are taken `slots` at a time by each of
+ * `phases` phases (phase p runs chunk groups p, p + phases, ...; with two
+ * phases one group's barrier is crossed while the other computes). */
+#define GBX_SWEEP_SLOTS 32
+#define GBX_SWEEP_PHASES 2
+#define GBX_SWEEP_CHUNKS 512           /* chunks of a graph, at most */
+#define GBX_SWEEP_SMEM_MAX (200 * 1024)
+#define GBX_SWEEP_TWO_LEVEL 64         /* widest row (entries) whose neighbours' lists are read for level 2 */
+#define GBX_SWEEP_TRACK_DEGREE 32      /* widest row of the tracking kernel */
+typedef struct {
+  gbx_expand_desc e;           /* adj: the caller's host array and adj_dev its device copy, or adj the
+                                  device copy already filled and adj_dev NULL */
+  const int *row_vertex;       /* device int[n] row -> vertex, or NULL: rows are vertices */
+  unsigned long long *buf;     /* [phases * slots][2][slot_words]; track: [2][slot_words] */
+  size_t slot_words;           /* words of a chunk of all rows; track: of all rows */
+  unsigned long long *start;   /* chunk c's bits of the start at start + c * start_stride */
+  size_t start_stride;
+  void *sync;                  /* gbx_sweep_sync_bytes(), zeroed once */
+  unsigned int *changed;       /* track: [2][n][2^word_log2], a bit per lane of the group */
+  gbx_small_rec *rec;          /* [nchunks], device address of pinned host memory */
+  unsigned int *abort_flag;    /* the same: GBX_ERR_TIMEOUT when a wait ran out */
+  unsigned long long limit_ns; /* longest wait of a CTA for the others */
+  int B, rows, nchunks, wc_log2, slots, phases;   /* rows: of a CTA, at most */
+  int track;                   /* grids: rows in spatial order, only changed lanes are visited */
+  int word_log2;               /* track: log2 of the changed words per row */
+  int wide;                    /* two CTAs per SM with more loads in flight each */
+  int two_level;               /* levels 1 and 2 from the neighbour lists */
+  int scratch_bits;            /* sources a warp marks at a time (a multiple of 8192, or all of them) */
+  int in_place;                /* the lists are built from the host array itself */
+  int set;                     /* which half of `sync`: alternate it from launch to launch */
+} gbx_sweep;
+size_t gbx_sweep_sync_bytes(void);
+/* Shared memory per CTA, and resident CTAs per SM with it (0: does not fit). */
+size_t gbx_sweep_smem(const gbx_sweep *a);
+int  gbx_sweep_blocks(const gbx_sweep *a, int *per_sm);
+int  gbx_sweep_launch(const gbx_sweep *a, int blocks, void *stream);
 
 /* Applies `count` writes, in stream order. */
 int  gbx_scatter(const gbx_write *d_writes, int count, void *stream);

@@ -58,6 +58,7 @@ void odp_tuning_defaults(odp_tuning *t, int batch)
   t->small_n = env_int("ODP_GB300_SMALL_N", 8192);
   t->small_cluster = env_int("ODP_GB300_SMALL_CLUSTER", 0);
   t->small_part = env_int("ODP_GB300_SMALL_PART", -1);
+  t->sweep = env_int("ODP_GB300_SWEEP", 1);
 }
 
 /* Chunk width (log2 words) for a graph whose whole level runs in shared
@@ -187,6 +188,65 @@ static void fill_degrees(const odp_shape *sh, int n, int *out)
       out[rotate_host(v, w, h, 4, 270)] = nd[i];
     }
   }
+}
+
+/* Position of cell (x, y) on the Hilbert curve over a 2^order x 2^order
+ * square (D. Hilbert, 1891): quadrant by quadrant from the coarsest, turning
+ * the square at each level so that the curve stays connected. */
+static unsigned long long hilbert_key(unsigned x, unsigned y, int order)
+{
+  unsigned long long key = 0;
+  for(int b = order - 1; b >= 0; b--){
+    const unsigned side = 1u << b, rx = (x >> b) & 1u, ry = (y >> b) & 1u;
+    key = key * 4 + (ry ? (rx ? 2 : 1) : (rx ? 3 : 0));
+    x &= side - 1;
+    y &= side - 1;
+    if(!ry){
+      if(rx){ x = side - 1 - x; y = side - 1 - y; }
+      const unsigned swap = x;
+      x = y;
+      y = swap;
+    }
+  }
+  return key;
+}
+
+typedef struct { unsigned long long key; int vertex; } curve_cell;
+
+static int cmp_curve(const void *a, const void *b)
+{
+  const unsigned long long x = ((const curve_cell *)a)->key, y = ((const curve_cell *)b)->key;
+  return (x > y) - (x < y);
+}
+
+/* Rows of a grid graph in the order of a Hilbert curve through its base
+ * region (the whole grid, the left half for s = 2, the lower-left quadrant
+ * for s = 4): vertex -> row, and row -> vertex.  The base rows come first, so
+ * the sources are rows [0, B) in curve order; the rotations of base row r
+ * are rows r + t*B, as in fill_itable. */
+static int fill_curve_rows(const odp_plan_graph *g, int *itable, int *row_vertex)
+{
+  const int bw = g->s == 1 ? g->width : g->width / 2;
+  const int bh = g->s == 4 ? g->height / 2 : g->height;
+  curve_cell *cell = malloc(sizeof(curve_cell) * (size_t)g->B);
+  if(!cell) return ODPX_ERR_MEMORY;
+  const int order = ilog2_ceil(bw > bh ? bw : bh);
+  for(int x = 0; x < bw; x++)
+    for(int y = 0; y < bh; y++){
+      curve_cell *c = &cell[(size_t)x * bh + y];
+      c->key = hilbert_key((unsigned)x, (unsigned)y, order);
+      c->vertex = x * g->height + y;
+    }
+  qsort(cell, (size_t)g->B, sizeof(curve_cell), cmp_curve);
+  for(int k = 0; k < g->B; k++)
+    for(int t = 0; t < g->s; t++){
+      const int v = t == 0 ? cell[k].vertex
+                           : rotate_host(cell[k].vertex, g->width, g->height, g->s, g->s == 2 ? 180 : 90 * t);
+      itable[v] = k + t * g->B;
+      row_vertex[k + t * g->B] = v;
+    }
+  free(cell);
+  return 0;
 }
 
 /* Source ordinals of a grid graph, ordered by square tiles of the base
@@ -390,6 +450,88 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
   return 0;
 }
 
+/* Whether a plan runs on the lockstep kernels (sweep.cu), and its shape.  One
+ * graph, no schedule setting, and a CTA's rows must fit in its shared memory
+ * beside their lane states.  Measured on GB300 against the persistent engine:
+ * n = 4096, d = 24: 27 against 67 us; n = 9999, s = 3: 48 against 108; n =
+ * 65536, d = 16: 1.65 against 2.63 ms; n = 262144, s = 64: 0.63 against 1.0;
+ * 97 x 103 grid: 0.34 against 0.76; 256 x 256: 5.3 against 18.5.
+ *  - Grids of degree up to 32 track changed lanes, 65536 sources at a time.
+ *  - Graphs whose bitset buffers take at most 64 MB, and a row 64 lanes, run
+ *    all chunks at once.  With at most one lane per thread of two CTAs per SM
+ *    they take the wide form.
+ *  - Larger ones keep the start's bits of all chunks (n * B / 8 bytes) apart
+ *    and run groups of chunks: 256-byte rows while both buffers of a chunk
+ *    stay within 70 MB, narrower above (n = 262144: 0.63 ms with 128-byte
+ *    rows, 0.94 with 256, 0.82 with 64); as many chunks in a phase as fit in
+ *    75 MB (n = 262144, two chunks of 67 MB: 1.07 ms); and two phases, one
+ *    computing while the other's barrier is crossed, where two chunks fit in
+ *    80 MB (n = 65536: two phases of two chunks 1.65 ms, of one 1.71, one
+ *    phase of two 1.69).
+ *  - Without symmetry, a compact adjacency of up to 1 MB is expanded straight
+ *    from host memory (n = 4096: 27.2 against 29.8 us); larger ones are copied
+ *    first, in wider pieces. */
+static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_sweep *sw, int *grid_out)
+{
+  const ODPX_Tune_entry *te = table_lookup(shape_n(sh), sh->degree, sh->grid);
+  if(!t->sweep || t->wc_log2 > 0 || t->slots > 0 || t->tile_rows > 0 || t->local_kb_explicit || t->blocks > 0 ||
+     t->activity != -2 || (te && (te->wc_log2 > 0 || te->tile_kb > 0 || te->local_kb > 0)))
+    return 0;
+  const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
+  memset(sw, 0, sizeof(*sw));
+  sw->e.dp = shape_dp(sh);
+  sw->B = n / sh->symmetries;
+  sw->phases = 1;
+  sw->track = sh->grid && sw->e.dp <= GBX_SWEEP_TRACK_DEGREE;
+  sw->two_level = sw->e.dp <= GBX_SWEEP_TWO_LEVEL;
+  sw->in_place = !sh->grid && sh->symmetries == 1 && (double)n * sh->degree * 4 <= 1e6;
+  sw->scratch_bits = sw->B <= 32768 ? (sw->B + 255) / 256 * 256 : 32768;
+  if(sw->track){
+    sw->wc_log2 = full_l2 < 5 ? full_l2 : 5;
+    sw->slots = (W + (1 << sw->wc_log2) - 1) >> sw->wc_log2;
+    if(sw->slots > GBX_SWEEP_SLOTS) sw->slots = GBX_SWEEP_SLOTS;
+  }
+  else if(16.0 * n * W <= 64e6 && W <= 256){
+    sw->wc_log2 = full_l2 < 6 ? full_l2 : 6;
+    sw->slots = (W + (1 << sw->wc_log2) - 1) >> sw->wc_log2;
+    sw->wide = (double)n * ((W + 3) / 4) <= 2.0 * 256 * sms;
+  }
+  else{
+    int wl = full_l2 < 5 ? full_l2 : 5;
+    while(wl > 2 && 16.0 * n * (1 << wl) > 70e6) wl--;
+    const double pair = 16.0 * n * (1 << wl);            /* both buffers of a chunk */
+    const int chunks = (W + (1 << wl) - 1) >> wl;
+    sw->phases = 2.0 * pair <= 80e6 && chunks > 1 ? 2 : 1;
+    int q = (int)(75e6 / pair);
+    if(q > (chunks + sw->phases - 1) / sw->phases) q = (chunks + sw->phases - 1) / sw->phases;
+    if(q > 8) q = 8;
+    sw->slots = q < 1 ? 1 : q;
+    sw->wc_log2 = wl;
+  }
+  sw->nchunks = (W + (1 << sw->wc_log2) - 1) >> sw->wc_log2;
+  if(sw->nchunks > GBX_SWEEP_CHUNKS) return 0;
+  for(int per_sm = sw->track || sw->wide ? 2 : 4; per_sm >= 1; per_sm--)
+    for(int q = sw->slots; q >= 1; q = q > 1 ? (q + 1) / 2 : 0){
+      gbx_sweep c = *sw;
+      int fit = 0;
+      c.slots = q;
+      c.rows = (n + per_sm * sms - 1) / (per_sm * sms);
+      while((32 << c.word_log2) < (q << (c.wc_log2 - 2))) c.word_log2++;
+      if(gbx_sweep_blocks(&c, &fit) == 0 && fit >= per_sm){
+        /* bitsets that would take more than half of the free memory are left
+         * to the engine, whose slots hold a few chunks only */
+        const double bitsets = 16.0 * n * c.phases * q * (1 << c.wc_log2) + (c.track ? 0.0 : 8.0 * n * W);
+        size_t room = 0;
+        if(gbx_mem_free(&room) || bitsets > 0.5 * (double)room) return 0;
+        *sw = c;
+        *grid_out = (n + c.rows - 1) / c.rows;
+        return 1;
+      }
+      if(!sw->track) break;
+    }
+  return 0;
+}
+
 #define CK(call) do{ int _e = (call); if(_e){ rc = ODPX_ERR_CUDA; goto fail; } }while(0)
 
 int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning, odp_plan **out)
@@ -420,6 +562,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   int *small_wl = calloc((size_t)count, sizeof(int));
   int small = choose_small(shapes, count, tuning, sms, small_wl, &p->small_cluster, &p->small_threads,
                            &p->small_smem, &p->small_part);
+  p->sweep = !small && count == 1 && choose_sweep(shapes, tuning, sms, &p->sw, &p->sweep_grid);
 
   /* Shapes, chunk widths, tiles. */
   int njobs = 0;
@@ -457,12 +600,13 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
     if(wl > 7) wl = 7;                 /* rows of at most 1 KB per chunk */
     if(wl > full_l2 && full_l2 >= 1) wl = full_l2;
     if(small) wl = small_wl[i];
+    if(p->sweep) wl = p->sw.wc_log2;
     g->wc_log2 = wl;
     const int wc = 1 << wl;
     g->nchunks = (g->W + wc - 1) / wc;
     g->has_ndeg = sh->num_degrees != NULL;
-    g->has_itable = g->grid_s;
-    g->has_srcpos = sh->grid;             /* grids: spatially compact source chunks */
+    g->has_itable = g->grid_s || (p->sweep && sh->grid);   /* the lockstep kernel's grid rows follow a curve */
+    g->has_srcpos = sh->grid && !p->sweep;   /* grids: spatially compact source chunks */
     g->adj_ints = (size_t)g->B * g->d;
     g->adj_off = p->adj_ints;       p->adj_ints += ALIGN_UP(g->adj_ints, 4);
     g->ndeg_off = p->ndeg_ints;     if(g->has_ndeg) p->ndeg_ints += ALIGN_UP((size_t)g->n, 4);
@@ -522,6 +666,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
       int tr = (int)(tile_bytes / per_row);
       g->tile_rows = ALIGN_UP(tr < rpp ? rpp : tr, rpp);
     }
+    if(p->sweep) g->tile_rows = p->sw.rows;
     if(g->tile_rows > g->n) g->tile_rows = g->n;
     if(g->tile_rows < 1) g->tile_rows = 1;
     g->ntiles = (g->n + g->tile_rows - 1) / g->tile_rows;
@@ -582,6 +727,8 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
     if(count > 1 && nslots < 64) nslots = 64;
     if(nslots > 512) nslots = 512;
   }
+  if(p->sweep) nslots = p->sw.phases * p->sw.slots;
+  const size_t buffers = (size_t)nslots;
   if(nslots > njobs) nslots = njobs;
   if(nslots < 1) nslots = 1;
   p->nslots = nslots;
@@ -600,7 +747,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   if(p->ndeg_ints) CK(gbx_malloc((void **)&p->d_ndeg, sizeof(int) * p->ndeg_ints));
   if(p->itable_ints) CK(gbx_malloc((void **)&p->d_itable, sizeof(int) * p->itable_ints));
   CK(gbx_malloc((void **)&p->d_nbr, sizeof(int) * (p->nbr_ints ? p->nbr_ints : 4)));
-  CK(gbx_malloc((void **)&p->d_slotbuf, sizeof(unsigned long long) * p->slot_words * 2 * (size_t)nslots));
+  CK(gbx_malloc((void **)&p->d_slotbuf, sizeof(unsigned long long) * p->slot_words * 2 * (p->sweep ? buffers : (size_t)nslots)));
   CK(gbx_malloc((void **)&p->d_slotmask, sizeof(unsigned int) * p->slot_rows * 2 * (size_t)nslots));
   if(p->srcpos_ints) CK(gbx_malloc((void **)&p->d_srcpos, sizeof(int) * p->srcpos_ints));
   CK(gbx_malloc((void **)&p->d_expand, sizeof(gbx_expand_desc) * (size_t)count));
@@ -609,9 +756,24 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   p->direct = tuning->direct && gbx_pageable_access();
   /* Small plans read their descriptors (and through them the adjacency)
    * from pinned host memory and write per-job records there. */
-  if(p->direct || small) CK(gbx_host_alloc((void **)&p->h_expand, sizeof(gbx_expand_desc) * (size_t)count));
+  if(p->direct || small || p->sweep) CK(gbx_host_alloc((void **)&p->h_expand, sizeof(gbx_expand_desc) * (size_t)count));
   if(!p->direct) CK(gbx_host_alloc((void **)&p->h_adj, sizeof(int) * (p->adj_ints ? p->adj_ints : 4)));
-  if(small){
+  if(p->sweep){
+    CK(gbx_host_alloc((void **)&p->h_small_rec, sizeof(gbx_small_rec) * (size_t)njobs));
+    memset(p->h_small_rec, 0, sizeof(gbx_small_rec) * (size_t)njobs);
+    CK(gbx_host_device_ptr(p->h_small_rec, (void **)&p->d_small_rec));
+    CK(gbx_host_alloc((void **)&p->h_abort, sizeof(unsigned int)));
+    *p->h_abort = 0;
+    CK(gbx_host_device_ptr(p->h_abort, (void **)&p->sw.abort_flag));
+    CK(gbx_malloc(&p->d_sync, gbx_sweep_sync_bytes()));
+    CK(gbx_memset(p->d_sync, 0, gbx_sweep_sync_bytes(), p->stream));
+    if(p->sw.track)
+      CK(gbx_malloc((void **)&p->d_changed, sizeof(unsigned int) * 2 * ((size_t)p->g[0].n << p->sw.word_log2)));
+    else if(njobs > p->sw.phases * p->sw.slots)   /* more than one group: the start's bits of every chunk apart */
+      CK(gbx_malloc((void **)&p->d_start, sizeof(unsigned long long) * p->slot_words * (size_t)njobs));
+    if(p->g[0].has_itable) CK(gbx_malloc((void **)&p->d_row_vertex, sizeof(int) * (size_t)p->g[0].n));
+  }
+  else if(small){
     CK(gbx_host_alloc((void **)&p->h_small_rec, sizeof(gbx_small_rec) * (size_t)njobs));
     memset(p->h_small_rec, 0, sizeof(gbx_small_rec) * (size_t)njobs);
     CK(gbx_host_device_ptr(p->h_small_rec, (void **)&p->d_small_rec));
@@ -625,6 +787,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   }
   CK(gbx_host_alloc((void **)&p->h_state_init, p->state_bytes));
   CK(gbx_host_alloc((void **)&p->h_state_out, p->out_bytes));
+  memset(p->h_state_out, 0, p->out_bytes);
 
   /* Static tables: degrees, row tables, expand descriptors, jobs. */
   {
@@ -641,7 +804,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
         for(int v = 0; v < g->n; v++) g->row_reads += (double)h_nd[g->ndeg_off + v] + 2.0;
       }
       else g->row_reads = (double)g->n * (g->d + 2);
-      if(g->has_itable) fill_itable(g->width, g->height, g->s, h_it + g->itable_off);
+      if(g->has_itable && !p->sweep) fill_itable(g->width, g->height, g->s, h_it + g->itable_off);
       if(g->has_srcpos) fill_srcpos(g, h_sp + g->srcpos_off);
       gbx_expand_desc *e = &ed[i];
       e->adj = p->d_adj + g->adj_off;
@@ -658,11 +821,45 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
       p->h_jobs[k].nbr = p->d_nbr + g->nbr_off;
       p->h_jobs[k].srcpos = g->has_srcpos ? p->d_srcpos + g->srcpos_off : NULL;
     }
+    if(p->sweep && p->g[0].has_itable){
+      int *h_rv = malloc(sizeof(int) * (size_t)p->g[0].n);
+      rc = h_rv ? fill_curve_rows(&p->g[0], h_it, h_rv) : ODPX_ERR_MEMORY;
+      if(!rc && (gbx_memcpy_h2d(p->d_row_vertex, h_rv, sizeof(int) * (size_t)p->g[0].n, p->stream) ||
+                 gbx_stream_sync(p->stream)))
+        rc = ODPX_ERR_CUDA;
+      free(h_rv);
+      if(rc){
+        free(h_nd); free(h_it); free(h_sp); free(ed);
+        goto fail;
+      }
+    }
     if(h_sp) CK(gbx_memcpy_h2d(p->d_srcpos, h_sp, sizeof(int) * p->srcpos_ints, p->stream));
     if(h_nd) CK(gbx_memcpy_h2d(p->d_ndeg, h_nd, sizeof(int) * p->ndeg_ints, p->stream));
     if(h_it) CK(gbx_memcpy_h2d(p->d_itable, h_it, sizeof(int) * p->itable_ints, p->stream));
     CK(gbx_memcpy_h2d(p->d_expand, ed, sizeof(gbx_expand_desc) * (size_t)count, p->stream));
-    if(small){
+    if(p->sweep){
+      /* the launch carries the descriptor: per call `adj` names the caller's
+       * array, which the kernel copies to `adj_dev`; without direct reads the
+       * call uploads it and `adj` names the device copy */
+      p->h_expand[0] = ed[0];
+      p->h_expand[0].adj_dev = p->direct ? (int *)ed[0].adj : NULL;
+      gbx_sweep *w = &p->sw;
+      w->row_vertex = p->d_row_vertex;
+      w->buf = p->d_slotbuf;
+      w->slot_words = p->slot_words * (w->track ? (size_t)w->slots : 1);
+      if(p->d_start){
+        w->start = p->d_start;
+        w->start_stride = p->slot_words;
+      }
+      else{                            /* the buffer that the first gathered level reads */
+        w->start = p->d_slotbuf + (w->two_level ? 0 : p->slot_words);
+        w->start_stride = 2 * p->slot_words;
+      }
+      w->sync = p->d_sync;
+      w->changed = p->d_changed;
+      w->rec = p->d_small_rec;
+    }
+    else if(small){
       /* the small-graph kernel reads `adj` itself: the caller's array (set
        * per call) or this plan's pinned staging copy */
       memcpy(p->h_expand, ed, sizeof(gbx_expand_desc) * (size_t)count);
@@ -704,6 +901,8 @@ void odp_plan_destroy(odp_plan *p)
   gbx_free(p->d_state_init);
   gbx_host_free(p->h_adj); gbx_host_free(p->h_expand); gbx_host_free(p->h_state_init); gbx_host_free(p->h_state_out);
   gbx_host_free(p->h_small_rec);
+  gbx_free(p->d_row_vertex); gbx_free(p->d_changed); gbx_free(p->d_sync); gbx_free(p->d_start);
+  gbx_host_free(p->h_abort);
   if(p->stream) gbx_stream_destroy(p->stream);
   free(p->h_jobs);
   free(p->g);
@@ -716,6 +915,16 @@ static int enqueue(odp_plan *p)
 {
   int e;
   if(p->small) return odp_plan_enqueue_engine(p);
+  if(p->sweep){
+    if(!p->direct &&
+       (e = gbx_memcpy_h2d(p->d_adj, p->h_adj, sizeof(int) * (p->adj_ints ? p->adj_ints : 4), p->stream)))
+      return e;
+    p->sw.e = p->h_expand[0];
+    p->sw.limit_ns = p->spin_limit_ns;
+    if((e = gbx_sweep_launch(&p->sw, p->sweep_grid, p->stream))) return e;
+    p->sw.set ^= 1;                    /* this launch clears the other half of the counters for the next */
+    return 0;
+  }
   if(p->direct){
     /* one kernel: this call's descriptors (their host pointers) from pinned
      * memory, the callers' arrays into the device copy that expand reads,
@@ -818,8 +1027,8 @@ void odp_plan_stage(odp_plan *p, const int *const *adjacency)
 
 int odp_plan_launch(odp_plan *p)
 {
-  /* a single-graph small plan passes this call's descriptor by value: never captured */
-  if(p->tuning.use_graph && !(p->small && p->ngraphs == 1)){
+  /* single-graph plans of one kernel pass this call's descriptor by value: never captured */
+  if(p->tuning.use_graph && !p->sweep && !(p->small && p->ngraphs == 1)){
     if(!p->graph_exec){
       if(gbx_capture_begin(p->stream)) return ODPX_ERR_CUDA;
       int e = enqueue(p);
@@ -876,7 +1085,7 @@ static int reorder_by_duration(odp_plan *p)
   return 0;
 }
 
-/* Small plans: the per-job records folded per graph, as the engine's
+/* Plans of one kernel: the per-job records folded per graph, as the engine's
  * accumulators fold them (sum of the jobs' sums, the largest level, stalled
  * if any job stalled); the levels and stamps also go to the per-job outcome
  * table that the introspection calls read. */
@@ -921,7 +1130,11 @@ static int finish_small(odp_plan *p, odp_result *results)
 int odp_plan_finish(odp_plan *p, odp_result *results)
 {
   if(gbx_stream_sync(p->stream)) return ODPX_ERR_CUDA;
-  if(p->small) return finish_small(p, results);
+  if(p->sweep && *p->h_abort){
+    *p->h_abort = 0;
+    return ODPX_ERR_TIMEOUT;
+  }
+  if(p->small || p->sweep) return finish_small(p, results);
   const gbx_ctrl *ctrl = (const gbx_ctrl *)p->h_state_out;
   unsigned int err = *(const unsigned int *)(p->h_state_out + sizeof(gbx_ctrl)) | ctrl->error;
   if(err & GBX_ERR_TIMEOUT) return ODPX_ERR_TIMEOUT;
@@ -965,8 +1178,8 @@ unsigned long long odp_plan_tiles(const odp_plan *p)
 
 unsigned int odp_plan_error(const odp_plan *p)
 {
-  if(p->small){
-    unsigned int err = 0;
+  if(p->small || p->sweep){
+    unsigned int err = p->sweep ? *p->h_abort : 0;
     for(int k = 0; k < p->njobs; k++) err |= p->h_small_rec[k].err;
     return err;
   }

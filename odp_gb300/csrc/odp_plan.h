@@ -35,6 +35,7 @@ typedef struct {
   int small_n;                 /* graphs of at most this many vertices may run in shared memory (0: never) */
   int small_cluster;           /* CTAs per small-kernel job: 1, 2, 4 or 8; 0 = automatic */
   int small_part;              /* small-kernel rows partitioned over the cluster: -1 when needed, 0 never, 1 always */
+  int sweep;                   /* single graphs run in lockstep on every SM where that fits (1, default) */
 } odp_tuning;
 
 typedef struct {
@@ -86,6 +87,14 @@ typedef struct odp_plan {
   gbx_small_rec *h_small_rec;  /* small plans: per-job records, pinned; the kernel writes them */
   gbx_small_rec *d_small_rec;  /*   the same memory, as the device addresses it */
   gbx_expand_desc *d_small_desc; /* small plans: h_expand as the device addresses it */
+  int sweep;                   /* the plan's one graph runs in the lockstep kernel */
+  gbx_sweep sw;                /* its launch arguments */
+  int sweep_grid;              /* CTAs */
+  unsigned long long *d_start; /* the start's bits of all chunks, where the slots hold only some */
+  int *d_row_vertex;           /* row -> vertex where the plan orders the rows */
+  unsigned int *d_changed;     /* the lockstep kernel's changed-lane masks */
+  void *d_sync;                /* its counters */
+  unsigned int *h_abort;       /* pinned: set when one of its waits ran out */
 } odp_plan;
 
 typedef struct {

@@ -1,0 +1,890 @@
+/*
+ * sweep.cu -- one graph per call, evaluated by every SM in lockstep.
+ *
+ * The persistent engine (aspl_engine.cu) hands every level of every job out
+ * in tiles through a ticket.  That suits many uneven graphs, but a single
+ * graph pays about 10 us per level for it on GB300 (read the ticket, fence,
+ * read the slot, stage the neighbour lists, gather, count, fence, close),
+ * where the level's traffic takes 1 to 5 us for a few thousand vertices.
+ * Here the rows are split over the CTAs once: each CTA keeps its rows'
+ * neighbour lists in shared memory for the whole call, and a level is one
+ * pass over its own rows and one grid-wide barrier, whose word also carries
+ * the level's bit count.  A call is one cooperative launch (all CTAs are
+ * resident, so they may wait for one another; every wait has a time limit).
+ *
+ * The unit of work is a lane: 32 bytes of a row (256 sources, one sector),
+ * moved by one 256-bit access.
+ *
+ * sweep_dense_kernel (general graphs): levels 1 and 2 come from the neighbour
+ * lists, marked in shared memory and stored once; from level 3 on every lane
+ * that is not full gathers, and stops as soon as it is.
+ *
+ * sweep_track_kernel (grids): rows and sources follow a Hilbert curve, so the
+ * 256 sources of a lane lie close together and a row's lane changes in a few
+ * levels only.  Every row keeps one bit per lane, "changed at this level"
+ * (65536 sources: one 32-byte sector per row); a lane with no changed
+ * neighbour is not visited, and one that is gathers its changed neighbours
+ * alone.
+ */
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdint.h>
+#include "odp_engine.h"
+#include "odp_device.cuh"
+
+#define SWEEP_THREADS 256
+#define SWEEP_WARPS (SWEEP_THREADS / 32)
+#define SWEEP_SLOTS GBX_SWEEP_SLOTS   /* column chunks a phase runs at once, at most */
+
+#define LANE_FULL 1u                  /* every source bit of the lane is set */
+#define LANE_CHANGED 2u               /* the older buffer does not hold the lane's words yet */
+
+#define ARRIVE_ONE (1ull << 48)       /* barrier words: CTAs done << 48 | bits counted */
+#define ARRIVE_BITS (ARRIVE_ONE - 1)
+
+namespace {
+
+/* Counters of one call; the call before clears them. */
+struct SweepSync {
+  unsigned ready[3];                                 /* CTAs past the copy, the expansion, the start */
+  unsigned err;                                      /* GBX_ERR_* */
+  unsigned pad[28];
+  unsigned long long arrive[GBX_SWEEP_PHASES][3][16];           /* step t's barrier word: [t % 3][0] */
+  unsigned long long count[GBX_SWEEP_PHASES][3][SWEEP_SLOTS];   /* bits per chunk of step t */
+  unsigned long long start1[GBX_SWEEP_CHUNKS], start2[GBX_SWEEP_CHUNKS];  /* bits at levels 1 and 2 */
+};
+
+/* A phase's progress, the same in every CTA but for `prev`, `sum` and
+ * `alive`, which CTA 0 keeps for the records. */
+struct SweepPhase {
+  unsigned long long total, full;                    /* bits set at the last level; bits of a complete group */
+  unsigned long long t_loaded;
+  int level, group;                                  /* level < 0: no group left */
+  unsigned step, alive;
+  unsigned long long prev[SWEEP_SLOTS];
+  long long sum[SWEEP_SLOTS];
+};
+
+struct SweepShared {
+  SweepPhase ph[GBX_SWEEP_PHASES];
+  unsigned cnt[SWEEP_SLOTS];                         /* this CTA's bits per chunk of the current step */
+  int todo;
+};
+
+#define TODO_DONE 0
+#define TODO_LEVEL 1
+#define TODO_ABORT 2
+
+__device__ __forceinline__ void ld_lane(unsigned (&r)[8], const void *p)
+{
+  asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "l"(p) : "memory");
+}
+
+__device__ __forceinline__ void st_lane(void *p, const unsigned (&r)[8])
+{
+  asm volatile("st.global.cg.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+               :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "l"(p)
+               : "memory");
+}
+
+/* Set bits of eight words: full adders (one three-input operation for each
+ * sum and carry) reduce them to four words of weights 1, 1, 2 and 4, as the
+ * bit count runs at a quarter of the logic's rate. */
+__device__ __forceinline__ unsigned popc_lane(const unsigned (&r)[8])
+{
+  const unsigned s1 = r[0] ^ r[1] ^ r[2], c1 = (r[0] & r[1]) | (r[2] & (r[0] | r[1]));
+  const unsigned s2 = r[3] ^ r[4] ^ r[5], c2 = (r[3] & r[4]) | (r[5] & (r[3] | r[4]));
+  const unsigned s3 = s1 ^ s2 ^ r[6], c3 = (s1 & s2) | (r[6] & (s1 | s2));
+  const unsigned t1 = c1 ^ c2 ^ c3, f1 = (c1 & c2) | (c3 & (c1 | c2));
+  return __popc(s3) + __popc(r[7]) + 2 * __popc(t1) + 4 * __popc(f1);
+}
+
+__device__ __forceinline__ unsigned and_lane(const unsigned (&r)[8])
+{
+  return r[0] & r[1] & r[2] & r[3] & r[4] & r[5] & r[6] & r[7];
+}
+
+/* One thread waits until `*word` reaches `target`; false past the limit. */
+template <typename T>
+__device__ __forceinline__ bool wait_for(const T *word, T target, T &seen, unsigned long long limit_ns)
+{
+  seen = vload(word);
+  if(seen < target){
+    const unsigned long long t0 = globaltimer();
+    do{
+      if(globaltimer() - t0 > limit_ns) return false;
+      seen = vload(word);
+    } while(seen < target);
+  }
+  __threadfence();
+  return true;
+}
+
+/* The whole grid passes; false (in every thread) past the limit. */
+__device__ __forceinline__ bool grid_pass(unsigned *word, SweepShared &sh, const gbx_sweep &a)
+{
+  __syncthreads();
+  if(threadIdx.x == 0){
+    unsigned seen;
+    __threadfence();
+    atomicAdd(word, 1u);
+    const bool ok = wait_for(word, gridDim.x, seen, a.limit_ns);
+    sh.todo = ok ? TODO_LEVEL : TODO_ABORT;
+    if(!ok) *a.abort_flag = GBX_ERR_TIMEOUT;           /* pinned host memory */
+  }
+  __syncthreads();
+  const bool ok = sh.todo != TODO_ABORT;
+  __syncthreads();                                     /* read before it is written again */
+  return ok;
+}
+
+__device__ __forceinline__ int lane_bits(int nsrc, int gl) { return min(max(nsrc - 256 * gl, 0), 256); }
+
+/* Sources of chunk c. */
+__device__ __forceinline__ int chunk_sources(const gbx_sweep &a, int c)
+{
+  const int C = 64 << a.wc_log2;
+  return c < a.nchunks ? min(C, a.B - c * C) : 0;
+}
+
+/* First chunk of the phase's group. */
+__device__ __forceinline__ int group_chunk(const gbx_sweep &a, int group, int ph)
+{
+  return (group * a.phases + ph) * a.slots;
+}
+
+/* A chunk's bits after `level` (CTA 0, the thread of the chunk): records the
+ * chunk when it is complete or stalled (then false), else adds the level's
+ * share of the distance sum. */
+__device__ __forceinline__ bool settle(const gbx_sweep &a, SweepPhase &p, const SweepSync &sy, int chunk, int q,
+                                       int level, unsigned long long c)
+{
+  const unsigned long long full = (unsigned long long)a.e.n * (unsigned long long)chunk_sources(a, chunk);
+  const bool complete = c == full;
+  const bool stalled = !complete && (c == p.prev[q] || level >= a.e.n);
+  if(!complete && !stalled){
+    p.sum[q] += (long long)(full - c) * a.e.s;
+    p.prev[q] = c;
+    return true;
+  }
+  gbx_small_rec r;
+  r.level = stalled ? -level : level;
+  r.err = __ldcg(&sy.err);
+  r.sum = p.sum[q];
+  r.t_loaded = p.t_loaded;
+  r.t_done = globaltimer();
+  a.rec[chunk] = r;
+  return false;
+}
+
+/* CTA 0, warp 0: the chunks' counts of step `step`, which ended `level`.
+ * `added`: the counts are of bits added. */
+__device__ __forceinline__ void settle_step(const gbx_sweep &a, SweepPhase &p, const SweepSync &sy, int ph,
+                                            unsigned step, int level, bool added)
+{
+  const int q = threadIdx.x;
+  bool go = (p.alive >> q) & 1u;
+  if(go){
+    unsigned long long c = __ldcg(&sy.count[ph][step % 3][q]);
+    if(added) c += p.prev[q];
+    go = settle(a, p, sy, group_chunk(a, p.group, ph) + q, q, level, c);
+  }
+  const unsigned alive = __ballot_sync(0xffffffffu, go);
+  if(q == 0) p.alive = alive;
+  __syncwarp();
+}
+
+/* Warp 0: a phase's state at the start of a group (no level counted yet). */
+__device__ __forceinline__ void group_state(const gbx_sweep &a, SweepPhase &p, int ph, int group)
+{
+  const int q = threadIdx.x;
+  const int nsrc = q < a.slots ? chunk_sources(a, group_chunk(a, group, ph) + q) : 0;
+  if(q < a.slots){
+    p.prev[q] = (unsigned long long)nsrc;
+    p.sum[q] = ((long long)a.e.n * nsrc - nsrc) * a.e.s;
+  }
+  const unsigned alive = __ballot_sync(0xffffffffu, nsrc > 0);
+  const unsigned all = __reduce_add_sync(0xffffffffu, (unsigned)nsrc);
+  if(q == 0){
+    p.group = group;
+    p.alive = alive;
+    p.total = all;
+    p.full = (unsigned long long)a.e.n * all;
+    p.level = alive ? 0 : -1;
+    p.t_loaded = globaltimer();
+  }
+  __syncwarp();
+}
+
+/* Warp 0 publishes the CTA's part of a step: the counts per chunk, then one
+ * barrier word with their total.  CTA 0 first clears the next step's words:
+ * their last readers (step - 2) have all arrived at step - 1, which this CTA
+ * has waited for, and nobody adds to them before it arrives. */
+__device__ __forceinline__ void arrive_step(const gbx_sweep &a, SweepShared &sh, SweepSync &sy, int ph)
+{
+  const int q = threadIdx.x;
+  const unsigned step = sh.ph[ph].step;
+  const unsigned c = q < a.slots ? sh.cnt[q] : 0u;
+  if(q < a.slots){
+    if(blockIdx.x == 0) sy.count[ph][(step + 1) % 3][q] = 0;
+    if(c) atomicAdd(&sy.count[ph][step % 3][q], (unsigned long long)c);
+    sh.cnt[q] = 0;
+  }
+  const unsigned total = __reduce_add_sync(0xffffffffu, c);   /* rows x lanes x 256 of one CTA: below 2^32 */
+  if(q == 0){
+    if(blockIdx.x == 0) sy.arrive[ph][(step + 1) % 3][0] = 0;
+    __threadfence();
+    atomicAdd(&sy.arrive[ph][step % 3][0], ARRIVE_ONE | total);
+    sh.ph[ph].step = step + 1;
+  }
+  __syncwarp();
+}
+
+/* Warp 0 waits for the phase's last step and takes its count (true), or past
+ * the limit gives up.  CTA 0 settles the step before meanwhile. */
+__device__ __forceinline__ bool wait_step(const gbx_sweep &a, SweepShared &sh, SweepSync &sy, int ph, bool added,
+                                          int first_level, unsigned long long &bits)
+{
+  SweepPhase &p = sh.ph[ph];
+  const unsigned step = p.step;
+  if(blockIdx.x == 0 && p.level > first_level) settle_step(a, p, sy, ph, step - 2, p.level - 1, added);
+  unsigned long long seen = 0;
+  bool ok = true;
+  if(threadIdx.x == 0) ok = wait_for(&sy.arrive[ph][(step - 1) % 3][0], ARRIVE_ONE * gridDim.x, seen, a.limit_ns);
+  ok = __all_sync(0xffffffffu, ok);
+  bits = __shfl_sync(0xffffffffu, seen, 0) & ARRIVE_BITS;
+  return ok;
+}
+
+/* Clears the other half of the counters for the next launch. */
+__device__ __forceinline__ SweepSync &sweep_begin(const gbx_sweep &a, SweepShared &sh)
+{
+  SweepSync *sy = reinterpret_cast<SweepSync *>(a.sync);
+  if(blockIdx.x == 0){
+    unsigned *other = reinterpret_cast<unsigned *>(sy + (a.set ^ 1));
+    for(int i = threadIdx.x; i < (int)(sizeof(SweepSync) / 4); i += SWEEP_THREADS) other[i] = 0;
+  }
+  if(threadIdx.x < SWEEP_SLOTS) sh.cnt[threadIdx.x] = 0;
+  if(threadIdx.x < GBX_SWEEP_PHASES) sh.ph[threadIdx.x].step = 0;
+  return sy[a.set];
+}
+
+/* The CTA's slice of the compact adjacency out of host memory; then the
+ * whole grid has the device copy.  False past the limit. */
+__device__ __forceinline__ bool pull_adjacency(const gbx_sweep &a, SweepShared &sh, SweepSync &sy)
+{
+  if(!a.e.adj_dev || a.in_place) return true;
+  const long long ints = (long long)a.B * a.e.d;
+  const long long t0 = (long long)blockIdx.x * SWEEP_THREADS + threadIdx.x;
+  const long long stride = (long long)gridDim.x * SWEEP_THREADS;
+  if(((reinterpret_cast<uintptr_t>(a.e.adj) | reinterpret_cast<uintptr_t>(a.e.adj_dev)) & 15) == 0){
+    const int4 *src = reinterpret_cast<const int4 *>(a.e.adj);
+    int4 *dst = reinterpret_cast<int4 *>(a.e.adj_dev);
+    for(long long i = t0; i < (ints >> 2); i += stride) dst[i] = src[i];
+    if(blockIdx.x == 0)
+      for(long long i = (ints & ~3LL) + threadIdx.x; i < ints; i += SWEEP_THREADS) a.e.adj_dev[i] = a.e.adj[i];
+  }
+  else
+    for(long long i = t0; i < ints; i += stride) a.e.adj_dev[i] = a.e.adj[i];
+  return grid_pass(&sy.ready[0], sh, a);
+}
+
+/* The neighbour lists of the CTA's rows row0 + i * drow, i < nr, in shared
+ * memory (and the table, if given).  2^lr threads share a row, eight rows in
+ * flight per thread. */
+__device__ __forceinline__ void expand_rows(const gbx_sweep &a, SweepSync &sy, int *list, int row0, int drow, int nr,
+                                            int *table)
+{
+  const int *adj = a.e.adj_dev && !a.in_place ? a.e.adj_dev : a.e.adj;
+  const int d = a.e.d, dp = a.e.dp;
+  int lr = 2;
+  while((1 << lr) < dp && lr < 5) lr++;
+  const int per = SWEEP_THREADS >> lr;
+  const int base = a.B;
+  const float inv = 1.0f / (float)base;
+  bool bad = false;
+  for(int j = threadIdx.x & ((1 << lr) - 1); j < dp; j += 1 << lr)
+    for(int i0 = threadIdx.x >> lr; i0 < nr; i0 += per * 8){
+      int val[8], back[8], deg[8];
+#pragma unroll
+      for(int k = 0; k < 8; k++){
+        const int i = i0 + k * per;
+        back[k] = val[k] = deg[k] = 0;
+        if(i < nr){
+          const int row = row0 + i * drow;
+          const int v = a.row_vertex ? __ldg(a.row_vertex + row) : row;
+          deg[k] = a.e.ndeg ? __ldg(a.e.ndeg + v) : d;
+          if(deg[k] < 0 || deg[k] > d){ bad = true; deg[k] = deg[k] < 0 ? 0 : d; }
+          if(a.e.grid_s){
+            if(j < deg[k]) val[k] = __ldcg(adj + entry_source(a.e, v, j, back[k]));
+          }
+          else{
+            /* entry_source's quotient v / base, estimated and put right */
+            int q = (int)((float)v * inv), m = v - q * base;
+            if(m < 0){ q--; m += base; }
+            if(m >= base){ q++; m -= base; }
+            back[k] = q * base;
+            if(j < deg[k]) val[k] = __ldcg(adj + (size_t)m * d + j);
+          }
+        }
+      }
+#pragma unroll
+      for(int k = 0; k < 8; k++){
+        const int i = i0 + k * per;
+        if(i < nr){
+          const int row = row0 + i * drow;
+          const int x = expand_value(a.e, val[k], back[k], j, deg[k], row, bad);
+          list[i * dp + j] = x;
+          if(table) __stcg(table + (size_t)row * dp + j, x);
+        }
+      }
+    }
+  if(bad) atomicOr(&sy.err, GBX_ERR_BAD_ADJ);
+}
+
+/* ---------------------------------------------------------------------- */
+/* General graphs.                                                         */
+/* ---------------------------------------------------------------------- */
+
+__device__ __forceinline__ void mark(unsigned *s, int o, int n)
+{
+  if((unsigned)o < (unsigned)n) atomicOr(s + (o >> 5), 1u << (o & 31));
+}
+
+/* Levels 1 and 2 of every chunk (of one group's chunks when the lists are too
+ * wide for level 2: then level 1 alone), a warp per row.  The warp marks the
+ * row, its neighbours and their neighbours in its scratch row (scratch_bits
+ * sources at a time) and stores each lane once.  A level-2 gather would read
+ * d whole rows per row, nearly all of them zeros; this reads d neighbour
+ * lists once for all chunks, and level 1 is never stored. */
+__device__ void start_rows(const gbx_sweep &a, const int *list, unsigned *scratch, unsigned *cnt1, unsigned *cnt2,
+                           int c0, int nc, int r0, int nr)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lL = a.wc_log2 - 2, L = 1 << lL;             /* lanes per row of a chunk */
+  const int dp = a.e.dp, d = a.e.d;
+  const int src0 = c0 << (lL + 8), nsrc = min(nc << (lL + 8), a.B - src0);
+  const int q4 = dp >> 2, magic = (65536 + q4 - 1) / q4;  /* i / q4 for i < 1024, q4 <= 16 */
+  unsigned *s = scratch + (size_t)warp * (a.scratch_bits >> 5);
+  for(int r = warp; r < nr; r += SWEEP_WARPS){
+    const int *ids = list + r * dp;
+    for(int sb = 0; sb < nsrc; sb += a.scratch_bits){
+      const int base = src0 + sb, sub = min(nsrc - sb, a.scratch_bits);
+      const int pieces = (sub + 255) >> 8;
+      uint4 *sv = reinterpret_cast<uint4 *>(s);
+      for(int i = lane; i < pieces * 2; i += 32) sv[i] = make_uint4(0u, 0u, 0u, 0u);
+      __syncwarp();
+      for(int i = lane; i <= dp; i += 32) mark(s, (i < dp ? ids[i] : r0 + r) - base, sub);
+      __syncwarp();
+      if(a.two_level){
+        for(int p0 = 0; p0 < pieces; p0 += 32){          /* level 1's counts */
+          const int p = p0 + lane;
+          unsigned v = 0;
+          if(p < pieces){
+            const uint4 x = sv[2 * p], y = sv[2 * p + 1];
+            v = popc4(x) + popc4(y);
+          }
+          for(int o = L >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if(v && (lane & (L - 1)) == 0) atomicAdd(cnt1 + (((sb >> 8) + p) >> lL), v);
+        }
+        __syncwarp();
+        /* six pieces of lists in flight per lane */
+        for(int i0 = lane; i0 < d * q4; i0 += 192){
+          int4 x[6];
+#pragma unroll
+          for(int k = 0; k < 6; k++){
+            const int i = i0 + 32 * k, j = (i * magic) >> 16;
+            if(i < d * q4) x[k] = __ldcg(reinterpret_cast<const int4 *>(a.e.nbr + (size_t)ids[j] * dp) + (i - j * q4));
+            else x[k] = make_int4(-1, -1, -1, -1);
+          }
+#pragma unroll
+          for(int k = 0; k < 6; k++){
+            mark(s, x[k].x - base, sub);
+            mark(s, x[k].y - base, sub);
+            mark(s, x[k].z - base, sub);
+            mark(s, x[k].w - base, sub);
+          }
+        }
+        __syncwarp();
+      }
+      for(int p0 = 0; p0 < pieces; p0 += 32){
+        const int p = p0 + lane;
+        unsigned w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        const int c = ((sb >> 8) + p) >> lL, gl = ((sb >> 8) + p) & (L - 1);
+        if(p < pieces){
+          *reinterpret_cast<uint4 *>(w) = sv[2 * p];
+          *reinterpret_cast<uint4 *>(w + 4) = sv[2 * p + 1];
+          char *to = reinterpret_cast<char *>(a.start + (size_t)c * a.start_stride);
+          st_lane(to + ((size_t)(r0 + r) << (a.wc_log2 + 3)) + (size_t)gl * 32, w);
+        }
+        unsigned v = popc_lane(w);
+        for(int o = L >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if(v && (lane & (L - 1)) == 0) atomicAdd(cnt2 + c, v);
+      }
+      __syncwarp();                                      /* the scratch row is read before it is cleared again */
+    }
+  }
+}
+
+/* A lane's words OR its neighbours', NB of them in flight. */
+template <int NB>
+__device__ __forceinline__ void gather_lane(unsigned (&acc)[8], const char *X, const int *ids, int d, unsigned rb)
+{
+  int j = 0;
+  for(; j + NB <= d; j += NB){
+    unsigned t[NB][8];
+#pragma unroll
+    for(int i = 0; i < NB; i += 4){
+      const int4 u = *reinterpret_cast<const int4 *>(ids + j + i);
+      ld_lane(t[i], X + (size_t)(unsigned)u.x * rb);
+      ld_lane(t[i + 1], X + (size_t)(unsigned)u.y * rb);
+      ld_lane(t[i + 2], X + (size_t)(unsigned)u.z * rb);
+      ld_lane(t[i + 3], X + (size_t)(unsigned)u.w * rb);
+    }
+#pragma unroll
+    for(int i = 0; i < NB; i += 2)
+#pragma unroll
+      for(int k = 0; k < 8; k++) acc[k] |= t[i][k] | t[i + 1][k];
+    if(and_lane(acc) == ~0u) return;
+  }
+  for(; j < d; j += 4){
+    const int4 u = *reinterpret_cast<const int4 *>(ids + j);
+    unsigned t0[8], t1[8] = {0, 0, 0, 0, 0, 0, 0, 0}, t2[8] = {0, 0, 0, 0, 0, 0, 0, 0},
+             t3[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    ld_lane(t0, X + (size_t)(unsigned)u.x * rb);
+    if(j + 1 < d) ld_lane(t1, X + (size_t)(unsigned)u.y * rb);
+    if(j + 2 < d) ld_lane(t2, X + (size_t)(unsigned)u.z * rb);
+    if(NB > 4 && j + 3 < d) ld_lane(t3, X + (size_t)(unsigned)u.w * rb);
+#pragma unroll
+    for(int k = 0; k < 8; k++) acc[k] |= (t0[k] | t1[k]) | (t2[k] | t3[k]);
+  }
+}
+
+/* One level of the phase's group over the CTA's rows: a thread keeps its lane
+ * and walks the rows.  `first`: the group's first gathered level, whose lanes
+ * have no state yet. */
+template <int NB>
+__device__ void level_rows(const gbx_sweep &a, SweepShared &sh, const int *list, unsigned char *flag, int ph,
+                           bool first, int r0, int nr)
+{
+  const int lL = a.wc_log2 - 2, L = 1 << lL, Q = a.slots, dp = a.e.dp, d = a.e.d;
+  const unsigned rb = 8u << a.wc_log2;
+  const int level = sh.ph[ph].level, c0 = group_chunk(a, sh.ph[ph].group, ph);
+  const int nsrc = min(Q << (lL + 8), a.B - (c0 << (lL + 8)));
+  const int lanes = (nsrc + 255) >> 8;                   /* at most SWEEP_THREADS */
+  const int rr = threadIdx.x / lanes, rs = SWEEP_THREADS / lanes;
+  unsigned cnt = 0;
+  int q = 0;
+  if(rr < rs){
+    const int at = threadIdx.x - rr * lanes, gl = at & (L - 1);
+    q = at >> lL;
+    const unsigned bits = (unsigned)lane_bits(nsrc, at);
+    const size_t words = a.slot_words;
+    const unsigned long long *x = first ? a.start + (size_t)(c0 + q) * a.start_stride
+                                        : a.buf + ((size_t)(ph * Q + q) * 2 + ((level & 1) ^ 1)) * words;
+    const char *X = reinterpret_cast<const char *>(x) + gl * 32;
+    char *Y = reinterpret_cast<char *>(a.buf + ((size_t)(ph * Q + q) * 2 + (level & 1)) * words) + gl * 32;
+    unsigned char *fl = flag + (((ph * Q + q) * a.rows) << lL) + gl;
+    for(int row = rr; row < nr; row += rs){
+      const unsigned f = first ? LANE_CHANGED : fl[row << lL];
+      unsigned acc[8];
+      if(f & LANE_FULL){
+        cnt += bits;
+        if(f & LANE_CHANGED){
+          if(bits == 256u){
+#pragma unroll
+            for(int k = 0; k < 8; k++) acc[k] = ~0u;
+          }
+          else ld_lane(acc, X + (size_t)(unsigned)(r0 + row) * rb);
+          st_lane(Y + (size_t)(unsigned)(r0 + row) * rb, acc);
+          fl[row << lL] = LANE_FULL;
+        }
+        continue;
+      }
+      ld_lane(acc, X + (size_t)(unsigned)(r0 + row) * rb);
+      gather_lane<NB>(acc, X, list + row * dp, d, rb);
+      st_lane(Y + (size_t)(unsigned)(r0 + row) * rb, acc);
+      const unsigned c = popc_lane(acc);
+      cnt += c;
+      if(first || c == bits) fl[row << lL] = LANE_CHANGED | (c == bits ? LANE_FULL : 0u);
+    }
+  }
+  if(Q == 1){
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if((threadIdx.x & 31) == 0) atomicAdd(&sh.cnt[0], cnt);
+  }
+  else if(cnt) atomicAdd(&sh.cnt[q], cnt);
+}
+
+/* Warp 0: what the phase does next.  After the group's last level (complete,
+ * or a level that added nothing) the next group begins. */
+__device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, SweepSync &sy, int ph)
+{
+  SweepPhase &p = sh.ph[ph];
+  const int base = a.two_level ? 2 : 1;                  /* the level that the start computed */
+  int todo = -1;
+  if(p.level > base){
+    unsigned long long bits;
+    if(!wait_step(a, sh, sy, ph, false, base + 1, bits)) todo = TODO_ABORT;
+    else{
+      if(bits == p.full || bits == p.total || p.level >= a.e.n){
+        if(blockIdx.x == 0) settle_step(a, p, sy, ph, p.step - 1, p.level, false);
+        group_state(a, p, ph, p.group + 1);
+      }
+      else{
+        todo = TODO_LEVEL;
+        if(threadIdx.x == 0){ p.total = bits; p.level++; }
+      }
+    }
+  }
+  while(todo < 0){
+    /* the group's levels up to `base`, counted at the start */
+    if(p.level < 0){ todo = TODO_DONE; break; }
+    const int q = threadIdx.x, chunk = group_chunk(a, p.group, ph) + q;
+    unsigned long long c1 = 0, c2 = 0;
+    bool go = (p.alive >> q) & 1u;
+    if(go){
+      if(a.two_level) c1 = __ldcg(&sy.start1[chunk]);
+      c2 = __ldcg(&sy.start2[chunk]);
+    }
+    unsigned long long t1 = c1, t2 = c2;
+    for(int o = 16; o > 0; o >>= 1){
+      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+    }
+    if(blockIdx.x == 0){
+      if(go && a.two_level) go = settle(a, p, sy, chunk, q, 1, c1);
+      if(go) go = settle(a, p, sy, chunk, q, base, c2);
+      const unsigned alive = __ballot_sync(0xffffffffu, go);
+      if(q == 0) p.alive = alive;
+    }
+    const unsigned long long t0 = p.total;
+    const bool over = (a.two_level && (t1 == p.full || t1 == t0 || a.e.n <= 1)) || t2 == p.full ||
+                      t2 == (a.two_level ? t1 : t0) || a.e.n <= base;
+    __syncwarp();
+    if(over) group_state(a, p, ph, p.group + 1);
+    else{
+      todo = TODO_LEVEL;
+      if(q == 0){ p.total = t2; p.level = base + 1; }
+    }
+    __syncwarp();
+  }
+  if(threadIdx.x == 0) sh.todo = todo;
+  __syncwarp();
+}
+
+template <int NB, int MIN_BLOCKS>
+__global__ void __launch_bounds__(SWEEP_THREADS, MIN_BLOCKS) sweep_dense_kernel(const gbx_sweep a)
+{
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  __shared__ SweepShared sh;
+  const int tid = threadIdx.x, dp = a.e.dp;
+  const int r0 = (int)blockIdx.x * a.rows, nr = min(a.rows, a.e.n - r0);
+  int *list = reinterpret_cast<int *>(sweep_smem);                               /* [rows][dp] */
+  unsigned *scratch = reinterpret_cast<unsigned *>(list + (size_t)a.rows * dp);  /* a row of marks per warp */
+  unsigned *cnt1 = scratch + SWEEP_WARPS * (a.scratch_bits >> 5), *cnt2 = cnt1 + a.nchunks;
+  unsigned char *flag = reinterpret_cast<unsigned char *>(cnt2 + a.nchunks);     /* [phases * slots][rows][lanes] */
+  SweepSync &sy = sweep_begin(a, sh);
+  for(int i = tid; i < 2 * a.nchunks; i += SWEEP_THREADS) cnt1[i] = 0;
+  if(!pull_adjacency(a, sh, sy)) return;
+  expand_rows(a, sy, list, r0, 1, nr, a.two_level ? a.e.nbr : nullptr);
+  if(a.two_level){
+    if(!grid_pass(&sy.ready[1], sh, a)) return;
+  }
+  else __syncthreads();
+  start_rows(a, list, scratch, cnt1, cnt2, 0, a.nchunks, r0, nr);
+  __syncthreads();
+  for(int c = tid; c < a.nchunks; c += SWEEP_THREADS){
+    if(cnt1[c]) atomicAdd(&sy.start1[c], (unsigned long long)cnt1[c]);
+    if(cnt2[c]) atomicAdd(&sy.start2[c], (unsigned long long)cnt2[c]);
+  }
+  if(!grid_pass(&sy.ready[2], sh, a)) return;
+  if(tid < 32)
+    for(int ph = 0; ph < a.phases; ph++) group_state(a, sh.ph[ph], ph, 0);
+
+  unsigned open = (1u << a.phases) - 1u;                 /* phases with groups left */
+  while(open)
+    for(int ph = 0; ph < a.phases; ph++){
+      if(!((open >> ph) & 1u)) continue;
+      __syncthreads();
+      if(tid < 32) plan_dense(a, sh, sy, ph);
+      __syncthreads();
+      const int todo = sh.todo;
+      if(todo == TODO_ABORT){
+        if(tid == 0) *a.abort_flag = GBX_ERR_TIMEOUT;
+        return;
+      }
+      if(todo == TODO_DONE){ open &= ~(1u << ph); continue; }
+      level_rows<NB>(a, sh, list, flag, ph, sh.ph[ph].level == (a.two_level ? 3 : 2), r0, nr);
+      __syncthreads();
+      if(tid < 32) arrive_step(a, sh, sy, ph);
+    }
+}
+
+/* ---------------------------------------------------------------------- */
+/* Grids.                                                                  */
+/* ---------------------------------------------------------------------- */
+
+#define TRACK_QUEUE 1024              /* 32 words of 32 lanes */
+
+/* Per-warp working memory of a step over 32 (row, word) pairs. */
+struct TrackWarp {
+  unsigned newc[32], newf[32];        /* lanes that changed, lanes now full */
+  unsigned short queue[TRACK_QUEUE];  /* pair << 5 | lane of the word */
+};
+
+struct TrackShared {
+  int *list;                          /* [rows][dp] */
+  unsigned *have, *full, *last;       /* per (row, word), a bit per lane: holds bits; is full; buffer of its words */
+  TrackWarp *warp;
+  unsigned *near;                     /* this warp's [dp][32]: the neighbours' changed words */
+};
+
+/* Level 0 of a group: every source's own bit.  Lanes that hold nothing are
+ * never stored or read. */
+__device__ void track_start(const gbx_sweep &a, const TrackShared &t, int src0, int nsrc, int nr)
+{
+  const int lw = a.word_log2, row_lanes = a.slots << (a.wc_log2 - 2);
+  for(int c = threadIdx.x; c < (nr << lw); c += SWEEP_THREADS){
+    const int row = (int)blockIdx.x + (c >> lw) * (int)gridDim.x, w = c & ((1 << lw) - 1);
+    const int o = row - src0, l = o >> 8;
+    unsigned bit = 0, full = 0;
+    if(row < a.B && (unsigned)o < (unsigned)nsrc && (l >> 5) == w){
+      unsigned x[8];
+#pragma unroll
+      for(int k = 0; k < 8; k++) x[k] = ((o >> 5) & 7) == k ? 1u << (o & 31) : 0u;
+      st_lane(reinterpret_cast<char *>(a.buf) + ((size_t)row * row_lanes + l) * 32, x);
+      bit = 1u << (l & 31);
+      if(lane_bits(nsrc, l) == 1) full = bit;
+    }
+    t.have[c] = bit;
+    t.full[c] = full;
+    t.last[c] = 0;
+    __stcg(a.changed + ((size_t)row << lw) + w, bit);
+  }
+}
+
+/* One level: warp by warp over 32 (row, word) pairs of the CTA's rows (row
+ * blockIdx.x + i * gridDim.x, so that the busy rows of a wavefront spread
+ * over the CTAs).  The pairs' lanes with a changed neighbour are queued and
+ * taken 32 at a time, whatever rows they come from.  A neighbour that did not
+ * change is not read: its words of the previous level may never have been
+ * stored, or lie in the other buffer.  (Reading a row of zeros in its place
+ * saves the predicates, but that row's sectors are then read by everybody: a
+ * 97 x 103 grid took 0.49 to 0.55 ms that way.) */
+template <int NB>
+__device__ void track_level(const gbx_sweep &a, SweepShared &sh, const TrackShared &t, int level, int nsrc, int nr)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lw = a.word_log2, lL = a.wc_log2 - 2, dp = a.e.dp, d = a.e.d, n = a.e.n;
+  const unsigned rb = (unsigned)(a.slots << lL) * 32u;   /* bytes of a row */
+  const size_t half = a.slot_words * 8;                  /* bytes of a buffer */
+  const unsigned *was = a.changed + (size_t)((level & 1) ^ 1) * ((size_t)n << lw);
+  unsigned *now = a.changed + (size_t)(level & 1) * ((size_t)n << lw);
+  const char *X = reinterpret_cast<const char *>(a.buf) + ((level & 1) ? 0 : half);
+  char *Y = reinterpret_cast<char *>(a.buf) + ((level & 1) ? half : 0);
+  TrackWarp &tw = t.warp[warp];
+  const int pairs = nr << lw;
+  const int per = min(32, (pairs + SWEEP_WARPS - 1) / SWEEP_WARPS);
+  for(int c0 = warp * per; c0 < pairs; c0 += SWEEP_WARPS * per){
+    const int m = min(per, pairs - c0), c = c0 + lane;
+    const int w = c & ((1 << lw) - 1);
+    unsigned act = 0;
+    if(lane < m){
+      const int *ids = t.list + (c >> lw) * dp;
+      for(int j0 = 0; j0 < d; j0 += 8){
+        unsigned x[8];
+#pragma unroll
+        for(int k = 0; k < 8; k++)
+          x[k] = j0 + k < d ? __ldcg(was + ((size_t)(unsigned)ids[j0 + k] << lw) + w) : 0u;
+#pragma unroll
+        for(int k = 0; k < 8; k++)
+          if(j0 + k < dp){
+            t.near[(j0 + k) * 32 + lane] = x[k];
+            act |= x[k];
+          }
+      }
+      act &= ~t.full[c];
+      tw.newc[lane] = tw.newf[lane] = 0;
+    }
+    const int mine = __popc(act);
+    int end = mine;
+    for(int o = 1; o < 32; o <<= 1){
+      const int x = __shfl_up_sync(0xffffffffu, end, o);
+      if(lane >= o) end += x;
+    }
+    const int total = __shfl_sync(0xffffffffu, end, 31);
+    int at = end - mine;
+    for(unsigned x = act; x; x &= x - 1) tw.queue[at++] = (unsigned short)(lane << 5 | (__ffs(x) - 1));
+    __syncwarp();
+    for(int i = lane; i < total; i += 32){
+      const int code = tw.queue[i], cl = code >> 5, b = code & 31, cc = c0 + cl;
+      const int l = ((cc & ((1 << lw) - 1)) << 5) | b;   /* lane of the row */
+      const int row = (int)blockIdx.x + (cc >> lw) * (int)gridDim.x;
+      const int *ids = t.list + (cc >> lw) * dp;
+      const unsigned *near = t.near + cl;
+      const size_t own = (size_t)(unsigned)row * rb + (unsigned)l * 32u;
+      const char *Xl = X + (unsigned)l * 32u;
+      unsigned old[8], acc[8];
+#pragma unroll
+      for(int e = 0; e < 8; e++) old[e] = 0;
+      if((t.have[cc] >> b) & 1u)
+        ld_lane(old, reinterpret_cast<const char *>(a.buf) + (((t.last[cc] >> b) & 1u) ? half : 0) + own);
+#pragma unroll
+      for(int e = 0; e < 8; e++) acc[e] = 0;
+      for(int j0 = 0; j0 < d; j0 += NB){
+        unsigned v[NB][8];
+#pragma unroll
+        for(int k = 0; k < NB; k++){
+#pragma unroll
+          for(int e = 0; e < 8; e++) v[k][e] = 0;
+          if(j0 + k < d && ((near[(j0 + k) * 32] >> b) & 1u))
+            ld_lane(v[k], Xl + (size_t)(unsigned)ids[j0 + k] * rb);
+        }
+#pragma unroll
+        for(int k = 0; k < NB; k += 2)
+#pragma unroll
+          for(int e = 0; e < 8; e++) acc[e] |= v[k][e] | v[k + 1][e];
+      }
+      unsigned diff[8];
+#pragma unroll
+      for(int e = 0; e < 8; e++){
+        diff[e] = acc[e] & ~old[e];
+        acc[e] |= old[e];
+      }
+      const unsigned added = popc_lane(diff);
+      if(added){
+        st_lane(Y + own, acc);
+        atomicOr(&tw.newc[cl], 1u << b);
+        const unsigned bits = (unsigned)lane_bits(nsrc, l);
+        if(bits == 256u ? and_lane(acc) == ~0u : popc_lane(acc) == bits) atomicOr(&tw.newf[cl], 1u << b);
+        atomicAdd(&sh.cnt[l >> lL], added);
+      }
+    }
+    __syncwarp();
+    if(lane < m){
+      const unsigned nc = tw.newc[lane];
+      __stcg(now + ((size_t)(unsigned)((int)blockIdx.x + (c >> lw) * (int)gridDim.x) << lw) + w, nc);
+      t.have[c] |= nc;
+      t.full[c] |= tw.newf[lane];
+      t.last[c] = (t.last[c] & ~nc) | ((level & 1) ? nc : 0u);
+    }
+    __syncwarp();
+  }
+}
+
+/* Warp 0: what comes next; level 0 (the sources themselves) starts a group. */
+__device__ __forceinline__ void plan_track(const gbx_sweep &a, SweepShared &sh, SweepSync &sy)
+{
+  SweepPhase &p = sh.ph[0];
+  int todo = TODO_LEVEL;
+  unsigned long long bits;
+  if(p.step > 0){
+    if(!wait_step(a, sh, sy, 0, true, 1, bits)) todo = TODO_ABORT;
+    else if(p.level > 0 && (p.total + bits == p.full || bits == 0 || p.level >= a.e.n)){
+      if(blockIdx.x == 0) settle_step(a, p, sy, 0, p.step - 1, p.level, true);
+      group_state(a, p, 0, p.group + 1);
+      if(p.level < 0) todo = TODO_DONE;
+    }
+    else if(threadIdx.x == 0){
+      p.total += bits;
+      p.level++;
+    }
+  }
+  if(threadIdx.x == 0) sh.todo = todo;
+  __syncwarp();
+}
+
+/* Two CTAs per SM and six neighbours in flight: 256 x 256, d = 6 took 5.26 ms
+ * (6.0 with three CTAs, 5.9 with four and four neighbours in flight; both
+ * spilled). */
+template <int NB>
+__global__ void __launch_bounds__(SWEEP_THREADS, 2) sweep_track_kernel(const gbx_sweep a)
+{
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  __shared__ SweepShared sh;
+  const int tid = threadIdx.x, dp = a.e.dp;
+  const int nr = (a.e.n - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  TrackShared t;
+  t.list = reinterpret_cast<int *>(sweep_smem);
+  t.have = reinterpret_cast<unsigned *>(t.list + (size_t)a.rows * dp);
+  t.full = t.have + ((size_t)a.rows << a.word_log2);
+  t.last = t.full + ((size_t)a.rows << a.word_log2);
+  t.near = t.last + ((size_t)a.rows << a.word_log2) + (tid >> 5) * 32 * dp;
+  t.warp = reinterpret_cast<TrackWarp *>(t.last + ((size_t)a.rows << a.word_log2) + SWEEP_WARPS * 32 * dp);
+  SweepSync &sy = sweep_begin(a, sh);
+  if(!pull_adjacency(a, sh, sy)) return;
+  expand_rows(a, sy, t.list, (int)blockIdx.x, (int)gridDim.x, nr, nullptr);
+  if(tid < 32) group_state(a, sh.ph[0], 0, 0);
+  for(;;){
+    __syncthreads();
+    if(tid < 32) plan_track(a, sh, sy);
+    __syncthreads();
+    const int todo = sh.todo, level = sh.ph[0].level, c0 = group_chunk(a, sh.ph[0].group, 0);
+    if(todo == TODO_DONE) return;
+    if(todo == TODO_ABORT){
+      if(tid == 0) *a.abort_flag = GBX_ERR_TIMEOUT;
+      return;
+    }
+    const int src0 = c0 * (64 << a.wc_log2), nsrc = min(a.slots * (64 << a.wc_log2), a.B - src0);
+    if(level == 0) track_start(a, t, src0, nsrc, nr);
+    else track_level<NB>(a, sh, t, level, nsrc, nr);
+    __syncthreads();
+    if(tid < 32) arrive_step(a, sh, sy, 0);
+  }
+}
+
+}  // namespace
+
+extern "C" {
+
+size_t gbx_sweep_sync_bytes(void) { return 2 * sizeof(SweepSync); }
+
+size_t gbx_sweep_smem(const gbx_sweep *a)
+{
+  const size_t rows = (size_t)a->rows, lists = rows * (size_t)a->e.dp * 4;
+  if(a->track)
+    return lists + 3 * (rows << a->word_log2) * 4 + SWEEP_WARPS * (32 * (size_t)a->e.dp * 4 + sizeof(TrackWarp));
+  return lists + SWEEP_WARPS * (size_t)a->scratch_bits / 8 + 8 * (size_t)a->nchunks +
+         (((size_t)a->phases * a->slots * rows) << (a->wc_log2 - 2));
+}
+
+/* The narrow form keeps four CTAs of 64 registers per SM, the wide one two of
+ * 128 with eight neighbours in flight per lane. */
+static const void *sweep_entry(const gbx_sweep *a)
+{
+  if(a->track) return (const void *)sweep_track_kernel<6>;
+  return a->wide ? (const void *)sweep_dense_kernel<8, 2> : (const void *)sweep_dense_kernel<4, 4>;
+}
+
+int gbx_sweep_blocks(const gbx_sweep *a, int *per_sm)
+{
+  *per_sm = 0;
+  const size_t smem = gbx_sweep_smem(a);
+  if(smem > GBX_SWEEP_SMEM_MAX) return (int)cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(sweep_entry(a), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       GBX_SWEEP_SMEM_MAX);
+  if(e != cudaSuccess) return (int)e;
+  return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, sweep_entry(a), SWEEP_THREADS, smem);
+}
+
+int gbx_sweep_launch(const gbx_sweep *a, int blocks, void *stream)
+{
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks, 1, 1);
+  cfg.blockDim = dim3(SWEEP_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = gbx_sweep_smem(a);
+  cfg.stream = (cudaStream_t)stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  gbx_sweep arg = *a;
+  void *args[1] = { &arg };
+  return (int)cudaLaunchKernelExC(&cfg, sweep_entry(a), args);
+}
+
+}  /* extern "C" */
