@@ -230,6 +230,28 @@ size_t gbx_sweep_smem(const gbx_sweep *a);
 int  gbx_sweep_blocks(const gbx_sweep *a, int *per_sm);
 int  gbx_sweep_launch(const gbx_sweep *a, int blocks, void *stream);
 
+/* Many graphs in one cooperative launch (team_kernel in sweep.cu).  Graph g's
+ * arguments are graphs[g] (one phase, one group; buf, start, changed, rows and
+ * limit_ns are set by the team).  order[queue[k] .. queue[k + 1]) are the
+ * graphs for teams of a 2^k-th of the grid, taken in that order. */
+#define GBX_TEAM_SPLITS 9              /* teams of 1/1 to 1/256 of the grid */
+typedef struct {
+  const gbx_sweep *graphs;
+  const int *order;
+  const unsigned long long *adj;       /* this call's host arrays (device memory), or NULL: graphs[g].e.adj */
+  unsigned int *next;                  /* [GBX_TEAM_SPLITS], zeroed before the launch, as are the nodes */
+  void *nodes;                         /* gbx_team_node_bytes() for each team of first_split .. last_split */
+  unsigned char *arena;                /* the teams' bitsets: arena_bytes >> k for each of 2^k teams */
+  size_t arena_bytes;                  /* a multiple of 256 << (GBX_TEAM_SPLITS - 1) */
+  unsigned int *abort_flag;
+  unsigned long long limit_ns;
+  int first_split, last_split;
+  int queue[GBX_TEAM_SPLITS + 1];
+} gbx_team;
+size_t gbx_team_node_bytes(void);
+int  gbx_team_blocks(size_t smem, int *per_sm);
+int  gbx_team_launch(const gbx_team *t, int blocks, size_t smem, void *stream);
+
 /* Applies `count` writes, in stream order. */
 int  gbx_scatter(const gbx_write *d_writes, int count, void *stream);
 int  gbx_event_query(void *ev);        /* 0: complete, 1: not yet, else an error */

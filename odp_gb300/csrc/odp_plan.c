@@ -59,6 +59,7 @@ void odp_tuning_defaults(odp_tuning *t, int batch)
   t->small_cluster = env_int("ODP_GB300_SMALL_CLUSTER", 0);
   t->small_part = env_int("ODP_GB300_SMALL_PART", -1);
   t->sweep = env_int("ODP_GB300_SWEEP", 1);
+  t->team = 0;
 }
 
 /* Chunk width (log2 words) for a graph whose whole level runs in shared
@@ -190,33 +191,27 @@ static void fill_degrees(const odp_shape *sh, int n, int *out)
   }
 }
 
-/* Position of cell (x, y) on the Hilbert curve over a 2^order x 2^order
- * square (D. Hilbert, 1891): quadrant by quadrant from the coarsest, turning
- * the square at each level so that the curve stays connected. */
-static unsigned long long hilbert_key(unsigned x, unsigned y, int order)
+/* Cells of a bw x bh rectangle along the Hilbert curve (D. Hilbert, 1891) of
+ * the square of side 2^order around it: quadrant by quadrant, the first and
+ * the last turned so that the curve stays connected; squares outside the
+ * rectangle are passed over.  A square is its origin and the directions of
+ * its two axes. */
+typedef struct { int bw, bh, count, *x, *y; } curve_walk;
+
+static void walk_curve(curve_walk *c, int order, int ox, int oy, int ux, int uy, int vx, int vy)
 {
-  unsigned long long key = 0;
-  for(int b = order - 1; b >= 0; b--){
-    const unsigned side = 1u << b, rx = (x >> b) & 1u, ry = (y >> b) & 1u;
-    key = key * 4 + (ry ? (rx ? 2 : 1) : (rx ? 3 : 0));
-    x &= side - 1;
-    y &= side - 1;
-    if(!ry){
-      if(rx){ x = side - 1 - x; y = side - 1 - y; }
-      const unsigned swap = x;
-      x = y;
-      y = swap;
-    }
+  const int far = (1 << order) - 1, ex = ox + far * (ux + vx), ey = oy + far * (uy + vy);
+  if((ox < ex ? ox : ex) >= c->bw || (oy < ey ? oy : ey) >= c->bh) return;
+  if(order == 0){
+    c->x[c->count] = ox;
+    c->y[c->count++] = oy;
+    return;
   }
-  return key;
-}
-
-typedef struct { unsigned long long key; int vertex; } curve_cell;
-
-static int cmp_curve(const void *a, const void *b)
-{
-  const unsigned long long x = ((const curve_cell *)a)->key, y = ((const curve_cell *)b)->key;
-  return (x > y) - (x < y);
+  const int side = 1 << (order - 1), last = side - 1;
+  walk_curve(c, order - 1, ox, oy, vx, vy, ux, uy);
+  walk_curve(c, order - 1, ox + side * vx, oy + side * vy, ux, uy, vx, vy);
+  walk_curve(c, order - 1, ox + side * (ux + vx), oy + side * (uy + vy), ux, uy, vx, vy);
+  walk_curve(c, order - 1, ox + side * ux + last * (ux + vx), oy + side * uy + last * (uy + vy), -vx, -vy, -ux, -uy);
 }
 
 /* Rows of a grid graph in the order of a Hilbert curve through its base
@@ -228,24 +223,19 @@ static int fill_curve_rows(const odp_plan_graph *g, int *itable, int *row_vertex
 {
   const int bw = g->s == 1 ? g->width : g->width / 2;
   const int bh = g->s == 4 ? g->height / 2 : g->height;
-  curve_cell *cell = malloc(sizeof(curve_cell) * (size_t)g->B);
-  if(!cell) return ODPX_ERR_MEMORY;
-  const int order = ilog2_ceil(bw > bh ? bw : bh);
-  for(int x = 0; x < bw; x++)
-    for(int y = 0; y < bh; y++){
-      curve_cell *c = &cell[(size_t)x * bh + y];
-      c->key = hilbert_key((unsigned)x, (unsigned)y, order);
-      c->vertex = x * g->height + y;
+  int *xy = malloc(sizeof(int) * 2 * (size_t)g->B);
+  if(!xy) return ODPX_ERR_MEMORY;
+  curve_walk c = { bw, bh, 0, xy, xy + g->B };
+  walk_curve(&c, ilog2_ceil(bw > bh ? bw : bh), 0, 0, 1, 0, 0, 1);
+  for(int k = 0; k < g->B; k++){
+    const int base = c.x[k] * g->height + c.y[k];
+    for(int r = 0; r < g->s; r++){
+      const int v = r == 0 ? base : rotate_host(base, g->width, g->height, g->s, g->s == 2 ? 180 : 90 * r);
+      itable[v] = k + r * g->B;
+      row_vertex[k + r * g->B] = v;
     }
-  qsort(cell, (size_t)g->B, sizeof(curve_cell), cmp_curve);
-  for(int k = 0; k < g->B; k++)
-    for(int t = 0; t < g->s; t++){
-      const int v = t == 0 ? cell[k].vertex
-                           : rotate_host(cell[k].vertex, g->width, g->height, g->s, g->s == 2 ? 180 : 90 * t);
-      itable[v] = k + t * g->B;
-      row_vertex[k + t * g->B] = v;
-    }
-  free(cell);
+  }
+  free(xy);
   return 0;
 }
 
@@ -450,6 +440,14 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
   return 0;
 }
 
+/* Whether no schedule setting asks for the persistent engine. */
+static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
+{
+  const ODPX_Tune_entry *te = table_lookup(shape_n(sh), sh->degree, sh->grid);
+  return t->sweep && t->wc_log2 <= 0 && t->slots <= 0 && t->tile_rows <= 0 && !t->local_kb_explicit &&
+         t->activity == -2 && !(te && (te->wc_log2 > 0 || te->tile_kb > 0 || te->local_kb > 0));
+}
+
 /* Whether a plan runs on the lockstep kernels (sweep.cu), and its shape.  One
  * graph, no schedule setting, and a CTA's rows must fit in its shared memory
  * beside their lane states.  Measured on GB300 against the persistent engine:
@@ -473,10 +471,7 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
  *    first, in wider pieces. */
 static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_sweep *sw, int *grid_out)
 {
-  const ODPX_Tune_entry *te = table_lookup(shape_n(sh), sh->degree, sh->grid);
-  if(!t->sweep || t->wc_log2 > 0 || t->slots > 0 || t->tile_rows > 0 || t->local_kb_explicit || t->blocks > 0 ||
-     t->activity != -2 || (te && (te->wc_log2 > 0 || te->tile_kb > 0 || te->local_kb > 0)))
-    return 0;
+  if(!lockstep_allowed(sh, t) || t->blocks > 0) return 0;
   const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
   memset(sw, 0, sizeof(*sw));
   sw->e.dp = shape_dp(sh);
@@ -532,6 +527,157 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
   return 0;
 }
 
+typedef struct {
+  double cost, latency;        /* us on the whole GPU; us whatever the team */
+  double need;                 /* bytes of its bitsets */
+  int split;
+} team_graph;
+
+/* Makespan (us) of the graphs on their teams: every team takes the next graph
+ * of its size when it is free, and splits when there is none. */
+static double team_makespan(const team_graph *g, const job_order *ord, int count)
+{
+  double at[1 << (GBX_TEAM_SPLITS - 1)] = {0};
+  double end = 0;
+  for(int k = 0; k < GBX_TEAM_SPLITS; k++){
+    const int teams = 1 << k;
+    if(k) for(int i = teams - 1; i >= 0; i--) at[i] = at[i >> 1];
+    for(int j = 0; j < count; j++){
+      const team_graph *x = &g[ord[j].job];
+      if(x->split != k) continue;
+      int first = 0;
+      for(int i = 1; i < teams; i++) if(at[i] < at[first]) first = i;
+      at[first] += x->cost * teams + x->latency;
+      if(at[first] > end) end = at[first];
+    }
+  }
+  return end;
+}
+
+/* Each graph's team: the smallest on which it takes at most `most` us, its
+ * rows fit a CTA and the teams' bitsets stay within 160 MB.  0 if some graph
+ * does not even fit the whole grid. */
+static int assign_teams(const odp_shape *shapes, int count, int grid, size_t smem_max, double most, gbx_sweep *gs,
+                        team_graph *g)
+{
+  for(int i = 0; i < count; i++){
+    g[i].split = -1;
+    for(int k = 0; k < GBX_TEAM_SPLITS && (1 << k) <= grid; k++){
+      gbx_sweep c = gs[i];
+      const int size = grid >> k;
+      c.rows = (shape_n(&shapes[i]) + size - 1) / size;
+      if(gbx_sweep_smem(&c) > smem_max || (k > 0 && (g[i].need * (1 << k) > 160e6 || g[i].cost * (1 << k) > most))) break;
+      g[i].split = k;
+      gs[i].rows = c.rows;
+    }
+    if(g[i].split < 0) return 0;
+  }
+  return 1;
+}
+
+/* Whether a plan runs on the team kernel, and which team each graph gets.
+ * Every graph must fit the lockstep kernels in one group (bitsets of at most
+ * 64 MB, 64 lanes a row, 256 for grids).  A graph's cost on the whole GPU is
+ * estimated from its traffic: a general graph's gathered levels at 20 TB/s;
+ * for grids about ten visits per row and lane, each reading d + 2 sectors, at
+ * 8 TB/s.  Its team is the smallest on which it takes no more
+ * than a share of all graphs' cost, its rows fit a CTA's shared memory and
+ * the teams' bitsets together stay within 160 MB; of several shares the one
+ * with the least makespan is taken. */
+static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, int sms, gbx_sweep *gs,
+                       gbx_team *tm, int *order, int *grid_out, size_t *smem_out)
+{
+  if(count == 1 && !t->team) return 0;
+  for(int i = 0; i < count; i++){
+    const double n = shape_n(&shapes[i]), W = shape_words(&shapes[i]);
+    if(!lockstep_allowed(&shapes[i], t) || 16.0 * n * W > 64e6 || W > (shapes[i].grid ? 1024 : 256)) return 0;
+  }
+  int fit = 0;
+  if(gbx_team_blocks(0, &fit) || fit < 2) return 0;
+  int grid = 2 * sms;
+  if(t->blocks > 0 && t->blocks < grid) grid = t->blocks;
+  const size_t smem_max = 100 * 1024;
+  team_graph *g = calloc((size_t)count, sizeof(team_graph));
+  job_order *ord = calloc((size_t)count, sizeof(job_order));
+  int ok = g && ord;
+  double all = 0;
+  for(int i = 0; i < count && ok; i++){
+    const odp_shape *sh = &shapes[i];
+    gbx_sweep *c = &gs[i];
+    const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
+    memset(c, 0, sizeof(*c));
+    c->e.dp = shape_dp(sh);
+    c->B = n / sh->symmetries;
+    c->phases = 1;
+    c->track = sh->grid && c->e.dp <= GBX_SWEEP_TRACK_DEGREE;
+    c->two_level = c->e.dp <= GBX_SWEEP_TWO_LEVEL && 8.0 * W * sh->degree > 5000;
+    c->scratch_bits = (c->B + 255) / 256 * 256;
+    c->wc_log2 = c->track ? (full_l2 < 5 ? full_l2 : 5) : (full_l2 < 6 ? full_l2 : 6);
+    c->nchunks = c->slots = (W + (1 << c->wc_log2) - 1) >> c->wc_log2;
+    while((32 << c->word_log2) < (c->slots << (c->wc_log2 - 2))) c->word_log2++;
+    if(!c->track && W > 256) ok = 0;
+    const double lanes = (c->B + 255) / 256;
+    if(c->track){
+      g[i].cost = n * lanes * 9.5 * (sh->degree + 2) * 32.0 / 8e6;
+      g[i].latency = 15.0 + 4.0 * (sh->width + sh->height) / 3.0;
+    }
+    else{
+      double levels = 2.0, ball = sh->degree + 1.0;      /* until a ball of branching d - 1 holds n, and one more */
+      for(const double grow = sh->degree > 3 ? sh->degree - 1.0 : 2.0; ball < n; ball *= grow) levels += 1.0;
+      g[i].cost = (n * 8.0 * W * (sh->degree + 1) * (levels > 3.0 ? levels - 2.5 : 0.5) + 4.0 * n * c->e.dp * sh->degree) / 20e6;
+      g[i].latency = 15.0 + 4.0 * levels;
+    }
+    g[i].need = 16.0 * ((double)n * c->slots * (1 << c->wc_log2)) + (c->track ? 8.0 * n * (1 << c->word_log2) : 0) + 1024;
+    all += g[i].cost;
+    ord[i].job = i;
+    ord[i].work = g[i].cost;
+  }
+  if(ok){
+    qsort(ord, (size_t)count, sizeof(job_order), cmp_work_desc);
+    static const double shares[] = { 0.1, 0.2, 0.35, 0.6, 1.0 };
+    double best = 0, best_share = 0;
+    for(int s = 0; s < 5 && ok; s++){
+      ok = assign_teams(shapes, count, grid, smem_max, shares[s] * all, gs, g);
+      const double m = ok ? team_makespan(g, ord, count) : 0;
+      if(s == 0 || m < best){ best = m; best_share = shares[s]; }
+    }
+    if(ok) ok = assign_teams(shapes, count, grid, smem_max, best_share * all, gs, g);
+  }
+  size_t smem = 0;
+  double arena = 0;
+  if(ok){
+    int at = 0;
+    tm->first_split = GBX_TEAM_SPLITS;
+    tm->last_split = 0;
+    for(int k = 0; k < GBX_TEAM_SPLITS; k++){
+      tm->queue[k] = at;
+      for(int j = 0; j < count; j++){
+        const int i = ord[j].job;
+        if(g[i].split != k) continue;
+        order[at++] = i;
+        if(k < tm->first_split) tm->first_split = k;
+        tm->last_split = k;
+        const size_t b = gbx_sweep_smem(&gs[i]);
+        if(b > smem) smem = b;
+        const double need = (double)ALIGN_UP((size_t)g[i].need, 256) + 512;
+        if(need * (1 << k) > arena) arena = need * (1 << k);
+      }
+    }
+    tm->queue[GBX_TEAM_SPLITS] = at;
+    /* parts of every split are whole multiples of 256 bytes, so that a team's
+     * part lies inside its parent's, whose other half may still be in use */
+    tm->arena_bytes = ALIGN_UP((size_t)arena, (size_t)256 << (GBX_TEAM_SPLITS - 1));
+    size_t room = 0;
+    ok = gbx_team_blocks(smem, &fit) == 0 && fit * sms >= grid && gbx_mem_free(&room) == 0 &&
+         arena <= 0.5 * (double)room;
+  }
+  *grid_out = grid;
+  *smem_out = smem;
+  free(g);
+  free(ord);
+  return ok;
+}
+
 #define CK(call) do{ int _e = (call); if(_e){ rc = ODPX_ERR_CUDA; goto fail; } }while(0)
 
 int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning, odp_plan **out)
@@ -563,6 +709,14 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   int small = choose_small(shapes, count, tuning, sms, small_wl, &p->small_cluster, &p->small_threads,
                            &p->small_smem, &p->small_part);
   p->sweep = !small && count == 1 && choose_sweep(shapes, tuning, sms, &p->sw, &p->sweep_grid);
+  int *team_order = NULL;
+  if(!small && !p->sweep){
+    p->h_teams = calloc((size_t)count, sizeof(gbx_sweep));
+    team_order = calloc((size_t)count, sizeof(int));
+    p->team = p->h_teams && team_order &&
+              choose_team(shapes, count, tuning, sms, p->h_teams, &p->tm, team_order, &p->sweep_grid, &p->team_smem);
+  }
+  const int lockstep = p->sweep || p->team;
 
   /* Shapes, chunk widths, tiles. */
   int njobs = 0;
@@ -601,12 +755,13 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
     if(wl > full_l2 && full_l2 >= 1) wl = full_l2;
     if(small) wl = small_wl[i];
     if(p->sweep) wl = p->sw.wc_log2;
+    if(p->team) wl = p->h_teams[i].wc_log2;
     g->wc_log2 = wl;
     const int wc = 1 << wl;
     g->nchunks = (g->W + wc - 1) / wc;
     g->has_ndeg = sh->num_degrees != NULL;
-    g->has_itable = g->grid_s || (p->sweep && sh->grid);   /* the lockstep kernel's grid rows follow a curve */
-    g->has_srcpos = sh->grid && !p->sweep;   /* grids: spatially compact source chunks */
+    g->has_itable = g->grid_s || (lockstep && sh->grid);   /* the lockstep kernels' grid rows follow a curve */
+    g->has_srcpos = sh->grid && !lockstep;   /* grids: spatially compact source chunks */
     g->adj_ints = (size_t)g->B * g->d;
     g->adj_off = p->adj_ints;       p->adj_ints += ALIGN_UP(g->adj_ints, 4);
     g->ndeg_off = p->ndeg_ints;     if(g->has_ndeg) p->ndeg_ints += ALIGN_UP((size_t)g->n, 4);
@@ -667,6 +822,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
       g->tile_rows = ALIGN_UP(tr < rpp ? rpp : tr, rpp);
     }
     if(p->sweep) g->tile_rows = p->sw.rows;
+    if(p->team) g->tile_rows = p->h_teams[i].rows;
     if(g->tile_rows > g->n) g->tile_rows = g->n;
     if(g->tile_rows < 1) g->tile_rows = 1;
     g->ntiles = (g->n + g->tile_rows - 1) / g->tile_rows;
@@ -689,7 +845,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
         j->tile_rows = g->tile_rows; j->ntiles = g->ntiles;
         j->flags = tracks_changes(tuning, count, g->grid, g->n, g->s) ? GBX_JOB_ACTIVE : 0;
         ord[k].job = k;
-        ord[k].work = (double)g->n * wc * (g->d + 2) * (count > 1 ? 1.0 : 0.0);
+        ord[k].work = (double)g->n * wc * (g->d + 2) * (count > 1 && !p->team ? 1.0 : 0.0);
       }
     }
   }
@@ -728,6 +884,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
     if(nslots > 512) nslots = 512;
   }
   if(p->sweep) nslots = p->sw.phases * p->sw.slots;
+  if(p->team) nslots = 1;
   const size_t buffers = (size_t)nslots;
   if(nslots > njobs) nslots = njobs;
   if(nslots < 1) nslots = 1;
@@ -747,7 +904,8 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   if(p->ndeg_ints) CK(gbx_malloc((void **)&p->d_ndeg, sizeof(int) * p->ndeg_ints));
   if(p->itable_ints) CK(gbx_malloc((void **)&p->d_itable, sizeof(int) * p->itable_ints));
   CK(gbx_malloc((void **)&p->d_nbr, sizeof(int) * (p->nbr_ints ? p->nbr_ints : 4)));
-  CK(gbx_malloc((void **)&p->d_slotbuf, sizeof(unsigned long long) * p->slot_words * 2 * (p->sweep ? buffers : (size_t)nslots)));
+  if(p->team) CK(gbx_malloc((void **)&p->d_slotbuf, p->tm.arena_bytes));
+  else CK(gbx_malloc((void **)&p->d_slotbuf, sizeof(unsigned long long) * p->slot_words * 2 * (p->sweep ? buffers : (size_t)nslots)));
   CK(gbx_malloc((void **)&p->d_slotmask, sizeof(unsigned int) * p->slot_rows * 2 * (size_t)nslots));
   if(p->srcpos_ints) CK(gbx_malloc((void **)&p->d_srcpos, sizeof(int) * p->srcpos_ints));
   CK(gbx_malloc((void **)&p->d_expand, sizeof(gbx_expand_desc) * (size_t)count));
@@ -756,22 +914,34 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   p->direct = tuning->direct && gbx_pageable_access();
   /* Small plans read their descriptors (and through them the adjacency)
    * from pinned host memory and write per-job records there. */
-  if(p->direct || small || p->sweep) CK(gbx_host_alloc((void **)&p->h_expand, sizeof(gbx_expand_desc) * (size_t)count));
+  if(p->direct || small || lockstep) CK(gbx_host_alloc((void **)&p->h_expand, sizeof(gbx_expand_desc) * (size_t)count));
   if(!p->direct) CK(gbx_host_alloc((void **)&p->h_adj, sizeof(int) * (p->adj_ints ? p->adj_ints : 4)));
-  if(p->sweep){
+  if(lockstep){
     CK(gbx_host_alloc((void **)&p->h_small_rec, sizeof(gbx_small_rec) * (size_t)njobs));
     memset(p->h_small_rec, 0, sizeof(gbx_small_rec) * (size_t)njobs);
     CK(gbx_host_device_ptr(p->h_small_rec, (void **)&p->d_small_rec));
     CK(gbx_host_alloc((void **)&p->h_abort, sizeof(unsigned int)));
     *p->h_abort = 0;
     CK(gbx_host_device_ptr(p->h_abort, (void **)&p->sw.abort_flag));
-    CK(gbx_malloc(&p->d_sync, gbx_sweep_sync_bytes()));
-    CK(gbx_memset(p->d_sync, 0, gbx_sweep_sync_bytes(), p->stream));
-    if(p->sw.track)
+    if(p->team){
+      /* the queue counters (256 bytes), then the teams' nodes */
+      const int nodes = (2 << p->tm.last_split) - (1 << p->tm.first_split);
+      p->team_node_bytes = 256 + gbx_team_node_bytes() * (size_t)nodes;
+      CK(gbx_malloc(&p->d_sync, p->team_node_bytes));
+      CK(gbx_malloc(&p->d_teams, (sizeof(gbx_sweep) + sizeof(int) + 2 * sizeof(unsigned long long)) * (size_t)count));
+      CK(gbx_host_alloc((void **)&p->h_ptrs, sizeof(unsigned long long) * (size_t)count));
+      if(p->itable_ints) CK(gbx_malloc((void **)&p->d_row_vertex, sizeof(int) * p->itable_ints));
+    }
+    else{
+      CK(gbx_malloc(&p->d_sync, gbx_sweep_sync_bytes()));
+      CK(gbx_memset(p->d_sync, 0, gbx_sweep_sync_bytes(), p->stream));
+    }
+    if(p->team){}
+    else if(p->sw.track)
       CK(gbx_malloc((void **)&p->d_changed, sizeof(unsigned int) * 2 * ((size_t)p->g[0].n << p->sw.word_log2)));
     else if(njobs > p->sw.phases * p->sw.slots)   /* more than one group: the start's bits of every chunk apart */
       CK(gbx_malloc((void **)&p->d_start, sizeof(unsigned long long) * p->slot_words * (size_t)njobs));
-    if(p->g[0].has_itable) CK(gbx_malloc((void **)&p->d_row_vertex, sizeof(int) * (size_t)p->g[0].n));
+    if(p->sweep && p->itable_ints) CK(gbx_malloc((void **)&p->d_row_vertex, sizeof(int) * p->itable_ints));
   }
   else if(small){
     CK(gbx_host_alloc((void **)&p->h_small_rec, sizeof(gbx_small_rec) * (size_t)njobs));
@@ -804,7 +974,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
         for(int v = 0; v < g->n; v++) g->row_reads += (double)h_nd[g->ndeg_off + v] + 2.0;
       }
       else g->row_reads = (double)g->n * (g->d + 2);
-      if(g->has_itable && !p->sweep) fill_itable(g->width, g->height, g->s, h_it + g->itable_off);
+      if(g->has_itable && !lockstep) fill_itable(g->width, g->height, g->s, h_it + g->itable_off);
       if(g->has_srcpos) fill_srcpos(g, h_sp + g->srcpos_off);
       gbx_expand_desc *e = &ed[i];
       e->adj = p->d_adj + g->adj_off;
@@ -821,10 +991,14 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
       p->h_jobs[k].nbr = p->d_nbr + g->nbr_off;
       p->h_jobs[k].srcpos = g->has_srcpos ? p->d_srcpos + g->srcpos_off : NULL;
     }
-    if(p->sweep && p->g[0].has_itable){
-      int *h_rv = malloc(sizeof(int) * (size_t)p->g[0].n);
-      rc = h_rv ? fill_curve_rows(&p->g[0], h_it, h_rv) : ODPX_ERR_MEMORY;
-      if(!rc && (gbx_memcpy_h2d(p->d_row_vertex, h_rv, sizeof(int) * (size_t)p->g[0].n, p->stream) ||
+    if(lockstep && p->itable_ints){
+      int *h_rv = malloc(sizeof(int) * p->itable_ints);
+      rc = h_rv ? 0 : ODPX_ERR_MEMORY;
+      for(int i = 0; i < count && !rc; i++){
+        const odp_plan_graph *g = &p->g[i];
+        if(g->has_itable) rc = fill_curve_rows(g, h_it + g->itable_off, h_rv + g->itable_off);
+      }
+      if(!rc && (gbx_memcpy_h2d(p->d_row_vertex, h_rv, sizeof(int) * p->itable_ints, p->stream) ||
                  gbx_stream_sync(p->stream)))
         rc = ODPX_ERR_CUDA;
       free(h_rv);
@@ -837,7 +1011,34 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
     if(h_nd) CK(gbx_memcpy_h2d(p->d_ndeg, h_nd, sizeof(int) * p->ndeg_ints, p->stream));
     if(h_it) CK(gbx_memcpy_h2d(p->d_itable, h_it, sizeof(int) * p->itable_ints, p->stream));
     CK(gbx_memcpy_h2d(p->d_expand, ed, sizeof(gbx_expand_desc) * (size_t)count, p->stream));
-    if(p->sweep){
+    if(p->team){
+      char *dev = p->d_teams;
+      const size_t args = sizeof(gbx_sweep) * (size_t)count, ptrs = sizeof(unsigned long long) * (size_t)count;
+      int job = 0;
+      for(int i = 0; i < count; i++){
+        gbx_sweep *w = &p->h_teams[i];
+        const odp_plan_graph *g = &p->g[i];
+        const size_t words = (size_t)g->n << g->wc_log2;
+        w->e = ed[i];
+        w->e.adj_dev = p->direct ? (int *)ed[i].adj : NULL;
+        w->row_vertex = g->has_itable ? p->d_row_vertex + g->itable_off : NULL;
+        w->slot_words = ALIGN_UP(words, 4) * (w->track ? (size_t)w->slots : 1);
+        w->rec = p->d_small_rec + job;
+        w->abort_flag = p->sw.abort_flag;
+        job += w->nchunks;
+      }
+      gbx_team *tm = &p->tm;
+      tm->graphs = (const gbx_sweep *)dev;
+      tm->adj = p->direct ? (const unsigned long long *)(dev + args) : NULL;
+      tm->order = (const int *)(dev + args + ptrs);
+      tm->next = (unsigned int *)p->d_sync;
+      tm->nodes = (char *)p->d_sync + 256;
+      tm->arena = (unsigned char *)p->d_slotbuf;
+      tm->abort_flag = p->sw.abort_flag;
+      CK(gbx_memcpy_h2d(dev, p->h_teams, args, p->stream));
+      CK(gbx_memcpy_h2d(dev + args + ptrs, team_order, sizeof(int) * (size_t)count, p->stream));
+    }
+    else if(p->sweep){
       /* the launch carries the descriptor: per call `adj` names the caller's
        * array, which the kernel copies to `adj_dev`; without direct reads the
        * call uploads it and `adj` names the device copy */
@@ -878,6 +1079,8 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
     CK(gbx_stream_sync(p->stream));
     free(h_nd); free(h_it); free(h_sp); free(ed);
   }
+  free(team_order);
+  team_order = NULL;
 
   fill_state_init(p);
   if(p->d_state_init){
@@ -888,6 +1091,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   return 0;
 
 fail:
+  free(team_order);
   odp_plan_destroy(p);
   return rc;
 }
@@ -902,7 +1106,9 @@ void odp_plan_destroy(odp_plan *p)
   gbx_host_free(p->h_adj); gbx_host_free(p->h_expand); gbx_host_free(p->h_state_init); gbx_host_free(p->h_state_out);
   gbx_host_free(p->h_small_rec);
   gbx_free(p->d_row_vertex); gbx_free(p->d_changed); gbx_free(p->d_sync); gbx_free(p->d_start);
-  gbx_host_free(p->h_abort);
+  gbx_host_free(p->h_abort); gbx_host_free(p->h_ptrs);
+  gbx_free(p->d_teams);
+  free(p->h_teams);
   if(p->stream) gbx_stream_destroy(p->stream);
   free(p->h_jobs);
   free(p->g);
@@ -915,6 +1121,14 @@ static int enqueue(odp_plan *p)
 {
   int e;
   if(p->small) return odp_plan_enqueue_engine(p);
+  if(p->team){
+    if(p->direct){
+      if((e = gbx_memcpy_h2d((void *)p->tm.adj, p->h_ptrs, sizeof(unsigned long long) * (size_t)p->ngraphs, p->stream)))
+        return e;
+    }
+    else if((e = gbx_memcpy_h2d(p->d_adj, p->h_adj, sizeof(int) * (p->adj_ints ? p->adj_ints : 4), p->stream))) return e;
+    return odp_plan_enqueue_engine(p);
+  }
   if(p->sweep){
     if(!p->direct &&
        (e = gbx_memcpy_h2d(p->d_adj, p->h_adj, sizeof(int) * (p->adj_ints ? p->adj_ints : 4), p->stream)))
@@ -944,6 +1158,12 @@ static int enqueue(odp_plan *p)
 
 int odp_plan_enqueue_engine(odp_plan *p)
 {
+  if(p->team){
+    int e = gbx_memset(p->d_sync, 0, p->team_node_bytes, p->stream);
+    if(e) return e;
+    p->tm.limit_ns = p->spin_limit_ns;
+    return gbx_team_launch(&p->tm, p->sweep_grid, p->team_smem, p->stream);
+  }
   if(p->small){
     /* one graph: its descriptor (this call's adjacency pointer) travels in
      * the launch's parameters, so the plan is launched directly each call */
@@ -992,6 +1212,8 @@ void odp_plan_stage(odp_plan *p, const int *const *adjacency)
     /* The device reads pageable host memory: no staging copy, only the
      * pointers (the arrays must stay unchanged until the run is finished). */
     for(int i = 0; i < p->ngraphs; i++) p->h_expand[i].adj = adjacency[i];
+    if(p->team)
+      for(int i = 0; i < p->ngraphs; i++) p->h_ptrs[i] = (unsigned long long)(uintptr_t)adjacency[i];
     return;
   }
   size_t total = sizeof(int) * p->adj_ints;
@@ -1101,26 +1323,28 @@ static int finish_small(odp_plan *p, odp_result *results)
   }
   if(err & GBX_ERR_BAD_ADJ) return ODPX_ERR_ADJACENCY;
   for(int i = 0; i < p->ngraphs; i++){
-    unsigned long long sum = 0;
-    int level = 0, stalled = 0;
-    for(int k = 0; k < p->njobs; k++){
-      const gbx_small_rec *r = &p->h_small_rec[k];
-      if(p->h_jobs[k].graph != i) continue;
-      sum += (unsigned long long)r->sum;
-      const int l = r->level < 0 ? -r->level : r->level;
-      if(l > level) level = l;
-      if(r->level < 0) stalled = 1;
-    }
+    results[i].sum = 0;
+    results[i].diameter = 0;
+    results[i].aspl = 0.0;                       /* set when a job stalled */
+  }
+  for(int k = 0; k < p->njobs; k++){
+    const gbx_small_rec *r = &p->h_small_rec[k];
+    odp_result *res = &results[p->h_jobs[k].graph];
+    const int l = r->level < 0 ? -r->level : r->level;
+    res->sum += (long)r->sum;
+    if(l > res->diameter) res->diameter = l;
+    if(r->level < 0) res->aspl = 1.0;
+  }
+  for(int i = 0; i < p->ngraphs; i++){
     const odp_plan_graph *g = &p->g[i];
     odp_result *res = &results[i];
-    if(stalled){
+    if(res->aspl != 0.0){
       res->diameter = INT_MAX;
       res->sum = LONG_MAX;
       res->aspl = DBL_MAX;
       continue;
     }
-    long total = (long)sum;
-    res->diameter = level;
+    const long total = res->sum;
     res->aspl = total / (((double)g->n - 1) * g->n);
     res->sum = (long)(total / 2.0);
   }
@@ -1130,11 +1354,11 @@ static int finish_small(odp_plan *p, odp_result *results)
 int odp_plan_finish(odp_plan *p, odp_result *results)
 {
   if(gbx_stream_sync(p->stream)) return ODPX_ERR_CUDA;
-  if(p->sweep && *p->h_abort){
+  if(p->h_abort && *p->h_abort){
     *p->h_abort = 0;
     return ODPX_ERR_TIMEOUT;
   }
-  if(p->small || p->sweep) return finish_small(p, results);
+  if(p->small || p->sweep || p->team) return finish_small(p, results);
   const gbx_ctrl *ctrl = (const gbx_ctrl *)p->h_state_out;
   unsigned int err = *(const unsigned int *)(p->h_state_out + sizeof(gbx_ctrl)) | ctrl->error;
   if(err & GBX_ERR_TIMEOUT) return ODPX_ERR_TIMEOUT;
@@ -1178,8 +1402,8 @@ unsigned long long odp_plan_tiles(const odp_plan *p)
 
 unsigned int odp_plan_error(const odp_plan *p)
 {
-  if(p->small || p->sweep){
-    unsigned int err = p->sweep ? *p->h_abort : 0;
+  if(p->small || p->sweep || p->team){
+    unsigned int err = p->h_abort ? *p->h_abort : 0;
     for(int k = 0; k < p->njobs; k++) err |= p->h_small_rec[k].err;
     return err;
   }

@@ -35,7 +35,8 @@ typedef struct {
   int small_n;                 /* graphs of at most this many vertices may run in shared memory (0: never) */
   int small_cluster;           /* CTAs per small-kernel job: 1, 2, 4 or 8; 0 = automatic */
   int small_part;              /* small-kernel rows partitioned over the cluster: -1 when needed, 0 never, 1 always */
-  int sweep;                   /* single graphs run in lockstep on every SM where that fits (1, default) */
+  int sweep;                   /* graphs run in lockstep on every SM, or on teams of CTAs, where that fits (1, default) */
+  int team;                    /* a single graph may run as a team of every CTA (annealing) */
 } odp_tuning;
 
 typedef struct {
@@ -90,6 +91,12 @@ typedef struct odp_plan {
   int sweep;                   /* the plan's one graph runs in the lockstep kernel */
   gbx_sweep sw;                /* its launch arguments */
   int sweep_grid;              /* CTAs */
+  int team;                    /* the plan's graphs run in the team kernel */
+  gbx_team tm;                 /* its launch arguments */
+  gbx_sweep *h_teams;          /* per graph: its arguments */
+  void *d_teams;               /* the same on the device, then the queue order */
+  size_t team_smem, team_node_bytes;
+  unsigned long long *h_ptrs;  /* pinned: this call's host arrays (direct plans) */
   unsigned long long *d_start; /* the start's bits of all chunks, where the slots hold only some */
   int *d_row_vertex;           /* row -> vertex where the plan orders the rows */
   unsigned int *d_changed;     /* the lockstep kernel's changed-lane masks */

@@ -1,5 +1,6 @@
 /*
- * sweep.cu -- one graph per call, evaluated by every SM in lockstep.
+ * sweep.cu -- graphs evaluated in lockstep: one graph by every SM, or many by
+ * teams of CTAs.
  *
  * The persistent engine (aspl_engine.cu) hands every level of every job out
  * in tiles through a ticket.  That suits many uneven graphs, but a single
@@ -44,15 +45,18 @@
 
 namespace {
 
-/* Counters of one call; the call before clears them. */
-struct SweepSync {
+/* Counters of one graph's evaluation by PH phases over at most CH chunks;
+ * the evaluation before clears them. */
+template <int PH, int CH>
+struct SyncT {
   unsigned ready[3];                                 /* CTAs past the copy, the expansion, the start */
   unsigned err;                                      /* GBX_ERR_* */
   unsigned pad[28];
-  unsigned long long arrive[GBX_SWEEP_PHASES][3][16];           /* step t's barrier word: [t % 3][0] */
-  unsigned long long count[GBX_SWEEP_PHASES][3][SWEEP_SLOTS];   /* bits per chunk of step t */
-  unsigned long long start1[GBX_SWEEP_CHUNKS], start2[GBX_SWEEP_CHUNKS];  /* bits at levels 1 and 2 */
+  unsigned long long arrive[PH][3][16];              /* step t's barrier word: [t % 3][0] */
+  unsigned long long count[PH][3][SWEEP_SLOTS];      /* bits per chunk of step t */
+  unsigned long long start1[CH], start2[CH];         /* bits at levels 1 and 2 */
 };
+typedef SyncT<GBX_SWEEP_PHASES, GBX_SWEEP_CHUNKS> SweepSync;
 
 /* A phase's progress, the same in every CTA but for `prev`, `sum` and
  * `alive`, which CTA 0 keeps for the records. */
@@ -69,6 +73,8 @@ struct SweepShared {
   SweepPhase ph[GBX_SWEEP_PHASES];
   unsigned cnt[SWEEP_SLOTS];                         /* this CTA's bits per chunk of the current step */
   int todo;
+  int rank, size;                                    /* of this CTA among those that evaluate the graph */
+  unsigned long long begin;                          /* when it began the graph */
 };
 
 #define TODO_DONE 0
@@ -130,7 +136,7 @@ __device__ __forceinline__ bool grid_pass(unsigned *word, SweepShared &sh, const
     unsigned seen;
     __threadfence();
     atomicAdd(word, 1u);
-    const bool ok = wait_for(word, gridDim.x, seen, a.limit_ns);
+    const bool ok = wait_for(word, (unsigned)sh.size, seen, a.limit_ns);
     sh.todo = ok ? TODO_LEVEL : TODO_ABORT;
     if(!ok) *a.abort_flag = GBX_ERR_TIMEOUT;           /* pinned host memory */
   }
@@ -158,7 +164,8 @@ __device__ __forceinline__ int group_chunk(const gbx_sweep &a, int group, int ph
 /* A chunk's bits after `level` (CTA 0, the thread of the chunk): records the
  * chunk when it is complete or stalled (then false), else adds the level's
  * share of the distance sum. */
-__device__ __forceinline__ bool settle(const gbx_sweep &a, SweepPhase &p, const SweepSync &sy, int chunk, int q,
+template <class Sync>
+__device__ __forceinline__ bool settle(const gbx_sweep &a, SweepPhase &p, const Sync &sy, int chunk, int q,
                                        int level, unsigned long long c)
 {
   const unsigned long long full = (unsigned long long)a.e.n * (unsigned long long)chunk_sources(a, chunk);
@@ -181,7 +188,8 @@ __device__ __forceinline__ bool settle(const gbx_sweep &a, SweepPhase &p, const 
 
 /* CTA 0, warp 0: the chunks' counts of step `step`, which ended `level`.
  * `added`: the counts are of bits added. */
-__device__ __forceinline__ void settle_step(const gbx_sweep &a, SweepPhase &p, const SweepSync &sy, int ph,
+template <class Sync>
+__device__ __forceinline__ void settle_step(const gbx_sweep &a, SweepPhase &p, const Sync &sy, int ph,
                                             unsigned step, int level, bool added)
 {
   const int q = threadIdx.x;
@@ -222,19 +230,20 @@ __device__ __forceinline__ void group_state(const gbx_sweep &a, SweepPhase &p, i
  * barrier word with their total.  CTA 0 first clears the next step's words:
  * their last readers (step - 2) have all arrived at step - 1, which this CTA
  * has waited for, and nobody adds to them before it arrives. */
-__device__ __forceinline__ void arrive_step(const gbx_sweep &a, SweepShared &sh, SweepSync &sy, int ph)
+template <class Sync>
+__device__ __forceinline__ void arrive_step(const gbx_sweep &a, SweepShared &sh, Sync &sy, int ph)
 {
   const int q = threadIdx.x;
   const unsigned step = sh.ph[ph].step;
   const unsigned c = q < a.slots ? sh.cnt[q] : 0u;
   if(q < a.slots){
-    if(blockIdx.x == 0) sy.count[ph][(step + 1) % 3][q] = 0;
+    if(sh.rank == 0) sy.count[ph][(step + 1) % 3][q] = 0;
     if(c) atomicAdd(&sy.count[ph][step % 3][q], (unsigned long long)c);
     sh.cnt[q] = 0;
   }
   const unsigned total = __reduce_add_sync(0xffffffffu, c);   /* rows x lanes x 256 of one CTA: below 2^32 */
   if(q == 0){
-    if(blockIdx.x == 0) sy.arrive[ph][(step + 1) % 3][0] = 0;
+    if(sh.rank == 0) sy.arrive[ph][(step + 1) % 3][0] = 0;
     __threadfence();
     atomicAdd(&sy.arrive[ph][step % 3][0], ARRIVE_ONE | total);
     sh.ph[ph].step = step + 1;
@@ -244,46 +253,69 @@ __device__ __forceinline__ void arrive_step(const gbx_sweep &a, SweepShared &sh,
 
 /* Warp 0 waits for the phase's last step and takes its count (true), or past
  * the limit gives up.  CTA 0 settles the step before meanwhile. */
-__device__ __forceinline__ bool wait_step(const gbx_sweep &a, SweepShared &sh, SweepSync &sy, int ph, bool added,
+template <class Sync>
+__device__ __forceinline__ bool wait_step(const gbx_sweep &a, SweepShared &sh, Sync &sy, int ph, bool added,
                                           int first_level, unsigned long long &bits)
 {
   SweepPhase &p = sh.ph[ph];
   const unsigned step = p.step;
-  if(blockIdx.x == 0 && p.level > first_level) settle_step(a, p, sy, ph, step - 2, p.level - 1, added);
+  if(sh.rank == 0 && p.level > first_level) settle_step(a, p, sy, ph, step - 2, p.level - 1, added);
   unsigned long long seen = 0;
   bool ok = true;
-  if(threadIdx.x == 0) ok = wait_for(&sy.arrive[ph][(step - 1) % 3][0], ARRIVE_ONE * gridDim.x, seen, a.limit_ns);
+  if(threadIdx.x == 0) ok = wait_for(&sy.arrive[ph][(step - 1) % 3][0], ARRIVE_ONE * (unsigned)sh.size, seen, a.limit_ns);
   ok = __all_sync(0xffffffffu, ok);
   bits = __shfl_sync(0xffffffffu, seen, 0) & ARRIVE_BITS;
   return ok;
 }
 
-/* Clears the other half of the counters for the next launch. */
-__device__ __forceinline__ SweepSync &sweep_begin(const gbx_sweep &a, SweepShared &sh)
+/* This CTA's place among those that evaluate the graph, and clean counts. */
+__device__ __forceinline__ void sweep_begin(SweepShared &sh, int rank, int size)
+{
+  if(threadIdx.x < SWEEP_SLOTS) sh.cnt[threadIdx.x] = 0;
+  if(threadIdx.x < GBX_SWEEP_PHASES) sh.ph[threadIdx.x].step = 0;
+  if(threadIdx.x == 0){
+    sh.rank = rank;
+    sh.size = size;
+    sh.begin = globaltimer();
+  }
+  __syncthreads();
+}
+
+/* A launch of one graph alternates between two sets of counters; CTA 0
+ * clears the other one for the next launch. */
+__device__ __forceinline__ SweepSync &launch_sync(const gbx_sweep &a)
 {
   SweepSync *sy = reinterpret_cast<SweepSync *>(a.sync);
   if(blockIdx.x == 0){
     unsigned *other = reinterpret_cast<unsigned *>(sy + (a.set ^ 1));
     for(int i = threadIdx.x; i < (int)(sizeof(SweepSync) / 4); i += SWEEP_THREADS) other[i] = 0;
   }
-  if(threadIdx.x < SWEEP_SLOTS) sh.cnt[threadIdx.x] = 0;
-  if(threadIdx.x < GBX_SWEEP_PHASES) sh.ph[threadIdx.x].step = 0;
   return sy[a.set];
 }
 
 /* The CTA's slice of the compact adjacency out of host memory; then the
  * whole grid has the device copy.  False past the limit. */
-__device__ __forceinline__ bool pull_adjacency(const gbx_sweep &a, SweepShared &sh, SweepSync &sy)
+template <class Sync>
+__device__ __forceinline__ bool pull_adjacency(const gbx_sweep &a, SweepShared &sh, Sync &sy)
 {
   if(!a.e.adj_dev || a.in_place) return true;
   const long long ints = (long long)a.B * a.e.d;
-  const long long t0 = (long long)blockIdx.x * SWEEP_THREADS + threadIdx.x;
-  const long long stride = (long long)gridDim.x * SWEEP_THREADS;
+  const long long t0 = (long long)sh.rank * SWEEP_THREADS + threadIdx.x;
+  const long long stride = (long long)sh.size * SWEEP_THREADS;
   if(((reinterpret_cast<uintptr_t>(a.e.adj) | reinterpret_cast<uintptr_t>(a.e.adj_dev)) & 15) == 0){
+    /* several reads in flight per thread: a small team's copy is bound by the
+     * host link's latency */
     const int4 *src = reinterpret_cast<const int4 *>(a.e.adj);
     int4 *dst = reinterpret_cast<int4 *>(a.e.adj_dev);
-    for(long long i = t0; i < (ints >> 2); i += stride) dst[i] = src[i];
-    if(blockIdx.x == 0)
+    const int q = (int)(ints >> 2), st = sh.size * SWEEP_THREADS;
+    for(int i0 = (int)t0; i0 < q; i0 += st * 8){
+      int4 x[8];
+#pragma unroll
+      for(int k = 0; k < 8; k++) x[k] = src[min(i0 + k * st, q - 1)];
+#pragma unroll
+      for(int k = 0; k < 8; k++) dst[min(i0 + k * st, q - 1)] = x[k];
+    }
+    if(sh.rank == 0)
       for(long long i = (ints & ~3LL) + threadIdx.x; i < ints; i += SWEEP_THREADS) a.e.adj_dev[i] = a.e.adj[i];
   }
   else
@@ -294,7 +326,8 @@ __device__ __forceinline__ bool pull_adjacency(const gbx_sweep &a, SweepShared &
 /* The neighbour lists of the CTA's rows row0 + i * drow, i < nr, in shared
  * memory (and the table, if given).  2^lr threads share a row, eight rows in
  * flight per thread. */
-__device__ __forceinline__ void expand_rows(const gbx_sweep &a, SweepSync &sy, int *list, int row0, int drow, int nr,
+template <class Sync>
+__device__ __forceinline__ void expand_rows(const gbx_sweep &a, Sync &sy, int *list, int row0, int drow, int nr,
                                             int *table)
 {
   const int *adj = a.e.adj_dev && !a.in_place ? a.e.adj_dev : a.e.adj;
@@ -520,7 +553,8 @@ __device__ void level_rows(const gbx_sweep &a, SweepShared &sh, const int *list,
 
 /* Warp 0: what the phase does next.  After the group's last level (complete,
  * or a level that added nothing) the next group begins. */
-__device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, SweepSync &sy, int ph)
+template <class Sync>
+__device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, Sync &sy, int ph)
 {
   SweepPhase &p = sh.ph[ph];
   const int base = a.two_level ? 2 : 1;                  /* the level that the start computed */
@@ -530,7 +564,7 @@ __device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, 
     if(!wait_step(a, sh, sy, ph, false, base + 1, bits)) todo = TODO_ABORT;
     else{
       if(bits == p.full || bits == p.total || p.level >= a.e.n){
-        if(blockIdx.x == 0) settle_step(a, p, sy, ph, p.step - 1, p.level, false);
+        if(sh.rank == 0) settle_step(a, p, sy, ph, p.step - 1, p.level, false);
         group_state(a, p, ph, p.group + 1);
       }
       else{
@@ -554,7 +588,7 @@ __device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, 
       t1 += __shfl_xor_sync(0xffffffffu, t1, o);
       t2 += __shfl_xor_sync(0xffffffffu, t2, o);
     }
-    if(blockIdx.x == 0){
+    if(sh.rank == 0){
       if(go && a.two_level) go = settle(a, p, sy, chunk, q, 1, c1);
       if(go) go = settle(a, p, sy, chunk, q, base, c2);
       const unsigned alive = __ballot_sync(0xffffffffu, go);
@@ -575,23 +609,22 @@ __device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, 
   __syncwarp();
 }
 
-template <int NB, int MIN_BLOCKS>
-__global__ void __launch_bounds__(SWEEP_THREADS, MIN_BLOCKS) sweep_dense_kernel(const gbx_sweep a)
+/* The whole evaluation by the CTAs of sh (all threads; false past a wait's
+ * limit).  after_pass() runs once, when every CTA has begun the graph. */
+template <int NB, class Sync, class AfterPass>
+__device__ bool dense_graph(const gbx_sweep &a, SweepShared &sh, Sync &sy, unsigned char *smem, AfterPass after_pass)
 {
-  extern __shared__ __align__(16) unsigned char sweep_smem[];
-  __shared__ SweepShared sh;
   const int tid = threadIdx.x, dp = a.e.dp;
-  const int r0 = (int)blockIdx.x * a.rows, nr = min(a.rows, a.e.n - r0);
-  int *list = reinterpret_cast<int *>(sweep_smem);                               /* [rows][dp] */
+  const int r0 = sh.rank * a.rows, nr = max(0, min(a.rows, a.e.n - r0));
+  int *list = reinterpret_cast<int *>(smem);                                     /* [rows][dp] */
   unsigned *scratch = reinterpret_cast<unsigned *>(list + (size_t)a.rows * dp);  /* a row of marks per warp */
   unsigned *cnt1 = scratch + SWEEP_WARPS * (a.scratch_bits >> 5), *cnt2 = cnt1 + a.nchunks;
   unsigned char *flag = reinterpret_cast<unsigned char *>(cnt2 + a.nchunks);     /* [phases * slots][rows][lanes] */
-  SweepSync &sy = sweep_begin(a, sh);
   for(int i = tid; i < 2 * a.nchunks; i += SWEEP_THREADS) cnt1[i] = 0;
-  if(!pull_adjacency(a, sh, sy)) return;
+  if(!pull_adjacency(a, sh, sy)) return false;
   expand_rows(a, sy, list, r0, 1, nr, a.two_level ? a.e.nbr : nullptr);
   if(a.two_level){
-    if(!grid_pass(&sy.ready[1], sh, a)) return;
+    if(!grid_pass(&sy.ready[1], sh, a)) return false;
   }
   else __syncthreads();
   start_rows(a, list, scratch, cnt1, cnt2, 0, a.nchunks, r0, nr);
@@ -600,9 +633,13 @@ __global__ void __launch_bounds__(SWEEP_THREADS, MIN_BLOCKS) sweep_dense_kernel(
     if(cnt1[c]) atomicAdd(&sy.start1[c], (unsigned long long)cnt1[c]);
     if(cnt2[c]) atomicAdd(&sy.start2[c], (unsigned long long)cnt2[c]);
   }
-  if(!grid_pass(&sy.ready[2], sh, a)) return;
+  if(!grid_pass(&sy.ready[2], sh, a)) return false;
+  after_pass();
   if(tid < 32)
-    for(int ph = 0; ph < a.phases; ph++) group_state(a, sh.ph[ph], ph, 0);
+    for(int ph = 0; ph < a.phases; ph++){
+      group_state(a, sh.ph[ph], ph, 0);
+      if(tid == 0) sh.ph[ph].t_loaded = sh.begin;
+    }
 
   unsigned open = (1u << a.phases) - 1u;                 /* phases with groups left */
   while(open)
@@ -614,41 +651,56 @@ __global__ void __launch_bounds__(SWEEP_THREADS, MIN_BLOCKS) sweep_dense_kernel(
       const int todo = sh.todo;
       if(todo == TODO_ABORT){
         if(tid == 0) *a.abort_flag = GBX_ERR_TIMEOUT;
-        return;
+        return false;
       }
       if(todo == TODO_DONE){ open &= ~(1u << ph); continue; }
       level_rows<NB>(a, sh, list, flag, ph, sh.ph[ph].level == (a.two_level ? 3 : 2), r0, nr);
       __syncthreads();
       if(tid < 32) arrive_step(a, sh, sy, ph);
     }
+  __syncthreads();
+  return true;
+}
+
+template <int NB, int MIN_BLOCKS>
+__global__ void __launch_bounds__(SWEEP_THREADS, MIN_BLOCKS) sweep_dense_kernel(const gbx_sweep a)
+{
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  __shared__ SweepShared sh;
+  SweepSync &sy = launch_sync(a);
+  sweep_begin(sh, (int)blockIdx.x, (int)gridDim.x);
+  dense_graph<NB>(a, sh, sy, sweep_smem, [] {});
 }
 
 /* ---------------------------------------------------------------------- */
 /* Grids.                                                                  */
 /* ---------------------------------------------------------------------- */
 
-#define TRACK_QUEUE 1024              /* 32 words of 32 lanes */
+#define TRACK_SOLO 1024               /* pairs of a CTA from which its warps work alone */
 
-/* Per-warp working memory of a step over 32 (row, word) pairs. */
-struct TrackWarp {
-  unsigned newc[32], newf[32];        /* lanes that changed, lanes now full */
-  unsigned short queue[TRACK_QUEUE];  /* pair << 5 | lane of the word */
+/* Working memory of a round over SWEEP_THREADS (row, word) pairs. */
+struct TrackRound {
+  unsigned newc[SWEEP_THREADS], newf[SWEEP_THREADS];   /* lanes that changed, lanes now full */
+  unsigned count[SWEEP_SLOTS * 8];                     /* bits added per chunk, in eight parts */
+  int warp_items[2][SWEEP_WARPS];
+  int next;                                            /* the level's next block of 32 pairs */
+  unsigned short queue[SWEEP_THREADS * 32];            /* pair << 5 | lane of the word */
 };
 
 struct TrackShared {
   int *list;                          /* [rows][dp] */
   unsigned *have, *full, *last;       /* per (row, word), a bit per lane: holds bits; is full; buffer of its words */
-  TrackWarp *warp;
-  unsigned *near;                     /* this warp's [dp][32]: the neighbours' changed words */
+  unsigned *near;                     /* [dp][SWEEP_THREADS]: the neighbours' changed words of the round's pairs */
+  TrackRound *round;
 };
 
 /* Level 0 of a group: every source's own bit.  Lanes that hold nothing are
  * never stored or read. */
-__device__ void track_start(const gbx_sweep &a, const TrackShared &t, int src0, int nsrc, int nr)
+__device__ void track_start(const gbx_sweep &a, const SweepShared &sh, const TrackShared &t, int src0, int nsrc, int nr)
 {
   const int lw = a.word_log2, row_lanes = a.slots << (a.wc_log2 - 2);
   for(int c = threadIdx.x; c < (nr << lw); c += SWEEP_THREADS){
-    const int row = (int)blockIdx.x + (c >> lw) * (int)gridDim.x, w = c & ((1 << lw) - 1);
+    const int row = sh.rank + (c >> lw) * sh.size, w = c & ((1 << lw) - 1);
     const int o = row - src0, l = o >> 8;
     unsigned bit = 0, full = 0;
     if(row < a.B && (unsigned)o < (unsigned)nsrc && (l >> 5) == w){
@@ -666,18 +718,21 @@ __device__ void track_start(const gbx_sweep &a, const TrackShared &t, int src0, 
   }
 }
 
-/* One level: warp by warp over 32 (row, word) pairs of the CTA's rows (row
- * blockIdx.x + i * gridDim.x, so that the busy rows of a wavefront spread
- * over the CTAs).  The pairs' lanes with a changed neighbour are queued and
- * taken 32 at a time, whatever rows they come from.  A neighbour that did not
- * change is not read: its words of the previous level may never have been
- * stored, or lie in the other buffer.  (Reading a row of zeros in its place
- * saves the predicates, but that row's sectors are then read by everybody: a
- * 97 x 103 grid took 0.49 to 0.55 ms that way.) */
+/* One level over the CTA's (row, word) pairs (row rank + i * size, so that the
+ * busy rows of a wavefront spread over the CTAs).  The pairs' lanes with a
+ * changed neighbour are queued and shared out over the threads, whatever rows
+ * they come from.  With few pairs the CTA goes round by round, a pair per
+ * thread and the queue shared out evenly over all of them; with many (solo)
+ * each warp takes blocks of 32 pairs by itself, with no barrier in between
+ * (256 x 256: 5.26 ms against 5.6; 97 x 103: 0.34 against 0.32).  A neighbour
+ * that did not change is not read: its words of the previous level may never
+ * have been stored, or lie in the other buffer.  (Reading a row of zeros in
+ * its place saves the predicates, but that row's sectors are then read by
+ * everybody: a 97 x 103 grid took 0.49 to 0.55 ms that way.) */
 template <int NB>
 __device__ void track_level(const gbx_sweep &a, SweepShared &sh, const TrackShared &t, int level, int nsrc, int nr)
 {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int lw = a.word_log2, lL = a.wc_log2 - 2, dp = a.e.dp, d = a.e.d, n = a.e.n;
   const unsigned rb = (unsigned)(a.slots << lL) * 32u;   /* bytes of a row */
   const size_t half = a.slot_words * 8;                  /* bytes of a buffer */
@@ -685,14 +740,27 @@ __device__ void track_level(const gbx_sweep &a, SweepShared &sh, const TrackShar
   unsigned *now = a.changed + (size_t)(level & 1) * ((size_t)n << lw);
   const char *X = reinterpret_cast<const char *>(a.buf) + ((level & 1) ? 0 : half);
   char *Y = reinterpret_cast<char *>(a.buf) + ((level & 1) ? half : 0);
-  TrackWarp &tw = t.warp[warp];
+  TrackRound &tr = *t.round;
   const int pairs = nr << lw;
-  const int per = min(32, (pairs + SWEEP_WARPS - 1) / SWEEP_WARPS);
-  for(int c0 = warp * per; c0 < pairs; c0 += SWEEP_WARPS * per){
-    const int m = min(per, pairs - c0), c = c0 + lane;
-    const int w = c & ((1 << lw) - 1);
+  const bool solo = pairs >= TRACK_SOLO;
+  const unsigned short *queue = tr.queue + (solo ? warp * 1024 : 0);
+  for(int x = tid; x < SWEEP_SLOTS * 8; x += SWEEP_THREADS) tr.count[x] = 0;
+  __syncthreads();
+  for(int round = 0;; round++){
+    /* pair of this thread: first + tid */
+    int first = round * SWEEP_THREADS;
+    if(solo){
+      int blk = 0;
+      if(lane == 0) blk = atomicAdd(&tr.next, 1);
+      blk = __shfl_sync(0xffffffffu, blk, 0);
+      if(blk * 32 >= pairs) break;
+      first = (blk - warp) * 32;
+    }
+    else if(first >= pairs) break;
+    const int c = first + tid, w = c & ((1 << lw) - 1);
+    const bool mine = c < pairs;
     unsigned act = 0;
-    if(lane < m){
+    if(mine){
       const int *ids = t.list + (c >> lw) * dp;
       for(int j0 = 0; j0 < d; j0 += 8){
         unsigned x[8];
@@ -702,27 +770,37 @@ __device__ void track_level(const gbx_sweep &a, SweepShared &sh, const TrackShar
 #pragma unroll
         for(int k = 0; k < 8; k++)
           if(j0 + k < dp){
-            t.near[(j0 + k) * 32 + lane] = x[k];
+            t.near[(j0 + k) * SWEEP_THREADS + tid] = x[k];
             act |= x[k];
           }
       }
       act &= ~t.full[c];
-      tw.newc[lane] = tw.newf[lane] = 0;
     }
-    const int mine = __popc(act);
-    int end = mine;
+    tr.newc[tid] = tr.newf[tid] = 0;
+    const int items = __popc(act);
+    int at = items;
     for(int o = 1; o < 32; o <<= 1){
-      const int x = __shfl_up_sync(0xffffffffu, end, o);
-      if(lane >= o) end += x;
+      const int x = __shfl_up_sync(0xffffffffu, at, o);
+      if(lane >= o) at += x;
     }
-    const int total = __shfl_sync(0xffffffffu, end, 31);
-    int at = end - mine;
-    for(unsigned x = act; x; x &= x - 1) tw.queue[at++] = (unsigned short)(lane << 5 | (__ffs(x) - 1));
-    __syncwarp();
-    for(int i = lane; i < total; i += 32){
-      const int code = tw.queue[i], cl = code >> 5, b = code & 31, cc = c0 + cl;
+    int total = __shfl_sync(0xffffffffu, at, 31);
+    at += (solo ? warp * 1024 : 0) - items;
+    if(!solo){
+      if(lane == 31) tr.warp_items[round & 1][warp] = total;
+      __syncthreads();
+      total = 0;
+      for(int k = 0; k < SWEEP_WARPS; k++){
+        if(k == warp) at += total;
+        total += tr.warp_items[round & 1][k];
+      }
+    }
+    for(unsigned x = act; x; x &= x - 1) tr.queue[at++] = (unsigned short)(tid << 5 | (__ffs(x) - 1));
+    if(solo) __syncwarp();
+    else __syncthreads();
+    for(int i = solo ? lane : tid; i < total; i += solo ? 32 : SWEEP_THREADS){
+      const int code = queue[i], cl = code >> 5, b = code & 31, cc = first + cl;
       const int l = ((cc & ((1 << lw) - 1)) << 5) | b;   /* lane of the row */
-      const int row = (int)blockIdx.x + (cc >> lw) * (int)gridDim.x;
+      const int row = sh.rank + (cc >> lw) * sh.size;
       const int *ids = t.list + (cc >> lw) * dp;
       const unsigned *near = t.near + cl;
       const size_t own = (size_t)(unsigned)row * rb + (unsigned)l * 32u;
@@ -740,7 +818,7 @@ __device__ void track_level(const gbx_sweep &a, SweepShared &sh, const TrackShar
         for(int k = 0; k < NB; k++){
 #pragma unroll
           for(int e = 0; e < 8; e++) v[k][e] = 0;
-          if(j0 + k < d && ((near[(j0 + k) * 32] >> b) & 1u))
+          if(j0 + k < d && ((near[(j0 + k) * SWEEP_THREADS] >> b) & 1u))
             ld_lane(v[k], Xl + (size_t)(unsigned)ids[j0 + k] * rb);
         }
 #pragma unroll
@@ -757,26 +835,34 @@ __device__ void track_level(const gbx_sweep &a, SweepShared &sh, const TrackShar
       const unsigned added = popc_lane(diff);
       if(added){
         st_lane(Y + own, acc);
-        atomicOr(&tw.newc[cl], 1u << b);
+        atomicOr(&tr.newc[cl], 1u << b);
         const unsigned bits = (unsigned)lane_bits(nsrc, l);
-        if(bits == 256u ? and_lane(acc) == ~0u : popc_lane(acc) == bits) atomicOr(&tw.newf[cl], 1u << b);
-        atomicAdd(&sh.cnt[l >> lL], added);
+        if(bits == 256u ? and_lane(acc) == ~0u : popc_lane(acc) == bits) atomicOr(&tr.newf[cl], 1u << b);
+        atomicAdd(&tr.count[(l >> lL) * 8 + (tid & 7)], added);
       }
     }
-    __syncwarp();
-    if(lane < m){
-      const unsigned nc = tw.newc[lane];
-      __stcg(now + ((size_t)(unsigned)((int)blockIdx.x + (c >> lw) * (int)gridDim.x) << lw) + w, nc);
+    if(solo) __syncwarp();
+    else __syncthreads();
+    if(mine){
+      const unsigned nc = tr.newc[tid];
+      __stcg(now + ((size_t)(unsigned)(sh.rank + (c >> lw) * sh.size) << lw) + w, nc);
       t.have[c] |= nc;
-      t.full[c] |= tw.newf[lane];
+      t.full[c] |= tr.newf[tid];
       t.last[c] = (t.last[c] & ~nc) | ((level & 1) ? nc : 0u);
     }
-    __syncwarp();
+  }
+  __syncthreads();
+  if(warp == 0 && lane < a.slots){
+    unsigned s = 0;
+#pragma unroll
+    for(int k = 0; k < 8; k++) s += tr.count[lane * 8 + k];
+    sh.cnt[lane] = s;
   }
 }
 
 /* Warp 0: what comes next; level 0 (the sources themselves) starts a group. */
-__device__ __forceinline__ void plan_track(const gbx_sweep &a, SweepShared &sh, SweepSync &sy)
+template <class Sync>
+__device__ __forceinline__ void plan_track(const gbx_sweep &a, SweepShared &sh, Sync &sy)
 {
   SweepPhase &p = sh.ph[0];
   int todo = TODO_LEVEL;
@@ -784,7 +870,7 @@ __device__ __forceinline__ void plan_track(const gbx_sweep &a, SweepShared &sh, 
   if(p.step > 0){
     if(!wait_step(a, sh, sy, 0, true, 1, bits)) todo = TODO_ABORT;
     else if(p.level > 0 && (p.total + bits == p.full || bits == 0 || p.level >= a.e.n)){
-      if(blockIdx.x == 0) settle_step(a, p, sy, 0, p.step - 1, p.level, true);
+      if(sh.rank == 0) settle_step(a, p, sy, 0, p.step - 1, p.level, true);
       group_state(a, p, 0, p.group + 1);
       if(p.level < 0) todo = TODO_DONE;
     }
@@ -797,6 +883,51 @@ __device__ __forceinline__ void plan_track(const gbx_sweep &a, SweepShared &sh, 
   __syncwarp();
 }
 
+/* The whole evaluation by the CTAs of sh, as dense_graph. */
+template <int NB, class Sync, class AfterPass>
+__device__ bool track_graph(const gbx_sweep &a, SweepShared &sh, Sync &sy, unsigned char *smem, AfterPass after_pass)
+{
+  const int tid = threadIdx.x, dp = a.e.dp;
+  const int nr = max(0, (a.e.n - sh.rank + sh.size - 1) / sh.size);
+  TrackShared t;
+  t.list = reinterpret_cast<int *>(smem);
+  t.have = reinterpret_cast<unsigned *>(t.list + (size_t)a.rows * dp);
+  t.full = t.have + ((size_t)a.rows << a.word_log2);
+  t.last = t.full + ((size_t)a.rows << a.word_log2);
+  t.near = t.last + ((size_t)a.rows << a.word_log2);
+  t.round = reinterpret_cast<TrackRound *>(t.near + SWEEP_THREADS * dp);
+  if(!pull_adjacency(a, sh, sy)) return false;
+  expand_rows(a, sy, t.list, sh.rank, sh.size, nr, nullptr);
+  if(tid < 32){
+    group_state(a, sh.ph[0], 0, 0);
+    if(tid == 0) sh.ph[0].t_loaded = sh.begin;
+  }
+  bool passed = false;
+  for(;;){
+    __syncthreads();
+    if(tid < 32) plan_track(a, sh, sy);
+    __syncthreads();
+    const int todo = sh.todo, level = sh.ph[0].level, c0 = group_chunk(a, sh.ph[0].group, 0);
+    if(todo == TODO_ABORT){
+      if(tid == 0) *a.abort_flag = GBX_ERR_TIMEOUT;
+      return false;
+    }
+    if(todo == TODO_DONE) break;
+    if(level > 0 && !passed){
+      passed = true;
+      after_pass();
+    }
+    const int src0 = c0 * (64 << a.wc_log2), nsrc = min(a.slots * (64 << a.wc_log2), a.B - src0);
+    if(level == 0) track_start(a, sh, t, src0, nsrc, nr);
+    else track_level<NB>(a, sh, t, level, nsrc, nr);
+    __syncthreads();
+    if(tid == 0) t.round->next = 0;
+    if(tid < 32) arrive_step(a, sh, sy, 0);
+  }
+  __syncthreads();
+  return true;
+}
+
 /* Two CTAs per SM and six neighbours in flight: 256 x 256, d = 6 took 5.26 ms
  * (6.0 with three CTAs, 5.9 with four and four neighbours in flight; both
  * spilled). */
@@ -805,34 +936,94 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) sweep_track_kernel(const gbx
 {
   extern __shared__ __align__(16) unsigned char sweep_smem[];
   __shared__ SweepShared sh;
-  const int tid = threadIdx.x, dp = a.e.dp;
-  const int nr = (a.e.n - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  TrackShared t;
-  t.list = reinterpret_cast<int *>(sweep_smem);
-  t.have = reinterpret_cast<unsigned *>(t.list + (size_t)a.rows * dp);
-  t.full = t.have + ((size_t)a.rows << a.word_log2);
-  t.last = t.full + ((size_t)a.rows << a.word_log2);
-  t.near = t.last + ((size_t)a.rows << a.word_log2) + (tid >> 5) * 32 * dp;
-  t.warp = reinterpret_cast<TrackWarp *>(t.last + ((size_t)a.rows << a.word_log2) + SWEEP_WARPS * 32 * dp);
-  SweepSync &sy = sweep_begin(a, sh);
-  if(!pull_adjacency(a, sh, sy)) return;
-  expand_rows(a, sy, t.list, (int)blockIdx.x, (int)gridDim.x, nr, nullptr);
-  if(tid < 32) group_state(a, sh.ph[0], 0, 0);
-  for(;;){
-    __syncthreads();
-    if(tid < 32) plan_track(a, sh, sy);
-    __syncthreads();
-    const int todo = sh.todo, level = sh.ph[0].level, c0 = group_chunk(a, sh.ph[0].group, 0);
-    if(todo == TODO_DONE) return;
-    if(todo == TODO_ABORT){
-      if(tid == 0) *a.abort_flag = GBX_ERR_TIMEOUT;
-      return;
+  SweepSync &sy = launch_sync(a);
+  sweep_begin(sh, (int)blockIdx.x, (int)gridDim.x);
+  track_graph<NB>(a, sh, sy, sweep_smem, [] {});
+}
+
+/* ---------------------------------------------------------------------- */
+/* Many graphs.                                                            */
+/* ---------------------------------------------------------------------- */
+
+/* Many graphs of uneven size by teams of CTAs.  A graph's team is a 2^k-th of
+ * the grid: the large graphs are taken first by the large teams, and a team
+ * that finds its size's queue empty splits in two, so that the small graphs
+ * fill in behind.  Within a team a graph runs as in the kernels above, with
+ * its barriers in the team's own words.  Against one grid-wide queue of tiles
+ * there is no hand-off per tile, the neighbour lists stay in shared memory
+ * over the levels, and one team's copy of its adjacency from host memory runs
+ * while others compute. */
+typedef SyncT<1, SWEEP_SLOTS> TeamSync;
+
+struct TeamNode {
+  TeamSync sync[2];                    /* by graph, alternating */
+  unsigned long long box[2][16];       /* graph `seq` of the team: (seq + 1) << 32 | graph + 1, or 0: none left */
+};
+
+__global__ void __launch_bounds__(SWEEP_THREADS, 2) team_kernel(const gbx_team t)
+{
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  __shared__ SweepShared sh;
+  __shared__ gbx_sweep a;
+  __shared__ int sh_graph;
+  const int tid = threadIdx.x, G = (int)gridDim.x, b = (int)blockIdx.x;
+  for(int k = t.first_split; k <= t.last_split; k++){
+    const int queued = t.queue[k + 1] - t.queue[k];
+    if(queued <= 0) continue;
+    /* team i of 2^k: CTAs [i * G >> k, (i + 1) * G >> k) */
+    const int i = (int)((((long long)(b + 1) << k) - 1) / G);
+    const int lo = (int)(((long long)i * G) >> k), hi = (int)(((long long)(i + 1) * G) >> k);
+    TeamNode &node = reinterpret_cast<TeamNode *>(t.nodes)[(1 << k) - (1 << t.first_split) + i];
+    /* CTA `lo` takes the next graph off the queue and posts it */
+    auto post = [&](int seq) {
+      const unsigned at = atomicAdd(t.next + k, 1u);
+      const unsigned g = at < (unsigned)queued ? (unsigned)t.order[t.queue[k] + (int)at] + 1u : 0u;
+      __threadfence();
+      atomicExch(&node.box[seq & 1][0], (unsigned long long)(seq + 1) << 32 | g);
+    };
+    if(b == lo && tid == 0) post(0);
+    for(int seq = 0;; seq++){
+      if(tid == 0){
+        unsigned long long seen = 0;
+        const bool ok = wait_for(&node.box[seq & 1][0], (unsigned long long)(seq + 1) << 32, seen, t.limit_ns);
+        if(!ok) *t.abort_flag = GBX_ERR_TIMEOUT;
+        sh_graph = ok ? (int)(unsigned)seen - 1 : -2;
+      }
+      __syncthreads();
+      const int g = sh_graph;
+      __syncthreads();                                   /* read before it is written again */
+      if(g == -2) return;
+      if(g < 0) break;
+      {
+        const unsigned *src = reinterpret_cast<const unsigned *>(t.graphs + g);
+        unsigned *dst = reinterpret_cast<unsigned *>(&a);
+        for(int x = tid; x < (int)(sizeof(gbx_sweep) / 4); x += SWEEP_THREADS) dst[x] = __ldg(src + x);
+      }
+      __syncthreads();
+      if(tid == 0){
+        a.limit_ns = t.limit_ns;
+        if(t.adj) a.e.adj = reinterpret_cast<const int *>(__ldcg(t.adj + g));
+        unsigned char *at = t.arena + (size_t)i * (t.arena_bytes >> k);   /* inside the parent's part: the size divides evenly */
+        a.buf = reinterpret_cast<unsigned long long *>(at);
+        a.start = a.buf + (a.two_level ? 0 : a.slot_words);
+        a.start_stride = 2 * a.slot_words;
+        a.changed = reinterpret_cast<unsigned *>(at + 16 * a.slot_words);
+        a.rows = (a.e.n + (hi - lo) - 1) / (hi - lo);
+      }
+      sweep_begin(sh, b - lo, hi - lo);
+      TeamSync &sy = node.sync[seq & 1];
+      auto clear = [&] {
+        /* every CTA has begun this graph, so the last one's counters and box are free */
+        if(b != lo) return;
+        unsigned *other = reinterpret_cast<unsigned *>(&node.sync[(seq + 1) & 1]);
+        for(int x = tid; x < (int)(sizeof(TeamSync) / 4); x += SWEEP_THREADS) other[x] = 0;
+      };
+      const bool ok = a.track ? track_graph<6>(a, sh, sy, sweep_smem, clear)
+                              : dense_graph<8>(a, sh, sy, sweep_smem, clear);
+      if(!ok) return;
+      /* taken only now: a graph taken ahead would wait for this one, however long, while another team is free */
+      if(b == lo && tid == 0) post(seq + 1);
     }
-    const int src0 = c0 * (64 << a.wc_log2), nsrc = min(a.slots * (64 << a.wc_log2), a.B - src0);
-    if(level == 0) track_start(a, t, src0, nsrc, nr);
-    else track_level<NB>(a, sh, t, level, nsrc, nr);
-    __syncthreads();
-    if(tid < 32) arrive_step(a, sh, sy, 0);
   }
 }
 
@@ -846,7 +1037,7 @@ size_t gbx_sweep_smem(const gbx_sweep *a)
 {
   const size_t rows = (size_t)a->rows, lists = rows * (size_t)a->e.dp * 4;
   if(a->track)
-    return lists + 3 * (rows << a->word_log2) * 4 + SWEEP_WARPS * (32 * (size_t)a->e.dp * 4 + sizeof(TrackWarp));
+    return lists + 3 * (rows << a->word_log2) * 4 + SWEEP_THREADS * (size_t)a->e.dp * 4 + sizeof(TrackRound);
   return lists + SWEEP_WARPS * (size_t)a->scratch_bits / 8 + 8 * (size_t)a->nchunks +
          (((size_t)a->phases * a->slots * rows) << (a->wc_log2 - 2));
 }
@@ -870,7 +1061,7 @@ int gbx_sweep_blocks(const gbx_sweep *a, int *per_sm)
   return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, sweep_entry(a), SWEEP_THREADS, smem);
 }
 
-int gbx_sweep_launch(const gbx_sweep *a, int blocks, void *stream)
+static int launch_all(const void *entry, void *arg, int blocks, size_t smem, cudaStream_t stream)
 {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -878,13 +1069,36 @@ int gbx_sweep_launch(const gbx_sweep *a, int blocks, void *stream)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks, 1, 1);
   cfg.blockDim = dim3(SWEEP_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = gbx_sweep_smem(a);
-  cfg.stream = (cudaStream_t)stream;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  void *args[1] = { arg };
+  return (int)cudaLaunchKernelExC(&cfg, entry, args);
+}
+
+int gbx_sweep_launch(const gbx_sweep *a, int blocks, void *stream)
+{
   gbx_sweep arg = *a;
-  void *args[1] = { &arg };
-  return (int)cudaLaunchKernelExC(&cfg, sweep_entry(a), args);
+  return launch_all(sweep_entry(a), &arg, blocks, gbx_sweep_smem(a), (cudaStream_t)stream);
+}
+
+size_t gbx_team_node_bytes(void) { return sizeof(TeamNode); }
+
+int gbx_team_blocks(size_t smem, int *per_sm)
+{
+  *per_sm = 0;
+  if(smem > GBX_SWEEP_SMEM_MAX) return (int)cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute((const void *)team_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       GBX_SWEEP_SMEM_MAX);
+  if(e != cudaSuccess) return (int)e;
+  return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, (const void *)team_kernel, SWEEP_THREADS, smem);
+}
+
+int gbx_team_launch(const gbx_team *t, int blocks, size_t smem, void *stream)
+{
+  gbx_team arg = *t;
+  return launch_all((const void *)team_kernel, &arg, blocks, smem, (cudaStream_t)stream);
 }
 
 }  /* extern "C" */

@@ -89,3 +89,47 @@ def test_bad_adjacency_and_wait_limit():
     for _ in range(3):
         assert same(b.run([adj])[0], want)
     b.close()
+
+
+def random_spec(rng, n_hi):
+    kind = rng.integers(0, 5)
+    if kind == 0:
+        w, h = int(rng.integers(2, 31)), int(rng.integers(2, 31))
+        s = int(rng.choice([1, 2])) if w % 2 == 0 else 1
+        d = int(rng.integers(1, 40))
+        base = w * h // s
+        cells = np.arange(base)
+        step = rng.integers(-3, 4, (base, d))
+        adj = np.clip(cells[:, None] + step, 0, w * h - 1).astype(np.int32)
+        return og.GraphSpec(adj, grid=True, width=w, height=h, symmetries=s)
+    s = int(rng.choice([1, 1, 2, 3, 7]))
+    base = int(np.exp(rng.uniform(0, np.log(n_hi // s)))) + (1 if kind == 1 else 0)
+    n, d = base * s, int(rng.integers(1, 13) if kind else rng.integers(60, 90))
+    adj = np.stack([rng.permutation(base) + base * rng.integers(0, s, base) for _ in range(d)], axis=1).astype(np.int32)
+    nd = rng.integers(0, d + 1, base).astype(np.int32) if kind == 2 else None
+    return og.GraphSpec(adj, nodes=n, symmetries=s, num_degrees=nd)
+
+
+@pytest.mark.parametrize("count,n_hi", [(2, 3000), (3, 40), (17, 6000), (60, 2000), (400, 300)])
+def test_batches(count, n_hi):
+    """Teams of every size: uneven graphs, two calls with other arrays, an
+    out-of-range entry and a wait that runs out in between."""
+    rng = np.random.default_rng(count)
+    specs = [random_spec(rng, n_hi) for _ in range(count)]
+    want = [oracle.aspl(g.adjacency, nodes=0 if g.grid else g.nodes, num_degrees=g.num_degrees,
+                        symmetries=g.symmetries, grid=g.grid, width=g.width, height=g.height) for g in specs]
+    b = og.Batch(specs)
+    b.set_wait_limit(5 * 10 ** 9)
+    for got in (b.run(), b.run()):
+        for k, (x, y) in enumerate(zip(got, want)):
+            assert same(x, y), (k, specs[k].grid, specs[k].nodes, specs[k].adjacency.shape, x, y)
+    k = int(np.argmax([g.adjacency.size if g.num_degrees is None else 0 for g in specs]))
+    bad = [g.adjacency for g in specs]
+    bad[k] = bad[k].copy()
+    bad[k][-1, -1] = specs[k].nodes
+    with pytest.raises(og.ODPError) as e:
+        b.run(bad)
+    assert e.value.code == og.ERR_ADJACENCY
+    turned = [np.ascontiguousarray(g.adjacency[:, ::-1]) if g.num_degrees is None else g.adjacency for g in specs]
+    assert all(same(x, y) for x, y in zip(b.run(turned), want))
+    b.close()
