@@ -24,7 +24,7 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc") if os.path.exists(os.path.join(CUDA_HOME, "bin", "nvcc")) else "nvcc"
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
-CU_SOURCES = ["aspl_engine.cu", "sweep.cu", "anneal.cu"]
+CU_SOURCES = ["aspl_engine.cu", "sweep.cu", "anneal.cu", "anneal_resident.cu"]
 C_SOURCES = ["odp_graph.c", "odp_io.c", "odp_plan.c", "odp_aspl.c", "odp_batch.c", "odp_serve.c", "odp_anneal.c"]
 
 SO_PATH = os.path.join(HERE, "libodp_gb300.so")

@@ -1,7 +1,7 @@
 /*
  * odp_device.cuh -- device helpers shared by the kernels: bit counting, the
- * timer, and the rules that turn the compact adjacency into row-space
- * neighbour entries.
+ * timer, the rules that turn the compact adjacency into row-space neighbour
+ * entries, and the lanes of the lockstep kernels.
  */
 #ifndef ODP_DEVICE_CUH
 #define ODP_DEVICE_CUH
@@ -97,6 +97,132 @@ __device__ __forceinline__ int expand_value(const gbx_expand_desc &e, int a, int
   int nb = a + back;
   if(nb >= e.n) nb -= e.n;
   return e.itable ? e.itable[nb] : nb;
+}
+
+
+/* ---------------------------------------------------------------------- */
+/* Lanes: 32 bytes (256 source bits, one sector) of a row, the unit of the  */
+/* lockstep kernels, moved by 256-bit accesses (L2 only: other SMs rewrite  */
+/* the buffers between levels).                                             */
+/* ---------------------------------------------------------------------- */
+
+#define LANE_FULL 1u                  /* every source bit of the lane is set */
+#define LANE_CHANGED 2u               /* the older buffer does not hold the lane's words yet */
+
+#define ARRIVE_ONE (1ull << 48)       /* barrier words: CTAs done << 48 | bits counted */
+#define ARRIVE_BITS (ARRIVE_ONE - 1)
+
+__device__ __forceinline__ void ld_lane(unsigned (&r)[8], const void *p)
+{
+  asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "l"(p) : "memory");
+}
+
+__device__ __forceinline__ void st_lane(void *p, const unsigned (&r)[8])
+{
+  asm volatile("st.global.cg.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+               :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "l"(p)
+               : "memory");
+}
+
+/* Set bits of eight words: full adders (one three-input operation for each
+ * sum and carry) reduce them to four words of weights 1, 1, 2 and 4, as the
+ * bit count runs at a quarter of the logic's rate. */
+__device__ __forceinline__ unsigned popc_lane(const unsigned (&r)[8])
+{
+  const unsigned s1 = r[0] ^ r[1] ^ r[2], c1 = (r[0] & r[1]) | (r[2] & (r[0] | r[1]));
+  const unsigned s2 = r[3] ^ r[4] ^ r[5], c2 = (r[3] & r[4]) | (r[5] & (r[3] | r[4]));
+  const unsigned s3 = s1 ^ s2 ^ r[6], c3 = (s1 & s2) | (r[6] & (s1 | s2));
+  const unsigned t1 = c1 ^ c2 ^ c3, f1 = (c1 & c2) | (c3 & (c1 | c2));
+  return __popc(s3) + __popc(r[7]) + 2 * __popc(t1) + 4 * __popc(f1);
+}
+
+__device__ __forceinline__ unsigned and_lane(const unsigned (&r)[8])
+{
+  return r[0] & r[1] & r[2] & r[3] & r[4] & r[5] & r[6] & r[7];
+}
+
+/* Barrier words.  A CTA arrives with arrive_word (one thread, after a CTA
+ * barrier: its release covers the CTA's stores) and one thread of it waits
+ * with wait_for until `*word` reaches `target`; false past the limit. */
+__device__ __forceinline__ void arrive_word(unsigned long long *word, unsigned long long v)
+{
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" :: "l"(word), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ void arrive_word(unsigned *word, unsigned v)
+{
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" :: "l"(word), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ unsigned long long acquire_word(const unsigned long long *p)
+{
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ unsigned acquire_word(const unsigned *p)
+{
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+template <typename T>
+__device__ __forceinline__ bool wait_for(const T *word, T target, T &seen, unsigned long long limit_ns)
+{
+  seen = acquire_word(word);
+  if(seen < target){
+    const unsigned long long t0 = globaltimer();
+    do{
+      if(globaltimer() - t0 > limit_ns) return false;
+      seen = acquire_word(word);
+    } while(seen < target);
+  }
+  return true;
+}
+
+__device__ __forceinline__ int lane_bits(int nsrc, int gl) { return min(max(nsrc - 256 * gl, 0), 256); }
+
+__device__ __forceinline__ void mark(unsigned *s, int o, int n)
+{
+  if((unsigned)o < (unsigned)n) atomicOr(s + (o >> 5), 1u << (o & 31));
+}
+
+/* A lane's words OR its neighbours', NB of them in flight. */
+template <int NB>
+__device__ __forceinline__ void gather_lane(unsigned (&acc)[8], const char *X, const int *ids, int d, unsigned rb)
+{
+  int j = 0;
+  for(; j + NB <= d; j += NB){
+    unsigned t[NB][8];
+#pragma unroll
+    for(int i = 0; i < NB; i += 4){
+      const int4 u = *reinterpret_cast<const int4 *>(ids + j + i);
+      ld_lane(t[i], X + (size_t)(unsigned)u.x * rb);
+      ld_lane(t[i + 1], X + (size_t)(unsigned)u.y * rb);
+      ld_lane(t[i + 2], X + (size_t)(unsigned)u.z * rb);
+      ld_lane(t[i + 3], X + (size_t)(unsigned)u.w * rb);
+    }
+#pragma unroll
+    for(int i = 0; i < NB; i += 2)
+#pragma unroll
+      for(int k = 0; k < 8; k++) acc[k] |= t[i][k] | t[i + 1][k];
+    if(and_lane(acc) == ~0u) return;
+  }
+  for(; j < d; j += 4){
+    const int4 u = *reinterpret_cast<const int4 *>(ids + j);
+    unsigned t0[8], t1[8] = {0, 0, 0, 0, 0, 0, 0, 0}, t2[8] = {0, 0, 0, 0, 0, 0, 0, 0},
+             t3[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    ld_lane(t0, X + (size_t)(unsigned)u.x * rb);
+    if(j + 1 < d) ld_lane(t1, X + (size_t)(unsigned)u.y * rb);
+    if(j + 2 < d) ld_lane(t2, X + (size_t)(unsigned)u.z * rb);
+    if(NB > 4 && j + 3 < d) ld_lane(t3, X + (size_t)(unsigned)u.w * rb);
+#pragma unroll
+    for(int k = 0; k < 8; k++) acc[k] |= (t0[k] | t1[k]) | (t2[k] | t3[k]);
+  }
 }
 
 }  // namespace

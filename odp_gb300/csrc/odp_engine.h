@@ -301,6 +301,24 @@ int  gbx_anneal_propose(gbx_chain *d_chains, int count, void *stream);
 int  gbx_anneal_decide(gbx_chain *d_chains, int count, const gbx_graph_acc *d_acc, const gbx_ctrl *d_ctrl,
                        const unsigned int *d_err, void *stream);
 
+/* Many steps of every running chain in one cooperative launch
+ * (anneal_resident.cu), for chains whose compact adjacency fits a CTA's shared
+ * memory as 16-bit vertices.  Chain k belongs to team k % teams; the teams
+ * share the grid evenly. */
+typedef struct {
+  gbx_chain *chains;
+  char *buf;                   /* bitsets: chain k's two buffers at buf + buf_offset[k] */
+  const unsigned long long *buf_offset;
+  void *sync;                  /* gbx_resident_sync_bytes() per team, zeroed before the launch */
+  unsigned long long limit_ns; /* longest wait of a CTA for its team */
+  int count, teams, steps;
+} gbx_resident;
+size_t gbx_resident_sync_bytes(void);
+/* Shared memory of a CTA that holds `rows` rows of a chain. */
+size_t gbx_resident_smem(int rows, int dp, int base, int d);
+int  gbx_resident_blocks(size_t smem, int *per_sm);
+int  gbx_resident_launch(const gbx_resident *r, int blocks, size_t smem, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -32,10 +32,16 @@
 #define MUT_FN static inline
 #endif
 
+/* The stored adjacency's element type: int, or a narrower unsigned one where
+ * every vertex fits (entries past a row's degree are never read). */
+#ifndef MUT_VERTEX
+#define MUT_VERTEX int
+#endif
+
 typedef struct {
   int n, d, s, base;          /* base = n / s rows stored */
   const int *ndeg;            /* per base row degree, or NULL (regular) */
-  int *adj;                   /* int[base][d] */
+  MUT_VERTEX *adj;            /* [base][d] */
   int nw;                     /* the last successful swap's writes: */
   int wrow[4], wslot[4];      /*   adj[wrow][wslot] was set (base rows) */
 } mut_general;
@@ -47,17 +53,22 @@ MUT_FN int mut_wrap(int x, int n)                 /* NORM, utils.c:171-177 */
   return x;
 }
 
+/* Base row of v and the rotation that brings it there (a multiple of base);
+ * no division without symmetry. */
+MUT_FN int mut_row(const mut_general *g, int v) { return g->s == 1 ? v : v % g->base; }
+MUT_FN int mut_turn(const mut_general *g, int v) { return g->s == 1 ? 0 : (v / g->base) * g->base; }
+
 /* adjacency[v][j] of the expanded graph (GLOBAL_ADJ_GENERAL, utils.c:180-186) */
 MUT_FN int mut_nbr(const mut_general *g, int v, int j)
 {
-  return mut_wrap(g->adj[(long long)(v % g->base) * g->d + j] + (v / g->base) * g->base, g->n);
+  return mut_wrap(g->adj[(long long)mut_row(g, v) * g->d + j] + mut_turn(g, v), g->n);
 }
 
 /* value to store in the row of `pos` so that it names global vertex v
  * (LOCAL_INDEX_GENERAL, utils.c:266-270) */
 MUT_FN int mut_rel(const mut_general *g, int v, int pos)
 {
-  return mut_wrap(v - (pos / g->base) * g->base, g->n);
+  return mut_wrap(v - mut_turn(g, pos), g->n);
 }
 
 MUT_FN int mut_antipodal(const mut_general *g, int u, int v)   /* IS_DIAMETER_GENERAL, utils.c:96-102 */
@@ -68,7 +79,7 @@ MUT_FN int mut_antipodal(const mut_general *g, int u, int v)   /* IS_DIAMETER_GE
 
 MUT_FN int mut_deg(const mut_general *g, int v)
 {
-  return g->ndeg ? g->ndeg[v % g->base] : g->d;
+  return g->ndeg ? g->ndeg[mut_row(g, v)] : g->d;
 }
 
 /* The slot of v's row that points back at u (get_degree_index_general,
@@ -84,9 +95,10 @@ MUT_FN int mut_back_slot(const mut_general *g, int u, int v, int u_slot)
     return u_slot;
   }
   else{
-    int dd = mut_deg(g, v);
+    const int dd = mut_deg(g, v), turn = mut_turn(g, v);
+    const MUT_VERTEX *row = g->adj + (long long)mut_row(g, v) * g->d;
     for(int i = 0; i < dd; i++)
-      if(mut_nbr(g, v, i) == u) return i;
+      if(mut_wrap(row[i] + turn, g->n) == u) return i;
   }
   return -1;
 }
@@ -99,15 +111,15 @@ MUT_FN int mut_same_orbit(const mut_general *g, int u0, int v0, int u1, int v1)
   int d0 = (u0 > v0) ? v0 - u0 + n : v0 - u0;
   int d1 = (u1 > v1) ? v1 - u1 + n : v1 - u1;
   int d2 = (u1 < v1) ? u1 - v1 + n : u1 - v1;
-  if(d0 == d1 && u0 % g->base == u1 % g->base) return 1;
-  if(d0 == d2 && u0 % g->base == v1 % g->base) return 1;
+  if(d0 == d1 && mut_row(g, u0) == mut_row(g, u1)) return 1;
+  if(d0 == d2 && mut_row(g, u0) == mut_row(g, v1)) return 1;
   return 0;
 }
 
 MUT_FN void mut_put(mut_general *g, int v, int slot, int value)
 {
-  int row = v % g->base;
-  g->adj[(long long)row * g->d + slot] = value;
+  int row = mut_row(g, v);
+  g->adj[(long long)row * g->d + slot] = (MUT_VERTEX)value;
   if(g->nw < 4){ g->wrow[g->nw] = row; g->wslot[g->nw] = slot; g->nw++; }
 }
 
@@ -266,7 +278,7 @@ typedef struct {              /* a (possibly rotation-symmetric) grid graph */
   int w, h, d, s, len, n;
   int bw, bh;                 /* base block: x < bw, y < bh */
   const int *ndeg;            /* per local row degree, or NULL */
-  int *adj;                   /* int[n/s][d], rows in local-index order */
+  MUT_VERTEX *adj;            /* [n/s][d], rows in local-index order */
   const int *xy;              /* optional (x, y) per vertex: saves divisions */
   int nw;                     /* the last successful swap's writes: */
   int wrow[4], wslot[4];      /*   adj[wrow][wslot] was set (local rows) */
@@ -344,7 +356,7 @@ MUT_FN void grid_put(mut_grid *g, int v, int slot, int u)
     else if(y >= g->bh){ row = grid_row(g, grid_rot(g, v, 180)); val = grid_rot(g, u, 180); }
     else{ row = grid_row(g, grid_rot(g, v, 90)); val = grid_rot(g, u, 90); }
   }
-  g->adj[(long long)row * d + slot] = val;
+  g->adj[(long long)row * d + slot] = (MUT_VERTEX)val;
   grid_record(g, row, slot);
 }
 

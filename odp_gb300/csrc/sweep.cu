@@ -37,12 +37,6 @@
 #define SWEEP_WARPS (SWEEP_THREADS / 32)
 #define SWEEP_SLOTS GBX_SWEEP_SLOTS   /* column chunks a phase runs at once, at most */
 
-#define LANE_FULL 1u                  /* every source bit of the lane is set */
-#define LANE_CHANGED 2u               /* the older buffer does not hold the lane's words yet */
-
-#define ARRIVE_ONE (1ull << 48)       /* barrier words: CTAs done << 48 | bits counted */
-#define ARRIVE_BITS (ARRIVE_ONE - 1)
-
 namespace {
 
 /* Counters of one graph's evaluation by PH phases over at most CH chunks;
@@ -81,61 +75,13 @@ struct SweepShared {
 #define TODO_LEVEL 1
 #define TODO_ABORT 2
 
-__device__ __forceinline__ void ld_lane(unsigned (&r)[8], const void *p)
-{
-  asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "l"(p) : "memory");
-}
-
-__device__ __forceinline__ void st_lane(void *p, const unsigned (&r)[8])
-{
-  asm volatile("st.global.cg.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
-               :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "l"(p)
-               : "memory");
-}
-
-/* Set bits of eight words: full adders (one three-input operation for each
- * sum and carry) reduce them to four words of weights 1, 1, 2 and 4, as the
- * bit count runs at a quarter of the logic's rate. */
-__device__ __forceinline__ unsigned popc_lane(const unsigned (&r)[8])
-{
-  const unsigned s1 = r[0] ^ r[1] ^ r[2], c1 = (r[0] & r[1]) | (r[2] & (r[0] | r[1]));
-  const unsigned s2 = r[3] ^ r[4] ^ r[5], c2 = (r[3] & r[4]) | (r[5] & (r[3] | r[4]));
-  const unsigned s3 = s1 ^ s2 ^ r[6], c3 = (s1 & s2) | (r[6] & (s1 | s2));
-  const unsigned t1 = c1 ^ c2 ^ c3, f1 = (c1 & c2) | (c3 & (c1 | c2));
-  return __popc(s3) + __popc(r[7]) + 2 * __popc(t1) + 4 * __popc(f1);
-}
-
-__device__ __forceinline__ unsigned and_lane(const unsigned (&r)[8])
-{
-  return r[0] & r[1] & r[2] & r[3] & r[4] & r[5] & r[6] & r[7];
-}
-
-/* One thread waits until `*word` reaches `target`; false past the limit. */
-template <typename T>
-__device__ __forceinline__ bool wait_for(const T *word, T target, T &seen, unsigned long long limit_ns)
-{
-  seen = vload(word);
-  if(seen < target){
-    const unsigned long long t0 = globaltimer();
-    do{
-      if(globaltimer() - t0 > limit_ns) return false;
-      seen = vload(word);
-    } while(seen < target);
-  }
-  __threadfence();
-  return true;
-}
-
 /* The whole grid passes; false (in every thread) past the limit. */
 __device__ __forceinline__ bool grid_pass(unsigned *word, SweepShared &sh, const gbx_sweep &a)
 {
   __syncthreads();
   if(threadIdx.x == 0){
     unsigned seen;
-    __threadfence();
-    atomicAdd(word, 1u);
+    arrive_word(word, 1u);
     const bool ok = wait_for(word, (unsigned)sh.size, seen, a.limit_ns);
     sh.todo = ok ? TODO_LEVEL : TODO_ABORT;
     if(!ok) *a.abort_flag = GBX_ERR_TIMEOUT;           /* pinned host memory */
@@ -145,8 +91,6 @@ __device__ __forceinline__ bool grid_pass(unsigned *word, SweepShared &sh, const
   __syncthreads();                                     /* read before it is written again */
   return ok;
 }
-
-__device__ __forceinline__ int lane_bits(int nsrc, int gl) { return min(max(nsrc - 256 * gl, 0), 256); }
 
 /* Sources of chunk c. */
 __device__ __forceinline__ int chunk_sources(const gbx_sweep &a, int c)
@@ -244,8 +188,7 @@ __device__ __forceinline__ void arrive_step(const gbx_sweep &a, SweepShared &sh,
   const unsigned total = __reduce_add_sync(0xffffffffu, c);   /* rows x lanes x 256 of one CTA: below 2^32 */
   if(q == 0){
     if(sh.rank == 0) sy.arrive[ph][(step + 1) % 3][0] = 0;
-    __threadfence();
-    atomicAdd(&sy.arrive[ph][step % 3][0], ARRIVE_ONE | total);
+    arrive_word(&sy.arrive[ph][step % 3][0], ARRIVE_ONE | total);
     sh.ph[ph].step = step + 1;
   }
   __syncwarp();
@@ -381,11 +324,6 @@ __device__ __forceinline__ void expand_rows(const gbx_sweep &a, Sync &sy, int *l
 /* General graphs.                                                         */
 /* ---------------------------------------------------------------------- */
 
-__device__ __forceinline__ void mark(unsigned *s, int o, int n)
-{
-  if((unsigned)o < (unsigned)n) atomicOr(s + (o >> 5), 1u << (o & 31));
-}
-
 /* Levels 1 and 2 of every chunk (of one group's chunks when the lists are too
  * wide for level 2: then level 1 alone), a warp per row.  The warp marks the
  * row, its neighbours and their neighbours in its scratch row (scratch_bits
@@ -458,40 +396,6 @@ __device__ void start_rows(const gbx_sweep &a, const int *list, unsigned *scratc
       }
       __syncwarp();                                      /* the scratch row is read before it is cleared again */
     }
-  }
-}
-
-/* A lane's words OR its neighbours', NB of them in flight. */
-template <int NB>
-__device__ __forceinline__ void gather_lane(unsigned (&acc)[8], const char *X, const int *ids, int d, unsigned rb)
-{
-  int j = 0;
-  for(; j + NB <= d; j += NB){
-    unsigned t[NB][8];
-#pragma unroll
-    for(int i = 0; i < NB; i += 4){
-      const int4 u = *reinterpret_cast<const int4 *>(ids + j + i);
-      ld_lane(t[i], X + (size_t)(unsigned)u.x * rb);
-      ld_lane(t[i + 1], X + (size_t)(unsigned)u.y * rb);
-      ld_lane(t[i + 2], X + (size_t)(unsigned)u.z * rb);
-      ld_lane(t[i + 3], X + (size_t)(unsigned)u.w * rb);
-    }
-#pragma unroll
-    for(int i = 0; i < NB; i += 2)
-#pragma unroll
-      for(int k = 0; k < 8; k++) acc[k] |= t[i][k] | t[i + 1][k];
-    if(and_lane(acc) == ~0u) return;
-  }
-  for(; j < d; j += 4){
-    const int4 u = *reinterpret_cast<const int4 *>(ids + j);
-    unsigned t0[8], t1[8] = {0, 0, 0, 0, 0, 0, 0, 0}, t2[8] = {0, 0, 0, 0, 0, 0, 0, 0},
-             t3[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    ld_lane(t0, X + (size_t)(unsigned)u.x * rb);
-    if(j + 1 < d) ld_lane(t1, X + (size_t)(unsigned)u.y * rb);
-    if(j + 2 < d) ld_lane(t2, X + (size_t)(unsigned)u.z * rb);
-    if(NB > 4 && j + 3 < d) ld_lane(t3, X + (size_t)(unsigned)u.w * rb);
-#pragma unroll
-    for(int k = 0; k < 8; k++) acc[k] |= (t0[k] | t1[k]) | (t2[k] | t3[k]);
   }
 }
 
