@@ -69,22 +69,25 @@ int  ODPX_Batch_time_mode(ODPX_Batch *batch, const int *const *adjacency, int re
 unsigned long long ODPX_Batch_tiles(const ODPX_Batch *batch);
 /* Introspection for benchmarks: jobs, slots, chunk width (log2 words) of graph i. */
 int  ODPX_Batch_info(const ODPX_Batch *batch, int graph, int *njobs, int *nslots, int *wc_log2, int *tile_rows);
-/* Which kernel evaluates the plan: 1 when every graph has at most
+/* Kind of the plan: 1 (small) when every graph has at most
  * ODP_GB300_SMALL_N (default 8192) vertices, both bitset buffers of a column
  * chunk of at least 128 sources fit in one CTA's shared memory beside its
- * share of the row table, and the plan's CTAs fit on the SMs in one wave, so
- * each job runs in the small-graph kernel, on the CTAs
- * of one thread-block cluster; 0 otherwise: larger single graphs run on every
- * SM in lockstep (ODP_GB300_SWEEP=0 turns that off), batches and plans with
- * explicit schedule settings or change tracking in the persistent engine.
- * Results are the same either way. */
+ * share of the row table, and the plan's CTAs fit on the SMs in one wave; 0
+ * otherwise.  A small plan runs in the small-graph kernel, each job on the
+ * CTAs of one thread-block cluster, except that a single graph runs in
+ * lockstep on every SM, as larger single graphs do, where that is faster and
+ * ODP_GB300_SMALL_CLUSTER and _PART do not ask for the cluster
+ * (ODP_GB300_SWEEP=0 turns lockstep off).  Batches run on teams of CTAs in
+ * lockstep; plans with explicit schedule settings or change tracking, or with
+ * graphs too large for a team, in the persistent engine.  Results are the
+ * same either way. */
 int  ODPX_Batch_kernel(const ODPX_Batch *batch);
-/* For a plan on the small-graph kernel: the CTAs of the thread-block cluster
+/* For a small plan: its shape on the small-graph kernel, the CTAs of the thread-block cluster
  * that runs each job (1, 2, 4 or 8; each CTA computes its share of the
  * rows), the threads per CTA, and whether the bitsets are partitioned over
  * the cluster (1: each CTA holds its own rows and reads the others' from
  * their shared memory; 0: each CTA holds the whole level).  Returns 0, or
- * ODPX_ERR_INVALID for a plan on the persistent engine.
+ * ODPX_ERR_INVALID for a plan of the other kind.
  * ODP_GB300_SMALL_CLUSTER forces the cluster size of plans created
  * afterwards (halved until the shape fits), ODP_GB300_SMALL_PART=0 or 1 the
  * layout. */

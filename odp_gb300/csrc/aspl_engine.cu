@@ -762,6 +762,11 @@ engine_kernel(const gbx_job *__restrict__ jobs, int njobs, gbx_slot *slots, int 
 #define SMALL_LOADS 8            /* host loads in flight per thread while the table is built */
 #define SMALL_CLUSTER_MAX GBX_SMALL_CLUSTER_MAX   /* CTAs sharing one job (portable cluster size) */
 
+__device__ __forceinline__ bool differ(const uint4 &a, const uint4 &b)
+{
+  return ((a.x ^ b.x) | (a.y ^ b.y) | (a.z ^ b.z) | (a.w ^ b.w)) != 0u;
+}
+
 struct SmallOutcome {
   long long sum;
   int level;
@@ -771,7 +776,8 @@ struct SmallOutcome {
 /* Per-CTA bookkeeping of the small kernel (static shared memory). */
 struct SmallShared {
   gbx_expand_desc desc;
-  unsigned long long total[3];                       /* bits of level k in total[k % 3], from every CTA */
+  unsigned total[3][SMALL_CLUSTER_MAX];              /* bits of level k in total[k % 3], by CTA */
+  unsigned warp_bits[SMALL_THREADS / 32];            /* this CTA's, by warp */
   unsigned bad[SMALL_CLUSTER_MAX];                   /* rank 0: every CTA's error flag */
 };
 
@@ -808,17 +814,20 @@ __device__ __forceinline__ uint4 dsmem_ld16(unsigned addr)
  *    (row-table entries name the owner and the row within its range), so a
  *    graph C times larger fits.  Every gather goes through the cluster's
  *    shared-memory window, own rows included: on GB300 a separate local path
- *    (a branch, or a generic address) measured no faster.
+ *    (a branch, or a generic address) measured no faster, and so did visiting
+ *    only the lanes with a changed neighbour (a byte per row exchanged per
+ *    level; queued and shared out over the threads: 90 x 90 0.73 ms against
+ *    0.66).
  * The same recurrence and bookkeeping as the engine: level 1 from the
  * neighbour lists, then P_k[v] = P_{k-1}[v] | OR_j P_{k-1}[nbr[v][j]], the
  * bits set per level counted, the job complete when all n * nsrc bits are
- * set and stalled when a level adds none (or the level reaches n).  Each warp
- * adds its count of a level into the level's total in every CTA (remote
- * atomics) and one cluster barrier per level orders the rows and the counts;
- * each CTA then reads the same total and takes the same decision.  The
- * totals rotate over three slots: the slot of level k + 1 is cleared during
- * level k, after the barrier that ended every read of it (level k - 2) and
- * before the barrier after which level k + 1 adds into it.  A CTA reads or
+ * set and stalled when a level adds none (or the level reaches n).  Each CTA
+ * stores its count of a level into every CTA and one cluster barrier per
+ * level orders the rows and the counts; each CTA then adds up the same counts
+ * and takes the same decision.  (A remote atomic per warp and CTA on one
+ * total cost more than the rows: 128 of them per level on a 50 x 50 grid.)
+ * The counts rotate over three slots: level k + 3 is written after the
+ * barrier of level k + 2, and level k is read before the one of level k + 1.  A CTA reads or
  * writes another's shared memory only between two barriers that both pass,
  * so none exits while another may still access it.  Thread 0 of each CTA
  * returns the job's outcome. */
@@ -827,13 +836,13 @@ __device__ void small_job(const gbx_job &jb, const int *idx, uint4 *b0, uint4 *b
                           SmallShared &sh, SmallOutcome &out)
 {
   typedef RowShape<WC> S;
-  constexpr int NB = S::V >= 8 ? 1 : 8 / S::V;
+  static_assert(S::V == 1, "a 16-byte vector per lane");
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks();
   const int n = jb.n, dp = jb.dp, d = jb.d, nsrc = jb.nsrc, src0 = jb.src0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int sub = lane / S::G, gl = lane % S::G;
-  const int nrows = r1 - r0;
+  const int nrows = r1 - r0, rank = (int)cl.block_rank();
 
   const unsigned long long full = (unsigned long long)n * (unsigned long long)nsrc;
   unsigned long long prev = (unsigned long long)nsrc;
@@ -845,65 +854,62 @@ __device__ void small_job(const gbx_job &jb, const int *idx, uint4 *b0, uint4 *b
     unsigned cnt = 0;
     for(int lr = warp * S::RPW + sub; lr < nrows; lr += nwarps * S::RPW){
       const int r = r0 + lr;
-      const int own = PART ? lr : r;                 /* the row's place in this CTA's buffers */
-      uint4 a[S::V];
+      const int own = PART ? lr : r;               /* the row's place in this CTA's buffers */
+      uint4 a = make_uint4(0u, 0u, 0u, 0u);
       const int *ip = idx + lr * dp;
       if(level == 1){
-#pragma unroll
-        for(int k = 0; k < S::V; k++) a[k] = make_uint4(0u, 0u, 0u, 0u);
-        mark_source<S>(a, source_of<SP>(jb.srcpos, r) - src0, nsrc, gl);
+        uint4 m[1] = { a };
+        mark_source<S>(m, source_of<SP>(jb.srcpos, r) - src0, nsrc, gl);
         for(int j = 0; j < dp; j++){
           int u = ip[j];
           if(PART) u = (u >> SMALL_OWNER_SHIFT) * R + (u & SMALL_LOCAL_MASK);
-          mark_source<S>(a, source_of<SP>(jb.srcpos, u) - src0, nsrc, gl);
+          mark_source<S>(m, source_of<SP>(jb.srcpos, u) - src0, nsrc, gl);
         }
+        a = m[0];
       }
       else{
+        a = X[(size_t)own * S::VPR + gl];
+        /* the words of neighbour row u */
+        auto words = [&](int u) {
+          if(PART)
+            return dsmem_ld16(dsmem_map(xs + 16u * (unsigned)((u & SMALL_LOCAL_MASK) * S::VPR),
+                                        (unsigned)(u >> SMALL_OWNER_SHIFT)));
+          return X[(size_t)u * S::VPR + gl];
+        };
+        int j = 0;
+        for(; j + 4 <= d; j += 4){
+          const int4 u = *reinterpret_cast<const int4 *>(ip + j);
+          const uint4 t0 = words(u.x), t1 = words(u.y), t2 = words(u.z), t3 = words(u.w);
+          or_into(a, t0);
+          or_into(a, t1);
+          or_into(a, t2);
+          or_into(a, t3);
+        }
+        for(; j < d; j++) or_into(a, words(ip[j]));
+      }
+      /* from level 3 on Y holds level k - 2: words that have not changed
+       * since are not stored (in every CTA's copy, replicated) */
+      uint4 *yr = Y + (size_t)own * S::VPR + gl;
+      if(level <= 2 || differ(a, *yr)){
+        if(PART) *yr = a;
+        else{
 #pragma unroll
-        for(int k = 0; k < S::V; k++) a[k] = X[(size_t)own * S::VPR + gl + k * S::G];
-        for(int j = 0; j < d; j += NB){
-          uint4 t[NB][S::V];
-#pragma unroll
-          for(int i = 0; i < NB; i++){
-            const bool ok = j + i < d;
-            const int u = ip[ok ? j + i : j];
-            if(PART){
-              /* a generic address: this CTA's own shared window for its own
-               * rows, the owner's window in the cluster for the others' */
-              const unsigned base = dsmem_map(xs + 16u * (unsigned)((u & SMALL_LOCAL_MASK) * S::VPR),
-                                              (unsigned)(u >> SMALL_OWNER_SHIFT));
-#pragma unroll
-              for(int k = 0; k < S::V; k++)
-                t[i][k] = ok ? dsmem_ld16(base + 16u * (unsigned)(k * S::G)) : make_uint4(0u, 0u, 0u, 0u);
-            }
-            else{
-              const uint4 *nr = X + (size_t)u * S::VPR + gl;
-#pragma unroll
-              for(int k = 0; k < S::V; k++) t[i][k] = ok ? nr[k * S::G] : make_uint4(0u, 0u, 0u, 0u);
-            }
-          }
-#pragma unroll
-          for(int i = 0; i < NB; i++)
-#pragma unroll
-            for(int k = 0; k < S::V; k++) or_into(a[k], t[i][k]);
+          for(int q = 0; q < SMALL_CLUSTER_MAX; q++)
+            if(q < C) *cl.map_shared_rank(yr, (unsigned)q) = a;
         }
       }
-      uint4 *yr = Y + (size_t)own * S::VPR + gl;
-#pragma unroll
-      for(int k = 0; k < S::V; k++){
-        if(PART) yr[k * S::G] = a[k];
-        else
-          for(int q = 0; q < C; q++) *cl.map_shared_rank(yr + k * S::G, (unsigned)q) = a[k];
-        cnt += popc4(a[k]);
-      }
+      cnt += popc4(a);
     }
     cnt = __reduce_add_sync(0xffffffffu, cnt);
-    unsigned long long *tot = &sh.total[level % 3];
-    if(lane == 0 && cnt)
-      for(int q = 0; q < C; q++) atomicAdd(cl.map_shared_rank(tot, (unsigned)q), (unsigned long long)cnt);
-    if(threadIdx.x == 0) sh.total[(level + 1) % 3] = 0;
+    if(lane == 0) sh.warp_bits[warp] = cnt;
+    __syncthreads();
+    if(warp == 0){
+      const unsigned mine = __reduce_add_sync(0xffffffffu, lane < nwarps ? sh.warp_bits[lane] : 0u);
+      if(lane < C) *cl.map_shared_rank(&sh.total[level % 3][rank], (unsigned)lane) = mine;
+    }
     cl.sync();
-    const unsigned long long c = *tot;
+    unsigned long long c = 0;
+    for(int q = 0; q < C; q++) c += sh.total[level % 3][q];
     const bool complete = c == full;
     const bool stalled = !complete && (c == prev || level >= n);
     if(complete || stalled){
@@ -943,7 +949,6 @@ small_kernel(const gbx_job *__restrict__ jobs, const gbx_expand_desc *descs, gbx
   if(threadIdx.x == 0){
     t_loaded = globaltimer();
     sh.desc = descs ? descs[jb.graph] : desc0;
-    sh.total[0] = sh.total[1] = sh.total[2] = 0;
   }
   /* every CTA of the cluster is running (its shared memory may be written)
    * and the descriptor is visible to the whole CTA */

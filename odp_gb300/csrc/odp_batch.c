@@ -98,11 +98,11 @@ int ODPX_Batch_info(const ODPX_Batch *batch, int graph, int *njobs, int *nslots,
   return 0;
 }
 
-int ODPX_Batch_kernel(const ODPX_Batch *batch) { return batch ? batch->small : ODPX_ERR_INVALID; }
+int ODPX_Batch_kernel(const ODPX_Batch *batch) { return batch ? batch->small_class : ODPX_ERR_INVALID; }
 
 int ODPX_Batch_small_shape(const ODPX_Batch *batch, int *cluster, int *threads, int *partitioned)
 {
-  if(!batch || !batch->small) return ODPX_ERR_INVALID;
+  if(!batch || !batch->small_class) return ODPX_ERR_INVALID;
   if(cluster) *cluster = batch->small_cluster;
   if(threads) *threads = batch->small_threads;
   if(partitioned) *partitioned = batch->small_part;

@@ -62,22 +62,6 @@ void odp_tuning_defaults(odp_tuning *t, int batch)
   t->team = 0;
 }
 
-/* Chunk width (log2 words) for a graph whose whole level runs in shared
- * memory on a cluster of `cluster` CTAs: the widest of at most 16 words, and
- * at most the graph's own width, whose two bitset buffers (whole in every
- * CTA, or with `part` only the CTA's rows) and row table (1/cluster of the
- * rows per CTA) fit; 0 if none does. */
-static int small_wc_log2(int n, int dp, int full_l2, int cluster, int part)
-{
-  const size_t rows = (size_t)(n + cluster - 1) / (size_t)cluster;
-  const size_t buf_rows = part ? rows : (size_t)n;
-  for(int wl = full_l2 < 4 ? full_l2 : 4; wl >= 1; wl--){
-    size_t bytes = 2 * buf_rows * ((size_t)8 << wl) + rows * (size_t)dp * 4;
-    if(bytes <= GBX_SMALL_SMEM_MAX) return wl;
-  }
-  return 0;
-}
-
 /* Shared memory per CTA of the small kernel when `cluster` CTAs share a job:
  * both bitset buffers (whole, or with `part` the CTA's 1/cluster of the
  * rows) and the row table of 1/cluster of the rows. */
@@ -85,6 +69,16 @@ static size_t small_bytes(int n, int dp, int wl, int cluster, int part)
 {
   const size_t rows = (size_t)(n + cluster - 1) / (size_t)cluster;
   return 2 * (part ? rows : (size_t)n) * ((size_t)8 << wl) + rows * (size_t)dp * 4;
+}
+
+/* Chunk width (log2 words) for a graph whose whole level runs in shared
+ * memory on a cluster of `cluster` CTAs: the widest of at most 16 words, and
+ * at most the graph's own width, that fits; 0 if none does. */
+static int small_wc_log2(int n, int dp, int full_l2, int cluster, int part)
+{
+  for(int wl = full_l2 < 4 ? full_l2 : 4; wl >= 1; wl--)
+    if(small_bytes(n, dp, wl, cluster, part) <= GBX_SMALL_SMEM_MAX) return wl;
+  return 0;
 }
 
 /* Threads per CTA for a CTA's rows: one lane per 16 bytes of a row (at most
@@ -440,6 +434,19 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
   return 0;
 }
 
+/* Whether a small plan of one graph is faster on the lockstep kernel (unless
+ * its cluster or layout is forced).  Measured on GB300, small kernel against
+ * lockstep (us): general graphs, each of whose jobs reads the adjacency from
+ * host memory, n = 512, d = 8: 18 / 21; 1024, 8: 19 / 22; 1024, 24: 27 / 17;
+ * 2048, 8: 33 / 25; 4096, 8: 51 / 29.  Grids, replicated: 50 x 50 117 / 177,
+ * 64 x 64 101 / 180; partitioned: 72 x 72 210 / 189, 80 x 80 298 / 283, 90 x 90
+ * 658 / 367. */
+static int small_yields(const odp_shape *sh, const odp_tuning *t, int part)
+{
+  if(t->small_cluster > 0 || t->small_part >= 0) return 0;
+  return sh->grid ? part : (long long)shape_n(sh) * shape_dp(sh) > 12000;
+}
+
 /* Whether no schedule setting asks for the persistent engine. */
 static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
 {
@@ -708,7 +715,10 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   int *small_wl = calloc((size_t)count, sizeof(int));
   int small = choose_small(shapes, count, tuning, sms, small_wl, &p->small_cluster, &p->small_threads,
                            &p->small_smem, &p->small_part);
-  p->sweep = !small && count == 1 && choose_sweep(shapes, tuning, sms, &p->sw, &p->sweep_grid);
+  p->small_class = small;
+  p->sweep = count == 1 && (!small || small_yields(shapes, tuning, p->small_part)) &&
+             choose_sweep(shapes, tuning, sms, &p->sw, &p->sweep_grid);
+  if(p->sweep) small = 0;
   int *team_order = NULL;
   if(!small && !p->sweep){
     p->h_teams = calloc((size_t)count, sizeof(gbx_sweep));

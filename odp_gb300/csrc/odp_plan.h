@@ -78,6 +78,7 @@ typedef struct odp_plan {
   int direct;                  /* the device pulls the callers' arrays (h_expand holds their pointers) */
   gbx_expand_desc *h_expand;   /* pinned copy of the expand descriptors (direct plans) */
   int small;                   /* every job runs in the small-graph kernel, in shared memory */
+  int small_class;             /* the plan fits the small-graph kernel, whichever kernel it runs on */
   size_t small_smem;           /* shared memory per CTA of the small-graph kernel */
   int small_cluster;           /* CTAs (one thread-block cluster) per job of the small-graph kernel */
   int small_threads;           /* threads per CTA of the small-graph kernel */
