@@ -434,17 +434,22 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
   return 0;
 }
 
-/* Whether a small plan of one graph is faster on the lockstep kernel (unless
- * its cluster or layout is forced).  Measured on GB300, small kernel against
- * lockstep (us): general graphs, each of whose jobs reads the adjacency from
- * host memory, n = 512, d = 8: 18 / 21; 1024, 8: 19 / 22; 1024, 24: 27 / 17;
- * 2048, 8: 33 / 25; 4096, 8: 51 / 29.  Grids, replicated: 50 x 50 117 / 177,
- * 64 x 64 101 / 180; partitioned: 72 x 72 210 / 189, 80 x 80 298 / 283, 90 x 90
- * 658 / 367. */
-static int small_yields(const odp_shape *sh, const odp_tuning *t, int part)
+/* Whether a small plan of one graph, in chunks of 2^wl words, is faster on the
+ * lockstep kernel (unless its cluster or layout is forced).  Every job of the
+ * small kernel reads the whole adjacency from host memory, so for general
+ * graphs the line lies at 450 KB read in all; measured on GB300, small kernel
+ * against lockstep (us): n = 512, d = 8 (66 KB) 18 / 21; n = 1182, d = 10, s =
+ * 2 (118 KB) 32 / 35 with the call around it; n = 1024, d = 8 (262 KB) 19 / 22;
+ * n = 1024, d = 24 (786 KB) 27 / 17; n = 2048, d = 8 (1 MB) 33 / 25; n = 4096, d
+ * = 8 (4 MB) 51 / 29.  Grids are bound by their levels: replicated 50 x 50 117
+ * / 177, 64 x 64 101 / 180; partitioned 72 x 72 210 / 189, 80 x 80 298 / 283, 90
+ * x 90 658 / 367. */
+static int small_yields(const odp_shape *sh, const odp_tuning *t, int part, int wl)
 {
   if(t->small_cluster > 0 || t->small_part >= 0) return 0;
-  return sh->grid ? part : (long long)shape_n(sh) * shape_dp(sh) > 12000;
+  if(sh->grid) return part;
+  const double jobs = (shape_words(sh) + (1 << wl) - 1) >> wl;
+  return jobs * 4.0 * (shape_n(sh) / sh->symmetries) * sh->degree > 450e3;
 }
 
 /* Whether no schedule setting asks for the persistent engine. */
@@ -716,7 +721,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   int small = choose_small(shapes, count, tuning, sms, small_wl, &p->small_cluster, &p->small_threads,
                            &p->small_smem, &p->small_part);
   p->small_class = small;
-  p->sweep = count == 1 && (!small || small_yields(shapes, tuning, p->small_part)) &&
+  p->sweep = count == 1 && (!small || small_yields(shapes, tuning, p->small_part, small_wl[0])) &&
              choose_sweep(shapes, tuning, sms, &p->sw, &p->sweep_grid);
   if(p->sweep) small = 0;
   int *team_order = NULL;
