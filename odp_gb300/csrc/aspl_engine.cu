@@ -937,7 +937,7 @@ __device__ void small_job(const gbx_job &jb, const int *idx, uint4 *b0, uint4 *b
  * (a single-graph call then reads no descriptor from host memory). */
 __global__ void __launch_bounds__(SMALL_THREADS, 1)
 small_kernel(const gbx_job *__restrict__ jobs, const gbx_expand_desc *descs, gbx_small_rec *rec,
-             const gbx_expand_desc desc0, const int part)
+             const gbx_expand_desc desc0, const int part, const unsigned seq)
 {
   extern __shared__ __align__(16) unsigned char small_smem[];
   __shared__ SmallShared sh;
@@ -1021,11 +1021,11 @@ small_kernel(const gbx_job *__restrict__ jobs, const gbx_expand_desc *descs, gbx
     for(int q = 0; q < C; q++) b |= sh.bad[q];
     gbx_small_rec r;
     r.level = o.stalled ? -o.level : o.level;
-    r.err = b ? GBX_ERR_BAD_ADJ : 0u;
+    r.err = (b ? GBX_ERR_BAD_ADJ : 0u) | seq << 8;
     r.sum = o.sum;
     r.t_loaded = t_loaded;
     r.t_done = globaltimer();
-    rec[job] = r;
+    store_record(rec + job, r);
   }
 }
 
@@ -1227,7 +1227,8 @@ int gbx_small_clusters(int cluster, int threads, size_t smem_bytes, int *active)
 }
 
 int gbx_small_launch(const gbx_job *d_jobs, int njobs, const gbx_expand_desc *descs, const gbx_expand_desc *desc0,
-                     gbx_small_rec *rec, size_t smem_bytes, int cluster, int threads, int part, void *stream)
+                     gbx_small_rec *rec, unsigned int seq, size_t smem_bytes, int cluster, int threads, int part,
+                     void *stream)
 {
   if(njobs <= 0) return 0;
   if(!small_shape_ok(cluster, threads, smem_bytes) || (!descs && !desc0)) return (int)cudaErrorInvalidValue;
@@ -1236,7 +1237,7 @@ int gbx_small_launch(const gbx_job *d_jobs, int njobs, const gbx_expand_desc *de
   gbx_expand_desc d0;
   if(desc0) d0 = *desc0;
   else memset(&d0, 0, sizeof(d0));
-  return (int)cudaLaunchKernelEx(&cfg, small_kernel, d_jobs, descs, rec, d0, part ? 1 : 0);
+  return (int)cudaLaunchKernelEx(&cfg, small_kernel, d_jobs, descs, rec, d0, part ? 1 : 0, (unsigned)seq);
 }
 
 int gbx_host_device_ptr(void *host, void **dev)

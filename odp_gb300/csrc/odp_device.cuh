@@ -100,6 +100,16 @@ __device__ __forceinline__ int expand_value(const gbx_expand_desc &e, int a, int
 }
 
 
+/* A record into pinned host memory: its error word last, released to the host. */
+__device__ __forceinline__ void store_record(gbx_small_rec *to, const gbx_small_rec &r)
+{
+  to->level = r.level;
+  to->sum = r.sum;
+  to->t_loaded = r.t_loaded;
+  to->t_done = r.t_done;
+  asm volatile("st.release.sys.global.u32 [%0], %1;" :: "l"(&to->err), "r"(r.err) : "memory");
+}
+
 /* ---------------------------------------------------------------------- */
 /* Lanes: 32 bytes (256 source bits, one sector) of a row, the unit of the  */
 /* lockstep kernels, moved by 256-bit accesses (L2 only: other SMs rewrite  */

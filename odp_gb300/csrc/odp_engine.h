@@ -158,9 +158,13 @@ int  gbx_engine_launch(const gbx_job *d_jobs, int njobs, gbx_slot *d_slots, int 
  * of 8), so a call needs no separate uploads for either. */
 int  gbx_pull(const gbx_expand_desc *h_descs, gbx_expand_desc *d_descs, int ndesc, void *d_state,
               const void *d_state_init, size_t state_bytes, void *stream);
-/* Outcome of one job of the small-graph kernel, written to pinned host
- * memory: its last level (negative: stalled), error bits (GBX_ERR_*), its
- * share of the graph's ordered distance sum, and %globaltimer stamps. */
+/* Outcome of one job of the one-launch kernels, written to pinned host
+ * memory: its last level (negative: stalled), error bits (GBX_ERR_*) below the
+ * launch's number, its share of the graph's ordered distance sum, and
+ * %globaltimer stamps.  `err` is stored last and released to the host, which
+ * may therefore take a record as soon as it carries the launch's number. */
+#define GBX_REC_ERR(e) ((e) & 0xffu)
+#define GBX_REC_SEQ(e) ((e) >> 8)
 typedef struct {
   int level;
   unsigned int err;
@@ -181,7 +185,8 @@ typedef struct {
  * With `part` set each CTA holds only its own rows of the bitset buffers
  * (1/cluster of them) and gathers the others' rows from their shared memory. */
 int  gbx_small_launch(const gbx_job *d_jobs, int njobs, const gbx_expand_desc *descs, const gbx_expand_desc *desc0,
-                      gbx_small_rec *rec, size_t smem_bytes, int cluster, int threads, int part, void *stream);
+                      gbx_small_rec *rec, unsigned int seq, size_t smem_bytes, int cluster, int threads, int part,
+                      void *stream);
 /* How many clusters of that shape the GPU holds at once (0: the shape does
  * not fit; then it cannot be launched). */
 int  gbx_small_clusters(int cluster, int threads, size_t smem_bytes, int *active);
@@ -223,6 +228,7 @@ typedef struct {
   int scratch_bits;            /* sources a warp marks at a time (a multiple of 8192, or all of them) */
   int in_place;                /* the lists are built from the host array itself */
   int set;                     /* which half of `sync`: alternate it from launch to launch */
+  unsigned int seq;            /* the launch's number, for the records */
 } gbx_sweep;
 size_t gbx_sweep_sync_bytes(void);
 /* Shared memory per CTA, and resident CTAs per SM with it (0: does not fit). */

@@ -89,6 +89,7 @@ typedef struct odp_plan {
   gbx_small_rec *h_small_rec;  /* small plans: per-job records, pinned; the kernel writes them */
   gbx_small_rec *d_small_rec;  /*   the same memory, as the device addresses it */
   gbx_expand_desc *d_small_desc; /* small plans: h_expand as the device addresses it */
+  unsigned int seq;            /* number of the last launch of a single graph's one kernel (0: none; 24 bits) */
   int sweep;                   /* the plan's one graph runs in the lockstep kernel */
   gbx_sweep sw;                /* its launch arguments */
   int sweep_grid;              /* CTAs */

@@ -122,11 +122,11 @@ __device__ __forceinline__ bool settle(const gbx_sweep &a, SweepPhase &p, const 
   }
   gbx_small_rec r;
   r.level = stalled ? -level : level;
-  r.err = __ldcg(&sy.err);
+  r.err = __ldcg(&sy.err) | a.seq << 8;
   r.sum = p.sum[q];
   r.t_loaded = p.t_loaded;
   r.t_done = globaltimer();
-  a.rec[chunk] = r;
+  store_record(a.rec + chunk, r);
   return false;
 }
 
