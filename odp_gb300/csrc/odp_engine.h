@@ -229,6 +229,8 @@ typedef struct {
   int in_place;                /* the lists are built from the host array itself */
   int set;                     /* which half of `sync`: alternate it from launch to launch */
   unsigned int seq;            /* the launch's number, for the records */
+  const gbx_write *writes;     /* teams: changes of the adjacency that precede the evaluation, or NULL */
+  int nwrites;
 } gbx_sweep;
 size_t gbx_sweep_sync_bytes(void);
 /* Shared memory per CTA, and resident CTAs per SM with it (0: does not fit). */
@@ -243,7 +245,7 @@ int  gbx_sweep_launch(const gbx_sweep *a, int blocks, void *stream);
 #define GBX_TEAM_SPLITS 9              /* teams of 1/1 to 1/256 of the grid */
 typedef struct {
   const gbx_sweep *graphs;
-  const int *order;
+  const int *order;                    /* NULL: graphs[] is in queue order */
   const unsigned long long *adj;       /* this call's host arrays (device memory), or NULL: graphs[g].e.adj */
   unsigned int *next;                  /* [GBX_TEAM_SPLITS], zeroed before the launch, as are the nodes */
   void *nodes;                         /* gbx_team_node_bytes() for each team of first_split .. last_split */

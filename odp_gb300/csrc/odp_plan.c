@@ -540,15 +540,44 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
   return 0;
 }
 
-typedef struct {
-  double cost, latency;        /* us on the whole GPU; us whatever the team */
-  double need;                 /* bytes of its bitsets */
-  int split;
-} team_graph;
+/* Whether the team kernel takes a graph of this shape: it must fit the lockstep
+ * kernels in one group (bitsets of at most 64 MB, 64 lanes a row, 256 for
+ * grids).  Its cost on the whole GPU is estimated from its traffic: a general
+ * graph's gathered levels at 20 TB/s; for grids about ten visits per row and
+ * lane, each reading d + 2 sectors, at 8 TB/s. */
+int odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_team_graph *g)
+{
+  const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
+  memset(c, 0, sizeof(*c));
+  if(!lockstep_allowed(sh, t) || 16.0 * n * W > 64e6 || W > (sh->grid ? 1024 : 256)) return 0;
+  c->e.dp = shape_dp(sh);
+  c->B = n / sh->symmetries;
+  c->phases = 1;
+  c->track = sh->grid && c->e.dp <= GBX_SWEEP_TRACK_DEGREE;
+  if(!c->track && W > 256) return 0;
+  c->two_level = c->e.dp <= GBX_SWEEP_TWO_LEVEL && 8.0 * W * sh->degree > 5000;
+  c->scratch_bits = (c->B + 255) / 256 * 256;
+  c->wc_log2 = c->track ? (full_l2 < 5 ? full_l2 : 5) : (full_l2 < 6 ? full_l2 : 6);
+  c->nchunks = c->slots = (W + (1 << c->wc_log2) - 1) >> c->wc_log2;
+  while((32 << c->word_log2) < (c->slots << (c->wc_log2 - 2))) c->word_log2++;
+  const double lanes = (c->B + 255) / 256;
+  if(c->track){
+    g->cost = n * lanes * 9.5 * (sh->degree + 2) * 32.0 / 8e6;
+    g->latency = 15.0 + 4.0 * (sh->width + sh->height) / 3.0;
+  }
+  else{
+    double levels = 2.0, ball = sh->degree + 1.0;      /* until a ball of branching d - 1 holds n, and one more */
+    for(const double grow = sh->degree > 3 ? sh->degree - 1.0 : 2.0; ball < n; ball *= grow) levels += 1.0;
+    g->cost = (n * 8.0 * W * (sh->degree + 1) * (levels > 3.0 ? levels - 2.5 : 0.5) + 4.0 * n * c->e.dp * sh->degree) / 20e6;
+    g->latency = 15.0 + 4.0 * levels;
+  }
+  g->need = 16.0 * ((double)n * c->slots * (1 << c->wc_log2)) + (c->track ? 8.0 * n * (1 << c->word_log2) : 0) + 1024;
+  return 1;
+}
 
 /* Makespan (us) of the graphs on their teams: every team takes the next graph
  * of its size when it is free, and splits when there is none. */
-static double team_makespan(const team_graph *g, const job_order *ord, int count)
+static double team_makespan(const odp_team_graph *g, const job_order *ord, int count)
 {
   double at[1 << (GBX_TEAM_SPLITS - 1)] = {0};
   double end = 0;
@@ -556,7 +585,7 @@ static double team_makespan(const team_graph *g, const job_order *ord, int count
     const int teams = 1 << k;
     if(k) for(int i = teams - 1; i >= 0; i--) at[i] = at[i >> 1];
     for(int j = 0; j < count; j++){
-      const team_graph *x = &g[ord[j].job];
+      const odp_team_graph *x = &g[ord[j].job];
       if(x->split != k) continue;
       int first = 0;
       for(int i = 1; i < teams; i++) if(at[i] < at[first]) first = i;
@@ -570,8 +599,8 @@ static double team_makespan(const team_graph *g, const job_order *ord, int count
 /* Each graph's team: the smallest on which it takes at most `most` us, its
  * rows fit a CTA and the teams' bitsets stay within 160 MB.  0 if some graph
  * does not even fit the whole grid. */
-static int assign_teams(const odp_shape *shapes, int count, int grid, size_t smem_max, double most, gbx_sweep *gs,
-                        team_graph *g)
+static int assign_teams(const odp_shape *shapes, int count, int grid, double most, gbx_sweep *gs,
+                        odp_team_graph *g)
 {
   for(int i = 0; i < count; i++){
     g[i].split = -1;
@@ -579,7 +608,7 @@ static int assign_teams(const odp_shape *shapes, int count, int grid, size_t sme
       gbx_sweep c = gs[i];
       const int size = grid >> k;
       c.rows = (shape_n(&shapes[i]) + size - 1) / size;
-      if(gbx_sweep_smem(&c) > smem_max || (k > 0 && (g[i].need * (1 << k) > 160e6 || g[i].cost * (1 << k) > most))) break;
+      if(gbx_sweep_smem(&c) > ODP_TEAM_SMEM || (k > 0 && (g[i].need * (1 << k) > 160e6 || g[i].cost * (1 << k) > most))) break;
       g[i].split = k;
       gs[i].rows = c.rows;
     }
@@ -589,11 +618,7 @@ static int assign_teams(const odp_shape *shapes, int count, int grid, size_t sme
 }
 
 /* Whether a plan runs on the team kernel, and which team each graph gets.
- * Every graph must fit the lockstep kernels in one group (bitsets of at most
- * 64 MB, 64 lanes a row, 256 for grids).  A graph's cost on the whole GPU is
- * estimated from its traffic: a general graph's gathered levels at 20 TB/s;
- * for grids about ten visits per row and lane, each reading d + 2 sectors, at
- * 8 TB/s.  Its team is the smallest on which it takes no more
+ * A graph's team is the smallest on which it takes no more
  * than a share of all graphs' cost, its rows fit a CTA's shared memory and
  * the teams' bitsets together stay within 160 MB; of several shares the one
  * with the least makespan is taken. */
@@ -601,46 +626,16 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
                        gbx_team *tm, int *order, int *grid_out, size_t *smem_out)
 {
   if(count == 1 && !t->team) return 0;
-  for(int i = 0; i < count; i++){
-    const double n = shape_n(&shapes[i]), W = shape_words(&shapes[i]);
-    if(!lockstep_allowed(&shapes[i], t) || 16.0 * n * W > 64e6 || W > (shapes[i].grid ? 1024 : 256)) return 0;
-  }
   int fit = 0;
   if(gbx_team_blocks(0, &fit) || fit < 2) return 0;
   int grid = 2 * sms;
   if(t->blocks > 0 && t->blocks < grid) grid = t->blocks;
-  const size_t smem_max = 100 * 1024;
-  team_graph *g = calloc((size_t)count, sizeof(team_graph));
+  odp_team_graph *g = calloc((size_t)count, sizeof(odp_team_graph));
   job_order *ord = calloc((size_t)count, sizeof(job_order));
   int ok = g && ord;
   double all = 0;
   for(int i = 0; i < count && ok; i++){
-    const odp_shape *sh = &shapes[i];
-    gbx_sweep *c = &gs[i];
-    const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
-    memset(c, 0, sizeof(*c));
-    c->e.dp = shape_dp(sh);
-    c->B = n / sh->symmetries;
-    c->phases = 1;
-    c->track = sh->grid && c->e.dp <= GBX_SWEEP_TRACK_DEGREE;
-    c->two_level = c->e.dp <= GBX_SWEEP_TWO_LEVEL && 8.0 * W * sh->degree > 5000;
-    c->scratch_bits = (c->B + 255) / 256 * 256;
-    c->wc_log2 = c->track ? (full_l2 < 5 ? full_l2 : 5) : (full_l2 < 6 ? full_l2 : 6);
-    c->nchunks = c->slots = (W + (1 << c->wc_log2) - 1) >> c->wc_log2;
-    while((32 << c->word_log2) < (c->slots << (c->wc_log2 - 2))) c->word_log2++;
-    if(!c->track && W > 256) ok = 0;
-    const double lanes = (c->B + 255) / 256;
-    if(c->track){
-      g[i].cost = n * lanes * 9.5 * (sh->degree + 2) * 32.0 / 8e6;
-      g[i].latency = 15.0 + 4.0 * (sh->width + sh->height) / 3.0;
-    }
-    else{
-      double levels = 2.0, ball = sh->degree + 1.0;      /* until a ball of branching d - 1 holds n, and one more */
-      for(const double grow = sh->degree > 3 ? sh->degree - 1.0 : 2.0; ball < n; ball *= grow) levels += 1.0;
-      g[i].cost = (n * 8.0 * W * (sh->degree + 1) * (levels > 3.0 ? levels - 2.5 : 0.5) + 4.0 * n * c->e.dp * sh->degree) / 20e6;
-      g[i].latency = 15.0 + 4.0 * levels;
-    }
-    g[i].need = 16.0 * ((double)n * c->slots * (1 << c->wc_log2)) + (c->track ? 8.0 * n * (1 << c->word_log2) : 0) + 1024;
+    ok = odp_team_shape(&shapes[i], t, &gs[i], &g[i]);
     all += g[i].cost;
     ord[i].job = i;
     ord[i].work = g[i].cost;
@@ -650,11 +645,11 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
     static const double shares[] = { 0.1, 0.2, 0.35, 0.6, 1.0 };
     double best = 0, best_share = 0;
     for(int s = 0; s < 5 && ok; s++){
-      ok = assign_teams(shapes, count, grid, smem_max, shares[s] * all, gs, g);
+      ok = assign_teams(shapes, count, grid, shares[s] * all, gs, g);
       const double m = ok ? team_makespan(g, ord, count) : 0;
       if(s == 0 || m < best){ best = m; best_share = shares[s]; }
     }
-    if(ok) ok = assign_teams(shapes, count, grid, smem_max, best_share * all, gs, g);
+    if(ok) ok = assign_teams(shapes, count, grid, best_share * all, gs, g);
   }
   size_t smem = 0;
   double arena = 0;

@@ -112,6 +112,16 @@ typedef struct {
   double aspl;
 } odp_result;
 
+/* Whether the team kernel can take a graph of this shape, and then its shape
+ * and estimates there. */
+typedef struct {
+  double cost, latency;        /* us on the whole GPU; us whatever the team */
+  double need;                 /* bytes of its bitsets */
+  int split;
+} odp_team_graph;
+#define ODP_TEAM_SMEM (100 * 1024)     /* of a CTA: two per SM */
+int  odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_team_graph *g);
+
 void odp_tuning_defaults(odp_tuning *t, int batch);
 /* The defaults for `count` graphs with the ODPX_Set_tuning overrides applied. */
 void odp_tuning_for(int count, odp_tuning *t);

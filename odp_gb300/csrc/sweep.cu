@@ -881,7 +881,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) team_kernel(const gbx_team t
     /* CTA `lo` takes the next graph off the queue and posts it */
     auto post = [&](int seq) {
       const unsigned at = atomicAdd(t.next + k, 1u);
-      const unsigned g = at < (unsigned)queued ? (unsigned)t.order[t.queue[k] + (int)at] + 1u : 0u;
+      const int from = t.queue[k] + (int)at;
+      const unsigned g = at < (unsigned)queued ? (unsigned)(t.order ? t.order[from] : from) + 1u : 0u;
       __threadfence();
       atomicExch(&node.box[seq & 1][0], (unsigned long long)(seq + 1) << 32 | g);
     };
@@ -914,6 +915,10 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) team_kernel(const gbx_team t
         a.changed = reinterpret_cast<unsigned *>(at + 16 * a.slot_words);
         a.rows = (a.e.n + (hi - lo) - 1) / (hi - lo);
       }
+      /* every CTA applies all of the graph's changes itself, the same values
+       * to the same places, and so needs no barrier of the team before it
+       * reads them */
+      for(int x = tid; x < a.nwrites; x += SWEEP_THREADS) *a.writes[x].at = a.writes[x].value;
       sweep_begin(sh, b - lo, hi - lo);
       TeamSync &sy = node.sync[seq & 1];
       auto clear = [&] {

@@ -199,3 +199,44 @@ def test_native_client_chains_match_their_graphs_alone():
         rep = json.loads(r.stdout.strip().splitlines()[-1])
         assert rep["checked"] == len(chains) and rep["mismatched"] == 0 and rep["errors"] == 0, rep
         assert rep["completed"] > 0
+
+
+@pytest.mark.parametrize("lanes,max_batch,memory_mb", [(1, 16, 256), (4, 5, 256), (7, 2, 256), (2, 16, 24)])
+def test_served_general_graphs_by_teams(lanes, max_batch, memory_mb):
+    """General graphs of a batch are evaluated by teams of CTAs that apply the
+    deltas themselves: batches of one graph up to the whole of them, rows
+    shorter than a lane and of several chunks, one and two start levels,
+    orders with symmetry, irregular rows, many deltas at once, and memory for
+    some of the graphs only (the others stay on the persistent engine)."""
+    rng = np.random.default_rng(lanes)
+    graphs = []
+    for i, (n, d, s) in enumerate([(20, 3, 1), (257, 5, 1), (1024, 8, 4), (1500, 80, 1), (2111, 9, 1), (4100, 6, 1),
+                                   (4352, 40, 17), (8192, 12, 1)]):
+        adj = og.conv_edge2adjacency_general(n, og.generate_random_general(n, d if n * d % 2 == 0 else d - 1, s, seed=70 + i),
+                                             d if n * d % 2 == 0 else d - 1, s)
+        deg = None
+        if s == 1 and i % 2:
+            deg = np.full(n, adj.shape[1], dtype=np.int32)
+            deg[rng.integers(0, n, 5)] -= 1
+        graphs.append((n, s, adj, deg))
+    srv = og.Server(lanes=lanes, max_batch=max_batch, max_nodes=8192, memory_mb=memory_mb)
+    handles = [srv.register(og.GraphSpec(a.copy(), nodes=n, symmetries=s, num_degrees=g)) for n, s, a, g in graphs]
+    alone_plans = [og.Batch([og.GraphSpec(a, nodes=n, symmetries=s, num_degrees=g)]) for n, s, a, g in graphs]
+    for step, many in enumerate((0, 1, 4, 300)):
+        ids = []
+        for h, (n, s, a, g) in zip(handles, graphs):
+            deltas = []
+            for _ in range(many):
+                row, slot = int(rng.integers(0, a.shape[0])), int(rng.integers(0, a.shape[1] - 1))
+                a[row, slot] = int(rng.integers(0, n))
+                deltas.append((row, slot, int(a[row, slot])))
+            ids.append(srv.submit(h, deltas))
+        for r, h, b, (n, s, a, g) in zip(ids, handles, alone_plans, graphs):
+            got = srv.wait(r)[:3]
+            assert same(got, b.run([a])[0]), (n, step)
+            if step in (0, 3) and n <= 2111:
+                assert same(got, oracle.aspl(a, nodes=n, symmetries=s, num_degrees=g)), (n, step)
+            assert np.array_equal(srv.adjacency(h), a)
+    for b in alone_plans:
+        b.close()
+    srv.close()
