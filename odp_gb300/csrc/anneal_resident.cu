@@ -84,6 +84,67 @@ __device__ __forceinline__ void swap_writes(ResidentShared &sh, const G &g)
     }
 }
 
+/* Thread 0: mut_two_opt's common way for regular general graphs without
+ * symmetry, where nothing turns or has an antipode: five draws, four distinct
+ * vertices, one exchange.  The draws, the two edges' slots and the rows that
+ * point back are loaded side by side; one after another behind the general
+ * form's branches they took 5k cycles a step, warm.  False, with nothing
+ * drawn, when a vertex repeats (the general form draws again) or an edge has
+ * no other end. */
+__device__ bool propose_regular(ResidentShared &sh)
+{
+  unsigned short *adj = sh.g.adj;
+  const int n = sh.g.n, d = sh.g.d, p = sh.rng.pos;
+  unsigned x[5];
+  int at[5];
+#pragma unroll
+  for(int k = 0; k < 5; k++){
+    at[k] = p + k < 31 ? p + k : p + k - 31;
+    const int q = at[k] >= 3 ? at[k] - 3 : at[k] + 28;
+    x[k] = sh.rng.ring[at[k]];
+    if(k < 3) x[k] += sh.rng.ring[q];
+  }
+  x[3] += x[0];
+  x[4] += x[1];
+  auto below = [&](int k, int max) { return (int)(((unsigned long long)(x[k] >> 1) * (unsigned long long)max) >> 31); };
+  const int u0 = below(0, n), u1 = below(1, n), s0 = below(2, d), s1 = below(3, d);
+  const int v0 = adj[u0 * d + s0], v1 = adj[u1 * d + s1];
+  if(u0 == u1 || v0 == u1 || v1 == u0 || v0 == v1 || v0 == u0 || v1 == u1) return false;
+  int b0 = -1, b1 = -1;
+  for(int i0 = (d - 1) & ~7; i0 >= 0; i0 -= 8){            /* the first of equal entries */
+    int e0[8], e1[8];
+#pragma unroll
+    for(int k = 0; k < 8; k++){
+      const int i = min(i0 + k, d - 1);
+      e0[k] = adj[v0 * d + i];
+      e1[k] = adj[v1 * d + i];
+    }
+#pragma unroll
+    for(int k = 7; k >= 0; k--){
+      if(e0[k] == u0) b0 = min(i0 + k, d - 1);
+      if(e1[k] == u1) b1 = min(i0 + k, d - 1);
+    }
+  }
+  if(b0 < 0 || b1 < 0) return false;
+  const bool cross = below(4, 2) != 0;                     /* u0--v1, v0--u1; else u0--u1, v0--v1 */
+  adj[u0 * d + s0] = (unsigned short)(cross ? v1 : u1);
+  adj[u1 * d + s1] = (unsigned short)(cross ? v0 : u0);
+  adj[v0 * d + b0] = (unsigned short)(cross ? u1 : v1);
+  adj[v1 * d + b1] = (unsigned short)(cross ? u0 : v0);
+#pragma unroll
+  for(int k = 0; k < 5; k++) sh.rng.ring[at[k]] = x[k];
+  sh.rng.pos = p + 5 < 31 ? p + 5 : p + 5 - 31;
+  sh.nw = 4;
+  sh.wrow[0] = u0; sh.wslot[0] = s0;
+  sh.wrow[1] = u1; sh.wslot[1] = s1;
+  sh.wrow[2] = v0; sh.wslot[2] = b0;
+  sh.wrow[3] = v1; sh.wslot[3] = b1;
+  ODP_Restore &r = sh.c.last;
+  r.u[0] = u0; r.u[1] = u1; r.v[0] = v0; r.v[1] = v1;
+  r.u_d[0] = s0; r.u_d[1] = s1; r.v_d[0] = b0; r.v_d[1] = b1;
+  return true;
+}
+
 /* Thread 0: the next swap into the shared adjacency; false when there is none.
  * The graph's record is a local copy: through shared memory every use of a
  * field would load it again, as the adjacency's stores might alias it. */
@@ -91,6 +152,7 @@ __device__ bool propose(ResidentShared &sh)
 {
   int e = 0;
   ODP_Restore last;
+  if(!sh.c.grid && sh.c.s == 1 && !sh.c.ndeg && propose_regular(sh)) return true;
   if(sh.c.grid){
     packed::mut_grid g = sh.gg;
     for(int attempt = 0; attempt < ANNEAL_MAX_ATTEMPTS && e == 0; attempt++) e = packed::mut_grid_two_opt(&sh.rng, &g, &last);

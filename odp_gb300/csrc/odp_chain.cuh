@@ -45,7 +45,19 @@ __device__ bool accept_move(gbx_chain &c, dev_rng *rng, int diameter, double asp
   if(aspl <= c.cur_aspl) return true;
   double diff = (c.cur_aspl - aspl) * c.n * (c.n - 1);
   if(c.s != 1) diff /= c.s;
-  const double u = ((double)rng_next(rng) + 1.0) / ((double)2147483647 + 2.0);
+  const int r = rng_next(rng);
+  /* In 32 bits first: the estimate of exp(diff / temp) is good to 1e-4 (the
+   * exponent, above -24, rounds by 4e-6, u by 1e-7), and below -24 the value is
+   * less than any u.  Only a u within 1e-3 of it needs the 64-bit form, whose
+   * divisions and exponential take 2k cycles. */
+  const float x = (float)diff / (float)c.temp, uf = ((float)r + 1.0f) * (1.0f / 2147483648.0f);
+  if(x < -24.0f) return false;
+  if(x <= 0.0f){
+    const float e = expf(x);
+    if(uf < e * 0.999f) return true;
+    if(uf > e * 1.001f) return false;
+  }
+  const double u = ((double)r + 1.0) / ((double)2147483647 + 2.0);
   return exp(diff / c.temp) > u;
 }
 
