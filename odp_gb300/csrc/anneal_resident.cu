@@ -12,8 +12,10 @@
  * the CTA's rows and one barrier per BFS level, and one decision.  Levels 1
  * and 2 come from the adjacency in shared memory (regular graphs without
  * symmetry; level 1 otherwise); later levels gather lanes as the lockstep
- * kernels do (sweep.cu).  Several teams run side by side in one cooperative
- * launch; every wait has a time limit.
+ * kernels do (sweep.cu).  Several teams run side by side.  A team of up to 16
+ * CTAs is a thread-block cluster: the counts go to every CTA's shared memory
+ * and a level's barrier is the cluster's.  Larger teams share one cooperative
+ * launch and meet in global memory; every wait there has a time limit.
  *
  * The moves, results and records are those of the stepwise kernels.
  */
@@ -21,11 +23,13 @@
 #include <climits>
 #include <cstdint>
 #include <cfloat>
+#include <cooperative_groups.h>
 #include "odp_engine.h"
 #include "odp_device.cuh"
 #include "odp_chain.cuh"
 
-#define RESIDENT_THREADS 256
+#define RESIDENT_THREADS GBX_RESIDENT_THREADS
+#define RESIDENT_CLUSTER GBX_RESIDENT_CLUSTER
 
 /* Rows marked at a time: 16 KB of them. */
 __host__ __device__ static inline int resident_block(int rows, int lanes)
@@ -57,7 +61,8 @@ struct ResidentShared {
   packed::mut_general g;
   packed::mut_grid gg;
   int nw, wrow[4], wslot[4];          /* the last swap's (or undo's) writes */
-  unsigned cnt, cnt1;                 /* this CTA's bits of the pass */
+  unsigned cnt[2], cnt1[2];           /* this CTA's bits of the pass, by the step's parity */
+  uint2 peer[2][RESIDENT_CLUSTER];    /* cluster: every CTA's cnt and cnt1, the same */
   unsigned long long bits, bits1;     /* the team's */
   int ok, accept, copy;
 };
@@ -186,10 +191,11 @@ __device__ void undo(ResidentShared &sh)
 
 /* The slots a swap or its undo wrote, into the CTA's lists (s orbit rows per
  * slot) and, by the team's first CTA, into the chain's adjacency. */
+template <int THREADS>
 __device__ void spread_writes(const ResidentShared &sh, const Resident &t)
 {
   const gbx_chain &c = sh.c;
-  for(int i = threadIdx.x; i < sh.nw * c.s; i += RESIDENT_THREADS){
+  for(int i = threadIdx.x; i < sh.nw * c.s; i += THREADS){
     const int k = i / c.s, turn = i - k * c.s;
     const int m = sh.wrow[k], slot = sh.wslot[k], a = t.adj[m * c.d + slot];
     int row, nb;
@@ -214,14 +220,33 @@ __device__ void spread_writes(const ResidentShared &sh, const Resident &t)
   }
 }
 
-/* The whole team passes: the level's bits from every CTA into sh.bits (and
- * level 1's into sh.bits1).  False past the limit. */
-__device__ bool team_pass(ResidentShared &sh, Resident &t, unsigned long long limit_ns, bool with_first = false)
+/* The whole team passes, with the level's bits of all CTAs (and level 1's, in
+ * the first pass of a step).  False past the limit (never in a cluster, whose
+ * barrier is the hardware's). */
+template <bool CLUSTER>
+__device__ bool team_pass(ResidentShared &sh, Resident &t, unsigned long long limit_ns, bool with_first,
+                          unsigned long long &bits, unsigned long long &bits1)
 {
+  const unsigned par = t.step & 1;
+  if(CLUSTER){
+    /* at most n * n < 2^32 bits */
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    __syncthreads();
+    if(threadIdx.x < t.size)
+      cl.map_shared_rank(&sh, threadIdx.x)->peer[par][t.rank] = make_uint2(sh.cnt[par], sh.cnt1[par]);
+    if(threadIdx.x == 0) sh.cnt[par ^ 1] = sh.cnt1[par ^ 1] = 0;     /* read before the last barrier */
+    t.step++;
+    cl.sync();
+    const unsigned lane = threadIdx.x & 31;
+    const uint2 c = lane < t.size ? sh.peer[par][lane] : make_uint2(0u, 0u);
+    bits = __reduce_add_sync(0xffffffffu, c.x);
+    bits1 = __reduce_add_sync(0xffffffffu, c.y);
+    return true;
+  }
   __syncthreads();
   if(threadIdx.x == 0){
-    const unsigned cnt = sh.cnt, cnt1 = sh.cnt1;
-    sh.cnt = sh.cnt1 = 0;
+    const unsigned cnt = sh.cnt[par], cnt1 = sh.cnt1[par];
+    sh.cnt[par] = sh.cnt1[par] = 0;
     sh.ok = 1;
     if(t.size == 1){
       sh.bits = cnt;
@@ -243,12 +268,15 @@ __device__ bool team_pass(ResidentShared &sh, Resident &t, unsigned long long li
   }
   t.step++;
   __syncthreads();
+  bits = sh.bits;
+  bits1 = sh.bits1;
   return sh.ok != 0;
 }
 
 /* Levels 1 and 2 (two) or level 1 of the CTA's rows, marked in shared memory
  * a block of rows at a time by all threads (a warp per row took 14k cycles of
  * latency for 64 rows of n = 1024, d = 8). */
+template <int THREADS>
 __device__ void first_rows(ResidentShared &sh, const Resident &t, bool two)
 {
   const gbx_chain &c = sh.c;
@@ -259,18 +287,18 @@ __device__ void first_rows(ResidentShared &sh, const Resident &t, bool two)
   for(int b0 = 0; b0 < t.nr; b0 += t.block){
     const int nb = min(t.block, t.nr - b0);
     uint4 *sv = reinterpret_cast<uint4 *>(t.scratch);
-    for(int i = tid; i < nb * t.lanes * 2; i += RESIDENT_THREADS) sv[i] = make_uint4(0u, 0u, 0u, 0u);
+    for(int i = tid; i < nb * t.lanes * 2; i += THREADS) sv[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     const int *ids = t.list + b0 * dp;
-    for(int i = tid; i < nb * dp; i += RESIDENT_THREADS) mark(t.scratch + (i / dp) * words, ids[i], c.base);
-    for(int r = tid; r < nb; r += RESIDENT_THREADS) mark(t.scratch + r * words, t.r0 + b0 + r, c.base);
+    for(int i = tid; i < nb * dp; i += THREADS) mark(t.scratch + (i / dp) * words, ids[i], c.base);
+    for(int r = tid; r < nb; r += THREADS) mark(t.scratch + r * words, t.r0 + b0 + r, c.base);
     __syncthreads();
     if(two){
-      for(int i = tid; i < nb * t.lanes * 2; i += RESIDENT_THREADS) n1 += popc4(sv[i]);
+      for(int i = tid; i < nb * t.lanes * 2; i += THREADS) n1 += popc4(sv[i]);
       __syncthreads();
       /* eight threads a row: entries part, part + 8, ... of its d * d */
       const int part = tid & 7;
-      for(int r = tid >> 3; r < nb; r += RESIDENT_THREADS / 8){
+      for(int r = tid >> 3; r < nb; r += THREADS / 8){
         unsigned *s = t.scratch + r * words;
         const int *row = ids + r * dp;
         for(int i0 = part; i0 < d * d; i0 += 64){          /* eight loaded before any is marked */
@@ -286,7 +314,7 @@ __device__ void first_rows(ResidentShared &sh, const Resident &t, bool two)
       }
       __syncthreads();
     }
-    for(int i = tid; i < nb * t.lanes; i += RESIDENT_THREADS){
+    for(int i = tid; i < nb * t.lanes; i += THREADS){
       const int r = i / t.lanes, p = i - r * t.lanes;
       unsigned w[8];
       *reinterpret_cast<uint4 *>(w) = sv[2 * i];
@@ -301,19 +329,20 @@ __device__ void first_rows(ResidentShared &sh, const Resident &t, bool two)
   n1 = __reduce_add_sync(0xffffffffu, n1);
   n2 = __reduce_add_sync(0xffffffffu, n2);
   if((tid & 31) == 0){
-    if(n1) atomicAdd(&sh.cnt1, n1);
-    if(n2) atomicAdd(&sh.cnt, n2);
+    if(n1) atomicAdd(&sh.cnt1[t.step & 1], n1);
+    if(n2) atomicAdd(&sh.cnt[t.step & 1], n2);
   }
 }
 
 /* A gathered level: a thread keeps its lane and walks the rows. */
+template <int THREADS>
 __device__ void next_rows(ResidentShared &sh, const Resident &t, int level)
 {
   const gbx_chain &c = sh.c;
   const unsigned rb = (unsigned)t.lanes * 32u;
   const size_t half = (size_t)c.n * rb;
   unsigned cnt = 0;
-  const int rr = threadIdx.x / t.lanes, rs = RESIDENT_THREADS / t.lanes;
+  const int rr = threadIdx.x / t.lanes, rs = THREADS / t.lanes;
   if(rr < rs){
     const int gl = threadIdx.x - rr * t.lanes;
     const unsigned bits = (unsigned)lane_bits(c.base, gl);
@@ -341,11 +370,12 @@ __device__ void next_rows(ResidentShared &sh, const Resident &t, int level)
     }
   }
   cnt = __reduce_add_sync(0xffffffffu, cnt);
-  if((threadIdx.x & 31) == 0 && cnt) atomicAdd(&sh.cnt, cnt);
+  if((threadIdx.x & 31) == 0 && cnt) atomicAdd(&sh.cnt[t.step & 1], cnt);
 }
 
 /* The graph's diameter (negative: some pair is unreachable) and ordered
  * distance sum, the same in every thread of the team; false past a wait's limit. */
+template <bool CLUSTER>
 __device__ bool evaluate(ResidentShared &sh, Resident &t, unsigned long long limit_ns, int &diameter, long long &sum)
 {
   const gbx_chain &c = sh.c;
@@ -368,14 +398,16 @@ __device__ bool evaluate(ResidentShared &sh, Resident &t, unsigned long long lim
     over = true;
     diameter = stalled ? -level : level;
   };
-  first_rows(sh, t, two);
-  if(!team_pass(sh, t, limit_ns, two)) return false;
-  if(two) settle(sh.bits1);
-  if(!over) settle(sh.bits);
+  constexpr int THREADS = CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESIDENT_THREADS;
+  first_rows<THREADS>(sh, t, two);
+  unsigned long long bits = 0, bits1 = 0;
+  if(!team_pass<CLUSTER>(sh, t, limit_ns, two, bits, bits1)) return false;
+  if(two) settle(bits1);
+  if(!over) settle(bits);
   while(!over){
-    next_rows(sh, t, level + 1);
-    if(!team_pass(sh, t, limit_ns)) return false;
-    settle(sh.bits);
+    next_rows<THREADS>(sh, t, level + 1);
+    if(!team_pass<CLUSTER>(sh, t, limit_ns, false, bits, bits1)) return false;
+    settle(bits);
   }
   return true;
 }
@@ -411,31 +443,34 @@ __device__ void decide(ResidentShared &sh, int level, long long total)
   c.temp *= c.cooling;
 }
 
-__global__ void __launch_bounds__(RESIDENT_THREADS, 2) anneal_resident_kernel(const gbx_resident p)
+template <bool CLUSTER>
+__global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESIDENT_THREADS, 2) anneal_resident_kernel(const gbx_resident p)
 {
   extern __shared__ __align__(16) unsigned char resident_smem[];
   __shared__ ResidentShared sh;
+  constexpr int THREADS = CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESIDENT_THREADS;
   const int tid = threadIdx.x, G = (int)gridDim.x;
-  /* team i: CTAs [i * G / teams, (i + 1) * G / teams) */
+  /* team i: CTAs [i * G / teams, (i + 1) * G / teams), a cluster of them */
   const int team = (int)((((long long)blockIdx.x + 1) * p.teams - 1) / G);
   const int lo = (int)((long long)team * G / p.teams), hi = (int)((long long)(team + 1) * G / p.teams);
   Resident t;
   t.rank = (int)blockIdx.x - lo;
   t.sync = reinterpret_cast<ResidentSync *>(p.sync) + team;
   t.step = 0;
+  if(CLUSTER) cooperative_groups::this_cluster().sync();   /* every CTA's shared memory is there */
   for(int chain = team; chain < p.count; chain += p.teams){
     __syncthreads();
     {
       const unsigned *src = reinterpret_cast<const unsigned *>(p.chains + chain);
       unsigned *dst = reinterpret_cast<unsigned *>(&sh.c);
-      for(int i = tid; i < (int)(sizeof(gbx_chain) / 4); i += RESIDENT_THREADS) dst[i] = src[i];
+      for(int i = tid; i < (int)(sizeof(gbx_chain) / 4); i += THREADS) dst[i] = src[i];
     }
     __syncthreads();
     const gbx_chain &c = sh.c;
     t.lanes = (c.base + 255) >> 8;
     /* a lane per thread is enough: more CTAs only lengthen the barrier */
-    const int want = (int)(((long long)c.n * t.lanes + RESIDENT_THREADS - 1) / RESIDENT_THREADS);
-    t.size = min(hi - lo, want);
+    const int want = (int)(((long long)c.n * t.lanes + THREADS - 1) / THREADS);
+    t.size = CLUSTER ? hi - lo : min(hi - lo, want);
     if(c.status || t.rank >= t.size) continue;           /* the same in the whole team / this CTA has no part */
     t.rows = (c.n + t.size - 1) / t.size;
     t.r0 = t.rank * t.rows;
@@ -446,12 +481,12 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, 2) anneal_resident_kernel(co
     t.block = resident_block(t.rows, t.lanes);
     t.adj = reinterpret_cast<unsigned short *>(t.scratch + t.block * t.lanes * 8);
     t.flag = reinterpret_cast<unsigned char *>(t.adj + ((c.base * c.d + 1) & ~1));
-    for(int i = tid; i < c.base * c.d; i += RESIDENT_THREADS) t.adj[i] = (unsigned short)__ldcg(c.adj + i);
-    for(int i = tid; i < t.nr * c.dp; i += RESIDENT_THREADS) t.list[i] = __ldcg(c.nbr + (size_t)t.r0 * c.dp + i);
+    for(int i = tid; i < c.base * c.d; i += THREADS) t.adj[i] = (unsigned short)__ldcg(c.adj + i);
+    for(int i = tid; i < t.nr * c.dp; i += THREADS) t.list[i] = __ldcg(c.nbr + (size_t)t.r0 * c.dp + i);
     if(tid < 31) sh.rng.ring[tid] = c.ring[tid];
     if(tid == 0){
       sh.rng.pos = c.ring_pos;
-      sh.cnt = sh.cnt1 = 0;
+      sh.cnt[0] = sh.cnt[1] = sh.cnt1[0] = sh.cnt1[1] = 0;
       sh.g.n = c.n; sh.g.d = c.d; sh.g.s = c.s; sh.g.base = c.base;
       sh.g.ndeg = c.ndeg; sh.g.adj = t.adj; sh.g.nw = 0;
       sh.gg.w = c.width; sh.gg.h = c.height; sh.gg.d = c.d; sh.gg.s = c.s; sh.gg.len = c.len; sh.gg.n = c.n;
@@ -459,7 +494,8 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, 2) anneal_resident_kernel(co
       sh.gg.ndeg = c.ndeg; sh.gg.adj = t.adj; sh.gg.xy = nullptr; sh.gg.nw = 0;
     }
     /* every CTA has its copy of the adjacency before the first one writes to it */
-    if(!team_pass(sh, t, p.limit_ns)){
+    unsigned long long bits, bits1;
+    if(!team_pass<CLUSTER>(sh, t, p.limit_ns, false, bits, bits1)){
       if(tid == 0) sh.c.status = GBX_CHAIN_ERR_EVAL;
       __syncthreads();
     }
@@ -471,11 +507,11 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, 2) anneal_resident_kernel(co
         __syncthreads();
         break;
       }
-      spread_writes(sh, t);
+      spread_writes<THREADS>(sh, t);
       __syncthreads();
       int level = 0;
       long long sum = 0;
-      if(!evaluate(sh, t, p.limit_ns, level, sum)){
+      if(!evaluate<CLUSTER>(sh, t, p.limit_ns, level, sum)){
         if(tid == 0) sh.c.status = GBX_CHAIN_ERR_EVAL;
         __syncthreads();
         break;
@@ -483,25 +519,25 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, 2) anneal_resident_kernel(co
       if(tid == 0) decide(sh, level, sum);
       __syncthreads();
       if(sh.copy && t.rank == 0)
-        for(int i = tid; i < c.base * c.d; i += RESIDENT_THREADS) c.best_adj[i] = __ldcg(c.adj + i);
+        for(int i = tid; i < c.base * c.d; i += THREADS) c.best_adj[i] = __ldcg(c.adj + i);
       if(!sh.accept){
         __syncthreads();                                 /* the copy has read the adjacency before the undo */
         if(tid == 0) undo(sh);
         __syncthreads();
-        spread_writes(sh, t);
+        spread_writes<THREADS>(sh, t);
         __syncthreads();
       }
     }
     /* the records and the neighbour table, for the host and the next launch */
     __syncthreads();
-    for(int i = tid; i < t.nr * c.dp; i += RESIDENT_THREADS) c.nbr[(size_t)t.r0 * c.dp + i] = t.list[i];
+    for(int i = tid; i < t.nr * c.dp; i += THREADS) c.nbr[(size_t)t.r0 * c.dp + i] = t.list[i];
     if(t.rank == 0){
       if(tid < 31) sh.c.ring[tid] = sh.rng.ring[tid];
       if(tid == 0) sh.c.ring_pos = sh.rng.pos;
       __syncthreads();
       unsigned *dst = reinterpret_cast<unsigned *>(p.chains + chain);
       const unsigned *src = reinterpret_cast<const unsigned *>(&sh.c);
-      for(int i = tid; i < (int)(sizeof(gbx_chain) / 4); i += RESIDENT_THREADS) dst[i] = src[i];
+      for(int i = tid; i < (int)(sizeof(gbx_chain) / 4); i += THREADS) dst[i] = src[i];
     }
   }
 }
@@ -522,28 +558,59 @@ int gbx_resident_blocks(size_t smem, int *per_sm)
 {
   *per_sm = 0;
   if(smem > GBX_SWEEP_SMEM_MAX) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute((const void *)anneal_resident_kernel,
+  cudaError_t e = cudaFuncSetAttribute((const void *)anneal_resident_kernel<false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, GBX_SWEEP_SMEM_MAX);
   if(e != cudaSuccess) return (int)e;
-  return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, (const void *)anneal_resident_kernel,
+  return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, (const void *)anneal_resident_kernel<false>,
                                                             RESIDENT_THREADS, smem);
 }
 
-int gbx_resident_launch(const gbx_resident *r, int blocks, size_t smem, void *stream)
+static void resident_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, int blocks, size_t smem, int cluster)
 {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cudaLaunchConfig_t cfg = {};
+  if(cluster){
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  }
+  else{
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  }
   cfg.gridDim = dim3((unsigned)blocks, 1, 1);
-  cfg.blockDim = dim3(RESIDENT_THREADS, 1, 1);
+  cfg.blockDim = dim3(cluster ? GBX_RESIDENT_CLUSTER_THREADS : RESIDENT_THREADS, 1, 1);
   cfg.dynamicSmemBytes = smem;
-  cfg.stream = (cudaStream_t)stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+}
+
+int gbx_resident_clusters(int cluster, size_t smem, int *active)
+{
+  *active = 0;
+  if(smem > GBX_SWEEP_SMEM_MAX || cluster > RESIDENT_CLUSTER) return (int)cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute((const void *)anneal_resident_kernel<true>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, GBX_SWEEP_SMEM_MAX);
+  if(e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void *)anneal_resident_kernel<true>,
+                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if(e != cudaSuccess) return (int)e;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = {};
+  resident_config(cfg, attr, cluster, smem, cluster);
+  e = cudaOccupancyMaxActiveClusters(active, (const void *)anneal_resident_kernel<true>, &cfg);
+  if(e != cudaSuccess) cudaGetLastError();
+  return (int)e;
+}
+
+int gbx_resident_launch(const gbx_resident *r, int blocks, size_t smem, int cluster, void *stream)
+{
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = {};
+  resident_config(cfg, attr, blocks, smem, cluster);
+  cfg.stream = (cudaStream_t)stream;
   gbx_resident arg = *r;
   void *args[1] = { &arg };
-  return (int)cudaLaunchKernelExC(&cfg, (const void *)anneal_resident_kernel, args);
+  return (int)cudaLaunchKernelExC(&cfg, cluster ? (const void *)anneal_resident_kernel<true>
+                                                : (const void *)anneal_resident_kernel<false>, args);
 }
 
 }  /* extern "C" */

@@ -35,7 +35,7 @@ struct odpx_anneal {
   void *steps_exec;            /* ANNEAL_GRAPH_STEPS steps captured as one CUDA graph */
   int resident;                /* the steps run in the resident kernel */
   gbx_resident res;
-  int res_blocks;
+  int res_blocks, res_cluster;
   size_t res_smem;
   void *d_res;                 /* its barrier words, bitset offsets and bitsets */
 };
@@ -84,13 +84,44 @@ void ODPX_Anneal_destroy(ODPX_Anneal *a)
   free(a);
 }
 
+/* CTAs of a cluster for every chain, or 0 for teams in a cooperative launch.  A
+ * cluster's barrier takes 0.6 us, the one in global memory 2.4; but a level
+ * on fewer CTAs takes longer than that saves, so a cluster has at least 7/8 of
+ * the grid's share of a chain (`range` CTAs) or a lane per thread (`lanes` in
+ * all), and every chain's runs at once.  Measured on GB300, teams against
+ * clusters, us a step: 32 chains of n = 300, d = 6: 14.7 / 11.8; 25 of n = 700,
+ * d = 16: 17.8 / 16.3; 16 of n = 1024, d = 8: 16.0 / 15.1 (13 CTAs); 4 of them:
+ * 16 / 12.  With too few CTAs, 16 of n = 2048, d = 8: 34 / 39 (13 of 19). */
+static int resident_cluster(const ODPX_Anneal *a, int range, long long lanes, size_t *smem_out)
+{
+  const odp_plan *p = a->p;
+  const long long enough = (lanes + GBX_RESIDENT_CLUSTER_THREADS - 1) / GBX_RESIDENT_CLUSTER_THREADS;
+  const long long want = (lanes + GBX_RESIDENT_THREADS - 1) / GBX_RESIDENT_THREADS;
+  const int share = (range * 7 + 7) / 8, least = enough < share ? (int)enough : share;
+  for(int c = want < range ? (int)want : range; c >= least && c >= 2; c--){
+    size_t smem = 0;
+    int active = 0;
+    if(c > GBX_RESIDENT_CLUSTER) continue;
+    for(int i = 0; i < a->count; i++){
+      const odp_plan_graph *g = &p->g[i];
+      const size_t s = gbx_resident_smem((g->n + c - 1) / c, g->dp, g->B, g->d);
+      if(s > smem) smem = s;
+    }
+    if(gbx_resident_clusters(c, smem, &active) == 0 && active >= a->count){
+      *smem_out = smem;
+      return c;
+    }
+  }
+  return 0;
+}
+
 /* Whether every chain fits the resident kernel: 16-bit vertices, and the
  * compact adjacency beside a CTA's share of the rows in shared memory.  The
  * teams share two CTAs per SM, or one where two do not fit; a part of the GPU
  * (ODP_GB300_BLOCKS, in engine CTAs, four per SM) becomes the same part of
  * them.  Measured on GB300 against four launches per step (us): 16 chains of
- * n = 1024, d = 8: 20 / 68; one of them: 18 / 48; 8 of n = 4096, d = 16: 90 /
- * 137; 32 of n = 300, d = 6: 18 / 64.  Allocates its memory; 0 if the chains
+ * n = 1024, d = 8: 15 / 68; one of them: 12 / 48; 8 of n = 4096, d = 16: 85 /
+ * 137; 32 of n = 300, d = 6: 12 / 64.  Allocates its memory; 0 if the chains
  * do not fit. */
 static int plan_resident(ODPX_Anneal *a, int blocks)
 {
@@ -104,6 +135,7 @@ static int plan_resident(ODPX_Anneal *a, int blocks)
     const int teams = a->count < grid ? a->count : grid, range = grid / teams;
     size_t smem = 0;
     unsigned long long words = 0;
+    long long most = 1;
     for(int i = 0; i < a->count; i++){
       const odp_plan_graph *g = &p->g[i];
       const long long lanes = (g->B + 255) / 256, want = ((long long)g->n * lanes + 255) / 256;
@@ -111,9 +143,11 @@ static int plan_resident(ODPX_Anneal *a, int blocks)
       const size_t s = gbx_resident_smem((g->n + size - 1) / size, g->dp, g->B, g->d);
       if(g->n > 65535 || lanes > 256) return 0;
       if(s > smem) smem = s;
+      if(g->n * lanes > most) most = g->n * lanes;
       words += 8ull * (unsigned long long)g->n * (unsigned long long)lanes;   /* two buffers, 4 words a lane */
     }
     if(gbx_resident_blocks(smem, &fit) || fit < per_sm) continue;
+    a->res_cluster = resident_cluster(a, range, most, &smem);
     const size_t sync = gbx_resident_sync_bytes() * (size_t)teams, offs = (sizeof(unsigned long long) * (size_t)a->count + 255) & ~(size_t)255;
     unsigned long long *off = malloc(sizeof(unsigned long long) * (size_t)a->count), at = 0;
     if(!off || gbx_malloc(&a->d_res, sync + offs + 8 * words)){
@@ -132,7 +166,7 @@ static int plan_resident(ODPX_Anneal *a, int blocks)
     a->res.limit_ns = p->spin_limit_ns;
     a->res.count = a->count;
     a->res.teams = teams;
-    a->res_blocks = grid;
+    a->res_blocks = a->res_cluster ? teams * a->res_cluster : grid;
     a->res_smem = smem;
     const int e = gbx_memcpy_h2d((void *)a->res.buf_offset, off, sizeof(unsigned long long) * (size_t)a->count, p->stream) ||
                   gbx_stream_sync(p->stream);
@@ -265,8 +299,9 @@ int ODPX_Anneal_run(ODPX_Anneal *a, int steps)
   if(a->resident){
     for(; s < steps; s += a->res.steps){
       a->res.steps = steps - s < RESIDENT_STEPS ? steps - s : RESIDENT_STEPS;
-      if(gbx_memset(a->res.sync, 0, gbx_resident_sync_bytes() * (size_t)a->res.teams, p->stream) ||
-         gbx_resident_launch(&a->res, a->res_blocks, a->res_smem, p->stream))
+      if((!a->res_cluster &&
+          gbx_memset(a->res.sync, 0, gbx_resident_sync_bytes() * (size_t)a->res.teams, p->stream)) ||
+         gbx_resident_launch(&a->res, a->res_blocks, a->res_smem, a->res_cluster, p->stream))
         return ODPX_ERR_CUDA;
     }
     return gbx_stream_sync(p->stream) ? ODPX_ERR_CUDA : 0;

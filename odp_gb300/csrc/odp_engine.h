@@ -309,10 +309,13 @@ int  gbx_anneal_propose(gbx_chain *d_chains, int count, void *stream);
 int  gbx_anneal_decide(gbx_chain *d_chains, int count, const gbx_graph_acc *d_acc, const gbx_ctrl *d_ctrl,
                        const unsigned int *d_err, void *stream);
 
-/* Many steps of every running chain in one cooperative launch
- * (anneal_resident.cu), for chains whose compact adjacency fits a CTA's shared
- * memory as 16-bit vertices.  Chain k belongs to team k % teams; the teams
- * share the grid evenly. */
+/* Many steps of every running chain in one launch (anneal_resident.cu), for
+ * chains whose compact adjacency fits a CTA's shared memory as 16-bit
+ * vertices.  Chain k belongs to team k % teams; the teams share the grid
+ * evenly, in a cooperative launch, or each is a cluster. */
+#define GBX_RESIDENT_THREADS 256       /* of a CTA in a cooperative launch */
+#define GBX_RESIDENT_CLUSTER_THREADS 320
+#define GBX_RESIDENT_CLUSTER 16        /* CTAs of a cluster, at most */
 typedef struct {
   gbx_chain *chains;
   char *buf;                   /* bitsets: chain k's two buffers at buf + buf_offset[k] */
@@ -325,7 +328,10 @@ size_t gbx_resident_sync_bytes(void);
 /* Shared memory of a CTA that holds `rows` rows of a chain. */
 size_t gbx_resident_smem(int rows, int dp, int base, int d);
 int  gbx_resident_blocks(size_t smem, int *per_sm);
-int  gbx_resident_launch(const gbx_resident *r, int blocks, size_t smem, void *stream);
+/* Clusters of that many CTAs that the GPU holds at once (0: none). */
+int  gbx_resident_clusters(int cluster, size_t smem, int *active);
+/* cluster: CTAs of a team, all teams alike, or 0 for a cooperative launch. */
+int  gbx_resident_launch(const gbx_resident *r, int blocks, size_t smem, int cluster, void *stream);
 
 #ifdef __cplusplus
 }
