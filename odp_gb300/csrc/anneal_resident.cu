@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
     /* a lane per thread is enough: more CTAs only lengthen the barrier */
     const int want = (int)(((long long)c.n * t.lanes + THREADS - 1) / THREADS);
     t.size = CLUSTER ? hi - lo : min(hi - lo, want);
-    if(c.status || t.rank >= t.size) continue;           /* the same in the whole team / this CTA has no part */
+    if(t.rank >= t.size) continue;                       /* this CTA has no part */
     t.rows = (c.n + t.size - 1) / t.size;
     t.r0 = t.rank * t.rows;
     t.nr = max(0, min(t.rows, c.n - t.r0));
@@ -528,16 +528,31 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
         __syncthreads();
       }
     }
-    /* the records and the neighbour table, for the host and the next launch */
+    /* the records and the neighbour table, for the host and the next launch;
+     * after a run the chain also goes to host memory, a part from each CTA:
+     * three copies and a synchronise per chain took 40 us */
+    if(p.host_chains && sh.c.status != GBX_CHAIN_ERR_EVAL) team_pass<CLUSTER>(sh, t, p.limit_ns, false, bits, bits1);
     __syncthreads();
+    if(p.host_chains){
+      const int ints = c.base * c.d;
+      int *to = p.host_graphs + p.host_offset[chain];
+      for(int i = t.rank * THREADS + tid; i < ints; i += t.size * THREADS){
+        to[i] = __ldcg(c.adj + i);
+        to[ints + i] = __ldcg(c.best_adj + i);
+      }
+    }
     for(int i = tid; i < t.nr * c.dp; i += THREADS) c.nbr[(size_t)t.r0 * c.dp + i] = t.list[i];
     if(t.rank == 0){
       if(tid < 31) sh.c.ring[tid] = sh.rng.ring[tid];
       if(tid == 0) sh.c.ring_pos = sh.rng.pos;
       __syncthreads();
       unsigned *dst = reinterpret_cast<unsigned *>(p.chains + chain);
+      unsigned *host = reinterpret_cast<unsigned *>(p.host_chains + chain);
       const unsigned *src = reinterpret_cast<const unsigned *>(&sh.c);
-      for(int i = tid; i < (int)(sizeof(gbx_chain) / 4); i += THREADS) dst[i] = src[i];
+      for(int i = tid; i < (int)(sizeof(gbx_chain) / 4); i += THREADS){
+        dst[i] = src[i];
+        if(p.host_chains) host[i] = src[i];
+      }
     }
   }
 }

@@ -25,6 +25,7 @@
 
 #define ANNEAL_GRAPH_STEPS 8   /* steps per replayed CUDA graph */
 #define RESIDENT_STEPS 512     /* steps per launch of the resident kernel */
+#define RESIDENT_HOST (64 << 20) /* pinned bytes of a group's records and graphs, at most */
 
 struct odpx_anneal {
   odp_plan *p;
@@ -37,7 +38,11 @@ struct odpx_anneal {
   gbx_resident res;
   int res_blocks, res_cluster;
   size_t res_smem;
-  void *d_res;                 /* its barrier words, bitset offsets and bitsets */
+  void *d_res;                 /* its barrier words, bitset and host offsets and bitsets */
+  char *h_res;                 /* pinned: the chains' records and graphs after a run, or NULL */
+  gbx_chain *dh_chains;
+  int h_current;               /* they are the chains' state */
+  unsigned long long *h_offset; /* in ints, chain k's graphs among them */
 };
 
 /* ODP_GB300_ANNEAL_RESIDENT=0 keeps the stepwise kernels. */
@@ -79,6 +84,8 @@ void ODPX_Anneal_destroy(ODPX_Anneal *a)
   if(a->steps_exec) gbx_graph_destroy(a->steps_exec);
   if(a->p) odp_plan_destroy(a->p);
   gbx_free(a->d_res);
+  gbx_host_free(a->h_res);
+  free(a->h_offset);
   gbx_free(a->d_chains); gbx_free(a->d_best); gbx_free(a->d_rowdeg); gbx_free(a->d_state_init);
   free(a->h_chains);
   free(a);
@@ -134,7 +141,7 @@ static int plan_resident(ODPX_Anneal *a, int blocks)
     if(grid > sms * per_sm) grid = sms * per_sm;
     const int teams = a->count < grid ? a->count : grid, range = grid / teams;
     size_t smem = 0;
-    unsigned long long words = 0;
+    unsigned long long words = 0, ints = 0;
     long long most = 1;
     for(int i = 0; i < a->count; i++){
       const odp_plan_graph *g = &p->g[i];
@@ -145,32 +152,39 @@ static int plan_resident(ODPX_Anneal *a, int blocks)
       if(s > smem) smem = s;
       if(g->n * lanes > most) most = g->n * lanes;
       words += 8ull * (unsigned long long)g->n * (unsigned long long)lanes;   /* two buffers, 4 words a lane */
+      ints += 2ull * (unsigned long long)g->B * (unsigned long long)g->d;
     }
     if(gbx_resident_blocks(smem, &fit) || fit < per_sm) continue;
     a->res_cluster = resident_cluster(a, range, most, &smem);
     const size_t sync = gbx_resident_sync_bytes() * (size_t)teams, offs = (sizeof(unsigned long long) * (size_t)a->count + 255) & ~(size_t)255;
-    unsigned long long *off = malloc(sizeof(unsigned long long) * (size_t)a->count), at = 0;
-    if(!off || gbx_malloc(&a->d_res, sync + offs + 8 * words)){
+    unsigned long long *off = calloc(1, 2 * offs), at = 0, to = 0;
+    if(!off || gbx_malloc(&a->d_res, sync + 2 * offs + 8 * words)){
       free(off);
       a->d_res = NULL;
       return 0;
     }
     for(int i = 0; i < a->count; i++){
-      off[i] = at;
+      off[i] = to;
+      off[offs / sizeof(off[0]) + (size_t)i] = at;
       at += 64ull * (unsigned long long)p->g[i].n * (unsigned long long)((p->g[i].B + 255) / 256);
+      to += 2ull * (unsigned long long)p->g[i].B * (unsigned long long)p->g[i].d;
     }
     a->res.chains = a->d_chains;
     a->res.sync = a->d_res;
-    a->res.buf_offset = (const unsigned long long *)((char *)a->d_res + sync);
-    a->res.buf = (char *)a->d_res + sync + offs;
+    a->res.host_offset = (const unsigned long long *)((char *)a->d_res + sync);
+    a->res.buf_offset = (const unsigned long long *)((char *)a->d_res + sync + offs);
+    a->res.buf = (char *)a->d_res + sync + 2 * offs;
     a->res.limit_ns = p->spin_limit_ns;
     a->res.count = a->count;
     a->res.teams = teams;
     a->res_blocks = a->res_cluster ? teams * a->res_cluster : grid;
     a->res_smem = smem;
-    const int e = gbx_memcpy_h2d((void *)a->res.buf_offset, off, sizeof(unsigned long long) * (size_t)a->count, p->stream) ||
-                  gbx_stream_sync(p->stream);
-    free(off);
+    const size_t recs = sizeof(gbx_chain) * (size_t)a->count;
+    if(recs + sizeof(int) * ints <= RESIDENT_HOST && gbx_host_alloc((void **)&a->h_res, recs + sizeof(int) * ints) == 0 &&
+       gbx_host_device_ptr(a->h_res, (void **)&a->dh_chains) == 0)
+      a->res.host_graphs = (int *)((char *)a->dh_chains + recs);
+    const int e = gbx_memcpy_h2d((char *)a->d_res + sync, off, 2 * offs, p->stream) || gbx_stream_sync(p->stream);
+    a->h_offset = off;
     return !e;
   }
   return 0;
@@ -297,14 +311,19 @@ int ODPX_Anneal_run(ODPX_Anneal *a, int steps)
   odp_plan *p = a->p;
   int s = 0;
   if(a->resident){
+    const int host = a->res.host_graphs && steps > 0;
+    if(steps > 0) a->h_current = 0;
     for(; s < steps; s += a->res.steps){
       a->res.steps = steps - s < RESIDENT_STEPS ? steps - s : RESIDENT_STEPS;
+      a->res.host_chains = host && s + a->res.steps == steps ? a->dh_chains : NULL;
       if((!a->res_cluster &&
           gbx_memset(a->res.sync, 0, gbx_resident_sync_bytes() * (size_t)a->res.teams, p->stream)) ||
          gbx_resident_launch(&a->res, a->res_blocks, a->res_smem, a->res_cluster, p->stream))
         return ODPX_ERR_CUDA;
     }
-    return gbx_stream_sync(p->stream) ? ODPX_ERR_CUDA : 0;
+    if(gbx_stream_sync(p->stream)) return ODPX_ERR_CUDA;
+    a->h_current |= host;
+    return 0;
   }
   if(steps >= ANNEAL_GRAPH_STEPS){
     /* full groups of steps replay one captured graph: a launch per group
@@ -326,28 +345,42 @@ int ODPX_Anneal_run(ODPX_Anneal *a, int steps)
   return gbx_stream_sync(p->stream) ? ODPX_ERR_CUDA : 0;
 }
 
+static void fill_state(const gbx_chain *c, ODPX_Chain_state *st)
+{
+  if(!st) return;
+  st->steps = c->steps;
+  st->accepted = c->accepted;
+  st->status = c->status;
+  st->diameter = c->cur_diameter;
+  st->sum = (long)c->cur_sum;
+  st->aspl = c->cur_aspl;
+  st->best_diameter = c->best_diameter;
+  st->best_sum = (long)c->best_sum;
+  st->best_aspl = c->best_aspl;
+  st->temp = c->temp;
+}
+
 int ODPX_Anneal_state(ODPX_Anneal *a, int chain, ODPX_Chain_state *st, int *adjacency, int *best_adjacency)
 {
   if(!a || chain < 0 || chain >= a->count) return ODPX_ERR_INVALID;
   odp_plan *p = a->p;
   gbx_chain *c = &a->h_chains[chain];
+  if(a->h_current){
+    const gbx_chain *now = (const gbx_chain *)a->h_res + chain;
+    const int *graphs = (const int *)((const gbx_chain *)a->h_res + a->count) + a->h_offset[chain];
+    const size_t ints = (size_t)now->base * now->d;
+    *c = *now;
+    if(adjacency) memcpy(adjacency, graphs, sizeof(int) * ints);
+    if(best_adjacency) memcpy(best_adjacency, graphs + ints, sizeof(int) * ints);
+    fill_state(c, st);
+    return 0;
+  }
   if(gbx_memcpy_d2h(c, a->d_chains + chain, sizeof(gbx_chain), p->stream)) return ODPX_ERR_CUDA;
   size_t words = (size_t)c->base * c->d;
   if(adjacency && gbx_memcpy_d2h(adjacency, c->adj, sizeof(int) * words, p->stream)) return ODPX_ERR_CUDA;
   if(best_adjacency && gbx_memcpy_d2h(best_adjacency, c->best_adj, sizeof(int) * words, p->stream))
     return ODPX_ERR_CUDA;
   if(gbx_stream_sync(p->stream)) return ODPX_ERR_CUDA;
-  if(st){
-    st->steps = c->steps;
-    st->accepted = c->accepted;
-    st->status = c->status;
-    st->diameter = c->cur_diameter;
-    st->sum = (long)c->cur_sum;
-    st->aspl = c->cur_aspl;
-    st->best_diameter = c->best_diameter;
-    st->best_sum = (long)c->best_sum;
-    st->best_aspl = c->best_aspl;
-    st->temp = c->temp;
-  }
+  fill_state(c, st);
   return 0;
 }

@@ -323,6 +323,9 @@ typedef struct {
   void *sync;                  /* gbx_resident_sync_bytes() per team, zeroed before the launch */
   unsigned long long limit_ns; /* longest wait of a CTA for its team */
   int count, teams, steps;
+  gbx_chain *host_chains;      /* device address of pinned memory that takes the records, or NULL */
+  int *host_graphs;            /* and the graphs: chain k's adj, then its best_adj, at host_offset[k] */
+  const unsigned long long *host_offset;
 } gbx_resident;
 size_t gbx_resident_sync_bytes(void);
 /* Shared memory of a CTA that holds `rows` rows of a chain. */
