@@ -205,6 +205,7 @@ int  gbx_small_prepare(void);
 #define GBX_SWEEP_PHASES 2
 #define GBX_SWEEP_CHUNKS 512           /* chunks of a graph, at most */
 #define GBX_SWEEP_SMEM_MAX (200 * 1024)
+#define GBX_SWEEP_BASE 10              /* levels from the lists, at most */
 #define GBX_SWEEP_TWO_LEVEL 64         /* widest row (entries) whose neighbours' lists are read for level 2 */
 #define GBX_SWEEP_TRACK_DEGREE 32      /* widest row of the tracking kernel */
 typedef struct {
@@ -224,8 +225,9 @@ typedef struct {
   int track;                   /* grids: rows in spatial order, only changed lanes are visited */
   int word_log2;               /* track: log2 of the changed words per row */
   int wide;                    /* two CTAs per SM with more loads in flight each */
-  int two_level;               /* levels 1 and 2 from the neighbour lists */
+  int base;                    /* levels from the neighbour lists: 1, 2 or, without symmetry, up to GBX_SWEEP_BASE */
   int scratch_bits;            /* sources a warp marks at a time (a multiple of 8192, or all of them) */
+  int scratch_rows, queue;     /* warps that mark; vertices in a warp's queue (base > 2) */
   int in_place;                /* the lists are built from the host array itself */
   int set;                     /* which half of `sync`: alternate it from launch to launch */
   unsigned int seq;            /* the launch's number, for the records */

@@ -453,6 +453,38 @@ static int small_yields(const odp_shape *sh, const odp_tuning *t, int part, int 
   return jobs * 4.0 * (shape_n(sh) / sh->symmetries) * sh->degree > 450e3;
 }
 
+/* How many levels of a general graph come from its neighbour lists (at least
+ * `base`, 1 or 2; `chunks` bounds the counters) and the scratch that takes.  A
+ * gathered level reads d + 1 lanes per row and 256 sources.  A level from the
+ * lists marks d (d - 1)^(k - 1) vertices a row and queued all before them, at
+ * about 0.7 of a lane each, and saves a barrier.  Measured on GB300, two levels
+ * against more (us): n = 65536, d = 16 (3 levels) 1656 / 1350; d = 6 (4) 2019 /
+ * 1547, 5 levels 1818; d = 3 (8) 3440 / 2528, 10 levels 3020; d = 20 (3) 1616 /
+ * 1548; d = 24 1796, 3 levels 2077; n = 30000, d = 8 (3) 374 / 320, 4 levels 343;
+ * n = 16384, d = 4 (5) 152 / 135; d = 12 115, 3 levels 117. */
+static void choose_start(const odp_shape *sh, int base, int chunks, gbx_sweep *c)
+{
+  const int n = shape_n(sh), d = sh->degree;
+  const double gathered = (d + 1.0) * ((c->B + 255) / 256);
+  c->base = base;
+  c->scratch_rows = 8;
+  c->scratch_bits = c->B <= 32768 ? (c->B + 255) / 256 * 256 : 32768;
+  if(base < 2 || sh->symmetries > 1 || n > 131072) return;
+  double marks = d * (d - 1.0);
+  int queue = 1 + d;
+  while(c->base < GBX_SWEEP_BASE && marks * d + queue <= 1.45 * gathered + 64.0 &&
+        (c->base + 1) * c->nchunks <= 2 * chunks){
+    queue += (int)marks;
+    marks *= d - 1.0;
+    c->base++;
+  }
+  if(c->base == 2) return;
+  c->queue = (queue + 3) / 4 * 4;
+  c->scratch_bits = (n + 255) / 256 * 256;
+  const int row = c->scratch_bits / 8 + 4 * c->queue;    /* four CTAs per SM */
+  while(c->scratch_rows > 1 && c->scratch_rows * row > 36 * 1024) c->scratch_rows--;
+}
+
 /* Whether no schedule setting asks for the persistent engine. */
 static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
 {
@@ -491,9 +523,7 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
   sw->B = n / sh->symmetries;
   sw->phases = 1;
   sw->track = sh->grid && sw->e.dp <= GBX_SWEEP_TRACK_DEGREE;
-  sw->two_level = sw->e.dp <= GBX_SWEEP_TWO_LEVEL;
   sw->in_place = !sh->grid && sh->symmetries == 1 && (double)n * sh->degree * 4 <= 1e6;
-  sw->scratch_bits = sw->B <= 32768 ? (sw->B + 255) / 256 * 256 : 32768;
   if(sw->track){
     sw->wc_log2 = full_l2 < 5 ? full_l2 : 5;
     sw->slots = (W + (1 << sw->wc_log2) - 1) >> sw->wc_log2;
@@ -517,6 +547,7 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
     sw->wc_log2 = wl;
   }
   sw->nchunks = (W + (1 << sw->wc_log2) - 1) >> sw->wc_log2;
+  if(!sw->track) choose_start(sh, sw->e.dp <= GBX_SWEEP_TWO_LEVEL ? 2 : 1, GBX_SWEEP_CHUNKS, sw);
   if(sw->nchunks > GBX_SWEEP_CHUNKS) return 0;
   for(int per_sm = sw->track || sw->wide ? 2 : 4; per_sm >= 1; per_sm--)
     for(int q = sw->slots; q >= 1; q = q > 1 ? (q + 1) / 2 : 0){
@@ -555,10 +586,9 @@ int odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_t
   c->phases = 1;
   c->track = sh->grid && c->e.dp <= GBX_SWEEP_TRACK_DEGREE;
   if(!c->track && W > 256) return 0;
-  c->two_level = c->e.dp <= GBX_SWEEP_TWO_LEVEL && 8.0 * W * sh->degree > 5000;
-  c->scratch_bits = (c->B + 255) / 256 * 256;
   c->wc_log2 = c->track ? (full_l2 < 5 ? full_l2 : 5) : (full_l2 < 6 ? full_l2 : 6);
   c->nchunks = c->slots = (W + (1 << c->wc_log2) - 1) >> c->wc_log2;
+  if(!c->track) choose_start(sh, c->e.dp <= GBX_SWEEP_TWO_LEVEL && 8.0 * W * sh->degree > 5000 ? 2 : 1, GBX_SWEEP_SLOTS, c);
   while((32 << c->word_log2) < (c->slots << (c->wc_log2 - 2))) c->word_log2++;
   const double lanes = (c->B + 255) / 256;
   if(c->track){
@@ -1064,7 +1094,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
         w->start_stride = p->slot_words;
       }
       else{                            /* the buffer that the first gathered level reads */
-        w->start = p->d_slotbuf + (w->two_level ? 0 : p->slot_words);
+        w->start = p->d_slotbuf + ((w->base & 1) ? p->slot_words : 0);
         w->start_stride = 2 * p->slot_words;
       }
       w->sync = p->d_sync;

@@ -48,7 +48,7 @@ struct SyncT {
   unsigned pad[28];
   unsigned long long arrive[PH][3][16];              /* step t's barrier word: [t % 3][0] */
   unsigned long long count[PH][3][SWEEP_SLOTS];      /* bits per chunk of step t */
-  unsigned long long start1[CH], start2[CH];         /* bits at levels 1 and 2 */
+  unsigned long long start[2 * CH];                  /* bits per chunk at levels 1 to `base`: [base][nchunks] */
 };
 typedef SyncT<GBX_SWEEP_PHASES, GBX_SWEEP_CHUNKS> SweepSync;
 
@@ -349,7 +349,7 @@ __device__ void start_rows(const gbx_sweep &a, const int *list, unsigned *scratc
       __syncwarp();
       for(int i = lane; i <= dp; i += 32) mark(s, (i < dp ? ids[i] : r0 + r) - base, sub);
       __syncwarp();
-      if(a.two_level){
+      if(a.base == 2){
         for(int p0 = 0; p0 < pieces; p0 += 32){          /* level 1's counts */
           const int p = p0 + lane;
           unsigned v = 0;
@@ -396,6 +396,144 @@ __device__ void start_rows(const gbx_sweep &a, const int *list, unsigned *scratc
       }
       __syncwarp();                                      /* the scratch row is read before it is cleared again */
     }
+  }
+}
+
+/* Levels 1 to `base` > 2 of every chunk, a warp per row: a search from the row
+ * over the neighbour table, the vertices reached as bits in the warp's scratch
+ * row and in its queue.  A gathered level reads d whole rows a row however few
+ * bits they hold: for n = 65536, d = 16 level 3 took 500 us gathered and takes
+ * 190 from the lists.  The counts of the levels before the last are of
+ * vertices added.  A vertex list longer than the queue (its size is that of
+ * symmetric lists) goes on from the bits: each lane keeps a copy of its
+ * pieces in the row's place in memory and expands what was there. */
+__device__ void ball_rows(const gbx_sweep &a, const int *list, unsigned *scratch, unsigned *cnt, int r0, int nr)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lL = a.wc_log2 - 2, L = 1 << lL;
+  const int dp = a.e.dp, n = a.e.n, last = a.base;
+  const int q4 = dp >> 2, magic = (65536 + q4 - 1) / q4;
+  const int words = a.scratch_bits >> 5, pieces = a.scratch_bits >> 8;
+  if(warp >= a.scratch_rows) return;
+  unsigned *s = scratch + (size_t)warp * (words + a.queue);
+  int *queue = reinterpret_cast<int *>(s + words);
+  uint4 *sv = reinterpret_cast<uint4 *>(s);
+  const unsigned below = (1u << lane) - 1u;
+  for(int r = warp; r < nr; r += a.scratch_rows){
+    const int own = r0 + r;
+    const int *ids = list + r * dp;
+    for(int i = lane; i < pieces * 2; i += 32) sv[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    if(lane == 0){
+      s[own >> 5] = 1u << (own & 31);
+      atomicAdd(cnt + (own >> (lL + 8)), 1u);
+    }
+    __syncwarp();
+    int lo = 0, hi = 0;                                  /* the last level's vertices in the queue (level 1: the row itself) */
+    int level = 1;
+    for(; level < last; level++){
+      unsigned *c = cnt + (level - 1) * a.nchunks;
+      const int total = level == 1 ? q4 : (hi - lo) * q4;
+      int end = hi;
+      for(int i0 = 0; i0 < total; i0 += 128){
+        int4 x[4];
+#pragma unroll
+        for(int k = 0; k < 4; k++){
+          const int i = i0 + 32 * k + lane;
+          if(i >= total) x[k] = make_int4(-1, -1, -1, -1);
+          else if(level == 1) x[k] = *reinterpret_cast<const int4 *>(ids + 4 * i);
+          else{
+            const int j = i < 1024 ? (i * magic) >> 16 : i / q4;
+            x[k] = __ldcg(reinterpret_cast<const int4 *>(a.e.nbr + (size_t)queue[lo + j] * dp) + (i - j * q4));
+          }
+        }
+#pragma unroll
+        for(int k = 0; k < 4; k++){
+          if(i0 + 32 * k >= total) break;
+          const int v[4] = { x[k].x, x[k].y, x[k].z, x[k].w };
+#pragma unroll
+          for(int m = 0; m < 4; m++){
+            bool add = false;
+            if((unsigned)v[m] < (unsigned)n){
+              const unsigned bit = 1u << (v[m] & 31);
+              add = !(atomicOr(s + (v[m] >> 5), bit) & bit);
+            }
+            const unsigned who = __ballot_sync(0xffffffffu, add);
+            if(add){
+              const int at = end + __popc(who & below);
+              if(at < a.queue) queue[at] = v[m];
+              atomicAdd(c + (v[m] >> (lL + 8)), 1u);
+            }
+            end += __popc(who);
+          }
+        }
+      }
+      __syncwarp();
+      lo = hi;
+      hi = end;
+      if(hi > a.queue) { level++; break; }
+    }
+    if(hi <= a.queue){
+      const int total = (hi - lo) * q4;
+      for(int i0 = lane; i0 < total; i0 += 192){
+        int4 x[6];
+#pragma unroll
+        for(int k = 0; k < 6; k++){
+          const int i = i0 + 32 * k, j = i < 1024 ? (i * magic) >> 16 : i / q4;
+          if(i < total) x[k] = __ldcg(reinterpret_cast<const int4 *>(a.e.nbr + (size_t)queue[lo + j] * dp) + (i - j * q4));
+          else x[k] = make_int4(-1, -1, -1, -1);
+        }
+#pragma unroll
+        for(int k = 0; k < 6; k++){
+          mark(s, x[k].x, n);
+          mark(s, x[k].y, n);
+          mark(s, x[k].z, n);
+          mark(s, x[k].w, n);
+        }
+      }
+    }
+    else
+      for(; level <= last; level++){
+        for(int p = lane; p < pieces; p += 32){
+          char *to = reinterpret_cast<char *>(a.start + (size_t)(p >> lL) * a.start_stride);
+          unsigned w[8];
+          *reinterpret_cast<uint4 *>(w) = sv[2 * p];
+          *reinterpret_cast<uint4 *>(w + 4) = sv[2 * p + 1];
+          st_lane(to + ((size_t)own << (a.wc_log2 + 3)) + (size_t)(p & (L - 1)) * 32, w);
+        }
+        __syncwarp();
+        for(int p = lane; p < pieces; p += 32){
+          const char *from = reinterpret_cast<const char *>(a.start + (size_t)(p >> lL) * a.start_stride);
+          const unsigned *w = reinterpret_cast<const unsigned *>(from + ((size_t)own << (a.wc_log2 + 3)) + (size_t)(p & (L - 1)) * 32);
+          for(int k = 0; k < 8; k++)
+            for(unsigned bits = __ldcg(w + k); bits; bits &= bits - 1u){
+              const int u = p * 256 + k * 32 + __ffs(bits) - 1;
+              for(int j = 0; j < a.e.d; j++){
+                const int v = __ldcg(a.e.nbr + (size_t)u * dp + j);
+                const unsigned bit = 1u << (v & 31);
+                if(!(atomicOr(s + (v >> 5), bit) & bit) && level < last)
+                  atomicAdd(cnt + (level - 1) * a.nchunks + (v >> (lL + 8)), 1u);
+              }
+            }
+        }
+        __syncwarp();
+      }
+    __syncwarp();
+    unsigned *c = cnt + (last - 1) * a.nchunks;
+    for(int p0 = 0; p0 < pieces; p0 += 32){
+      const int p = p0 + lane, q = p >> lL;
+      unsigned w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if(p < pieces){
+        *reinterpret_cast<uint4 *>(w) = sv[2 * p];
+        *reinterpret_cast<uint4 *>(w + 4) = sv[2 * p + 1];
+        char *to = reinterpret_cast<char *>(a.start + (size_t)q * a.start_stride);
+        st_lane(to + ((size_t)own << (a.wc_log2 + 3)) + (size_t)(p & (L - 1)) * 32, w);
+      }
+      unsigned v = popc_lane(w);
+      for(int o = L >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if(v && (lane & (L - 1)) == 0) atomicAdd(c + q, v);
+    }
+    __syncwarp();
   }
 }
 
@@ -461,7 +599,7 @@ template <class Sync>
 __device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, Sync &sy, int ph)
 {
   SweepPhase &p = sh.ph[ph];
-  const int base = a.two_level ? 2 : 1;                  /* the level that the start computed */
+  const int base = a.base;                               /* the level that the start computed */
   int todo = -1;
   if(p.level > base){
     unsigned long long bits;
@@ -481,31 +619,26 @@ __device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, 
     /* the group's levels up to `base`, counted at the start */
     if(p.level < 0){ todo = TODO_DONE; break; }
     const int q = threadIdx.x, chunk = group_chunk(a, p.group, ph) + q;
-    unsigned long long c1 = 0, c2 = 0;
-    bool go = (p.alive >> q) & 1u;
-    if(go){
-      if(a.two_level) c1 = __ldcg(&sy.start1[chunk]);
-      c2 = __ldcg(&sy.start2[chunk]);
-    }
-    unsigned long long t1 = c1, t2 = c2;
-    for(int o = 16; o > 0; o >>= 1){
-      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
-      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+    const bool mine = (p.alive >> q) & 1u;
+    unsigned long long t1 = p.total;
+    bool go = mine, over = false;
+    for(int j = 1; j <= base; j++){
+      const unsigned long long c = mine ? __ldcg(&sy.start[(j - 1) * a.nchunks + chunk]) : 0ull;
+      unsigned long long t2 = c;
+      for(int o = 16; o > 0; o >>= 1) t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+      if(sh.rank == 0 && go) go = settle(a, p, sy, chunk, q, j, c);
+      over |= t2 == p.full || t2 == t1 || a.e.n <= j;
+      t1 = t2;
     }
     if(sh.rank == 0){
-      if(go && a.two_level) go = settle(a, p, sy, chunk, q, 1, c1);
-      if(go) go = settle(a, p, sy, chunk, q, base, c2);
       const unsigned alive = __ballot_sync(0xffffffffu, go);
       if(q == 0) p.alive = alive;
     }
-    const unsigned long long t0 = p.total;
-    const bool over = (a.two_level && (t1 == p.full || t1 == t0 || a.e.n <= 1)) || t2 == p.full ||
-                      t2 == (a.two_level ? t1 : t0) || a.e.n <= base;
     __syncwarp();
     if(over) group_state(a, p, ph, p.group + 1);
     else{
       todo = TODO_LEVEL;
-      if(q == 0){ p.total = t2; p.level = base + 1; }
+      if(q == 0){ p.total = t1; p.level = base + 1; }
     }
     __syncwarp();
   }
@@ -522,20 +655,25 @@ __device__ bool dense_graph(const gbx_sweep &a, SweepShared &sh, Sync &sy, unsig
   const int r0 = sh.rank * a.rows, nr = max(0, min(a.rows, a.e.n - r0));
   int *list = reinterpret_cast<int *>(smem);                                     /* [rows][dp] */
   unsigned *scratch = reinterpret_cast<unsigned *>(list + (size_t)a.rows * dp);  /* a row of marks per warp */
-  unsigned *cnt1 = scratch + SWEEP_WARPS * (a.scratch_bits >> 5), *cnt2 = cnt1 + a.nchunks;
-  unsigned char *flag = reinterpret_cast<unsigned char *>(cnt2 + a.nchunks);     /* [phases * slots][rows][lanes] */
-  for(int i = tid; i < 2 * a.nchunks; i += SWEEP_THREADS) cnt1[i] = 0;
+  unsigned *cnt = scratch + a.scratch_rows * ((a.scratch_bits >> 5) + a.queue);  /* [base][nchunks] */
+  unsigned char *flag = reinterpret_cast<unsigned char *>(cnt + a.base * a.nchunks);  /* [phases * slots][rows][lanes] */
+  for(int i = tid; i < a.base * a.nchunks; i += SWEEP_THREADS) cnt[i] = 0;
   if(!pull_adjacency(a, sh, sy)) return false;
-  expand_rows(a, sy, list, r0, 1, nr, a.two_level ? a.e.nbr : nullptr);
-  if(a.two_level){
+  expand_rows(a, sy, list, r0, 1, nr, a.base > 1 ? a.e.nbr : nullptr);
+  if(a.base > 1){
     if(!grid_pass(&sy.ready[1], sh, a)) return false;
   }
   else __syncthreads();
-  start_rows(a, list, scratch, cnt1, cnt2, 0, a.nchunks, r0, nr);
+  if(a.base > 2) ball_rows(a, list, scratch, cnt, r0, nr);
+  else start_rows(a, list, scratch, cnt, cnt + (a.base - 1) * a.nchunks, 0, a.nchunks, r0, nr);
   __syncthreads();
   for(int c = tid; c < a.nchunks; c += SWEEP_THREADS){
-    if(cnt1[c]) atomicAdd(&sy.start1[c], (unsigned long long)cnt1[c]);
-    if(cnt2[c]) atomicAdd(&sy.start2[c], (unsigned long long)cnt2[c]);
+    unsigned sum = 0;
+    for(int j = 0; j < a.base; j++){
+      const unsigned x = cnt[j * a.nchunks + c];
+      sum = a.base > 2 && j < a.base - 1 ? sum + x : x;  /* ball_rows counts what a level adds, but for the last */
+      if(sum) atomicAdd(&sy.start[j * a.nchunks + c], (unsigned long long)sum);
+    }
   }
   if(!grid_pass(&sy.ready[2], sh, a)) return false;
   after_pass();
@@ -558,7 +696,7 @@ __device__ bool dense_graph(const gbx_sweep &a, SweepShared &sh, Sync &sy, unsig
         return false;
       }
       if(todo == TODO_DONE){ open &= ~(1u << ph); continue; }
-      level_rows<NB>(a, sh, list, flag, ph, sh.ph[ph].level == (a.two_level ? 3 : 2), r0, nr);
+      level_rows<NB>(a, sh, list, flag, ph, sh.ph[ph].level == a.base + 1, r0, nr);
       __syncthreads();
       if(tid < 32) arrive_step(a, sh, sy, ph);
     }
@@ -910,7 +1048,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) team_kernel(const gbx_team t
         if(t.adj) a.e.adj = reinterpret_cast<const int *>(__ldcg(t.adj + g));
         unsigned char *at = t.arena + (size_t)i * (t.arena_bytes >> k);   /* inside the parent's part: the size divides evenly */
         a.buf = reinterpret_cast<unsigned long long *>(at);
-        a.start = a.buf + (a.two_level ? 0 : a.slot_words);
+        a.start = a.buf + ((a.base & 1) ? a.slot_words : 0);
         a.start_stride = 2 * a.slot_words;
         a.changed = reinterpret_cast<unsigned *>(at + 16 * a.slot_words);
         a.rows = (a.e.n + (hi - lo) - 1) / (hi - lo);
@@ -947,7 +1085,7 @@ size_t gbx_sweep_smem(const gbx_sweep *a)
   const size_t rows = (size_t)a->rows, lists = rows * (size_t)a->e.dp * 4;
   if(a->track)
     return lists + 3 * (rows << a->word_log2) * 4 + SWEEP_THREADS * (size_t)a->e.dp * 4 + sizeof(TrackRound);
-  return lists + SWEEP_WARPS * (size_t)a->scratch_bits / 8 + 8 * (size_t)a->nchunks +
+  return lists + (size_t)a->scratch_rows * ((size_t)a->scratch_bits / 8 + 4 * (size_t)a->queue) + 4 * (size_t)a->base * (size_t)a->nchunks +
          (((size_t)a->phases * a->slots * rows) << (a->wc_log2 - 2));
 }
 

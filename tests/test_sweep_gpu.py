@@ -133,3 +133,36 @@ def test_batches(count, n_hi):
     turned = [np.ascontiguousarray(g.adjacency[:, ::-1]) if g.num_degrees is None else g.adjacency for g in specs]
     assert all(same(x, y) for x, y in zip(b.run(turned), want))
     b.close()
+
+
+@pytest.mark.parametrize("n,d,kind", [(2048, 3, "undirected"), (5000, 4, "directed"), (8600, 3, "undirected"),
+                                      (8601, 3, "directed"), (6000, 6, "irregular"), (7000, 2, "rings"),
+                                      (5001, 5, "halves"), (20000, 5, "undirected"), (33000, 9, "directed"),
+                                      (70000, 3, "halves")])
+def test_levels_from_the_lists(n, d, kind, monkeypatch):
+    """Three and more levels from the neighbour lists: queues that suffice
+    (undirected lists) and that run over (directed ones), rows of two lengths,
+    levels that end early (rings of 40, components), one group and several."""
+    rng = np.random.default_rng(n)
+    nd = None
+    if kind == "undirected":
+        adj = og.conv_edge2adjacency_general(n, og.generate_random_general(n, d - (n * d) % 2, seed=n), d - (n * d) % 2)
+    elif kind == "rings":
+        v = np.arange(n)
+        adj = np.stack([v // 40 * 40 + (v + 1) % 40, v // 40 * 40 + (v + 39) % 40], axis=1).astype(np.int32)
+        adj = np.minimum(adj, n - 1)
+    else:
+        half = n // 2 if kind == "halves" else n
+        adj = np.stack([np.concatenate([rng.permutation(half), half + rng.permutation(n - half)]) for _ in range(d)],
+                       axis=1).astype(np.int32)
+        if kind == "irregular":
+            nd = rng.integers(d - 2, d + 1, n).astype(np.int32)
+    b = og.Batch([og.GraphSpec(adj, nodes=n, num_degrees=nd)])
+    got = b.run()[0]
+    b.close()
+    if n <= 9000:
+        assert same(got, oracle.aspl(adj, nodes=n, num_degrees=nd))
+    monkeypatch.setenv("ODP_GB300_SWEEP", "0")
+    b = og.Batch([og.GraphSpec(adj, nodes=n, num_degrees=nd)])
+    assert same(got, b.run()[0])
+    b.close()
