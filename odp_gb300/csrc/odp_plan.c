@@ -18,6 +18,7 @@
 #include <string.h>
 #include <limits.h>
 #include <float.h>
+#include <math.h>
 #include <pthread.h>
 #include <unistd.h>
 #include <time.h>
@@ -443,12 +444,15 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
  * 2 (118 KB) 32 / 35 with the call around it; n = 1024, d = 8 (262 KB) 19 / 22;
  * n = 1024, d = 24 (786 KB) 27 / 17; n = 2048, d = 8 (1 MB) 33 / 25; n = 4096, d
  * = 8 (4 MB) 51 / 29.  Grids are bound by their levels: replicated 50 x 50 117
- * / 177, 64 x 64 101 / 180; partitioned 72 x 72 210 / 189, 80 x 80 298 / 283, 90
- * x 90 658 / 367. */
+ * / 177, 64 x 64 101 / 180.  Partitioned, a level's time grows with n and d in
+ * the small kernel and hardly in lockstep, less so the longer the grid, where
+ * fewer rows change: 75 x 75, d = 4 211 / 279, d = 8 226 / 218, d = 10 230 / 165;
+ * 90 x 90, d = 4 533 / 371; 171 x 33, d = 4 186 / 241, d = 8 328 / 391, d = 10 264
+ * / 227; 190 x 36, d = 4 359 / 470, d = 8 297 / 292; 200 x 41, d = 4 509 / 509. */
 static int small_yields(const odp_shape *sh, const odp_tuning *t, int part, int wl)
 {
   if(t->small_cluster > 0 || t->small_part >= 0) return 0;
-  if(sh->grid) return part;
+  if(sh->grid) return part && 2.0 * pow(shape_n(sh), 1.5) * (sh->degree + 2) > 46e3 * (sh->width + sh->height);
   const double jobs = (shape_words(sh) + (1 << wl) - 1) >> wl;
   return jobs * 4.0 * (shape_n(sh) / sh->symmetries) * sh->degree > 450e3;
 }
