@@ -377,6 +377,32 @@ static long long small_job_count(const odp_shape *shapes, int count, const int *
  * d = 24: 304 against 83 us).  A cluster size forced by
  * ODP_GB300_SMALL_CLUSTER is used if the graphs fit at it (else halved),
  * whatever the SM count; ODP_GB300_SMALL_PART=0 or 1 forces the layout. */
+/* Shared memory and threads of a CTA for chunks of 2^wl[i] words. */
+static void small_shape(const odp_shape *shapes, int count, const int *wl, int c, int part, size_t *smem, int *threads)
+{
+  *smem = 0;
+  *threads = 64;
+  for(int i = 0; i < count; i++){
+    const size_t b = small_bytes(shape_n(&shapes[i]), shape_dp(&shapes[i]), wl[i], c, part);
+    const int th = small_threads_for(shape_n(&shapes[i]), wl[i], c);
+    if(b > *smem) *smem = b;
+    if(th > *threads) *threads = th;
+  }
+}
+
+/* Whether all jobs run at once: by the SMs and, for a single graph, by the
+ * clusters that the GPU's parts really hold (with a CTA per SM, 36 of 4 and 15
+ * of 8: 64 x 64 in 16 clusters of 8 took two turns, 184 us against 115). */
+static int small_at_once(const odp_shape *shapes, int count, const int *wl, long long jobs, int c, int part, int sms)
+{
+  size_t smem;
+  int threads, active = 0;
+  if(jobs * c > sms) return 0;
+  if(count > 1) return 1;
+  small_shape(shapes, count, wl, c, part, &smem, &threads);
+  return smem <= GBX_SMALL_SMEM_MAX && gbx_small_clusters(c, threads, smem, &active) == 0 && active >= jobs;
+}
+
 static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t, int sms, int *wl,
                         int *cluster_out, int *threads_out, size_t *smem_out, int *part_out)
 {
@@ -392,8 +418,24 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
   const int want = t->small_cluster > 0 && t->small_cluster <= GBX_SMALL_CLUSTER_MAX ? t->small_cluster : 0;
   int all_grids = 1;
   for(int i = 0; i < count; i++) all_grids &= shapes[i].grid != 0;
-  for(int part = t->small_part > 0 ? 1 : 0; part <= (t->small_part == 0 ? 0 : 1); part++){
-    for(int c = want ? want : GBX_SMALL_CLUSTER_MAX; c >= 1; c >>= 1){
+  /* A single grid of 1800 vertices or more first tries clusters of 4 with chunks
+   * of two words (clusters of 8 have half the rows a CTA, but chunks twice as
+   * wide, and send every changed word to twice the peers), partitioned up to
+   * degree 4, and then clusters of 8, partitioned; but a grid more than twice as
+   * high as wide, whose rows of a CTA (a few columns) border on every other
+   * CTA's, replicated first.  Measured on GB300, us, clusters of 8 against 4
+   * replicated and 4 and 8 partitioned: 50 x 50, d = 4 125 / 90 / 85 / 86, d = 10
+   * 81 / 77 / 84 / 96; 64 x 64, d = 4 268 / 124 / 115 / 184, d = 8 233 / 131 / 133
+   * / 202; 200 x 12, d = 4 264 / 177 / 179 / 212;
+   * 20 x 195, d = 6 262 partitioned against 195; 110 x 45, d = 4 448 / 290 / 213
+   * / 202 (2 CTAs, replicated: 245); but 40 x 40, d = 8 49 / 54 / 55 / 53. */
+  const int one_grid = count == 1 && all_grids && !want && t->small_part < 0 && shape_n(shapes) >= 1800;
+  const int tall = one_grid && shapes->height > 2 * shapes->width;
+  for(int turn = one_grid ? 0 : 1; turn < 3; turn++){
+    const int part = turn == 0 ? shapes->degree <= 4 && !tall : one_grid ? (turn == 1) != tall : turn - 1;
+    if(turn == 0 && 2 * shape_words(shapes) > sms) continue;
+    if(!one_grid && ((part && t->small_part == 0) || (!part && t->small_part > 0))) continue;
+    for(int c = want ? want : turn == 0 ? 4 : GBX_SMALL_CLUSTER_MAX; c >= (turn == 0 ? 4 : 1); c >>= 1){
       if(part && c == 1) continue;                 /* one CTA: the replicated layout */
       if(part && t->small_part < 0 && !all_grids) continue;
       int ok = 1;
@@ -404,7 +446,7 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
       }
       if(!ok) continue;
       long long jobs = small_job_count(shapes, count, wl);
-      if(!want && jobs * c > sms) continue;
+      if(!want && !small_at_once(shapes, count, wl, jobs, c, part, sms)) continue;
       for(;;){                                   /* narrower chunks while the jobs fit on the SMs */
         int k = -1;
         for(int i = 0; i < count; i++)
@@ -412,18 +454,12 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
         if(k < 0) break;
         wl[k]--;
         const long long more = small_job_count(shapes, count, wl);
-        if(more * c > sms){ wl[k]++; break; }
+        if(want ? more * c > sms : !small_at_once(shapes, count, wl, more, c, part, sms)){ wl[k]++; break; }
         jobs = more;
       }
-      size_t smem = 0;
-      int threads = 64;
-      for(int i = 0; i < count; i++){
-        const size_t b = small_bytes(shape_n(&shapes[i]), shape_dp(&shapes[i]), wl[i], c, part);
-        const int th = small_threads_for(shape_n(&shapes[i]), wl[i], c);
-        if(b > smem) smem = b;
-        if(th > threads) threads = th;
-      }
-      int active = 0;
+      size_t smem;
+      int threads, active = 0;
+      small_shape(shapes, count, wl, c, part, &smem, &threads);
       if(smem <= GBX_SMALL_SMEM_MAX && gbx_small_clusters(c, threads, smem, &active) == 0 && active > 0){
         *cluster_out = c;
         *threads_out = threads;
@@ -448,11 +484,15 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
  * the small kernel and hardly in lockstep, less so the longer the grid, where
  * fewer rows change: 75 x 75, d = 4 211 / 279, d = 8 226 / 218, d = 10 230 / 165;
  * 90 x 90, d = 4 533 / 371; 171 x 33, d = 4 186 / 241, d = 8 328 / 391, d = 10 264
- * / 227; 190 x 36, d = 4 359 / 470, d = 8 297 / 292; 200 x 41, d = 4 509 / 509. */
+ * / 227; 190 x 36, d = 4 359 / 470, d = 8 297 / 292; 200 x 41, d = 4 509 / 509.
+ * Grids more than twice as high as wide, whose CTAs border on all others: 33 x
+ * 171, d = 4 379 / 423, d = 8 500 / 391; 25 x 200, d = 6 561 / 415. */
 static int small_yields(const odp_shape *sh, const odp_tuning *t, int part, int wl)
 {
   if(t->small_cluster > 0 || t->small_part >= 0) return 0;
-  if(sh->grid) return part && 2.0 * pow(shape_n(sh), 1.5) * (sh->degree + 2) > 46e3 * (sh->width + sh->height);
+  if(sh->grid)
+    return part && 2.0 * pow(shape_n(sh), 1.5) * (sh->degree + 2) >
+                   (sh->height > 2 * sh->width ? 25e3 : 46e3) * (sh->width + sh->height);
   const double jobs = (shape_words(sh) + (1 << wl) - 1) >> wl;
   return jobs * 4.0 * (shape_n(sh) / sh->symmetries) * sh->degree > 450e3;
 }
