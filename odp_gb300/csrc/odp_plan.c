@@ -618,8 +618,10 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
 /* Whether the team kernel takes a graph of this shape: it must fit the lockstep
  * kernels in one group (bitsets of at most 64 MB, 64 lanes a row, 256 for
  * grids).  Its cost on the whole GPU is estimated from its traffic: a general
- * graph's gathered levels at 20 TB/s; for grids about ten visits per row and
- * lane, each reading d + 2 sectors, at 8 TB/s. */
+ * graph's gathered levels and lists at 10 TB/s; for grids 6.5 visits per row and
+ * lane, each reading d + 2 sectors, at 8 TB/s; its latency from its levels.
+ * The constants are fitted to 785 graphs of seven batches on teams of 1/2 to
+ * 1/256 of the GPU (error of a graph's time 25 %). */
 int odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_team_graph *g)
 {
   const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
@@ -636,14 +638,14 @@ int odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_t
   while((32 << c->word_log2) < (c->slots << (c->wc_log2 - 2))) c->word_log2++;
   const double lanes = (c->B + 255) / 256;
   if(c->track){
-    g->cost = n * lanes * 9.5 * (sh->degree + 2) * 32.0 / 8e6;
-    g->latency = 15.0 + 4.0 * (sh->width + sh->height) / 3.0;
+    g->cost = n * lanes * 6.5 * (sh->degree + 2) * 32.0 / 8e6;
+    g->latency = 1.1 * (sh->width + sh->height);
   }
   else{
     double levels = 2.0, ball = sh->degree + 1.0;      /* until a ball of branching d - 1 holds n, and one more */
     for(const double grow = sh->degree > 3 ? sh->degree - 1.0 : 2.0; ball < n; ball *= grow) levels += 1.0;
-    g->cost = (n * 8.0 * W * (sh->degree + 1) * (levels > 3.0 ? levels - 2.5 : 0.5) + 4.0 * n * c->e.dp * sh->degree) / 20e6;
-    g->latency = 15.0 + 4.0 * levels;
+    g->cost = (n * 8.0 * W * (sh->degree + 1) * (levels > 3.0 ? levels - 2.5 : 0.5) + 4.0 * n * c->e.dp * sh->degree) / 10e6;
+    g->latency = 10.0 * levels;
   }
   g->need = 16.0 * ((double)n * c->slots * (1 << c->wc_log2)) + (c->track ? 8.0 * n * (1 << c->word_log2) : 0) + 1024;
   return 1;
@@ -695,7 +697,9 @@ static int assign_teams(const odp_shape *shapes, int count, int grid, double mos
  * A graph's team is the smallest on which it takes no more
  * than a share of all graphs' cost, its rows fit a CTA's shared memory and
  * the teams' bitsets together stay within 160 MB; of several shares the one
- * with the least makespan is taken. */
+ * with the least makespan is taken.  Shares above 1 let a few graphs of many
+ * levels run side by side on small teams: 18 graphs of n = 360 to 2880, 366 ->
+ * 207 us on GB300 with the fitted estimates. */
 static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, int sms, gbx_sweep *gs,
                        gbx_team *tm, int *order, int *grid_out, size_t *smem_out)
 {
@@ -716,9 +720,9 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
   }
   if(ok){
     qsort(ord, (size_t)count, sizeof(job_order), cmp_work_desc);
-    static const double shares[] = { 0.1, 0.2, 0.35, 0.6, 1.0 };
+    static const double shares[] = { 0.1, 0.2, 0.35, 0.6, 1.0, 2.0, 4.0, 8.0 };
     double best = 0, best_share = 0;
-    for(int s = 0; s < 5 && ok; s++){
+    for(int s = 0; s < 8 && ok; s++){
       ok = assign_teams(shapes, count, grid, shares[s] * all, gs, g);
       const double m = ok ? team_makespan(g, ord, count) : 0;
       if(s == 0 || m < best){ best = m; best_share = shares[s]; }
