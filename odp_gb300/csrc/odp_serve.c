@@ -14,8 +14,8 @@
  * admitted while others are running overlaps with them on the device.  A
  * batch of general graphs that fit there is one launch of the team kernel,
  * which reads its arguments and the deltas from pinned memory, applies the
- * deltas to the compact adjacency and writes its records to pinned memory.
- * The others run on the persistent engine, in stream order: the deltas are
+ * deltas and writes its records to pinned memory.  The others, and all
+ * batches formed while one of those is in flight, run on the persistent engine, in stream order: the deltas are
  * applied by one scatter kernel (to the compact adjacency and to every
  * neighbour-table row they touch), the jobs and engine state are uploaded, the
  * engine runs, and the per-graph accumulators come back.  A graph is never in
@@ -215,7 +215,6 @@ static int delta_writes(serve_graph *g, const ODPX_Delta *dl, gbx_write *w)
   int k = 0, m = dl->row, j = dl->slot, a = dl->value;
   w[k].at = g->d_adj + (size_t)m * g->d + j; w[k].value = a; k++;
   g->h_adj[(size_t)m * g->d + j] = a;
-  if(g->team) return k;                                  /* the lists are built from the adjacency */
   if(!g->grid_s){
     for(int t = 0; t < g->s; t++){
       int row = m + t * g->B, nb = a + t * g->B;
@@ -365,6 +364,11 @@ static int form_batch(odp_server *s, serve_lane *l, double max_seed_cost)
 {
   int nreq = 0, njobs = 0, nw = 0;
   double seed_cost = 0;
+  /* A cooperative launch waits until all its CTAs fit, and the engine's CTAs
+   * stay for a whole batch, so no team batch is issued beside an engine's:
+   * with chains of n = 16384 and 32768 on the other lanes it waited 12 ms. */
+  int engine = 0;
+  for(int i = 0; i < s->cfg.lanes; i++) engine |= s->lanes[i].busy && !s->lanes[i].team;
   for(long long id = s->next_pending; id < s->nreqs && nreq < l->max_batch; id++){
     serve_req *r = &s->reqs[id];
     if(r->state != 0) continue;
@@ -373,15 +377,15 @@ static int form_batch(odp_server *s, serve_lane *l, double max_seed_cost)
     /* A batch holds requests of similar cost (within 4x of the oldest one it
      * takes): a request completes only when its whole batch does, so a small
      * graph batched with a large one would wait for it. */
-    int other_class = nreq > 0 ? (g->cost > 4.0 * seed_cost || 4.0 * g->cost < seed_cost || g->team != l->team)
+    int other_class = nreq > 0 ? (g->cost > 4.0 * seed_cost || 4.0 * g->cost < seed_cost || (l->team && !g->team))
                                : g->cost > max_seed_cost;
     if(g->busy || other_class || njobs + g->nchunks > l->max_jobs || nw + need_w > l->max_writes) continue;
-    if(nreq == 0){ seed_cost = g->cost; l->team = g->team; }
+    if(nreq == 0){ seed_cost = g->cost; l->team = g->team && !engine; }
     const int w0 = nw;
     for(int k = 0; k < r->ndelta; k++) nw += delta_writes(g, &r->deltas[k], l->h_writes + nw);
     free(r->deltas);
     r->deltas = NULL;
-    if(g->team){
+    if(l->team){
       /* largest first, as the teams take them */
       int at = nreq++;
       for(; at > 0 && member(s, l, at - 1)->est.cost < g->est.cost; at--){
