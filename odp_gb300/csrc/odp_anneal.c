@@ -25,6 +25,7 @@
 
 #define ANNEAL_GRAPH_STEPS 8   /* steps per replayed CUDA graph */
 #define RESIDENT_STEPS 512     /* steps per launch of the resident kernel */
+#define RESIDENT_LANES 32      /* lanes a thread walks per level, at most */
 #define RESIDENT_HOST (64 << 20) /* pinned bytes of a group's records and graphs, at most */
 
 struct odpx_anneal {
@@ -128,8 +129,11 @@ static int resident_cluster(const ODPX_Anneal *a, int range, long long lanes, si
  * (ODP_GB300_BLOCKS, in engine CTAs, four per SM) becomes the same part of
  * them.  Measured on GB300 against four launches per step (us): 16 chains of
  * n = 1024, d = 8: 15 / 68; one of them: 12 / 48; 8 of n = 4096, d = 16: 85 /
- * 137; 32 of n = 300, d = 6: 12 / 64.  Allocates its memory; 0 if the chains
- * do not fit. */
+ * 137; 32 of n = 300, d = 6: 12 / 64.  With few CTAs for large graphs the
+ * engine's four CTAs per SM are faster: 16 chains on a quarter of the GPU, n =
+ * 2048, d = 16 (32 lanes a thread) 122 / 130, n = 3000, d = 12 (70) 360 / 270, n
+ * = 4096, d = 8 (128) 466 / 348.  Allocates its memory; 0 if the chains do not
+ * fit. */
 static int plan_resident(ODPX_Anneal *a, int blocks)
 {
   const odp_plan *p = a->p;
@@ -148,7 +152,7 @@ static int plan_resident(ODPX_Anneal *a, int blocks)
       const long long lanes = (g->B + 255) / 256, want = ((long long)g->n * lanes + 255) / 256;
       const int size = range < want ? range : (int)want;
       const size_t s = gbx_resident_smem((g->n + size - 1) / size, g->dp, g->B, g->d);
-      if(g->n > 65535 || lanes > 256) return 0;
+      if(g->n > 65535 || lanes > 256 || (long long)g->n * lanes > RESIDENT_LANES * 256ll * size) return 0;
       if(s > smem) smem = s;
       if(g->n * lanes > most) most = g->n * lanes;
       words += 8ull * (unsigned long long)g->n * (unsigned long long)lanes;   /* two buffers, 4 words a lane */
