@@ -7,10 +7,11 @@ s in {1, 2, 4}), each the reference generator's graph for its seed, evaluated
 together by the batched engine (ODP_Set_aspl_batch).
 
 Reported on rank 0 as one JSON line:
-  value        batched evals/s of the engine on resident inputs (device time,
-               CUDA events on the plan's stream, L2 flushed before each run)
+  value        batched evals/s on the device (the team kernel, which reads the
+               adjacency from host memory itself; device time, CUDA events on
+               the plan's stream, L2 flushed before each run)
   e2e          batched evals/s through ODP_Set_aspl_batch with the adjacency in
-               host memory (upload, expand, engine, read back, decode)
+               host memory (one kernel, read back, decode)
   per_call     evals/s of one graph per call on the same GPU over the same 512
                graphs: a plan per graph (ODPX_Batch_run), the drop-in
                Init/Set/Finalize cycle, and the reference's own libodp_cuda.a
@@ -21,7 +22,7 @@ Reported on rank 0 as one JSON line:
                roofline fraction, and the reference's CPU (libodp_threads.a)
                and GPU (libodp_cuda.a) times for the same graph
   single_graph the n=65536, d=16 graph, autotuned
-  roofline     the batched engine kernel against the L2 read ceiling (its
+  roofline     the batched team kernel against the L2 read ceiling (its
                bitsets are L2-resident): bytes actually read from L2 per second
                over the ceiling measured live by a streaming probe; the
                algorithmic bytes, the DRAM traffic and the HBM peak beside it
@@ -64,18 +65,18 @@ L2_NOTE = "GPU arm: L2 flushed (512 MB write) before every timed device run"
 # same for the reference generators (baseline/ref_bench.c gen) and the
 # library's own; both arms check it, so they evaluate identical graphs.
 BATCH_SHA256 = "cb594241cefc45d1"
-# ncu counters of one engine_kernel launch per leg, per algorithmic byte of the
+# ncu counters of one launch per leg, per algorithmic byte of the
 # same launch (ncu --metrics dram__bytes_read.sum, dram__bytes_write.sum,
 # l1tex__m_xbar2l1tex_read_bytes.sum, one launch per leg selected by its NVTX
 # range with --nvtx, bytes_alg from ODPX_Batch_bytes_alg):
-# "batch" is the 512-graph batch with the saved autotuned schedule, C2, C3 and
-# G the configuration graphs with the default schedule.  A launch's L2 read
+# "batch" is the 512-graph batch, C2, C3 and G the configuration graphs, all
+# with the default schedule (profiles/lockstep_kernels.md).  A launch's L2 read
 # bytes and DRAM traffic are taken as its algorithmic bytes times these ratios.
 NCU_RATIOS = {
-    "batch": {"l2_read": 0.641194, "dram": 0.092754},
-    "C2": {"l2_read": 0.654699, "dram": 0.106574},
-    "C3": {"l2_read": 0.784801, "dram": 0.145122},
-    "G": {"l2_read": 0.261177, "dram": 0.095565},
+    "batch": {"kernel": "team_kernel", "l2_read": 0.305860, "dram": 0.013813},
+    "C2": {"kernel": "sweep_dense_kernel", "l2_read": 0.266805, "dram": 0.053653},
+    "C3": {"kernel": "sweep_dense_kernel", "l2_read": 0.480601, "dram": 0.031746},
+    "G": {"kernel": "sweep_track_kernel", "l2_read": 0.064507, "dram": 0.026707},
 }
 
 
@@ -402,7 +403,7 @@ def time_configs(args, l2_gbs, hbm_gbs, l2_bytes, nvtx):
             moved, dram = balg * ratio["l2_read"], balg * ratio["dram"]
             l2f = moved / (ms * 1e-3) / 1e9 / l2_gbs
             dramf = dram / (ms * 1e-3) / 1e9 / hbm_gbs
-            rec.update({"l2_read_bytes": moved, "l2_read_gbs": moved / (ms * 1e-3) / 1e9, "l2_read_frac": l2f,
+            rec.update({"kernel": ratio["kernel"], "l2_read_bytes": moved, "l2_read_gbs": moved / (ms * 1e-3) / 1e9, "l2_read_frac": l2f,
                         "dram_bytes": dram, "dram_gbs": dram / (ms * 1e-3) / 1e9, "dram_frac_of_hbm": dramf,
                         "bound": "l2" if l2f >= dramf else "hbm", "frac": max(l2f, dramf)})
         else:
@@ -786,16 +787,16 @@ def run_own(args):
     if not args.no_anneal and world == 1:
         line["anneal"] = anneal(args.serve_seconds)
 
-    # ---- roofline of the headline kernel: the batched engine against L2 ----
+    # ---- roofline of the headline kernel: the batched team kernel against L2 ----
     rat = NCU_RATIOS["batch"]
     moved = balg * rat["l2_read"]
     achieved = moved / (ms * 1e-3) / 1e9
     line["roofline"] = {"bound": "l2", "achieved": achieved, "peak": l2_gbs, "unit": "GB/s",
                         "frac": achieved / l2_gbs, "traffic": balg * rat["dram"],
-                        "kernel": "engine_kernel",
+                        "kernel": rat["kernel"],
                         "achieved_source": "bytes read from L2 by the SMs per launch (ncu "
                                            "l1tex__m_xbar2l1tex_read_bytes.sum per algorithmic byte, one launch of "
-                                           "the tuned 512-graph batch, times this launch's algorithmic bytes) / the "
+                                           "the 512-graph batch, times this launch's algorithmic bytes) / the "
                                            "launch's CUDA-event time",
                         "peak_source": "L2 read ceiling measured live in this run by a streaming probe of 16-byte "
                                        "L2-only loads over a 48 MB L2-resident buffer (MEASURED_PEAKS.json has no "

@@ -61,7 +61,6 @@ void odp_tuning_defaults(odp_tuning *t, int batch)
   t->small_cluster = env_int("ODP_GB300_SMALL_CLUSTER", 0);
   t->small_part = env_int("ODP_GB300_SMALL_PART", -1);
   t->sweep = env_int("ODP_GB300_SWEEP", 1);
-  t->team = 0;
 }
 
 /* Shared memory per CTA of the small kernel when `cluster` CTAs share a job:
@@ -541,7 +540,7 @@ static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
  * graph, no schedule setting, and a CTA's rows must fit in its shared memory
  * beside their lane states.  Measured on GB300 against the persistent engine:
  * n = 4096, d = 24: 27 against 67 us; n = 9999, s = 3: 48 against 108; n =
- * 65536, d = 16: 1.65 against 2.63 ms; n = 262144, s = 64: 0.63 against 1.0;
+ * 65536, d = 16: 1.34 against 2.63 ms; n = 262144, s = 64: 0.63 against 1.0;
  * 97 x 103 grid: 0.34 against 0.76; 256 x 256: 5.3 against 18.5.
  *  - Grids of degree up to 32 track changed lanes, 65536 sources at a time.
  *  - Graphs whose bitset buffers take at most 64 MB, and a row 64 lanes, run
@@ -553,8 +552,8 @@ static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
  *    rows, 0.94 with 256, 0.82 with 64); as many chunks in a phase as fit in
  *    75 MB (n = 262144, two chunks of 67 MB: 1.07 ms); and two phases, one
  *    computing while the other's barrier is crossed, where two chunks fit in
- *    80 MB (n = 65536: two phases of two chunks 1.65 ms, of one 1.71, one
- *    phase of two 1.69).
+ *    80 MB (n = 65536, with two levels from the lists: two phases of two
+ *    chunks 1.65 ms, of one 1.71, one phase of two 1.69).
  *  - Without symmetry, a compact adjacency of up to 1 MB is expanded straight
  *    from host memory (n = 4096: 27.2 against 29.8 us); larger ones are copied
  *    first, in wider pieces. */
@@ -703,7 +702,7 @@ static int assign_teams(const odp_shape *shapes, int count, int grid, double mos
 static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, int sms, gbx_sweep *gs,
                        gbx_team *tm, int *order, int *grid_out, size_t *smem_out)
 {
-  if(count == 1 && !t->team) return 0;
+  if(count == 1) return 0;
   int fit = 0;
   if(gbx_team_blocks(0, &fit) || fit < 2) return 0;
   int grid = 2 * sms;

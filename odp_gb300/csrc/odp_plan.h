@@ -36,7 +36,6 @@ typedef struct {
   int small_cluster;           /* CTAs per small-kernel job: 1, 2, 4 or 8; 0 = automatic */
   int small_part;              /* small-kernel rows partitioned over the cluster: -1 when needed, 0 never, 1 always */
   int sweep;                   /* graphs run in lockstep on every SM, or on teams of CTAs, where that fits (1, default) */
-  int team;                    /* a single graph may run as a team of every CTA (annealing) */
 } odp_tuning;
 
 typedef struct {

@@ -324,30 +324,28 @@ __device__ __forceinline__ void expand_rows(const gbx_sweep &a, Sync &sy, int *l
 /* General graphs.                                                         */
 /* ---------------------------------------------------------------------- */
 
-/* Levels 1 and 2 of every chunk (of one group's chunks when the lists are too
- * wide for level 2: then level 1 alone), a warp per row.  The warp marks the
+/* Levels 1 and 2 of every chunk (level 1 alone for base 1), a warp per row.  The warp marks the
  * row, its neighbours and their neighbours in its scratch row (scratch_bits
  * sources at a time) and stores each lane once.  A level-2 gather would read
  * d whole rows per row, nearly all of them zeros; this reads d neighbour
  * lists once for all chunks, and level 1 is never stored. */
 __device__ void start_rows(const gbx_sweep &a, const int *list, unsigned *scratch, unsigned *cnt1, unsigned *cnt2,
-                           int c0, int nc, int r0, int nr)
+                           int r0, int nr)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lL = a.wc_log2 - 2, L = 1 << lL;             /* lanes per row of a chunk */
   const int dp = a.e.dp, d = a.e.d;
-  const int src0 = c0 << (lL + 8), nsrc = min(nc << (lL + 8), a.B - src0);
   const int q4 = dp >> 2, magic = (65536 + q4 - 1) / q4;  /* i / q4 for i < 1024, q4 <= 16 */
   unsigned *s = scratch + (size_t)warp * (a.scratch_bits >> 5);
   for(int r = warp; r < nr; r += SWEEP_WARPS){
     const int *ids = list + r * dp;
-    for(int sb = 0; sb < nsrc; sb += a.scratch_bits){
-      const int base = src0 + sb, sub = min(nsrc - sb, a.scratch_bits);
+    for(int sb = 0; sb < a.B; sb += a.scratch_bits){
+      const int sub = min(a.B - sb, a.scratch_bits);
       const int pieces = (sub + 255) >> 8;
       uint4 *sv = reinterpret_cast<uint4 *>(s);
       for(int i = lane; i < pieces * 2; i += 32) sv[i] = make_uint4(0u, 0u, 0u, 0u);
       __syncwarp();
-      for(int i = lane; i <= dp; i += 32) mark(s, (i < dp ? ids[i] : r0 + r) - base, sub);
+      for(int i = lane; i <= dp; i += 32) mark(s, (i < dp ? ids[i] : r0 + r) - sb, sub);
       __syncwarp();
       if(a.base == 2){
         for(int p0 = 0; p0 < pieces; p0 += 32){          /* level 1's counts */
@@ -372,10 +370,10 @@ __device__ void start_rows(const gbx_sweep &a, const int *list, unsigned *scratc
           }
 #pragma unroll
           for(int k = 0; k < 6; k++){
-            mark(s, x[k].x - base, sub);
-            mark(s, x[k].y - base, sub);
-            mark(s, x[k].z - base, sub);
-            mark(s, x[k].w - base, sub);
+            mark(s, x[k].x - sb, sub);
+            mark(s, x[k].y - sb, sub);
+            mark(s, x[k].z - sb, sub);
+            mark(s, x[k].w - sb, sub);
           }
         }
         __syncwarp();
@@ -665,7 +663,7 @@ __device__ bool dense_graph(const gbx_sweep &a, SweepShared &sh, Sync &sy, unsig
   }
   else __syncthreads();
   if(a.base > 2) ball_rows(a, list, scratch, cnt, r0, nr);
-  else start_rows(a, list, scratch, cnt, cnt + (a.base - 1) * a.nchunks, 0, a.nchunks, r0, nr);
+  else start_rows(a, list, scratch, cnt, cnt + (a.base - 1) * a.nchunks, r0, nr);
   __syncthreads();
   for(int c = tid; c < a.nchunks; c += SWEEP_THREADS){
     unsigned sum = 0;
