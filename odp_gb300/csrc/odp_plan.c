@@ -562,6 +562,7 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
   if(!lockstep_allowed(sh, t) || t->blocks > 0) return 0;
   const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
   memset(sw, 0, sizeof(*sw));
+  sw->e.d = sh->degree;
   sw->e.dp = shape_dp(sh);
   sw->B = n / sh->symmetries;
   sw->phases = 1;

@@ -970,7 +970,8 @@ __device__ bool track_graph(const gbx_sweep &a, SweepShared &sh, Sync &sy, unsig
 
 /* Two CTAs per SM and six neighbours in flight: 256 x 256, d = 6 took 5.26 ms
  * (6.0 with three CTAs, 5.9 with four and four neighbours in flight; both
- * spilled). */
+ * spilled).  Eight in flight where that saves a turn: 190 x 190, d = 8 2069 ->
+ * 1884 us, 100 x 100 335 -> 318; at d = 4 to 6 they cost 1 to 2 %. */
 template <int NB>
 __global__ void __launch_bounds__(SWEEP_THREADS, 2) sweep_track_kernel(const gbx_sweep a)
 {
@@ -1091,7 +1092,8 @@ size_t gbx_sweep_smem(const gbx_sweep *a)
  * 128 with eight neighbours in flight per lane. */
 static const void *sweep_entry(const gbx_sweep *a)
 {
-  if(a->track) return (const void *)sweep_track_kernel<6>;
+  if(a->track)
+    return (a->e.d + 7) / 8 < (a->e.d + 5) / 6 ? (const void *)sweep_track_kernel<8> : (const void *)sweep_track_kernel<6>;
   return a->wide ? (const void *)sweep_dense_kernel<8, 2> : (const void *)sweep_dense_kernel<4, 4>;
 }
 

@@ -166,3 +166,10 @@ def test_levels_from_the_lists(n, d, kind, monkeypatch):
     b = og.Batch([og.GraphSpec(adj, nodes=n, num_degrees=nd)])
     assert same(got, b.run()[0])
     b.close()
+
+
+@pytest.mark.parametrize("w,h,d,length", [(61, 47, 7, 4), (100, 90, 8, 4), (40, 33, 14, 5), (45, 40, 20, 6), (33, 30, 32, 8)])
+def test_grids_with_eight_neighbours_in_flight(w, h, d, length):
+    d -= (w * h * d) % 2
+    adjs = [og.conv_edge2adjacency_grid(w, h, og.generate_random_grid(w, h, d, length, 1, seed=k), d, 1) for k in (3, 4)]
+    check(og.GraphSpec(adjs[0], grid=True, width=w, height=h), adjs)
