@@ -542,7 +542,12 @@ static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
  * n = 4096, d = 24: 27 against 67 us; n = 9999, s = 3: 48 against 108; n =
  * 65536, d = 16: 1.34 against 2.63 ms; n = 262144, s = 64: 0.63 against 1.0;
  * 97 x 103 grid: 0.34 against 0.76; 256 x 256: 5.3 against 18.5.
- *  - Grids of degree up to 32 track changed lanes, 65536 sources at a time.
+ *  - Grids of degree up to 32 track changed lanes, 65536 sources at a time, in
+ *    the wide form while two CTAs per SM have a thread for every word of their
+ *    rows' changes; past that a level takes a second round, and three narrower
+ *    CTAs are faster (us): 135 x 135, d = 4 536 / 554; 140 x 140, d = 4 1031 /
+ *    872; 150 x 150, d = 6 910 / 823; 190 x 190, d = 10 1913 / 1756; 256 x 256, d
+ *    = 6 5431 / 5281.
  *  - Graphs whose bitset buffers take at most 64 MB, and a row 64 lanes, run
  *    all chunks at once.  With at most one lane per thread of two CTAs per SM
  *    they take the wide form.
@@ -572,6 +577,9 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
     sw->wc_log2 = full_l2 < 5 ? full_l2 : 5;
     sw->slots = (W + (1 << sw->wc_log2) - 1) >> sw->wc_log2;
     if(sw->slots > GBX_SWEEP_SLOTS) sw->slots = GBX_SWEEP_SLOTS;
+    int words = 1;
+    while(32 * words < (sw->slots << (sw->wc_log2 - 2))) words *= 2;
+    sw->wide = (double)n * words <= 2.0 * 256 * sms;
   }
   else if(16.0 * n * W <= 64e6 && W <= 256){
     sw->wc_log2 = full_l2 < 6 ? full_l2 : 6;
@@ -593,7 +601,7 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
   sw->nchunks = (W + (1 << sw->wc_log2) - 1) >> sw->wc_log2;
   if(!sw->track) choose_start(sh, sw->e.dp <= GBX_SWEEP_TWO_LEVEL ? 2 : 1, GBX_SWEEP_CHUNKS, sw);
   if(sw->nchunks > GBX_SWEEP_CHUNKS) return 0;
-  for(int per_sm = sw->track || sw->wide ? 2 : 4; per_sm >= 1; per_sm--)
+  for(int per_sm = sw->wide ? 2 : sw->track ? 3 : 4; per_sm >= 1; per_sm--)
     for(int q = sw->slots; q >= 1; q = q > 1 ? (q + 1) / 2 : 0){
       gbx_sweep c = *sw;
       int fit = 0;

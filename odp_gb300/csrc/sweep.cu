@@ -968,12 +968,13 @@ __device__ bool track_graph(const gbx_sweep &a, SweepShared &sh, Sync &sy, unsig
   return true;
 }
 
-/* Two CTAs per SM and six neighbours in flight: 256 x 256, d = 6 took 5.26 ms
- * (6.0 with three CTAs, 5.9 with four and four neighbours in flight; both
- * spilled).  Eight in flight where that saves a turn: 190 x 190, d = 8 2069 ->
- * 1884 us, 100 x 100 335 -> 318; at d = 4 to 6 they cost 1 to 2 %. */
-template <int NB>
-__global__ void __launch_bounds__(SWEEP_THREADS, 2) sweep_track_kernel(const gbx_sweep a)
+/* The wide form has two CTAs per SM and six neighbours in flight, or eight where
+ * that saves a turn: 190 x 190, d = 8 2069 -> 1884 us, 100 x 100 335 -> 318; at d
+ * = 4 to 6 they cost 1 to 2 %.  The narrow one has three CTAs and four in
+ * flight (79 registers; three with six in flight, and four CTAs, spilled: 256 x
+ * 256, d = 6 6.0 and 5.9 ms against 5.3). */
+template <int NB, int MIN_BLOCKS>
+__global__ void __launch_bounds__(SWEEP_THREADS, MIN_BLOCKS) sweep_track_kernel(const gbx_sweep a)
 {
   extern __shared__ __align__(16) unsigned char sweep_smem[];
   __shared__ SweepShared sh;
@@ -1088,12 +1089,14 @@ size_t gbx_sweep_smem(const gbx_sweep *a)
          (((size_t)a->phases * a->slots * rows) << (a->wc_log2 - 2));
 }
 
-/* The narrow form keeps four CTAs of 64 registers per SM, the wide one two of
- * 128 with eight neighbours in flight per lane. */
+/* The dense kernel's narrow form keeps four CTAs of 64 registers per SM, the
+ * wide one two of 128 with eight neighbours in flight per lane. */
 static const void *sweep_entry(const gbx_sweep *a)
 {
+  if(a->track && !a->wide) return (const void *)sweep_track_kernel<4, 3>;
   if(a->track)
-    return (a->e.d + 7) / 8 < (a->e.d + 5) / 6 ? (const void *)sweep_track_kernel<8> : (const void *)sweep_track_kernel<6>;
+    return (a->e.d + 7) / 8 < (a->e.d + 5) / 6 ? (const void *)sweep_track_kernel<8, 2>
+                                               : (const void *)sweep_track_kernel<6, 2>;
   return a->wide ? (const void *)sweep_dense_kernel<8, 2> : (const void *)sweep_dense_kernel<4, 4>;
 }
 

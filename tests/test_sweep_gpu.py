@@ -173,3 +173,16 @@ def test_grids_with_eight_neighbours_in_flight(w, h, d, length):
     d -= (w * h * d) % 2
     adjs = [og.conv_edge2adjacency_grid(w, h, og.generate_random_grid(w, h, d, length, 1, seed=k), d, 1) for k in (3, 4)]
     check(og.GraphSpec(adjs[0], grid=True, width=w, height=h), adjs)
+
+
+@pytest.mark.parametrize("w,h,d,length", [(139, 140, 4, 5), (140, 140, 6, 6), (100, 230, 3, 6)])
+def test_grids_of_three_ctas_per_sm(w, h, d, length, monkeypatch):
+    """On both sides of the line where a level takes a second round."""
+    adj = og.conv_edge2adjacency_grid(w, h, og.generate_random_grid(w, h, d, length, 1, seed=5), d, 1)
+    b = og.Batch([og.GraphSpec(adj, grid=True, width=w, height=h)])
+    got = b.run()[0]
+    b.close()
+    monkeypatch.setenv("ODP_GB300_SWEEP", "0")
+    b = og.Batch([og.GraphSpec(adj, grid=True, width=w, height=h)])
+    assert same(got, b.run()[0])
+    b.close()
