@@ -76,7 +76,7 @@ NCU_RATIOS = {
     "batch": {"kernel": "team_kernel", "l2_read": 0.305860, "dram": 0.013813},
     "C2": {"kernel": "sweep_dense_kernel", "l2_read": 0.266805, "dram": 0.053653},
     "C3": {"kernel": "sweep_dense_kernel", "l2_read": 0.480601, "dram": 0.031746},
-    "G": {"kernel": "sweep_track_kernel", "l2_read": 0.064507, "dram": 0.026707},
+    "G": {"kernel": "sweep_track_kernel", "l2_read": 0.064522, "dram": 0.026699},
 }
 
 
