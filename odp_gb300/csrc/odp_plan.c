@@ -499,12 +499,12 @@ static int small_yields(const odp_shape *sh, const odp_tuning *t, int part, int 
 /* How many levels of a general graph come from its neighbour lists (at least
  * `base`, 1 or 2; `chunks` bounds the counters) and the scratch that takes.  A
  * gathered level reads d + 1 lanes per row and 256 sources.  A level from the
- * lists marks d (d - 1)^(k - 1) vertices a row and queued all before them, at
- * about 0.7 of a lane each, and saves a barrier.  Measured on GB300, two levels
+ * lists marks up to d^k vertices a row (symmetric lists reach fewer) and queued
+ * all before them, at about 0.6 of a lane each, and saves a barrier; at least
+ * three warps of a CTA need their scratch rows.  Measured on GB300, two levels
  * against more (us): n = 65536, d = 16 (3 levels) 1656 / 1350; d = 6 (4) 2019 /
- * 1547, 5 levels 1818; d = 3 (8) 3440 / 2528, 10 levels 3020; d = 20 (3) 1616 /
- * 1548; d = 24 1796, 3 levels 2077; n = 30000, d = 8 (3) 374 / 320, 4 levels 343;
- * n = 16384, d = 4 (5) 152 / 135; d = 12 115, 3 levels 117. */
+ * 1547, 5 levels 1818; d = 20 (3) 1616 / 1548; d = 24 1796, 3 levels 2077; n =
+ * 30000, d = 8 (3) 374 / 320, 4 levels 343; n = 16384, d = 12 115, 3 levels 117. */
 static void choose_start(const odp_shape *sh, int base, int chunks, gbx_sweep *c)
 {
   const int n = shape_n(sh), d = sh->degree;
@@ -512,20 +512,21 @@ static void choose_start(const odp_shape *sh, int base, int chunks, gbx_sweep *c
   c->base = base;
   c->scratch_rows = 8;
   c->scratch_bits = c->B <= 32768 ? (c->B + 255) / 256 * 256 : 32768;
-  if(base < 2 || sh->symmetries > 1 || n > 131072) return;
-  double marks = d * (d - 1.0);
-  int queue = 1 + d;
-  while(c->base < GBX_SWEEP_BASE && marks * d + queue <= 1.45 * gathered + 64.0 &&
-        (c->base + 1) * c->nchunks <= 2 * chunks){
+  if(base < 2 || sh->symmetries > 1) return;
+  const double most = 1.57 * gathered + 64.0;
+  double marks = (double)d * d;
+  int queue = 1 + d, levels = 2;
+  while(levels < GBX_SWEEP_BASE && marks * d + queue + marks <= most && (levels + 1) * c->nchunks <= 2 * chunks){
     queue += (int)marks;
-    marks *= d - 1.0;
-    c->base++;
+    marks *= d;
+    levels++;
   }
-  if(c->base == 2) return;
+  const int bits = (n + 255) / 256 * 256, row = bits / 8 + (queue + 3) / 4 * 16;
+  if(levels == 2 || 3 * row > 36 * 1024) return;
+  c->base = levels;
   c->queue = (queue + 3) / 4 * 4;
-  c->scratch_bits = (n + 255) / 256 * 256;
-  const int row = c->scratch_bits / 8 + 4 * c->queue;    /* four CTAs per SM */
-  while(c->scratch_rows > 1 && c->scratch_rows * row > 36 * 1024) c->scratch_rows--;
+  c->scratch_bits = bits;
+  while(c->scratch_rows * row > 36 * 1024) c->scratch_rows--;      /* four CTAs per SM */
 }
 
 /* Whether no schedule setting asks for the persistent engine. */

@@ -402,9 +402,8 @@ __device__ void start_rows(const gbx_sweep &a, const int *list, unsigned *scratc
  * row and in its queue.  A gathered level reads d whole rows a row however few
  * bits they hold: for n = 65536, d = 16 level 3 took 500 us gathered and takes
  * 190 from the lists.  The counts of the levels before the last are of
- * vertices added.  A vertex list longer than the queue (its size is that of
- * symmetric lists) goes on from the bits: each lane keeps a copy of its
- * pieces in the row's place in memory and expands what was there. */
+ * vertices added.  The queue holds a whole tree of the levels before the last,
+ * whether or not the lists are symmetric. */
 __device__ void ball_rows(const gbx_sweep &a, const int *list, unsigned *scratch, unsigned *cnt, int r0, int nr)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -428,8 +427,7 @@ __device__ void ball_rows(const gbx_sweep &a, const int *list, unsigned *scratch
     }
     __syncwarp();
     int lo = 0, hi = 0;                                  /* the last level's vertices in the queue (level 1: the row itself) */
-    int level = 1;
-    for(; level < last; level++){
+    for(int level = 1; level < last; level++){
       unsigned *c = cnt + (level - 1) * a.nchunks;
       const int total = level == 1 ? q4 : (hi - lo) * q4;
       int end = hi;
@@ -458,8 +456,7 @@ __device__ void ball_rows(const gbx_sweep &a, const int *list, unsigned *scratch
             }
             const unsigned who = __ballot_sync(0xffffffffu, add);
             if(add){
-              const int at = end + __popc(who & below);
-              if(at < a.queue) queue[at] = v[m];
+              queue[end + __popc(who & below)] = v[m];
               atomicAdd(c + (v[m] >> (lL + 8)), 1u);
             }
             end += __popc(who);
@@ -469,9 +466,8 @@ __device__ void ball_rows(const gbx_sweep &a, const int *list, unsigned *scratch
       __syncwarp();
       lo = hi;
       hi = end;
-      if(hi > a.queue) { level++; break; }
     }
-    if(hi <= a.queue){
+    {
       const int total = (hi - lo) * q4;
       for(int i0 = lane; i0 < total; i0 += 192){
         int4 x[6];
@@ -490,32 +486,6 @@ __device__ void ball_rows(const gbx_sweep &a, const int *list, unsigned *scratch
         }
       }
     }
-    else
-      for(; level <= last; level++){
-        for(int p = lane; p < pieces; p += 32){
-          char *to = reinterpret_cast<char *>(a.start + (size_t)(p >> lL) * a.start_stride);
-          unsigned w[8];
-          *reinterpret_cast<uint4 *>(w) = sv[2 * p];
-          *reinterpret_cast<uint4 *>(w + 4) = sv[2 * p + 1];
-          st_lane(to + ((size_t)own << (a.wc_log2 + 3)) + (size_t)(p & (L - 1)) * 32, w);
-        }
-        __syncwarp();
-        for(int p = lane; p < pieces; p += 32){
-          const char *from = reinterpret_cast<const char *>(a.start + (size_t)(p >> lL) * a.start_stride);
-          const unsigned *w = reinterpret_cast<const unsigned *>(from + ((size_t)own << (a.wc_log2 + 3)) + (size_t)(p & (L - 1)) * 32);
-          for(int k = 0; k < 8; k++)
-            for(unsigned bits = __ldcg(w + k); bits; bits &= bits - 1u){
-              const int u = p * 256 + k * 32 + __ffs(bits) - 1;
-              for(int j = 0; j < a.e.d; j++){
-                const int v = __ldcg(a.e.nbr + (size_t)u * dp + j);
-                const unsigned bit = 1u << (v & 31);
-                if(!(atomicOr(s + (v >> 5), bit) & bit) && level < last)
-                  atomicAdd(cnt + (level - 1) * a.nchunks + (v >> (lL + 8)), 1u);
-              }
-            }
-        }
-        __syncwarp();
-      }
     __syncwarp();
     unsigned *c = cnt + (last - 1) * a.nchunks;
     for(int p0 = 0; p0 < pieces; p0 += 32){

@@ -140,9 +140,9 @@ def test_batches(count, n_hi):
                                       (5001, 5, "halves"), (20000, 5, "undirected"), (33000, 9, "directed"),
                                       (70000, 3, "halves")])
 def test_levels_from_the_lists(n, d, kind, monkeypatch):
-    """Three and more levels from the neighbour lists: queues that suffice
-    (undirected lists) and that run over (directed ones), rows of two lengths,
-    levels that end early (rings of 40, components), one group and several."""
+    """Three and more levels from the neighbour lists: undirected and directed
+    lists (whose trees fill the queue), rows of several lengths, levels that end
+    early (rings of 40, components), one group and several."""
     rng = np.random.default_rng(n)
     nd = None
     if kind == "undirected":
