@@ -159,6 +159,7 @@ __device__ __forceinline__ void group_state(const gbx_sweep &a, SweepPhase &p, i
   }
   const unsigned alive = __ballot_sync(0xffffffffu, nsrc > 0);
   const unsigned all = __reduce_add_sync(0xffffffffu, (unsigned)nsrc);
+  __syncwarp();                                        /* every lane has read the last group's state */
   if(q == 0){
     p.group = group;
     p.alive = alive;
@@ -186,6 +187,7 @@ __device__ __forceinline__ void arrive_step(const gbx_sweep &a, SweepShared &sh,
     sh.cnt[q] = 0;
   }
   const unsigned total = __reduce_add_sync(0xffffffffu, c);   /* rows x lanes x 256 of one CTA: below 2^32 */
+  __syncwarp();          /* lane 0's release covers the other lanes' counts (a reduction orders no memory) */
   if(q == 0){
     if(sh.rank == 0) sy.arrive[ph][(step + 1) % 3][0] = 0;
     arrive_word(&sy.arrive[ph][step % 3][0], ARRIVE_ONE | total);
@@ -195,7 +197,10 @@ __device__ __forceinline__ void arrive_step(const gbx_sweep &a, SweepShared &sh,
 }
 
 /* Warp 0 waits for the phase's last step and takes its count (true), or past
- * the limit gives up.  CTA 0 settles the step before meanwhile. */
+ * the limit gives up.  CTA 0 settles the step before meanwhile.  Lane 0
+ * acquires the barrier word; the warp barrier hands that on to the lanes that
+ * read the chunks' counts, and has them past their reads of the phase's state
+ * before lane 0 writes the next one. */
 template <class Sync>
 __device__ __forceinline__ bool wait_step(const gbx_sweep &a, SweepShared &sh, Sync &sy, int ph, bool added,
                                           int first_level, unsigned long long &bits)
@@ -206,6 +211,7 @@ __device__ __forceinline__ bool wait_step(const gbx_sweep &a, SweepShared &sh, S
   unsigned long long seen = 0;
   bool ok = true;
   if(threadIdx.x == 0) ok = wait_for(&sy.arrive[ph][(step - 1) % 3][0], ARRIVE_ONE * (unsigned)sh.size, seen, a.limit_ns);
+  __syncwarp();
   ok = __all_sync(0xffffffffu, ok);
   bits = __shfl_sync(0xffffffffu, seen, 0) & ARRIVE_BITS;
   return ok;
@@ -573,7 +579,9 @@ __device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, 
     unsigned long long bits;
     if(!wait_step(a, sh, sy, ph, false, base + 1, bits)) todo = TODO_ABORT;
     else{
-      if(bits == p.full || bits == p.total || p.level >= a.e.n){
+      const bool over = bits == p.full || bits == p.total || p.level >= a.e.n;
+      __syncwarp();
+      if(over){
         if(sh.rank == 0) settle_step(a, p, sy, ph, p.step - 1, p.level, false);
         group_state(a, p, ph, p.group + 1);
       }
@@ -602,7 +610,7 @@ __device__ __forceinline__ void plan_dense(const gbx_sweep &a, SweepShared &sh, 
       const unsigned alive = __ballot_sync(0xffffffffu, go);
       if(q == 0) p.alive = alive;
     }
-    __syncwarp();
+    __syncwarp();                                      /* read before it is written */
     if(over) group_state(a, p, ph, p.group + 1);
     else{
       todo = TODO_LEVEL;
@@ -879,14 +887,18 @@ __device__ __forceinline__ void plan_track(const gbx_sweep &a, SweepShared &sh, 
   unsigned long long bits;
   if(p.step > 0){
     if(!wait_step(a, sh, sy, 0, true, 1, bits)) todo = TODO_ABORT;
-    else if(p.level > 0 && (p.total + bits == p.full || bits == 0 || p.level >= a.e.n)){
-      if(sh.rank == 0) settle_step(a, p, sy, 0, p.step - 1, p.level, true);
-      group_state(a, p, 0, p.group + 1);
-      if(p.level < 0) todo = TODO_DONE;
-    }
-    else if(threadIdx.x == 0){
-      p.total += bits;
-      p.level++;
+    else{
+      const bool over = p.level > 0 && (p.total + bits == p.full || bits == 0 || p.level >= a.e.n);
+      __syncwarp();
+      if(over){
+        if(sh.rank == 0) settle_step(a, p, sy, 0, p.step - 1, p.level, true);
+        group_state(a, p, 0, p.group + 1);
+        if(p.level < 0) todo = TODO_DONE;
+      }
+      else if(threadIdx.x == 0){
+        p.total += bits;
+        p.level++;
+      }
     }
   }
   if(threadIdx.x == 0) sh.todo = todo;

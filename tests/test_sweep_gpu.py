@@ -186,3 +186,34 @@ def test_grids_of_three_ctas_per_sm(w, h, d, length, monkeypatch):
     b = og.Batch([og.GraphSpec(adj, grid=True, width=w, height=h)])
     assert same(got, b.run()[0])
     b.close()
+
+
+@pytest.mark.parametrize("kind", ["at once", "two phases", "tracking", "teams"])
+def test_chunk_counts_meet_the_barrier(kind, monkeypatch):
+    """Every lane of a CTA's first warp adds the counts of a chunk of its own
+    and one lane arrives for all of them: graphs of several chunks per barrier,
+    launched often, against the persistent engine."""
+    rng = np.random.default_rng(11)
+
+    def lists(n, d):
+        return np.stack([rng.permutation(n) for _ in range(d)], axis=1).astype(np.int32)
+
+    if kind == "tracking":
+        w, h = 150, 131
+        adj = og.conv_edge2adjacency_grid(w, h, og.generate_random_grid(w, h, 6, 6, 1, seed=9), 6, 1)
+        specs = [og.GraphSpec(adj, grid=True, width=w, height=h)]
+    elif kind == "teams":
+        specs = [og.GraphSpec(lists(n, 7), nodes=n) for n in (16000, 9000, 12289, 8193, 5000)]
+    else:
+        n = 16000 if kind == "at once" else 40000
+        specs = [og.GraphSpec(lists(n, 6), nodes=n)]
+    b = og.Batch(specs)
+    b.set_wait_limit(5 * 10 ** 9)
+    got = [b.run() for _ in range(40)]
+    b.close()
+    monkeypatch.setenv("ODP_GB300_SWEEP", "0")
+    b = og.Batch(specs)
+    want = b.run()
+    b.close()
+    for run in got:
+        assert all(same(x, y) for x, y in zip(run, want))
