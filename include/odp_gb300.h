@@ -261,6 +261,9 @@ int  ODPX_Anneal_run(ODPX_Anneal *anneal, int steps);
  * graphs (int[nodes/symmetries][degree] each; NULL to skip). */
 int  ODPX_Anneal_state(ODPX_Anneal *anneal, int chain, ODPX_Chain_state *state, int *adjacency,
                        int *best_adjacency);
+/* Longest wait of a CTA for the others of its chain, or for work of the engine
+ * (default 60 s).  A chain whose wait ran out stops with its status set. */
+void ODPX_Anneal_set_wait_limit(ODPX_Anneal *anneal, unsigned long long ns);
 void ODPX_Anneal_destroy(ODPX_Anneal *anneal);
 
 const char *ODPX_Version(void);

@@ -711,6 +711,8 @@ def _bind_anneal(lib):
     lib.ODPX_Anneal_run.argtypes = [P, ctypes.c_int]
     lib.ODPX_Anneal_state.restype = ctypes.c_int
     lib.ODPX_Anneal_state.argtypes = [P, ctypes.c_int, ctypes.POINTER(ChainState), P, P]
+    lib.ODPX_Anneal_set_wait_limit.restype = None
+    lib.ODPX_Anneal_set_wait_limit.argtypes = [P, ctypes.c_ulonglong]
     lib.ODPX_Anneal_destroy.restype = None
     lib.ODPX_Anneal_destroy.argtypes = [P]
     lib._anneal_bound = True
@@ -768,6 +770,9 @@ class Anneal:
         if graphs:
             out["adjacency"], out["best_adjacency"] = cur, best
         return out
+
+    def set_wait_limit(self, ns):
+        load().ODPX_Anneal_set_wait_limit(self._h, int(ns))
 
     def close(self):
         if self._h:

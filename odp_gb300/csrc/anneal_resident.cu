@@ -471,7 +471,10 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
     /* a lane per thread is enough: more CTAs only lengthen the barrier */
     const int want = (int)(((long long)c.n * t.lanes + THREADS - 1) / THREADS);
     t.size = CLUSTER ? hi - lo : min(hi - lo, want);
-    if(t.rank >= t.size) continue;                       /* this CTA has no part */
+    /* This CTA has no part in the chain.  Its step counter stays behind the
+     * team's, so it may have none in any other: a team of several CTAs has one
+     * chain, and several chains share a team only where teams have one CTA. */
+    if(t.rank >= t.size) continue;
     t.rows = (c.n + t.size - 1) / t.size;
     t.r0 = t.rank * t.rows;
     t.nr = max(0, min(t.rows, c.n - t.r0));
@@ -495,11 +498,8 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
     }
     /* every CTA has its copy of the adjacency before the first one writes to it */
     unsigned long long bits, bits1;
-    if(!team_pass<CLUSTER>(sh, t, p.limit_ns, false, bits, bits1)){
-      if(tid == 0) sh.c.status = GBX_CHAIN_ERR_EVAL;
-      __syncthreads();
-    }
-    for(int step = 0; step < p.steps && !sh.c.status; step++){
+    bool met = team_pass<CLUSTER>(sh, t, p.limit_ns, false, bits, bits1);
+    for(int step = 0; met && step < p.steps && !sh.c.status; step++){
       if(tid == 0) sh.ok = propose(sh);
       __syncthreads();
       if(!sh.ok){                                        /* in every CTA: out of draws */
@@ -511,11 +511,8 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
       __syncthreads();
       int level = 0;
       long long sum = 0;
-      if(!evaluate<CLUSTER>(sh, t, p.limit_ns, level, sum)){
-        if(tid == 0) sh.c.status = GBX_CHAIN_ERR_EVAL;
-        __syncthreads();
-        break;
-      }
+      met = evaluate<CLUSTER>(sh, t, p.limit_ns, level, sum);
+      if(!met) break;
       if(tid == 0) decide(sh, level, sum);
       __syncthreads();
       if(sh.copy && t.rank == 0)
@@ -528,12 +525,21 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
         __syncthreads();
       }
     }
+    /* A CTA whose wait ran out left with the rows it had, perhaps before a
+     * decision that all others took: the first CTA then misses it here, if not
+     * before, and the chain is stopped. */
+    if(met && sh.c.status != GBX_CHAIN_ERR_EVAL) met = team_pass<CLUSTER>(sh, t, p.limit_ns, false, bits, bits1);
+    if(!met && tid == 0){
+      sh.c.status = GBX_CHAIN_ERR_EVAL;
+      *p.late = 1u;
+    }
+    __syncthreads();
     /* the records and the neighbour table, for the host and the next launch;
      * after a run the chain also goes to host memory, a part from each CTA:
-     * three copies and a synchronise per chain took 40 us */
-    if(p.host_chains && sh.c.status != GBX_CHAIN_ERR_EVAL) team_pass<CLUSTER>(sh, t, p.limit_ns, false, bits, bits1);
-    __syncthreads();
-    if(p.host_chains){
+     * three copies and a synchronise per chain took 40 us.  A CTA that has not
+     * met the others copies nothing: the first one may still be writing the
+     * graph. */
+    if(met && p.host_chains){
       const int ints = c.base * c.d;
       int *to = p.host_graphs + p.host_offset[chain];
       for(int i = t.rank * THREADS + tid; i < ints; i += t.size * THREADS){

@@ -43,6 +43,7 @@ struct odpx_anneal {
   char *h_res;                 /* pinned: the chains' records and graphs after a run, or NULL */
   gbx_chain *dh_chains;
   int h_current;               /* they are the chains' state */
+  unsigned int *h_late;        /* pinned: a wait of the last run ran out */
   unsigned long long *h_offset; /* in ints, chain k's graphs among them */
 };
 
@@ -86,6 +87,7 @@ void ODPX_Anneal_destroy(ODPX_Anneal *a)
   if(a->p) odp_plan_destroy(a->p);
   gbx_free(a->d_res);
   gbx_host_free(a->h_res);
+  gbx_host_free(a->h_late);
   free(a->h_offset);
   gbx_free(a->d_chains); gbx_free(a->d_best); gbx_free(a->d_rowdeg); gbx_free(a->d_state_init);
   free(a->h_chains);
@@ -162,7 +164,8 @@ static int plan_resident(ODPX_Anneal *a, int blocks)
     a->res_cluster = resident_cluster(a, range, most, &smem);
     const size_t sync = gbx_resident_sync_bytes() * (size_t)teams, offs = (sizeof(unsigned long long) * (size_t)a->count + 255) & ~(size_t)255;
     unsigned long long *off = calloc(1, 2 * offs), at = 0, to = 0;
-    if(!off || gbx_malloc(&a->d_res, sync + 2 * offs + 8 * words)){
+    if(!off || (!a->h_late && gbx_host_alloc((void **)&a->h_late, sizeof(unsigned int))) ||
+       gbx_host_device_ptr(a->h_late, (void **)&a->res.late) || gbx_malloc(&a->d_res, sync + 2 * offs + 8 * words)){
       free(off);
       a->d_res = NULL;
       return 0;
@@ -173,6 +176,7 @@ static int plan_resident(ODPX_Anneal *a, int blocks)
       at += 64ull * (unsigned long long)p->g[i].n * (unsigned long long)((p->g[i].B + 255) / 256);
       to += 2ull * (unsigned long long)p->g[i].B * (unsigned long long)p->g[i].d;
     }
+    *a->h_late = 0;
     a->res.chains = a->d_chains;
     a->res.sync = a->d_res;
     a->res.host_offset = (const unsigned long long *)((char *)a->d_res + sync);
@@ -326,7 +330,9 @@ int ODPX_Anneal_run(ODPX_Anneal *a, int steps)
         return ODPX_ERR_CUDA;
     }
     if(gbx_stream_sync(p->stream)) return ODPX_ERR_CUDA;
-    a->h_current |= host;
+    /* after a wait that ran out the state is read from the device, as that of the stepwise kernels */
+    a->h_current |= host && !*a->h_late;
+    *a->h_late = 0;
     return 0;
   }
   if(steps >= ANNEAL_GRAPH_STEPS){
@@ -347,6 +353,19 @@ int ODPX_Anneal_run(ODPX_Anneal *a, int steps)
   for(; s < steps; s++)
     if(enqueue_step(a)) return ODPX_ERR_CUDA;
   return gbx_stream_sync(p->stream) ? ODPX_ERR_CUDA : 0;
+}
+
+void ODPX_Anneal_set_wait_limit(ODPX_Anneal *a, unsigned long long ns)
+{
+  if(!a || a->p->spin_limit_ns == ns) return;
+  a->p->spin_limit_ns = ns;
+  a->res.limit_ns = ns;
+  /* the limit is an argument of the captured engine launches: capture anew */
+  if(a->steps_exec){
+    gbx_stream_sync(a->p->stream);
+    gbx_graph_destroy(a->steps_exec);
+    a->steps_exec = NULL;
+  }
 }
 
 static void fill_state(const gbx_chain *c, ODPX_Chain_state *st)

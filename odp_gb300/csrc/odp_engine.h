@@ -324,6 +324,8 @@ typedef struct {
   const unsigned long long *buf_offset;
   void *sync;                  /* gbx_resident_sync_bytes() per team, zeroed before the launch */
   unsigned long long limit_ns; /* longest wait of a CTA for its team */
+  unsigned int *late;          /* device address of pinned memory: set when a wait ran out, and the host's
+                                  graphs are then not the chains' */
   int count, teams, steps;
   gbx_chain *host_chains;      /* device address of pinned memory that takes the records, or NULL */
   int *host_graphs;            /* and the graphs: chain k's adj, then its best_adj, at host_offset[k] */

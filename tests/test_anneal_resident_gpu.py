@@ -65,3 +65,29 @@ def test_resident_steps_equal_the_stepwise_kernels(name, monkeypatch):
             assert x == y, (name, k, steps)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,d,count", [(4096, 16, 1), (1500, 12, 3)])
+def test_a_wait_that_runs_out_stops_the_chain(n, d, count):
+    """A limit of 1 ns ends the waits of a chain's CTAs for one another: the
+    chain stops with its status set, counts no step, and the state that is
+    reported is the graph it holds (each edge in both its rows, at most one
+    proposal away from the last one), not what its CTAs copied without having
+    met."""
+    kw = dict(max_temp=50.0, min_temp=0.5, ncalcs=200)
+    a = og.Anneal([og.Chain(general(n, d, 1, k), nodes=n, seed=k + 1, **kw) for k in range(count)])
+    a.run(6)
+    before = [a.state(k, graphs=True) for k in range(count)]
+    assert all(x["status"] == 0 and x["steps"] == 6 for x in before)
+    a.set_wait_limit(1)
+    for _ in range(2):
+        a.run(3)
+        for k in range(count):
+            x = a.state(k, graphs=True)
+            assert x["status"] == 2 and x["steps"] == 6, x["status"]
+            assert np.count_nonzero(x["adjacency"] != before[k]["adjacency"]) <= 4
+            assert np.array_equal(x["best_adjacency"], before[k]["best_adjacency"])
+            u = np.repeat(np.arange(n), d)
+            pairs = np.stack([u, x["adjacency"].ravel()])
+            assert np.array_equal(np.sort(pairs[0] * n + pairs[1]), np.sort(pairs[1] * n + pairs[0]))
+    a.close()
