@@ -499,6 +499,7 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
     /* every CTA has its copy of the adjacency before the first one writes to it */
     unsigned long long bits, bits1;
     bool met = team_pass<CLUSTER>(sh, t, p.limit_ns, false, bits, bits1);
+    __syncthreads();                                     /* sh.ok is read before the proposal writes it */
     for(int step = 0; met && step < p.steps && !sh.c.status; step++){
       if(tid == 0) sh.ok = propose(sh);
       __syncthreads();

@@ -91,3 +91,20 @@ def test_a_wait_that_runs_out_stops_the_chain(n, d, count):
             pairs = np.stack([u, x["adjacency"].ravel()])
             assert np.array_equal(np.sort(pairs[0] * n + pairs[1]), np.sort(pairs[1] * n + pairs[0]))
     a.close()
+
+
+@pytest.mark.parametrize("n,d,count", [(64, 4, 3), (1024, 8, 16), (4096, 16, 1), (90, 5, 700)])
+def test_a_graph_without_return_edges_stops_at_its_first_proposal(n, d, count):
+    """Every thread of a team takes the same way when the proposal fails: one
+    CTA a chain, clusters and teams in global memory."""
+    rng = np.random.default_rng(n)
+    v = np.arange(n)
+    adj = np.stack([(v + s) % n for s in rng.permutation(n // 2 - 1)[:d] + 1], axis=1).astype(np.int32)   # one way round
+    a = og.Anneal([og.Chain(adj, nodes=n, seed=k + 1, max_temp=50.0, min_temp=0.5, ncalcs=200) for k in range(count)])
+    for _ in range(2):
+        a.run(3)
+        for k in range(count):
+            x = a.state(k, graphs=True)
+            assert x["status"] == 1 and x["steps"] == 0
+            assert np.array_equal(x["adjacency"], adj) and np.array_equal(x["best_adjacency"], adj)
+    a.close()
