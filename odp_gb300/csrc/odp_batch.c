@@ -224,6 +224,7 @@ int ODPX_Batch_time_mode(ODPX_Batch *p, const int *const *adjacency, int repeats
   for(int i = 0; i < 2 * repeats; i++) gbx_event_destroy(ev[i]);
   free(ev);
   if(!rc && (odp_plan_error(p) & GBX_ERR_TIMEOUT)) rc = ODPX_ERR_TIMEOUT;
+  if(p->h_abort) *p->h_abort = 0;              /* reported: the next run starts afresh */
   *ms_per_run = (float)(total / repeats);
   return rc;
 }

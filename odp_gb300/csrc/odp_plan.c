@@ -1497,12 +1497,22 @@ static int take_records(odp_plan *p)
   return 0;
 }
 
+/* Whether every record is the last launch's. */
+static int records_current(const odp_plan *p)
+{
+  for(int k = 0; k < p->njobs; k++)
+    if(GBX_REC_SEQ(__atomic_load_n(&p->h_small_rec[k].err, __ATOMIC_ACQUIRE)) != p->seq) return 0;
+  return 1;
+}
+
 int odp_plan_finish(odp_plan *p, odp_result *results)
 {
   if(p->seq ? take_records(p) : gbx_stream_sync(p->stream)) return ODPX_ERR_CUDA;
   if(p->h_abort && *p->h_abort){
+    /* a wait that ran out behind the last record (a CTA with nothing left to
+     * do; perhaps the launch's before this one) has spoiled nothing */
     *p->h_abort = 0;
-    return ODPX_ERR_TIMEOUT;
+    if(!p->seq || !records_current(p)) return ODPX_ERR_TIMEOUT;
   }
   if(p->small || p->sweep || p->team) return finish_small(p, results);
   const gbx_ctrl *ctrl = (const gbx_ctrl *)p->h_state_out;

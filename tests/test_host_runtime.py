@@ -1,0 +1,97 @@
+"""The host runtime (plans, batches, servers, annealing) over a CUDA layer
+without a GPU (c/fake_gpu.c): what it does when launches fail, and which
+kernels it launches."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import odp_gb300 as og
+from conftest import ROOT
+from odp_gb300 import build
+
+KINDS = ("engine", "small", "sweep", "team", "resident", "step", "pull")
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    subprocess.run(["gcc", "-O1", "-std=gnu11", "-fPIC", "-shared", "-w", "-I", build.INCLUDE, "-I", build.CSRC, "-o", so,
+                    os.path.join(ROOT, "tests", "c", "fake_gpu.c")] +
+                   [os.path.join(build.CSRC, f) for f in build.C_SOURCES] + ["-lm", "-lpthread"], check=True)
+    return so
+
+
+class Fake:
+    """The fake layer's counters and switches, in the loaded library."""
+
+    def __init__(self, lib):
+        object.__setattr__(self, "lib", lib)
+        self.counts = 0
+
+    def __setattr__(self, name, value):
+        if name == "counts":
+            (ctypes.c_int * len(KINDS)).in_dll(self.lib, "fake_launches")[:] = [value] * len(KINDS)
+        else:
+            ctypes.c_int.in_dll(self.lib, "fake_" + name).value = value
+
+    def __getattr__(self, name):
+        if name == "counts":
+            return {k: v for k, v in zip(KINDS, (ctypes.c_int * len(KINDS)).in_dll(self.lib, "fake_launches")) if v}
+        return ctypes.c_int.in_dll(self.lib, "fake_" + name).value
+
+
+@pytest.fixture
+def fake(library, monkeypatch):
+    """The package on the fake layer, without CUDA graphs."""
+    monkeypatch.setattr(og, "LIB_PATH", library)
+    monkeypatch.setattr(og, "_lib", None)
+    monkeypatch.setenv("ODP_GB300_GRAPH", "0")
+    f = Fake(og.load())
+    yield f
+    f.abort_at = f.late_at = f.pending = 0
+
+
+def ring(n, d=4):
+    v = np.arange(n)
+    return np.stack([(v + 1 + k) % n for k in range(d)], axis=1).astype(np.int32)
+
+
+def timed_out(call):
+    with pytest.raises(og.ODPError) as e:
+        call()
+    return e.value.code == og.ERR_TIMEOUT
+
+
+def plans():
+    return {"sweep": [og.GraphSpec(ring(6000), nodes=6000)],
+            "team": [og.GraphSpec(ring(n), nodes=n) for n in (6000, 9000, 700)]}
+
+
+@pytest.mark.parametrize("kind", ["sweep", "team"])
+def test_a_wait_that_ran_out_fails_its_own_call_only(fake, kind):
+    """In a run, and in a timed launch after a warm one."""
+    b = og.Batch(plans()[kind])
+    b.run()
+    assert fake.counts == {kind: 1}
+    fake.abort_at = fake.total + 1
+    assert timed_out(b.run)
+    b.run()
+    fake.abort_at = fake.total + 3
+    assert timed_out(lambda: b.time(4))
+    b.run()
+    b.close()
+
+
+def test_a_wait_that_ran_out_behind_the_last_record_is_no_failure(fake):
+    """All records of a launch are its results, also when a CTA that had nothing
+    left to do gave up its wait for the last barrier, before or after the host
+    looked."""
+    b = og.Batch(plans()["sweep"])
+    want = b.run()
+    fake.late_at = fake.total + 1
+    assert b.run() == want
+    assert b.run() == want
+    b.close()

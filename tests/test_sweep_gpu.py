@@ -217,3 +217,26 @@ def test_chunk_counts_meet_the_barrier(kind, monkeypatch):
     b.close()
     for run in got:
         assert all(same(x, y) for x, y in zip(run, want))
+
+
+@pytest.mark.parametrize("count,n_hi", [(2, 3000), (17, 6000), (60, 2000)])
+def test_batches_after_a_wait_that_runs_out(count, n_hi):
+    """The teams give up their waits for one another, and the plan's next runs
+    start from clean counters."""
+    rng = np.random.default_rng(count + 1)
+    specs = [random_spec(rng, n_hi) for _ in range(count)]
+    b = og.Batch(specs)
+    b.set_wait_limit(5 * 10 ** 9)
+    want = b.run()
+    for _ in range(2):
+        b.set_wait_limit(1)
+        with pytest.raises(og.ODPError) as e:
+            b.run()
+        assert e.value.code == og.ERR_TIMEOUT
+        with pytest.raises(og.ODPError) as e:
+            b.time(3)
+        assert e.value.code == og.ERR_TIMEOUT
+        b.set_wait_limit(5 * 10 ** 9)
+        for _ in range(2):
+            assert all(same(x, y) for x, y in zip(b.run(), want))
+    b.close()
