@@ -582,9 +582,11 @@ int gbx_resident_blocks(size_t smem, int *per_sm)
   if(smem > GBX_SWEEP_SMEM_MAX) return (int)cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute((const void *)anneal_resident_kernel<false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, GBX_SWEEP_SMEM_MAX);
-  if(e != cudaSuccess) return (int)e;
-  return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, (const void *)anneal_resident_kernel<false>,
-                                                            RESIDENT_THREADS, smem);
+  if(e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, (const void *)anneal_resident_kernel<false>,
+                                                      RESIDENT_THREADS, smem);
+  if(e != cudaSuccess) cudaGetLastError();
+  return (int)e;
 }
 
 static void resident_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, int blocks, size_t smem, int cluster)
@@ -614,7 +616,10 @@ int gbx_resident_clusters(int cluster, size_t smem, int *active)
   if(e == cudaSuccess)
     e = cudaFuncSetAttribute((const void *)anneal_resident_kernel<true>,
                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if(e != cudaSuccess) return (int)e;
+  if(e != cudaSuccess){
+    cudaGetLastError();
+    return (int)e;
+  }
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = {};
   resident_config(cfg, attr, cluster, smem, cluster);

@@ -1139,14 +1139,22 @@ int gbx_l2_read_probe(size_t bytes, int reps, double *gbs)
   return (int)e;
 }
 
-int gbx_malloc(void **p, size_t bytes) { return (int)cudaMalloc(p, bytes ? bytes : 256); }
+/* The result of a call whose failure the caller may live with: it is also the
+ * thread's last error, which the next launch would take for its own. */
+static int refused(cudaError_t e)
+{
+  if(e != cudaSuccess) cudaGetLastError();
+  return (int)e;
+}
+
+int gbx_malloc(void **p, size_t bytes) { return refused(cudaMalloc(p, bytes ? bytes : 256)); }
 int gbx_mem_free(size_t *bytes)
 {
   size_t total = 0;
-  return (int)cudaMemGetInfo(bytes, &total);
+  return refused(cudaMemGetInfo(bytes, &total));
 }
 int gbx_free(void *p) { return p ? (int)cudaFree(p) : 0; }
-int gbx_host_alloc(void **p, size_t bytes) { return (int)cudaMallocHost(p, bytes ? bytes : 64); }
+int gbx_host_alloc(void **p, size_t bytes) { return refused(cudaMallocHost(p, bytes ? bytes : 64)); }
 int gbx_host_free(void *p) { return p ? (int)cudaFreeHost(p) : 0; }
 
 int gbx_stream_create(void **stream)
@@ -1223,7 +1231,7 @@ int gbx_small_clusters(int cluster, int threads, size_t smem_bytes, int *active)
   if(!small_shape_ok(cluster, threads, smem_bytes)) return (int)cudaErrorInvalidValue;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = small_config(1, cluster, threads, smem_bytes, 0, attr);
-  return (int)cudaOccupancyMaxActiveClusters(active, small_kernel, &cfg);
+  return refused(cudaOccupancyMaxActiveClusters(active, small_kernel, &cfg));
 }
 
 int gbx_small_launch(const gbx_job *d_jobs, int njobs, const gbx_expand_desc *descs, const gbx_expand_desc *desc0,
@@ -1242,7 +1250,7 @@ int gbx_small_launch(const gbx_job *d_jobs, int njobs, const gbx_expand_desc *de
 
 int gbx_host_device_ptr(void *host, void **dev)
 {
-  return (int)cudaHostGetDevicePointer(dev, host, 0);
+  return refused(cudaHostGetDevicePointer(dev, host, 0));
 }
 
 int gbx_pull(const gbx_expand_desc *h_descs, gbx_expand_desc *d_descs, int ndesc, void *d_state,

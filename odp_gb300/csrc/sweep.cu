@@ -1060,6 +1060,16 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) team_kernel(const gbx_team t
 
 extern "C" {
 
+/* Resident CTAs per SM of `entry` with that much shared memory: an answer, not
+ * an error that the next launch would take for its own. */
+static int resident(const void *entry, size_t smem, int *per_sm)
+{
+  cudaError_t e = cudaFuncSetAttribute(entry, cudaFuncAttributeMaxDynamicSharedMemorySize, GBX_SWEEP_SMEM_MAX);
+  if(e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, entry, SWEEP_THREADS, smem);
+  if(e != cudaSuccess) cudaGetLastError();
+  return (int)e;
+}
+
 size_t gbx_sweep_sync_bytes(void) { return 2 * sizeof(SweepSync); }
 
 size_t gbx_sweep_smem(const gbx_sweep *a)
@@ -1087,10 +1097,7 @@ int gbx_sweep_blocks(const gbx_sweep *a, int *per_sm)
   *per_sm = 0;
   const size_t smem = gbx_sweep_smem(a);
   if(smem > GBX_SWEEP_SMEM_MAX) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(sweep_entry(a), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       GBX_SWEEP_SMEM_MAX);
-  if(e != cudaSuccess) return (int)e;
-  return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, sweep_entry(a), SWEEP_THREADS, smem);
+  return resident(sweep_entry(a), smem, per_sm);
 }
 
 static int launch_all(const void *entry, void *arg, int blocks, size_t smem, cudaStream_t stream)
@@ -1121,10 +1128,7 @@ int gbx_team_blocks(size_t smem, int *per_sm)
 {
   *per_sm = 0;
   if(smem > GBX_SWEEP_SMEM_MAX) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute((const void *)team_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       GBX_SWEEP_SMEM_MAX);
-  if(e != cudaSuccess) return (int)e;
-  return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, (const void *)team_kernel, SWEEP_THREADS, smem);
+  return resident((const void *)team_kernel, smem, per_sm);
 }
 
 int gbx_team_launch(const gbx_team *t, int blocks, size_t smem, void *stream)

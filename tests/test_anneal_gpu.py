@@ -204,3 +204,21 @@ def test_bad_chains_are_refused():
     with pytest.raises(og.ODPError) as ei:
         og.Anneal([og.Chain(adj, 64, max_temp=0.0)])
     assert ei.value.code == og.ERR_INVALID
+
+
+def test_an_allocation_that_failed_fails_no_later_launch(monkeypatch):
+    """The chains fall back to the stepwise kernels where the resident kernel's
+    memory cannot be had; the failed allocation must not remain as the error
+    that their launches then report."""
+    import ctypes
+    monkeypatch.setenv("ODP_GB300_ANNEAL_RESIDENT", "0")
+    n, d = 300, 6
+    adj = og.conv_edge2adjacency_general(n, og.generate_random_general(n, d, seed=3), d)
+    a = og.Anneal([og.Chain(adj, nodes=n, seed=4)])
+    p = ctypes.c_void_p()
+    lib = og.load()
+    lib.gbx_malloc.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t]
+    assert lib.gbx_malloc(ctypes.byref(p), 1 << 60) != 0
+    a.run(2)
+    assert a.state(0)["steps"] == 2
+    a.close()
