@@ -11,15 +11,16 @@
  * was rejected.  A scheduler thread admits pending requests into lanes.  A
  * lane is a CUDA stream with its own pool of bitset memory (the budget is
  * divided among lanes) and launches sized to its share of the GPU, so a batch
- * admitted while others are running overlaps with them on the device.  A
- * batch of general graphs that fit there is one launch of the team kernel,
- * which reads its arguments and the deltas from pinned memory, applies the
- * deltas and writes its records to pinned memory.  The others, and all
- * batches formed while one of those is in flight, run on the persistent engine, in stream order: the deltas are
- * applied by one scatter kernel (to the compact adjacency and to every
- * neighbour-table row they touch), the jobs and engine state are uploaded, the
- * engine runs, and the per-graph accumulators come back.  A graph is never in
- * two batches at once, so a delta never races an evaluation of the same graph.
+ * admitted while others are running overlaps with them on the device.  While
+ * every registered graph is a general one that fits there, a batch is one
+ * launch of the team kernel, which reads its arguments and the deltas from
+ * pinned memory, applies the deltas and writes its records to pinned memory.
+ * Otherwise all batches run on the persistent engine, in stream order: the
+ * deltas are applied by one scatter kernel (to the compact adjacency and to
+ * every neighbour-table row they touch), the jobs and engine state are
+ * uploaded, the engine runs, and the per-graph accumulators come back.  A
+ * graph is never in two batches at once, so a delta never races an evaluation
+ * of the same graph.
  *
  * Results are bit-identical to ODP_Init_aspl_* + ODP_Set_aspl on the updated
  * adjacency.
@@ -116,6 +117,7 @@ struct odp_server {
   int team_grid;               /* CTAs of the team kernel on the whole GPU (0: not used) */
   double l2_lane_bytes;        /* bitset working set a lane keeps active at once (L2 share) */
   double min_cost, max_cost;   /* over the registered graphs */
+  int mixed;                   /* some registered graph does not fit the team kernel */
   ODPX_Serve_counters stats;
 };
 
@@ -364,11 +366,6 @@ static int form_batch(odp_server *s, serve_lane *l, double max_seed_cost)
 {
   int nreq = 0, njobs = 0, nw = 0;
   double seed_cost = 0;
-  /* A cooperative launch waits until all its CTAs fit, and the engine's CTAs
-   * stay for a whole batch, so no team batch is issued beside an engine's:
-   * with chains of n = 16384 and 32768 on the other lanes it waited 12 ms. */
-  int engine = 0;
-  for(int i = 0; i < s->cfg.lanes; i++) engine |= s->lanes[i].busy && !s->lanes[i].team;
   for(long long id = s->next_pending; id < s->nreqs && nreq < l->max_batch; id++){
     serve_req *r = &s->reqs[id];
     if(r->state != 0) continue;
@@ -377,10 +374,9 @@ static int form_batch(odp_server *s, serve_lane *l, double max_seed_cost)
     /* A batch holds requests of similar cost (within 4x of the oldest one it
      * takes): a request completes only when its whole batch does, so a small
      * graph batched with a large one would wait for it. */
-    int other_class = nreq > 0 ? (g->cost > 4.0 * seed_cost || 4.0 * g->cost < seed_cost || (l->team && !g->team))
-                               : g->cost > max_seed_cost;
+    int other_class = nreq > 0 ? (g->cost > 4.0 * seed_cost || 4.0 * g->cost < seed_cost) : g->cost > max_seed_cost;
     if(g->busy || other_class || njobs + g->nchunks > l->max_jobs || nw + need_w > l->max_writes) continue;
-    if(nreq == 0){ seed_cost = g->cost; l->team = g->team && !engine; }
+    if(nreq == 0){ seed_cost = g->cost; l->team = !s->mixed; }
     const int w0 = nw;
     for(int k = 0; k < r->ndelta; k++) nw += delta_writes(g, &r->deltas[k], l->h_writes + nw);
     free(r->deltas);
@@ -677,10 +673,12 @@ int ODPX_Serve_register(ODPX_Server *s, const ODP_Graph *gr, int *handle)
   odp_tuning tuning;
   odp_tuning_for(2, &tuning);
   const int team_blocks = s->lanes[0].team_blocks;
-  /* The team kernel takes general graphs that fit a lane when they have it to
-   * themselves: one launch in place of five operations, and no hand-off per
-   * tile.  32 chains of n = 1024 to 4096, d = 16: 617 -> 392 us a round; one
-   * request alone 70 -> 46 us (n = 1024), 107 -> 66 us (n = 4096). */
+  /* The team kernel takes general graphs that fit a lane: one launch in place
+   * of five operations, and no hand-off per tile.  32 chains of n = 1024 to
+   * 4096, d = 16: 617 -> 392 us a round; one request alone 70 -> 46 us (n =
+   * 1024), 107 -> 66 us (n = 4096).  With a graph for the engine among them
+   * all stay on the engine: an engine batch keeps the SMs that it finds free
+   * when it starts, and a team kernel takes half of an SM's registers a CTA. */
   if(!gr->grid && team_blocks > 0 && odp_team_shape(&sh, &tuning, &g.sw, &g.est) && g.sw.nchunks <= TEAM_RECS){
     g.sw.rows = (n + team_blocks - 1) / team_blocks;
     g.team = gbx_sweep_smem(&g.sw) <= ODP_TEAM_SMEM && g.est.need + 1024.0 <= (double)s->lanes[0].arena_bytes;
@@ -758,6 +756,7 @@ int ODPX_Serve_register(ODPX_Server *s, const ODP_Graph *gr, int *handle)
     s->graphs = realloc(s->graphs, sizeof(serve_graph) * (size_t)s->cap_graphs);
   }
   s->graphs[s->ngraphs] = g;
+  s->mixed |= !g.team;
   if(s->ngraphs == 0 || g.cost < s->min_cost) s->min_cost = g.cost;
   if(s->ngraphs == 0 || g.cost > s->max_cost) s->max_cost = g.cost;
   *handle = s->ngraphs++;

@@ -95,3 +95,24 @@ def test_a_wait_that_ran_out_behind_the_last_record_is_no_failure(fake):
     assert b.run() == want
     assert b.run() == want
     b.close()
+
+
+def served(server, graphs):
+    handles = [server.register(g) for g in graphs]
+    for _ in range(2):
+        for r in [server.submit(h, []) for h in handles]:
+            server.wait(r)
+
+
+def test_a_server_with_graphs_for_the_engine_keeps_all_on_it(fake):
+    """Team batches take SMs from an engine batch that starts beside them."""
+    general = [og.GraphSpec(ring(n), nodes=n) for n in (300, 2000)]
+    grid = og.GraphSpec(ring(400), grid=True, width=20, height=20)
+    srv = og.Server(max_nodes=2000, memory_mb=64)
+    served(srv, general)
+    assert set(fake.counts) == {"team"}
+    fake.counts = 0
+    served(srv, [grid])
+    served(srv, general)
+    assert set(fake.counts) == {"engine"}
+    srv.close()
