@@ -249,6 +249,7 @@ typedef struct {
   const gbx_sweep *graphs;
   const int *order;                    /* NULL: graphs[] is in queue order */
   const unsigned long long *adj;       /* this call's host arrays (device memory), or NULL: graphs[g].e.adj */
+  int page_ints;                       /* of a page of host memory */
   unsigned int *next;                  /* [GBX_TEAM_SPLITS], zeroed before the launch, as are the nodes */
   void *nodes;                         /* gbx_team_node_bytes() for each team of first_split .. last_split */
   unsigned char *arena;                /* the teams' bitsets: arena_bytes >> k for each of 2^k teams */

@@ -1154,6 +1154,8 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
       tm->nodes = (char *)p->d_sync + 256;
       tm->arena = (unsigned char *)p->d_slotbuf;
       tm->abort_flag = p->sw.abort_flag;
+      const long page = sysconf(_SC_PAGESIZE);
+      tm->page_ints = (int)((page > 0 ? page : 4096) / (long)sizeof(int));
       CK(gbx_memcpy_h2d(dev, p->h_teams, args, p->stream));
       CK(gbx_memcpy_h2d(dev + args + ptrs, team_order, sizeof(int) * (size_t)count, p->stream));
     }

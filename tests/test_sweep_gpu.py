@@ -240,3 +240,33 @@ def test_batches_after_a_wait_that_runs_out(count, n_hi):
         for _ in range(2):
             assert all(same(x, y) for x, y in zip(b.run(), want))
     b.close()
+
+
+def test_batches_of_arrays_anywhere():
+    """Every page of the arrays is asked for before the graphs are taken: arrays
+    off 16-byte boundaries, ending with a page and a word behind one, new ones on
+    each run, and one without entries."""
+    import mmap
+    rng = np.random.default_rng(21)
+    page = mmap.PAGESIZE // 4
+    shapes = [(2048, 8), (page // 4, 4), (page // 4 + 1, 4), (5000, 13), (97, 5), (100, 0), (6001, 11)]
+    want = None
+    for run in range(3):
+        arrays, keep = [], []
+        for n, d in shapes:
+            m = mmap.mmap(-1, (n * d * 4 // mmap.PAGESIZE + 2) * mmap.PAGESIZE)
+            keep.append(m)
+            at = len(m) - 4 * n * d if run == 0 else 4 * run       # the last entries of the mapping, then odd offsets
+            a = np.frombuffer(m, dtype=np.int32, count=n * d, offset=at).reshape(n, d)
+            if want is None:
+                a[:] = np.stack([rng.permutation(n) for _ in range(d)], axis=1) if d else 0
+            else:
+                a[:] = first[len(arrays)]
+            arrays.append(a)
+        if want is None:
+            first = [a.copy() for a in arrays]
+            want = [oracle.aspl(a, nodes=n) if d else (2**31 - 1, 2**63 - 1, float(np.finfo(np.float64).max))
+                    for a, (n, d) in zip(arrays, shapes)]
+            b = og.Batch([og.GraphSpec(a, nodes=n) for a, (n, d) in zip(first, shapes)])
+        assert all(same(x, y) for x, y in zip(b.run(arrays), want)), run
+    b.close()
