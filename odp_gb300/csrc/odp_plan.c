@@ -660,50 +660,74 @@ int odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_t
   return 1;
 }
 
+/* The smallest of `at`, a heap of n, is to move down to its place. */
+static void sift_down(double *at, int n, int i)
+{
+  const double x = at[i];
+  for(int c; (c = 2 * i + 1) < n; i = c){
+    if(c + 1 < n && at[c + 1] < at[c]) c++;
+    if(at[c] >= x) break;
+    at[i] = at[c];
+  }
+  at[i] = x;
+}
+
 /* Makespan (us) of the graphs on their teams: every team takes the next graph
  * of its size when it is free, and splits when there is none.  *last: the graph
- * that ends it. */
-static double team_makespan(const odp_team_graph *g, const job_order *ord, int count, int *last)
+ * that ends it.  `ord` holds the graphs, largest first; `list` takes them by
+ * size of team.  The times at which the teams of a size are free are a heap. */
+static double team_makespan(const odp_team_graph *g, const job_order *ord, int count, int *list, int *last)
 {
   double at[1 << (GBX_TEAM_SPLITS - 1)] = {0};
+  int first_of[GBX_TEAM_SPLITS] = {0};
   double end = 0;
-  for(int k = 0; k < GBX_TEAM_SPLITS; k++){
-    const int teams = 1 << k;
+  for(int j = 0; j < count; j++) first_of[g[j].split]++;
+  for(int k = 1; k < GBX_TEAM_SPLITS; k++) first_of[k] += first_of[k - 1];
+  for(int j = count - 1; j >= 0; j--) list[--first_of[g[ord[j].job].split]] = ord[j].job;
+  for(int k = 0; k < GBX_TEAM_SPLITS && first_of[k] < count; k++){
+    const int teams = 1 << k, from = first_of[k], to = k + 1 < GBX_TEAM_SPLITS ? first_of[k + 1] : count;
     if(k) for(int i = teams - 1; i >= 0; i--) at[i] = at[i >> 1];
-    for(int j = 0; j < count; j++){
-      const odp_team_graph *x = &g[ord[j].job];
-      if(x->split != k) continue;
-      int first = 0;
-      for(int i = 1; i < teams; i++) if(at[i] < at[first]) first = i;
-      at[first] += x->cost * teams + x->latency;
-      if(at[first] > end){
-        end = at[first];
-        *last = ord[j].job;
+    if(from < to) for(int i = teams / 2 - 1; i >= 0; i--) sift_down(at, teams, i);
+    for(int j = from; j < to; j++){
+      const odp_team_graph *x = &g[list[j]];
+      at[0] += x->cost * teams + x->latency;
+      if(at[0] > end){
+        end = at[0];
+        *last = list[j];
       }
+      sift_down(at, teams, 0);
     }
   }
   return end;
 }
 
-/* Each graph's team: the smallest on which it takes at most `most` us, its
- * rows fit a CTA and the teams' bitsets stay within 160 MB.  0 if some graph
- * does not even fit the whole grid. */
-static int assign_teams(const odp_shape *shapes, int count, int grid, double most, gbx_sweep *gs,
-                        odp_team_graph *g)
+/* The smallest team (of a grid of `grid` CTAs) that each graph fits: its rows a
+ * CTA, the teams' bitsets 160 MB.  0 if some graph does not even fit the whole
+ * grid. */
+static int fit_teams(const odp_shape *shapes, int count, int grid, const gbx_sweep *gs, odp_team_graph *g)
 {
   for(int i = 0; i < count; i++){
-    g[i].split = -1;
+    g[i].fits = -1;
     for(int k = 0; k < GBX_TEAM_SPLITS && (1 << k) <= grid; k++){
       gbx_sweep c = gs[i];
       const int size = grid >> k;
       c.rows = (shape_n(&shapes[i]) + size - 1) / size;
-      if(gbx_sweep_smem(&c) > ODP_TEAM_SMEM || (k > 0 && (g[i].need * (1 << k) > 160e6 || g[i].cost * (1 << k) > most))) break;
-      g[i].split = k;
-      gs[i].rows = c.rows;
+      if(gbx_sweep_smem(&c) > ODP_TEAM_SMEM || (k > 0 && g[i].need * (1 << k) > 160e6)) break;
+      g[i].fits = k;
     }
-    if(g[i].split < 0) return 0;
+    if(g[i].fits < 0) return 0;
   }
   return 1;
+}
+
+/* Each graph's team: the smallest that it fits and on which it takes at most
+ * `most` us. */
+static void assign_teams(int count, double most, odp_team_graph *g)
+{
+  for(int i = 0; i < count; i++){
+    g[i].split = 0;
+    while(g[i].split < g[i].fits && g[i].cost * (2 << g[i].split) <= most) g[i].split++;
+  }
 }
 
 /* Whether a plan runs on the team kernel, and which team each graph gets.
@@ -723,7 +747,8 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
   if(t->blocks > 0 && t->blocks < grid) grid = t->blocks;
   odp_team_graph *g = calloc((size_t)count, sizeof(odp_team_graph));
   job_order *ord = calloc((size_t)count, sizeof(job_order));
-  int ok = g && ord;
+  int *list = calloc((size_t)count, sizeof(int));
+  int ok = g && ord && list;
   double all = 0;
   for(int i = 0; i < count && ok; i++){
     ok = odp_team_shape(&shapes[i], t, &gs[i], &g[i]);
@@ -731,30 +756,33 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
     ord[i].job = i;
     ord[i].work = g[i].cost;
   }
+  if(ok) ok = fit_teams(shapes, count, grid, gs, g);
   if(ok){
     qsort(ord, (size_t)count, sizeof(job_order), cmp_work_desc);
     static const double shares[] = { 0.1, 0.2, 0.35, 0.6, 1.0, 2.0, 4.0, 8.0 };
     double best = 0, best_share = 0;
     int last = 0;
-    for(int s = 0; s < 8 && ok; s++){
-      ok = assign_teams(shapes, count, grid, shares[s] * all, gs, g);
-      const double m = ok ? team_makespan(g, ord, count, &last) : 0;
+    for(int s = 0; s < 8; s++){
+      assign_teams(count, shares[s] * all, g);
+      const double m = team_makespan(g, ord, count, list, &last);
       if(s == 0 || m < best){ best = m; best_share = shares[s]; }
     }
-    if(ok) ok = assign_teams(shapes, count, grid, best_share * all, gs, g);
+    assign_teams(count, best_share * all, g);
     /* then larger teams for the graphs that end the run, while that shortens it
      * (256 graphs 2.87 -> 2.74 ms, 17 of n = 688 to 4128 392 -> 327 us) */
-    if(ok) best = team_makespan(g, ord, count, &last);
-    for(int tries = count < 64 ? 2 * count : 128; ok && tries > 0; tries--){
+    best = team_makespan(g, ord, count, list, &last);
+    for(int tries = count < 64 ? 2 * count : 128; tries > 0; tries--){
       const int i = last;
       if(g[i].split == 0) break;
       g[i].split--;
-      const double m = team_makespan(g, ord, count, &last);
+      const double m = team_makespan(g, ord, count, list, &last);
       if(m >= best){
         g[i].split++;
         break;
       }
       best = m;
+    }
+    for(int i = 0; i < count; i++){
       const int size = grid >> g[i].split;
       gs[i].rows = (shape_n(&shapes[i]) + size - 1) / size;
     }
@@ -791,6 +819,7 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
   *smem_out = smem;
   free(g);
   free(ord);
+  free(list);
   return ok;
 }
 

@@ -116,7 +116,7 @@ typedef struct {
 typedef struct {
   double cost, latency;        /* us on the whole GPU; us whatever the team */
   double need;                 /* bytes of its bitsets */
-  int split;
+  int split, fits;             /* teams of 1/2^split of the grid; the smallest it fits */
 } odp_team_graph;
 #define ODP_TEAM_SMEM (100 * 1024)     /* of a CTA: two per SM */
 int  odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_team_graph *g);

@@ -116,3 +116,13 @@ def test_a_server_with_graphs_for_the_engine_keeps_all_on_it(fake):
     served(srv, general)
     assert set(fake.counts) == {"engine"}
     srv.close()
+
+
+def test_choosing_teams_is_linear_in_the_graphs(fake):
+    """Each graph's fit is looked at once per size of team, whatever the shares
+    and teams that are tried."""
+    specs = [og.GraphSpec(np.zeros((64 * (k % 50) + 300, 6), np.int32), nodes=64 * (k % 50) + 300) for k in range(700)]
+    asked = fake.asked
+    b = og.Batch(specs)
+    assert fake.asked - asked <= 12 * len(specs)
+    b.close()
