@@ -86,11 +86,15 @@ int ODPX_Batch_run(ODPX_Batch *batch, const int *const *adjacency, int *diameter
   return rc;
 }
 
-unsigned long long ODPX_Batch_tiles(const ODPX_Batch *batch) { return batch ? odp_plan_tiles(batch) : 0; }
+/* The plan that the last run took: what it ran is reported of that one. */
+static const odp_plan *last_run(const odp_plan *p) { return p->ran ? p->ran : p; }
+
+unsigned long long ODPX_Batch_tiles(const ODPX_Batch *batch) { return batch ? odp_plan_tiles(last_run(batch)) : 0; }
 
 int ODPX_Batch_info(const ODPX_Batch *batch, int graph, int *njobs, int *nslots, int *wc_log2, int *tile_rows)
 {
   if(!batch || graph < 0 || graph >= batch->ngraphs) return ODPX_ERR_INVALID;
+  batch = last_run(batch);
   if(njobs) *njobs = batch->njobs;
   if(nslots) *nslots = batch->nslots;
   if(wc_log2) *wc_log2 = batch->g[graph].wc_log2;
@@ -188,6 +192,7 @@ int ODPX_Batch_time_mode(ODPX_Batch *p, const int *const *adjacency, int repeats
                          float *ms_per_run)
 {
   if(!p || repeats <= 0) return ODPX_ERR_INVALID;
+  p->ran = p;
   if(adjacency) odp_plan_stage(p, adjacency);
   odp_result *tmp = malloc(sizeof(odp_result) * (size_t)p->ngraphs);
   int rc = odp_plan_launch(p);                 /* warm: builds the CUDA graph, expands tables */
@@ -237,6 +242,7 @@ int ODPX_Batch_time(ODPX_Batch *batch, const int *const *adjacency, int repeats,
 int ODPX_Batch_job_levels(const ODPX_Batch *batch, int *levels, int max_jobs)
 {
   if(!batch) return ODPX_ERR_STATE;
+  batch = last_run(batch);
   const gbx_job_out *jo = odp_plan_job_out(batch);
   int n = batch->njobs < max_jobs ? batch->njobs : max_jobs;
   for(int i = 0; i < n; i++) levels[i] = jo[i].level;
@@ -246,6 +252,7 @@ int ODPX_Batch_job_levels(const ODPX_Batch *batch, int *levels, int max_jobs)
 int ODPX_Batch_job_profile(const ODPX_Batch *batch, int *graph, double *loaded_us, double *done_us, int max_jobs)
 {
   if(!batch) return ODPX_ERR_STATE;
+  batch = last_run(batch);
   const gbx_job_out *jo = odp_plan_job_out(batch);
   int n = batch->njobs < max_jobs ? batch->njobs : max_jobs;
   /* time origin: the engine's start, or the earliest stamp (the small-graph
@@ -269,6 +276,7 @@ void ODPX_Batch_set_wait_limit(ODPX_Batch *batch, unsigned long long ns)
 {
   if(!batch || batch->spin_limit_ns == ns) return;
   batch->spin_limit_ns = ns;
+  ODPX_Batch_set_wait_limit(batch->beside, ns);
   /* the limit is an argument of the captured engine launch: capture anew */
   if(batch->graph_exec){
     gbx_stream_sync(batch->stream);
@@ -277,7 +285,7 @@ void ODPX_Batch_set_wait_limit(ODPX_Batch *batch, unsigned long long ns)
   }
 }
 
-double ODPX_Batch_bytes_alg(const ODPX_Batch *batch) { return batch ? odp_plan_bytes_alg(batch) : 0.0; }
+double ODPX_Batch_bytes_alg(const ODPX_Batch *batch) { return batch ? odp_plan_bytes_alg(last_run(batch)) : 0.0; }
 
 double ODPX_Measure_l2_read_gbs(int megabytes, int reps)
 {

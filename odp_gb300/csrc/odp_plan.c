@@ -825,6 +825,22 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
 
 #define CK(call) do{ int _e = (call); if(_e){ rc = ODPX_ERR_CUDA; goto fail; } }while(0)
 
+/* Copies the shapes of a lockstep plan, from which `beside` is made. */
+static int keep_shapes(odp_plan *p, const odp_shape *shapes)
+{
+  if(!(p->shapes = calloc((size_t)p->ngraphs, sizeof(odp_shape)))) return ODPX_ERR_MEMORY;
+  for(int i = 0; i < p->ngraphs; i++){
+    const size_t bytes = sizeof(int) * (size_t)p->g[i].B;
+    p->shapes[i] = shapes[i];
+    if(!shapes[i].num_degrees) continue;
+    int *nd = malloc(bytes);
+    if(nd) memcpy(nd, shapes[i].num_degrees, bytes);
+    p->shapes[i].num_degrees = nd;
+    if(!nd) return ODPX_ERR_MEMORY;
+  }
+  return 0;
+}
+
 int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning, odp_plan **out)
 {
   int rc = 0;
@@ -1231,6 +1247,7 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   }
   free(team_order);
   team_order = NULL;
+  if(lockstep && (rc = keep_shapes(p, shapes))) goto fail;
 
   fill_state_init(p);
   if(p->d_state_init){
@@ -1249,6 +1266,9 @@ fail:
 void odp_plan_destroy(odp_plan *p)
 {
   if(!p) return;
+  odp_plan_destroy(p->beside);
+  for(int i = 0; p->shapes && i < p->ngraphs; i++) free((void *)p->shapes[i].num_degrees);
+  free(p->shapes);
   if(p->graph_exec) gbx_graph_destroy(p->graph_exec);
   gbx_free(p->d_adj); gbx_free(p->d_ndeg); gbx_free(p->d_itable); gbx_free(p->d_nbr);
   gbx_free(p->d_slotbuf); gbx_free(p->d_slotmask); gbx_free(p->d_srcpos); gbx_free(p->d_expand); gbx_free(p->d_jobs); gbx_free(p->d_state);
@@ -1574,12 +1594,34 @@ int odp_plan_finish(odp_plan *p, odp_result *results)
   return 0;
 }
 
+/* The plan that a call of p runs.  A cooperative launch waits until all of its
+ * CTAs fit on the GPU at once, and behind a busy server's long batches it waits
+ * for all lanes to be free together, where the other kernels' CTAs start as
+ * soon as one leaves.  So beside such batches a lockstep plan's call runs on
+ * the kernels that its shapes take without lockstep (a plan of its own, made the
+ * first time).  Measured on GB300, us, n = 4096, d = 24 through ODP_Set_aspl,
+ * lockstep against this, beside chains of n = 8192: 966 / 395; 16384: 2618 / 155;
+ * 32768: 7262 / 163; 90 x 90 grids: 6678 / 142; alone 33 / 76. */
+static odp_plan *plan_for_call(odp_plan *p)
+{
+  if(!p->shapes || !odp_serving()) return p;
+  if(!p->beside){
+    odp_tuning t = p->tuning;
+    t.sweep = 0;
+    if(odp_plan_create(p->shapes, p->ngraphs, &t, &p->beside)) return p;
+    p->beside->spin_limit_ns = p->spin_limit_ns;
+  }
+  return p->beside;
+}
+
 int odp_plan_run(odp_plan *p, const int *const *adjacency, odp_result *results)
 {
-  odp_plan_stage(p, adjacency);
-  int rc = odp_plan_launch(p);
+  odp_plan *q = plan_for_call(p);
+  p->ran = q;
+  odp_plan_stage(q, adjacency);
+  int rc = odp_plan_launch(q);
   if(rc) return rc;
-  return odp_plan_finish(p, results);
+  return odp_plan_finish(q, results);
 }
 
 unsigned long long odp_plan_tiles(const odp_plan *p)

@@ -103,6 +103,9 @@ typedef struct odp_plan {
   unsigned int *d_changed;     /* the lockstep kernel's changed-lane masks */
   void *d_sync;                /* its counters */
   unsigned int *h_abort;       /* pinned: set when one of its waits ran out */
+  odp_shape *shapes;           /* lockstep plans: the shapes, with degree tables of their own */
+  struct odp_plan *beside;     /* the same shapes without lockstep, for calls beside a busy server */
+  struct odp_plan *ran;        /* the plan that the last call ran, this one or `beside` */
 } odp_plan;
 
 typedef struct {
@@ -124,6 +127,9 @@ int  odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_
 void odp_tuning_defaults(odp_tuning *t, int batch);
 /* The defaults for `count` graphs with the ODPX_Set_tuning overrides applied. */
 void odp_tuning_for(int count, odp_tuning *t);
+/* Batches in flight, of all servers of the process, that hold their part of
+ * the GPU for long. */
+int  odp_serving(void);
 /* Returns 0 on success, else an ODPX_ERR_* code (include/odp_gb300.h). */
 int  odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning, odp_plan **out);
 void odp_plan_destroy(odp_plan *p);

@@ -84,6 +84,7 @@ typedef struct {
   long long *members;          /* request ids of the running batch */
   int *b_first, *b_count;      /* a team batch's members' writes */
   int nmembers;
+  int holds;                   /* the batch counts among those of odp_serving */
   /* the batch formed and not yet issued */
   int b_nw, b_njobs, b_nslots;
   size_t b_slots_off, b_jobs_off, b_outcomes_off, b_acc_bytes;
@@ -240,6 +241,23 @@ static int delta_writes(serve_graph *g, const ODPX_Delta *dl, gbx_write *w)
   return k;
 }
 
+/* Batches in flight that hold their part of the GPU for long, of all servers:
+ * those of the engine, and team batches by their estimate.  Plans ask
+ * (odp_plan.c).  Calls in lockstep against without, us, beside 16 chains of n =
+ * 4096 (an estimate of 170): n = 4096 202 / 184, 20000 341 / 474, 97 x 103 grid
+ * 491 / 853; beside 32 of n = 8192 (1000): 966 / 395, 1278 / 1280, 1077 / 2096, 40
+ * graphs of n = 300 to 2000 1556 / 861. */
+#define HOLD_US 300.0
+static int g_serving = 0;
+
+int odp_serving(void) { return __atomic_load_n(&g_serving, __ATOMIC_RELAXED); }
+
+static void hold(serve_lane *l, int on)
+{
+  if(l->holds != on) __atomic_add_fetch(&g_serving, on - l->holds, __ATOMIC_RELAXED);
+  l->holds = on;
+}
+
 /* Whether all records of lane l's team batch have arrived. */
 static int records_done(const serve_lane *l)
 {
@@ -294,6 +312,7 @@ static void finish_batch(odp_server *s, serve_lane *l)
     if(r->waiter) pthread_cond_signal(r->waiter);
   }
   s->stats.requests_done += l->nmembers;
+  hold(l, 0);
   l->busy = 0;
   l->nmembers = 0;
 }
@@ -334,6 +353,7 @@ static void form_team(odp_server *s, serve_lane *l, int count)
     const double end = one > all ? one : all;
     if(k == 0 || end < best){ best = end; split = k; l->b_smem = smem; }
   }
+  hold(l, best > HOLD_US);
   gbx_team *tm = &l->tm;
   memset(tm, 0, sizeof(*tm));
   tm->graphs = l->dh_args;
@@ -421,6 +441,7 @@ static int form_batch(odp_server *s, serve_lane *l, double max_seed_cost)
     form_team(s, l, nreq);
     return nreq;
   }
+  hold(l, 1);
 
   /* Active slots: as many leading jobs as fit the lane's share of L2 (at
    * least one).  Lanes run at the same time, so their bitsets together must
@@ -496,6 +517,7 @@ static void fail_batch(odp_server *s, serve_lane *l)
     s->graphs[r->graph].busy = 0;
     if(r->waiter) pthread_cond_signal(r->waiter);
   }
+  hold(l, 0);
   l->busy = 0;
   l->nmembers = 0;
 }
@@ -897,7 +919,10 @@ void ODPX_Serve_destroy(ODPX_Server *s)
   pthread_cond_broadcast(&s->cv_work);
   pthread_mutex_unlock(&s->mu);
   if(s->started) pthread_join(s->thread, NULL);
-  for(int i = 0; i < s->cfg.lanes; i++) lane_free(&s->lanes[i]);
+  for(int i = 0; i < s->cfg.lanes; i++){
+    lane_free(&s->lanes[i]);
+    hold(&s->lanes[i], 0);
+  }
   free(s->lanes);
   for(int i = 0; i < s->ngraphs; i++){
     serve_graph *g = &s->graphs[i];

@@ -126,3 +126,57 @@ def test_choosing_teams_is_linear_in_the_graphs(fake):
     b = og.Batch(specs)
     assert fake.asked - asked <= 12 * len(specs)
     b.close()
+
+
+@pytest.mark.parametrize("kind", ["sweep", "team"])
+def test_calls_beside_a_servers_long_batches_take_no_cooperative_launch(fake, kind):
+    """Such a launch waits for the whole GPU.  With the server idle again, or
+    closed with its batch in flight, the call takes it again."""
+    nd = np.full(6000, 4, np.int32)
+    nd[5] = 3
+    specs = plans()[kind]
+    specs[0] = og.GraphSpec(ring(6000), nodes=6000, num_degrees=nd)
+    b = og.Batch(specs)
+    nd[:] = 0                                            # the plan keeps its own
+    want = b.run()
+    assert fake.counts == {kind: 1}
+    for closed in (0, 1):
+        srv = og.Server(max_nodes=2000, memory_mb=64)
+        h = srv.register(og.GraphSpec(ring(400), grid=True, width=20, height=20))
+        fake.pending = 1
+        r = srv.submit(h, [])
+        while "engine" not in fake.counts:
+            pass
+        fake.counts = 0
+        assert b.run() == want and b.run() == want
+        assert set(fake.counts) == {"engine", "pull"} and fake.counts["engine"] == 2
+        assert len(b.job_levels()) == b.info(0)["njobs"] and (b.job_levels() == 1).all()
+        fake.pending = 0
+        if not closed:
+            srv.wait(r)
+        else:
+            fake.pending = 1
+            r = srv.submit(h, [])
+        srv.close()
+        fake.pending = fake.counts = 0
+        assert b.run() == want and fake.counts == {kind: 1}
+    b.close()
+
+
+def test_calls_beside_a_servers_short_team_batches_stay_in_lockstep(fake):
+    b = og.Batch(plans()["sweep"])
+    srv = og.Server(max_nodes=2000, memory_mb=64)
+    h = srv.register(og.GraphSpec(ring(2000), nodes=2000))
+    fake.abort_at = fake.total + 1                       # no records: in flight until its event is complete
+    fake.pending = 1
+    r = srv.submit(h, [])
+    while "team" not in fake.counts:
+        pass
+    fake.counts = fake.abort_at = 0
+    b.run()
+    assert fake.counts == {"sweep": 1}
+    fake.pending = 0
+    with pytest.raises(og.ODPError):
+        srv.wait(r)
+    srv.close()
+    b.close()
