@@ -412,6 +412,22 @@ __device__ bool evaluate(ResidentShared &sh, Resident &t, unsigned long long lim
   return true;
 }
 
+/* store(i, src[i]) for i = first, first + stride, ... below n, eight loads in
+ * flight (a store into shared or host memory might alias the source, so loads
+ * one by one would each wait for the one before). */
+template <class Store>
+__device__ __forceinline__ void each_int(const int *src, int n, int first, int stride, Store store)
+{
+  for(int i0 = first; i0 < n; i0 += 8 * stride){
+    int x[8];
+#pragma unroll
+    for(int k = 0; k < 8; k++) x[k] = __ldcg(src + min(i0 + k * stride, n - 1));
+#pragma unroll
+    for(int k = 0; k < 8; k++)
+      if(i0 + k * stride < n) store(i0 + k * stride, x[k]);
+  }
+}
+
 /* Thread 0: the step's outcome, as anneal_decide_kernel. */
 __device__ void decide(ResidentShared &sh, int level, long long total)
 {
@@ -484,8 +500,8 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
     t.block = resident_block(t.rows, t.lanes);
     t.adj = reinterpret_cast<unsigned short *>(t.scratch + t.block * t.lanes * 8);
     t.flag = reinterpret_cast<unsigned char *>(t.adj + ((c.base * c.d + 1) & ~1));
-    for(int i = tid; i < c.base * c.d; i += THREADS) t.adj[i] = (unsigned short)__ldcg(c.adj + i);
-    for(int i = tid; i < t.nr * c.dp; i += THREADS) t.list[i] = __ldcg(c.nbr + (size_t)t.r0 * c.dp + i);
+    each_int(c.adj, c.base * c.d, tid, THREADS, [&](int i, int x) { t.adj[i] = (unsigned short)x; });
+    each_int(c.nbr + (size_t)t.r0 * c.dp, t.nr * c.dp, tid, THREADS, [&](int i, int x) { t.list[i] = x; });
     if(tid < 31) sh.rng.ring[tid] = c.ring[tid];
     if(tid == 0){
       sh.rng.pos = c.ring_pos;
@@ -517,7 +533,7 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
       if(tid == 0) decide(sh, level, sum);
       __syncthreads();
       if(sh.copy && t.rank == 0)
-        for(int i = tid; i < c.base * c.d; i += THREADS) c.best_adj[i] = __ldcg(c.adj + i);
+        each_int(c.adj, c.base * c.d, tid, THREADS, [best = c.best_adj](int i, int x) { best[i] = x; });
       if(!sh.accept){
         __syncthreads();                                 /* the copy has read the adjacency before the undo */
         if(tid == 0) undo(sh);
@@ -543,10 +559,8 @@ __global__ void __launch_bounds__(CLUSTER ? GBX_RESIDENT_CLUSTER_THREADS : RESID
     if(met && p.host_chains){
       const int ints = c.base * c.d;
       int *to = p.host_graphs + p.host_offset[chain];
-      for(int i = t.rank * THREADS + tid; i < ints; i += t.size * THREADS){
-        to[i] = __ldcg(c.adj + i);
-        to[ints + i] = __ldcg(c.best_adj + i);
-      }
+      each_int(c.adj, ints, t.rank * THREADS + tid, t.size * THREADS, [to](int i, int x) { to[i] = x; });
+      each_int(c.best_adj, ints, t.rank * THREADS + tid, t.size * THREADS, [to, ints](int i, int x) { to[ints + i] = x; });
     }
     for(int i = tid; i < t.nr * c.dp; i += THREADS) c.nbr[(size_t)t.r0 * c.dp + i] = t.list[i];
     if(t.rank == 0){
