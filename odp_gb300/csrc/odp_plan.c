@@ -1619,6 +1619,7 @@ int odp_plan_run(odp_plan *p, const int *const *adjacency, odp_result *results)
   odp_plan *q = plan_for_call(p);
   p->ran = q;
   odp_plan_stage(q, adjacency);
+  if(q != p) odp_plan_stage(p, adjacency);       /* a timing call may ask for the last run's arrays */
   int rc = odp_plan_launch(q);
   if(rc) return rc;
   return odp_plan_finish(q, results);

@@ -13,6 +13,7 @@ int fake_launches[KINDS];
 int fake_total;                /* launches of the evaluation kernels so far */
 int fake_abort_at;             /* that launch (from 1): a wait runs out, no record is written */
 int fake_late_at;              /* that launch: complete, and then a wait runs out all the same */
+const int *fake_adjacency;     /* of the last lockstep launch */
 int fake_pending;              /* events are not complete while set */
 
 static int next(int kind)
@@ -102,6 +103,7 @@ int gbx_sweep_launch(const gbx_sweep *a, int blocks, void *s)
 {
   (void)blocks; (void)s;
   const int k = next(SWEEP);
+  fake_adjacency = a->e.adj;
   if(k != fake_abort_at) record(a->rec, a->nchunks, a->seq);
   if(k == fake_abort_at || k == fake_late_at) *a->abort_flag = GBX_ERR_TIMEOUT;
   return 0;

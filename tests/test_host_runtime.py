@@ -180,3 +180,26 @@ def test_calls_beside_a_servers_short_team_batches_stay_in_lockstep(fake):
         srv.wait(r)
     srv.close()
     b.close()
+
+
+def test_timing_after_a_call_beside_a_server_reads_that_calls_arrays(fake):
+    """ODPX_Batch_time without arrays times the last run's."""
+    b = og.Batch(plans()["sweep"])
+    first, second = ring(6000), ring(6000, 4)[:, ::-1].copy()
+    b.run([first])
+    srv = og.Server(max_nodes=2000, memory_mb=64)
+    h = srv.register(og.GraphSpec(ring(400), grid=True, width=20, height=20))
+    fake.pending = 1
+    r = srv.submit(h, [])
+    while "engine" not in fake.counts:
+        pass
+    fake.counts = 0
+    b.run([second])
+    assert fake.counts["engine"] == 1 and "sweep" not in fake.counts
+    fake.pending = 0
+    srv.wait(r)
+    srv.close()
+    ms = ctypes.c_float()
+    assert og.load().ODPX_Batch_time_mode(b._h, None, 2, 0, 0, ctypes.byref(ms)) == 0
+    assert ctypes.c_void_p.in_dll(fake.lib, "fake_adjacency").value == second.ctypes.data
+    b.close()
