@@ -62,7 +62,9 @@ void ODPX_Batch_destroy(ODPX_Batch *batch);
  * the plan keeps only their addresses). */
 int  ODPX_Batch_time(ODPX_Batch *batch, const int *const *adjacency, int repeats, float *ms_per_run);
 /* mode 0: whole per-call sequence (upload, expand, engine, read back);
- * mode 1: engine on resident inputs.  flush_mb > 0 overwrites a buffer of
+ * mode 1: engine on resident inputs.  Plans on the other kernels (see
+ * ODPX_Batch_path) are one kernel that reads the arrays from host memory: both
+ * modes time that.  flush_mb > 0 overwrites a buffer of
  * that size before each run, outside the timed interval. */
 int  ODPX_Batch_time_mode(ODPX_Batch *batch, const int *const *adjacency, int repeats, int mode, int flush_mb,
                           float *ms_per_run);
@@ -82,6 +84,13 @@ int  ODPX_Batch_info(const ODPX_Batch *batch, int graph, int *njobs, int *nslots
  * graphs too large for a team, in the persistent engine.  Results are the
  * same either way. */
 int  ODPX_Batch_kernel(const ODPX_Batch *batch);
+/* The kernels that evaluate the plan (the last run, if one went to others
+ * because a server of the process was busy with long batches). */
+#define ODPX_PATH_ENGINE   0   /* pull or upload, expand, persistent engine */
+#define ODPX_PATH_SMALL    1   /* small-graph kernel */
+#define ODPX_PATH_LOCKSTEP 2   /* one graph on every SM */
+#define ODPX_PATH_TEAMS    3   /* many graphs on teams of CTAs */
+int  ODPX_Batch_path(const ODPX_Batch *batch);
 /* For a small plan: its shape on the small-graph kernel, the CTAs of the thread-block cluster
  * that runs each job (1, 2, 4 or 8; each CTA computes its share of the
  * rows), the threads per CTA, and whether the bitsets are partitioned over

@@ -104,6 +104,7 @@ def load():
         "ODPX_Batch_set_wait_limit": (None, [P, ctypes.c_ulonglong]),
         "ODPX_Batch_bytes_alg": (ctypes.c_double, [P]),
         "ODPX_Batch_kernel": (I, [P]),
+        "ODPX_Batch_path": (I, [P]),
         "ODPX_Batch_small_shape": (I, [P, IP, IP, IP]),
         "ODPX_Measure_l2_read_gbs": (ctypes.c_double, [I, I]),
         "ODPX_Set_tuning": (None, [I, I, I, I, I, I]),
@@ -476,7 +477,9 @@ class Batch:
         return _results(d, s, a)
 
     def time(self, repeats, mode=1, flush_mb=0, adjacency=None):
-        """Average device ms per run (CUDA events on the plan's stream)."""
+        """Average device ms per run (CUDA events on the plan's stream): the whole
+        call (mode 0) or the engine on resident inputs (mode 1); the whole kernel in
+        both for plans on other kernels."""
         ms = ctypes.c_float()
         rc = load().ODPX_Batch_time_mode(self._h, self._adj_ptrs(adjacency), repeats, mode, flush_mb,
                                          ctypes.byref(ms))
@@ -492,8 +495,14 @@ class Batch:
         return dict(njobs=v[0].value, nslots=v[1].value, wc_log2=v[2].value, tile_rows=v[3].value)
 
     def kernel(self):
-        """'small' when every job runs in the small-graph kernel, else 'engine'."""
+        """'small' for a plan of the small class (its graphs fit the small-graph
+        kernel), else 'engine'.  path() says which kernels run."""
         return "small" if load().ODPX_Batch_kernel(self._h) == 1 else "engine"
+
+    def path(self):
+        """The kernels that evaluate the plan: 'engine', 'small', 'lockstep' (one
+        graph on every SM) or 'teams' (many graphs on teams of CTAs)."""
+        return ("engine", "small", "lockstep", "teams")[load().ODPX_Batch_path(self._h)]
 
     def small_shape(self):
         """(cluster CTAs per job, threads per CTA, partitioned 0/1) of a plan on the small-graph kernel."""

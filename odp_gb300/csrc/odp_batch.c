@@ -1,7 +1,6 @@
 /*
  * odp_batch.c -- ODP_Set_aspl_batch and the ODPX_Batch_* plan API: many
- * graphs of uneven size, degree and symmetry evaluated in one persistent
- * engine launch.  Each graph's results are bit-identical to evaluating it
+ * graphs of uneven size, degree and symmetry evaluated in one launch.  Each graph's results are bit-identical to evaluating it
  * alone through ODP_Init_aspl_* + ODP_Set_aspl.  No counterpart in the
  * reference, whose clients evaluate one graph per call.
  */
@@ -104,6 +103,13 @@ int ODPX_Batch_info(const ODPX_Batch *batch, int graph, int *njobs, int *nslots,
 
 int ODPX_Batch_kernel(const ODPX_Batch *batch) { return batch ? batch->small_class : ODPX_ERR_INVALID; }
 
+int ODPX_Batch_path(const ODPX_Batch *batch)
+{
+  if(!batch) return ODPX_ERR_INVALID;
+  batch = last_run(batch);
+  return batch->sweep ? ODPX_PATH_LOCKSTEP : batch->team ? ODPX_PATH_TEAMS : batch->small ? ODPX_PATH_SMALL : ODPX_PATH_ENGINE;
+}
+
 int ODPX_Batch_small_shape(const ODPX_Batch *batch, int *cluster, int *threads, int *partitioned)
 {
   if(!batch || !batch->small_class) return ODPX_ERR_INVALID;
@@ -182,7 +188,8 @@ int ODP_Set_aspl_batch(int count, const ODP_Graph *graphs, int *diameter, long *
 /* Device time per run of the plan's GPU work, averaged over `repeats` runs
  * timed with CUDA events on the plan's stream.  mode 0: the whole per-call
  * sequence (adjacency upload, expand, engine, read back); mode 1: the engine
- * alone on resident inputs (state reset + engine kernel).  When flush_mb > 0
+ * alone on resident inputs (state reset + engine kernel).  Plans on the other
+ * kernels are one kernel, timed in both modes.  When flush_mb > 0
  * a buffer of that size is overwritten before every run, outside the timed
  * interval, so no run starts with the previous run's data in L2. */
 static void *g_flush = NULL;

@@ -108,3 +108,43 @@ def test_a_graph_without_return_edges_stops_at_its_first_proposal(n, d, count):
             assert x["status"] == 1 and x["steps"] == 0
             assert np.array_equal(x["adjacency"], adj) and np.array_equal(x["best_adjacency"], adj)
     a.close()
+
+
+def test_a_cta_walks_several_chains(monkeypatch):
+    """All of 700 chains, two or three to a CTA."""
+    kw = dict(max_temp=50.0, min_temp=0.5, ncalcs=200)
+    made = [og.Chain(general(60 + k % 5 * 12, 4, 1, k), nodes=60 + k % 5 * 12, seed=k, **kw) for k in range(700)]
+    monkeypatch.setenv("ODP_GB300_ANNEAL_RESIDENT", "1")
+    a = og.Anneal(made)
+    monkeypatch.setenv("ODP_GB300_ANNEAL_RESIDENT", "0")
+    b = og.Anneal(made)
+    for steps in (1, 13):
+        a.run(steps)
+        b.run(steps)
+        for k in range(len(made)):
+            x, y = a.state(k, graphs=True), b.state(k, graphs=True)
+            assert np.array_equal(x.pop("adjacency"), y.pop("adjacency")), (k, steps)
+            assert np.array_equal(x.pop("best_adjacency"), y.pop("best_adjacency")), (k, steps)
+            assert x == y, (k, steps)
+    a.close()
+    b.close()
+
+
+def test_a_run_of_several_launches(monkeypatch):
+    """More steps than a launch takes; only the last one leaves the state on the host."""
+    kw = dict(max_temp=20.0, min_temp=0.1, ncalcs=2000)
+    made = [og.Chain(general(n, 5, 1, n), nodes=n, seed=n, **kw) for n in (40, 64, 130)]
+    monkeypatch.setenv("ODP_GB300_ANNEAL_RESIDENT", "1")
+    a = og.Anneal(made)
+    monkeypatch.setenv("ODP_GB300_ANNEAL_RESIDENT", "0")
+    b = og.Anneal(made)
+    for steps in (513, 512, 1100):
+        a.run(steps)
+        b.run(steps)
+        for k in range(len(made)):
+            x, y = a.state(k, graphs=True), b.state(k, graphs=True)
+            assert np.array_equal(x.pop("adjacency"), y.pop("adjacency")), (k, steps)
+            assert np.array_equal(x.pop("best_adjacency"), y.pop("best_adjacency")), (k, steps)
+            assert x == y, (k, steps)
+    a.close()
+    b.close()

@@ -203,3 +203,20 @@ def test_timing_after_a_call_beside_a_server_reads_that_calls_arrays(fake):
     assert og.load().ODPX_Batch_time_mode(b._h, None, 2, 0, 0, ctypes.byref(ms)) == 0
     assert ctypes.c_void_p.in_dll(fake.lib, "fake_adjacency").value == second.ctypes.data
     b.close()
+
+
+@pytest.mark.parametrize("graphs,env,path", [
+    ([(300, 4)], {}, "small"), ([(4000, 24)], {}, "lockstep"), ([(4000, 24)], {"ODP_GB300_SWEEP": "0"}, "engine"),
+    ([(2000, 8)], {}, "lockstep"), ([(2000, 8)], {"ODP_GB300_SWEEP": "0"}, "small"), ([(2000, 8)], {"ODP_GB300_SMALL_CLUSTER": "8"}, "small"),
+    ([(6000, 4), (700, 4)], {}, "teams"), ([(6000, 4), (700, 4)], {"ODP_GB300_SWEEP": "0"}, "engine"),
+    ([(6000, 4)], {"ODP_GB300_SLOTS": "3"}, "engine")])
+def test_the_path_names_the_kernels_that_run(fake, graphs, env, path, monkeypatch):
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    b = og.Batch([og.GraphSpec(ring(n, d), nodes=n) for n, d in graphs])
+    assert b.path() == path
+    fake.counts = 0
+    b.run()
+    assert set(fake.counts) - {"pull"} == {{"lockstep": "sweep", "teams": "team"}.get(path, path)}
+    assert b.path() == path
+    b.close()
