@@ -537,6 +537,23 @@ static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
          t->activity == -2 && !(te && (te->wc_log2 > 0 || te->tile_kb > 0 || te->local_kb > 0));
 }
 
+/* Whether a single graph of very many rows and few sources is faster on the
+ * engine, which moves rows of 16 bytes where lockstep moves 32 (up to 128
+ * sources), and whole rows of up to 128 bytes where lockstep, whose two
+ * buffers are to stay in L2, takes 32 bytes of each at a time (up to 1024).
+ * Measured on GB300, lockstep against engine (us): 16 to 128 sources, n = 120000,
+ * d = 4 132 / 158, d = 8 121 / 121, n = 140000, d = 4 148 / 161, d = 8 139 / 133, d =
+ * 12 139 / 131, n = 200000, d = 4 186 / 168, n = 262144, d = 8 220 / 183, n = 10^6, d
+ * = 4 751 / 404; but 140 sources, n = 200000 186 / 231; 1000 sources, n = 400000, d =
+ * 8 461 / 445, d = 16 faster by 1.25; n = 450000, d = 8 520 / 476, d = 12 542 / 539; n
+ * = 600000, d = 8 813 / 601, n = 10^6, d = 4 1385 / 1117; but 1500 sources, n =
+ * 600000 1061 / 1381. */
+static int few_sources(const odp_shape *sh)
+{
+  const int n = shape_n(sh), W = shape_words(sh);
+  return (W <= 2 && n > (sh->degree > 4 ? 130000 : 170000)) || (W <= 16 && n > 420000 && sh->degree <= 10);
+}
+
 /* Whether a plan runs on the lockstep kernels (sweep.cu), and its shape.  One
  * graph, no schedule setting, and a CTA's rows must fit in its shared memory
  * beside their lane states.  Measured on GB300 against the persistent engine:
@@ -565,7 +582,7 @@ static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
  *    first, in wider pieces. */
 static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_sweep *sw, int *grid_out)
 {
-  if(!lockstep_allowed(sh, t) || t->blocks > 0) return 0;
+  if(!lockstep_allowed(sh, t) || t->blocks > 0 || few_sources(sh)) return 0;
   const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
   memset(sw, 0, sizeof(*sw));
   sw->e.d = sh->degree;

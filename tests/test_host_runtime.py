@@ -220,3 +220,14 @@ def test_the_path_names_the_kernels_that_run(fake, graphs, env, path, monkeypatc
     assert set(fake.counts) - {"pull"} == {{"lockstep": "sweep", "teams": "team"}.get(path, path)}
     assert b.path() == path
     b.close()
+
+
+@pytest.mark.parametrize("n,s,d,path", [(262144, 4096, 8, "engine"), (262144, 1024, 8, "lockstep"), (130000, 1300, 8, "lockstep"), (130100, 1301, 8, "engine"),
+                                        (160000, 1600, 4, "lockstep"), (800000, 800, 6, "engine"), (800000, 500, 6, "lockstep"), (420000, 420, 6, "lockstep")])
+def test_graphs_of_many_rows_and_few_sources_stay_on_the_engine(fake, n, s, d, path):
+    """Both sides of the lines where the engine is the faster one."""
+    adj = np.zeros((n // s, d), np.int32)
+    b = og.Batch([og.GraphSpec(adj, nodes=n, symmetries=s)])
+    assert b.path() == path
+    b.run()
+    b.close()
