@@ -747,6 +747,23 @@ static void assign_teams(int count, double most, odp_team_graph *g)
   }
 }
 
+/* What a row of a graph with many rows a source costs more on a small team than
+ * on the engine (us): the lists and the start are work a row, and the team
+ * kernel has half of the engine's warps on an SM.  Of 20 graphs with 4 rows a
+ * source or more, ns a row, teams / engine, d = 8: up to 128 sources, n = 20000
+ * .83 / .46, 50000 .68 / .34; 500 sources .95 / .68, .70 / .61; 2000 sources, n =
+ * 8000 1.84 / 1.46, but 20000 1.37 / 1.21.  Other graphs gain about a fifth of
+ * their cost, and a call 20 us, 40 where few graphs have large teams (3 graphs
+ * of n = 8000 to 20000 1.3 to 1.9 times faster).  A batch that would lose more
+ * than it gains stays on the engine: 40 of n = 20000, s = 100 578 -> 431 us, 50 of
+ * n = 8000, s = 4 551 -> 483, 20 of n = 2000 and 3 of n = 200000, s = 2000 432 -> 333. */
+static double team_slower(const odp_shape *sh)
+{
+  const int W = shape_words(sh);
+  if(sh->grid || sh->symmetries < 4 || W > 32) return 0;
+  return W <= 2 ? 0.25e-3 : W <= 16 ? 0.2e-3 : 0.15e-3;
+}
+
 /* Whether a plan runs on the team kernel, and which team each graph gets.
  * A graph's team is the smallest on which it takes no more
  * than a share of all graphs' cost, its rows fit a CTA's shared memory and
@@ -766,13 +783,17 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
   job_order *ord = calloc((size_t)count, sizeof(job_order));
   int *list = calloc((size_t)count, sizeof(int));
   int ok = g && ord && list;
-  double all = 0;
+  double all = 0, lost = 0, won = count <= 4 ? 40.0 : 20.0;
   for(int i = 0; i < count && ok; i++){
     ok = odp_team_shape(&shapes[i], t, &gs[i], &g[i]);
     all += g[i].cost;
     ord[i].job = i;
     ord[i].work = g[i].cost;
+    const double slower = team_slower(&shapes[i]);
+    if(slower > 0) lost += slower * shape_n(&shapes[i]);
+    else won += 0.2 * g[i].cost;
   }
+  ok = ok && lost <= won;
   if(ok) ok = fit_teams(shapes, count, grid, gs, g);
   if(ok){
     qsort(ord, (size_t)count, sizeof(job_order), cmp_work_desc);

@@ -231,3 +231,13 @@ def test_graphs_of_many_rows_and_few_sources_stay_on_the_engine(fake, n, s, d, p
     assert b.path() == path
     b.run()
     b.close()
+
+
+@pytest.mark.parametrize("graphs,path", [
+    ([(20000, 100, 8)] * 40, "engine"), ([(8000, 4, 8)] * 50, "engine"), ([(8000, 4, 8)] * 10, "teams"), ([(20000, 100, 8)] * 3, "teams"),
+    ([(2000, 1, 8)] * 20 + [(200000, 2000, 8)] * 3, "engine"), ([(8000, 1, 8)] * 60 + [(8000, 4, 8)] * 30, "teams")])
+def test_batches_that_lose_on_teams_stay_on_the_engine(fake, graphs, path):
+    """Graphs of many rows a source, alone and among others."""
+    b = og.Batch([og.GraphSpec(np.zeros((n // s, d), np.int32), nodes=n, symmetries=s) for n, s, d in graphs])
+    assert b.path() == path
+    b.close()
