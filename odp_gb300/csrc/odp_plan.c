@@ -537,6 +537,11 @@ static int lockstep_allowed(const odp_shape *sh, const odp_tuning *t)
          t->activity == -2 && !(te && (te->wc_log2 > 0 || te->tile_kb > 0 || te->local_kb > 0));
 }
 
+/* A grid of more neighbours than the tracking kernel takes: its levels gather
+ * every lane that is not full, however many they are, where the engine tracks
+ * changes. */
+static int dense_grid(const odp_shape *sh) { return sh->grid && shape_dp(sh) > GBX_SWEEP_TRACK_DEGREE; }
+
 /* Whether a single graph of very many rows and few sources is faster on the
  * engine, which moves rows of 16 bytes where lockstep moves 32 (up to 128
  * sources), and whole rows of up to 128 bytes where lockstep, whose two
@@ -577,12 +582,17 @@ static int few_sources(const odp_shape *sh)
  *    computing while the other's barrier is crossed, where two chunks fit in
  *    80 MB (n = 65536, with two levels from the lists: two phases of two
  *    chunks 1.65 ms, of one 1.71, one phase of two 1.69).
+ *  - Dense grids of more than 25000 sources stay on the engine; lockstep against
+ *    it (ms), edges up to 2 to 10 columns long: 150 x 150, d = 34 5.7 / 8.0, d = 40
+ *    19.5 / 23.1; 170 x 170 13.9 / 12.0, 46.5 / 34.9, d = 64 6.5 / 7.9; 200 x 200 33.0 /
+ *    26.8, 113 / 80; 256 x 256 159 / 84, 550 / 251, s = 2 30.9 / 20.6, s = 4 0.94 / 1.88.
  *  - Without symmetry, a compact adjacency of up to 1 MB is expanded straight
  *    from host memory (n = 4096: 27.2 against 29.8 us); larger ones are copied
  *    first, in wider pieces. */
 static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_sweep *sw, int *grid_out)
 {
   if(!lockstep_allowed(sh, t) || t->blocks > 0 || few_sources(sh)) return 0;
+  if(dense_grid(sh) && shape_n(sh) / sh->symmetries > 25000) return 0;
   const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
   memset(sw, 0, sizeof(*sw));
   sw->e.d = sh->degree;
@@ -644,7 +654,7 @@ static int choose_sweep(const odp_shape *sh, const odp_tuning *t, int sms, gbx_s
 /* Whether the team kernel takes a graph of this shape: it must fit the lockstep
  * kernels in one group (bitsets of at most 64 MB, 64 lanes a row, 256 for
  * grids).  Its cost on the whole GPU is estimated from its traffic: a general
- * graph's gathered levels and lists at 10 TB/s; for grids 6.5 visits per row and
+ * graph's gathered levels and lists at 10 TB/s; for tracked grids 6.5 visits per row and
  * lane, each reading d + 2 sectors, at 8 TB/s; its latency from its levels.
  * The constants are fitted to 785 graphs of seven batches on teams of 1/2 to
  * 1/256 of the GPU (error of a graph's time 25 %). */
@@ -653,6 +663,9 @@ int odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_t
   const int n = shape_n(sh), W = shape_words(sh), full_l2 = ilog2_ceil(W < 4 ? 4 : W);
   memset(c, 0, sizeof(*c));
   if(!lockstep_allowed(sh, t) || 16.0 * n * W > 64e6 || W > (sh->grid ? 1024 : 256)) return 0;
+  /* ten dense grids, teams / engine, us: 40 x 60, d = 36 938 / 1085, 52 x 52 1279 /
+   * 1297, 56 x 56 1891 / 1580, 60 x 60 2730 / 1940, 90 x 90, d = 40 20.2 / 15.3 ms */
+  if(dense_grid(sh) && n > 3000) return 0;
   c->e.dp = shape_dp(sh);
   c->B = n / sh->symmetries;
   c->phases = 1;

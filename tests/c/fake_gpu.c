@@ -98,7 +98,7 @@ int gbx_small_launch(const gbx_job *j, int nj, const gbx_expand_desc *d, const g
 size_t gbx_sweep_sync_bytes(void){ return 65536; }
 int fake_asked;                /* gbx_sweep_smem calls */
 size_t gbx_sweep_smem(const gbx_sweep *a){ fake_asked++; return (size_t)a->rows * (size_t)a->e.dp * 4 + 8192; }
-int gbx_sweep_blocks(const gbx_sweep *a, int *per_sm){ *per_sm = gbx_sweep_smem(a) <= 56000 ? 4 : 0; return 0; }
+int gbx_sweep_blocks(const gbx_sweep *a, int *per_sm){ *per_sm = gbx_sweep_smem(a) <= 56000 ? 4 : gbx_sweep_smem(a) <= 200000 ? 1 : 0; return 0; }
 int gbx_sweep_launch(const gbx_sweep *a, int blocks, void *s)
 {
   (void)blocks; (void)s;

@@ -241,3 +241,14 @@ def test_batches_that_lose_on_teams_stay_on_the_engine(fake, graphs, path):
     b = og.Batch([og.GraphSpec(np.zeros((n // s, d), np.int32), nodes=n, symmetries=s) for n, s, d in graphs])
     assert b.path() == path
     b.close()
+
+
+@pytest.mark.parametrize("w,h,d,s,count,path", [(150, 150, 40, 1, 1, "lockstep"), (170, 170, 40, 1, 1, "engine"), (170, 170, 32, 1, 1, "lockstep"),
+                                                (256, 256, 36, 4, 1, "lockstep"), (256, 256, 36, 2, 1, "engine"), (54, 55, 36, 1, 40, "teams"),
+                                                (56, 56, 36, 1, 40, "engine"), (56, 56, 32, 1, 40, "teams")])
+def test_dense_grids_that_lose_in_lockstep_stay_on_the_engine(fake, w, h, d, s, count, path):
+    """Both sides of the lines, and grids whose changes are tracked."""
+    adj = np.zeros((w * h // s, d), np.int32)
+    b = og.Batch([og.GraphSpec(adj, grid=True, width=w, height=h, symmetries=s)] * count)
+    assert b.path() == path
+    b.close()
