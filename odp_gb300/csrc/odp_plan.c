@@ -770,7 +770,7 @@ static void assign_teams(int count, double most, odp_team_graph *g)
  * of n = 8000 to 20000 1.3 to 1.9 times faster).  A batch that would lose more
  * than it gains stays on the engine: 40 of n = 20000, s = 100 578 -> 431 us, 50 of
  * n = 8000, s = 4 551 -> 483, 20 of n = 2000 and 3 of n = 200000, s = 2000 432 -> 333. */
-static double team_slower(const odp_shape *sh)
+double odp_team_slower(const odp_shape *sh)
 {
   const int W = shape_words(sh);
   if(sh->grid || sh->symmetries < 4 || W > 32) return 0;
@@ -802,7 +802,7 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
     all += g[i].cost;
     ord[i].job = i;
     ord[i].work = g[i].cost;
-    const double slower = team_slower(&shapes[i]);
+    const double slower = odp_team_slower(&shapes[i]);
     if(slower > 0) lost += slower * shape_n(&shapes[i]);
     else won += 0.2 * g[i].cost;
   }

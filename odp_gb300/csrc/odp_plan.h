@@ -123,6 +123,8 @@ typedef struct {
 } odp_team_graph;
 #define ODP_TEAM_SMEM (100 * 1024)     /* of a CTA: two per SM */
 int  odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_team_graph *g);
+/* What a row costs more on a small team than on the engine, us (0: no more). */
+double odp_team_slower(const odp_shape *sh);
 
 void odp_tuning_defaults(odp_tuning *t, int batch);
 /* The defaults for `count` graphs with the ODPX_Set_tuning overrides applied. */

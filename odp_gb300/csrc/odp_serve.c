@@ -699,11 +699,14 @@ int ODPX_Serve_register(ODPX_Server *s, const ODP_Graph *gr, int *handle)
    * of five operations, and no hand-off per tile.  32 chains of n = 1024 to
    * 4096, d = 16: 617 -> 392 us a round; one request alone 70 -> 46 us (n =
    * 1024), 107 -> 66 us (n = 4096).  With a graph for the engine among them
-   * all stay on the engine: an engine batch keeps the SMs that it finds free
+   * all stay on the engine (also with one of up to 1024 sources whose rows are
+   * many: 16 of n = 50000, s = 500 392 us a round against 724, of n = 8000, s = 125
+   * 140 / 176, of n = 20000, s = 100 317 / 371, s = 20 437 / 444): an engine batch keeps the SMs that it finds free
    * when it starts, and a team kernel takes half of an SM's registers a CTA. */
   if(!gr->grid && team_blocks > 0 && odp_team_shape(&sh, &tuning, &g.sw, &g.est) && g.sw.nchunks <= TEAM_RECS){
     g.sw.rows = (n + team_blocks - 1) / team_blocks;
-    g.team = gbx_sweep_smem(&g.sw) <= ODP_TEAM_SMEM && g.est.need + 1024.0 <= (double)s->lanes[0].arena_bytes;
+    g.team = gbx_sweep_smem(&g.sw) <= ODP_TEAM_SMEM && g.est.need + 1024.0 <= (double)s->lanes[0].arena_bytes &&
+             !(g.W <= 16 && odp_team_slower(&sh) * n > 1.5);
   }
   size_t adj_ints = (size_t)g.B * g.d;
   g.h_adj = malloc(sizeof(int) * adj_ints);

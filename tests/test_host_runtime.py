@@ -252,3 +252,12 @@ def test_dense_grids_that_lose_in_lockstep_stay_on_the_engine(fake, w, h, d, s, 
     b = og.Batch([og.GraphSpec(adj, grid=True, width=w, height=h, symmetries=s)] * count)
     assert b.path() == path
     b.close()
+
+
+@pytest.mark.parametrize("n,s,kernel", [(8000, 125, "engine"), (4000, 62, "team"), (20000, 100, "engine"), (20000, 10, "team"), (2000, 4, "team")])
+def test_served_graphs_of_many_rows_a_source_stay_on_the_engine(fake, n, s, kernel):
+    n = n // s * s
+    srv = og.Server(max_nodes=n, memory_mb=512)
+    served(srv, [og.GraphSpec(np.zeros((n // s, 8), np.int32), nodes=n, symmetries=s)])
+    assert set(fake.counts) == {kernel}
+    srv.close()
