@@ -13,6 +13,10 @@ winners:
 * chunk width and tile traffic per (ceil log2 n, degree class, grid) bucket
   through ODPX_Set_tuning_table, which every plan created afterwards uses.
 
+All of these are settings of the persistent engine, and a plan with one runs
+there.  The default schedule of most plans runs on the lockstep and team
+kernels, which have none: the search keeps it unless the engine is faster.
+
 Typical use: ``report = tune_batch(specs)`` before timing a batch, or
 ``tune_single(spec)`` for one large graph.
 """

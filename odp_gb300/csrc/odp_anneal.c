@@ -130,10 +130,10 @@ static int resident_cluster(const ODPX_Anneal *a, int range, long long lanes, si
  * teams share two CTAs per SM, or one where two do not fit; a part of the GPU
  * (ODP_GB300_BLOCKS, in engine CTAs, four per SM) becomes the same part of
  * them.  Measured on GB300 against four launches per step (us): 16 chains of
- * n = 1024, d = 8: 15 / 68; one of them: 12 / 48; 8 of n = 4096, d = 16: 85 /
- * 137; 32 of n = 300, d = 6: 12 / 64.  With few CTAs for large graphs the
+ * n = 1024, d = 8: 14.5 / 70; one of them: 11.4 / 49; 8 of n = 4096, d = 16: 75 /
+ * 141; 32 of n = 300, d = 6: 12 / 64.  With few CTAs for large graphs the
  * engine's four CTAs per SM are faster: 16 chains on a quarter of the GPU, n =
- * 2048, d = 16 (32 lanes a thread) 122 / 130, n = 3000, d = 12 (70) 360 / 270, n
+ * 2048, d = 16 (32 lanes a thread) 116 / 132, n = 3000, d = 12 (70) 360 / 270, n
  * = 4096, d = 8 (128) 466 / 348.  Allocates its memory; 0 if the chains do not
  * fit. */
 static int plan_resident(ODPX_Anneal *a, int blocks)

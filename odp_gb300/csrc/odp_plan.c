@@ -1,10 +1,12 @@
 /*
  * odp_plan.c -- builds and runs execution plans (odp_plan.h) on the CUDA
- * layer.  This is the host runtime of the library: it sizes column chunks so
- * the live bitsets stay in L2, orders jobs, lays out device memory, and
- * replays one CUDA graph per evaluation so a call costs one host->device
- * copy, two kernels and one small device->host copy, with no host round trip
- * per BFS level (the reference does one per level, aspl_cuda.cu:62-82).
+ * layer.  This is the host runtime of the library: it chooses the kernels of a
+ * plan, sizes column chunks so the live bitsets stay in L2, orders jobs and lays
+ * out device memory.  A call is one kernel that reads the callers' arrays from
+ * host memory and leaves its records in pinned memory (small, lockstep and team
+ * plans), or a replayed CUDA graph of pull, expand, engine and one copy back,
+ * with no host round trip per BFS level (the reference does one per level,
+ * aspl_cuda.cu:62-82).
  *
  * Result semantics follow the reference exactly (aspl_cuda.cu:84-85,
  * 121-125, 256-260): the ordered sum is accumulated in 64-bit integers,
@@ -350,32 +352,6 @@ static long long small_job_count(const odp_shape *shapes, int count, const int *
   return jobs;
 }
 
-/* Whether a plan runs on the small-graph kernel, and its shape: the chunk
- * width of each graph (wl), the CTAs per job (one thread-block cluster), the
- * threads and shared memory per CTA.  Every graph must have at most small_n
- * vertices and no schedule setting or change tracking may ask for the
- * engine.  The cluster is the largest power of two up to 8 at which every
- * graph fits and every CTA of the plan gets its own SM; for each graph the
- * widest chunk that fits is halved, widest first, while the jobs still fit on
- * the SMs (the n = 1024, d = 8 graph: 8 jobs of 2 words on clusters of 8
- * CTAs, 64 SMs).  Plans that would need more than one wave of CTAs stay on
- * the persistent engine: every job reads its graph's adjacency from host
- * memory, and on GB300 the n = 4096, d = 24 and 32 graphs (32 jobs on
- * clusters of 8, two waves) took 151 and 257 us in the small kernel against
- * 84 and 95 us in the engine, while one-wave graphs up to n = 4096 gained
- * (n = 4096, d = 8: 55 against 85 us; a 64 x 64 grid: 176 against 418 us).
- * The replicated layout (every CTA holds the whole level) is tried first.
- * Plans of grid graphs whose whole level does not fit in one CTA take the
- * partitioned layout (each CTA holds its rows, neighbour rows are read from
- * the CTA that owns them through distributed shared memory), which fits
- * graphs up to `cluster` times larger.  Its gathers run at about one 16-byte
- * request per clock per SM, so it pays only where levels are many and
- * light: on GB300, grids of n = 5184, 6400 and 8100 (diameters 49 to 74)
- * took 265, 301 and 655 us against 547, 626 and 888 us in the engine, while
- * general graphs lost (n = 8192, d = 8: 339 against 122 us; n = 4096,
- * d = 24: 304 against 83 us).  A cluster size forced by
- * ODP_GB300_SMALL_CLUSTER is used if the graphs fit at it (else halved),
- * whatever the SM count; ODP_GB300_SMALL_PART=0 or 1 forces the layout. */
 /* Shared memory and threads of a CTA for chunks of 2^wl[i] words. */
 static void small_shape(const odp_shape *shapes, int count, const int *wl, int c, int part, size_t *smem, int *threads)
 {
@@ -402,6 +378,27 @@ static int small_at_once(const odp_shape *shapes, int count, const int *wl, long
   return smem <= GBX_SMALL_SMEM_MAX && gbx_small_clusters(c, threads, smem, &active) == 0 && active >= jobs;
 }
 
+/* Whether a plan is of the small class, for the small-graph kernel, and its
+ * shape there: the chunk width of each graph (wl), the CTAs per job (one
+ * thread-block cluster), the threads and shared memory per CTA.  Every graph
+ * must have at most small_n vertices and no schedule setting or change tracking
+ * may ask for the engine.  The cluster is the largest power of two up to 8 at
+ * which every graph fits and all jobs run at once; for each graph the widest
+ * chunk that fits is halved, widest first, while they still do (the n = 1024, d
+ * = 8 graph: 8 jobs of 2 words on clusters of 8 CTAs, 64 SMs).  Plans of more
+ * than one wave are for the other kernels: every job reads its graph's adjacency
+ * from host memory, and 32 jobs on clusters of 8 (n = 4096, d = 24 and 32) take
+ * 147 and 216 us against 38 and 41 in lockstep.  The replicated layout (every CTA
+ * holds the whole level) is tried first.  Plans of grid graphs whose whole level
+ * does not fit in one CTA take the partitioned layout (each CTA holds its rows,
+ * neighbour rows are read from the CTA that owns them through distributed shared
+ * memory), which fits graphs up to `cluster` times larger.  Its gathers run at
+ * about one 16-byte request per clock per SM, so it pays only where levels are
+ * many and light: grids of 72 x 72 and 80 x 80, d = 4, 207 and 249 us against 276
+ * and 298 in lockstep, but general graphs lose (n = 8192, d = 8: 260 against 63; n
+ * = 4096, d = 24: 183 against 38).  A cluster size forced by
+ * ODP_GB300_SMALL_CLUSTER is used if the graphs fit at it (else halved),
+ * whatever the SM count; ODP_GB300_SMALL_PART=0 or 1 forces the layout. */
 static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t, int sms, int *wl,
                         int *cluster_out, int *threads_out, size_t *smem_out, int *part_out)
 {
@@ -474,18 +471,20 @@ static int choose_small(const odp_shape *shapes, int count, const odp_tuning *t,
 /* Whether a small plan of one graph, in chunks of 2^wl words, is faster on the
  * lockstep kernel (unless its cluster or layout is forced).  Every job of the
  * small kernel reads the whole adjacency from host memory, so for general
- * graphs the line lies at 450 KB read in all; measured on GB300, small kernel
- * against lockstep (us): n = 512, d = 8 (66 KB) 18 / 21; n = 1182, d = 10, s =
- * 2 (118 KB) 32 / 35 with the call around it; n = 1024, d = 8 (262 KB) 19 / 22;
- * n = 1024, d = 24 (786 KB) 27 / 17; n = 2048, d = 8 (1 MB) 33 / 25; n = 4096, d
- * = 8 (4 MB) 51 / 29.  Grids are bound by their levels: replicated 50 x 50 117
- * / 177, 64 x 64 101 / 180.  Partitioned, a level's time grows with n and d in
- * the small kernel and hardly in lockstep, less so the longer the grid, where
- * fewer rows change: 75 x 75, d = 4 211 / 279, d = 8 226 / 218, d = 10 230 / 165;
- * 90 x 90, d = 4 533 / 371; 171 x 33, d = 4 186 / 241, d = 8 328 / 391, d = 10 264
- * / 227; 190 x 36, d = 4 359 / 470, d = 8 297 / 292; 200 x 41, d = 4 509 / 509.
- * Grids more than twice as high as wide, whose CTAs border on all others: 33 x
- * 171, d = 4 379 / 423, d = 8 500 / 391; 25 x 200, d = 6 561 / 415. */
+ * graphs the line lies at 450 KB read in all; measured on GB300 through
+ * ODPX_Batch_run, small kernel against lockstep (us): n = 512, d = 8 (66 KB) 29 /
+ * 33; n = 1182, d = 10, s = 2 (118 KB) 33 / 36; n = 1024, d = 8 (262 KB) 30 / 33; n =
+ * 1024, d = 24 (786 KB) 37 / 29; n = 2048, d = 8 (1 MB) 43 / 36; n = 4096, d = 8 (4
+ * MB) 65 / 41.  Grids are bound by their levels: replicated 40 x 40, d = 8 62 / 135,
+ * 64 x 64, d = 8 157 / 216; partitioned 50 x 50, d = 4 90 / 186, 64 x 64 119 / 233.
+ * Partitioned, a level's time grows with n and d in the small kernel and hardly
+ * in lockstep, less so the longer the grid, where fewer rows change: 75 x 75, d =
+ * 4 217 / 286, d = 8 268 / 270, d = 10 335 / 297; 80 x 80, d = 4 249 / 298; 90 x 90
+ * 341 to 533 / 371; 171 x 33, d = 4 295 / 423, d = 8 334 / 374, d = 10 405 / 415; 190 x
+ * 36, d = 4 366 / 477, d = 8 418 / 419.  Grids more than twice as high as wide,
+ * whose CTAs border on all others: 33 x 171, d = 4 384 / 430, d = 8 506 / 374; 25 x
+ * 200, d = 6 560 / 422.  (General graphs with the levels
+ * of a grid lose a little: 64 x 64 as one 192 / 208.) */
 static int small_yields(const odp_shape *sh, const odp_tuning *t, int part, int wl)
 {
   if(t->small_cluster > 0 || t->small_part >= 0) return 0;
@@ -673,6 +672,10 @@ int odp_team_shape(const odp_shape *sh, const odp_tuning *t, gbx_sweep *c, odp_t
   if(!c->track && W > 256) return 0;
   c->wc_log2 = c->track ? (full_l2 < 5 ? full_l2 : 5) : (full_l2 < 6 ? full_l2 : 6);
   c->nchunks = c->slots = (W + (1 << c->wc_log2) - 1) >> c->wc_log2;
+  /* Two levels from the lists where a gathered level 2 would read more than 5000
+   * bytes a row (d rows of 8 W), nearly all zeros; below that the marks cost a team
+   * more than the level.  256 graphs 2.86 ms, never two levels 2.92; by the single
+   * graphs' rule drawn batches went from 277 us (geometric mean) to 320 or more. */
   if(!c->track) choose_start(sh, c->e.dp <= GBX_SWEEP_TWO_LEVEL && 8.0 * W * sh->degree > 5000 ? 2 : 1, GBX_SWEEP_SLOTS, c);
   while((32 << c->word_log2) < (c->slots << (c->wc_log2 - 2))) c->word_log2++;
   const double lanes = (c->B + 255) / 256;
@@ -914,8 +917,8 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
 
   /* A small plan: every job runs in the small-graph kernel, its bitsets and
    * row table in the shared memory of one thread-block cluster, with no
-   * device-wide hand-off per level.  Mixed plans keep every job in the
-   * persistent engine, whose short jobs fill the end of a run. */
+   * device-wide hand-off per level.  Other plans, and single graphs past the
+   * line, run in lockstep or on teams where they fit, else on the engine. */
   const int sms = g_sm_count > 0 ? g_sm_count : 1;
   int *small_wl = calloc((size_t)count, sizeof(int));
   int small = choose_small(shapes, count, tuning, sms, small_wl, &p->small_cluster, &p->small_threads,

@@ -16,9 +16,10 @@
  * The unit of work is a lane: 32 bytes of a row (256 sources, one sector),
  * moved by one 256-bit access.
  *
- * sweep_dense_kernel (general graphs): levels 1 and 2 come from the neighbour
- * lists, marked in shared memory and stored once; from level 3 on every lane
- * that is not full gathers, and stops as soon as it is.
+ * sweep_dense_kernel (general graphs): the first levels (one, two, or without
+ * symmetry up to GBX_SWEEP_BASE) come from the neighbour lists, marked in shared
+ * memory and stored once; after them every lane that is not full gathers, and
+ * stops as soon as it is.
  *
  * sweep_track_kernel (grids): rows and sources follow a Hilbert curve, so the
  * 256 sources of a lane lie close together and a row's lane changes in a few
