@@ -80,8 +80,9 @@ int  ODPX_Batch_info(const ODPX_Batch *batch, int graph, int *njobs, int *nslots
  * lockstep on every SM, as larger single graphs do, where that is faster and
  * ODP_GB300_SMALL_CLUSTER and _PART do not ask for the cluster
  * (ODP_GB300_SWEEP=0 turns lockstep off).  Batches run on teams of CTAs in
- * lockstep; plans with explicit schedule settings or change tracking, or with
- * graphs too large for a team, in the persistent engine.  Results are the
+ * lockstep; plans with explicit schedule settings or change tracking, with
+ * graphs too large for a team, or of shapes that are faster there, in the
+ * persistent engine.  Results are the
  * same either way. */
 int  ODPX_Batch_kernel(const ODPX_Batch *batch);
 /* The kernels that evaluate the plan (the last run, if one went to others

@@ -4,6 +4,7 @@ kernels it launches."""
 import ctypes
 import os
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -57,6 +58,14 @@ def fake(library, monkeypatch):
 def ring(n, d=4):
     v = np.arange(n)
     return np.stack([(v + 1 + k) % n for k in range(d)], axis=1).astype(np.int32)
+
+
+def launched(fake, kind):
+    """Waits for the server's thread to launch its batch."""
+    stop = time.monotonic() + 30
+    while kind not in fake.counts and time.monotonic() < stop:
+        time.sleep(1e-4)
+    assert kind in fake.counts
 
 
 def timed_out(call):
@@ -145,8 +154,7 @@ def test_calls_beside_a_servers_long_batches_take_no_cooperative_launch(fake, ki
         h = srv.register(og.GraphSpec(ring(400), grid=True, width=20, height=20))
         fake.pending = 1
         r = srv.submit(h, [])
-        while "engine" not in fake.counts:
-            pass
+        launched(fake, "engine")
         fake.counts = 0
         assert b.run() == want and b.run() == want
         assert set(fake.counts) == {"engine", "pull"} and fake.counts["engine"] == 2
@@ -170,8 +178,7 @@ def test_calls_beside_a_servers_short_team_batches_stay_in_lockstep(fake):
     fake.abort_at = fake.total + 1                       # no records: in flight until its event is complete
     fake.pending = 1
     r = srv.submit(h, [])
-    while "team" not in fake.counts:
-        pass
+    launched(fake, "team")
     fake.counts = fake.abort_at = 0
     b.run()
     assert fake.counts == {"sweep": 1}
@@ -191,8 +198,7 @@ def test_timing_after_a_call_beside_a_server_reads_that_calls_arrays(fake):
     h = srv.register(og.GraphSpec(ring(400), grid=True, width=20, height=20))
     fake.pending = 1
     r = srv.submit(h, [])
-    while "engine" not in fake.counts:
-        pass
+    launched(fake, "engine")
     fake.counts = 0
     b.run([second])
     assert fake.counts["engine"] == 1 and "sweep" not in fake.counts
