@@ -788,7 +788,7 @@ double odp_team_slower(const odp_shape *sh)
  * levels run side by side on small teams: 18 graphs of n = 360 to 2880, 366 ->
  * 207 us on GB300 with the fitted estimates. */
 static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, int sms, gbx_sweep *gs,
-                       gbx_team *tm, int *order, int *grid_out, size_t *smem_out)
+                       gbx_team *tm, int *order, int *grid_out, size_t *smem_out, double *estimate)
 {
   if(count == 1) return 0;
   int fit = 0;
@@ -836,6 +836,7 @@ static int choose_team(const odp_shape *shapes, int count, const odp_tuning *t, 
       }
       best = m;
     }
+    *estimate = best;
     for(int i = 0; i < count; i++){
       const int size = grid >> g[i].split;
       gs[i].rows = (shape_n(&shapes[i]) + size - 1) / size;
@@ -926,13 +927,18 @@ int odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning
   p->small_class = small;
   p->sweep = count == 1 && (!small || small_yields(shapes, tuning, p->small_part, small_wl[0])) &&
              choose_sweep(shapes, tuning, sms, &p->sw, &p->sweep_grid);
-  if(p->sweep) small = 0;
+  if(p->sweep){
+    gbx_sweep c;
+    odp_team_graph g;
+    p->estimate = odp_team_shape(shapes, tuning, &c, &g) ? g.cost + g.latency : HUGE_VAL;
+    small = 0;
+  }
   int *team_order = NULL;
   if(!small && !p->sweep){
     p->h_teams = calloc((size_t)count, sizeof(gbx_sweep));
     team_order = calloc((size_t)count, sizeof(int));
     p->team = p->h_teams && team_order &&
-              choose_team(shapes, count, tuning, sms, p->h_teams, &p->tm, team_order, &p->sweep_grid, &p->team_smem);
+              choose_team(shapes, count, tuning, sms, p->h_teams, &p->tm, team_order, &p->sweep_grid, &p->team_smem, &p->estimate);
   }
   const int lockstep = p->sweep || p->team;
 
@@ -1655,10 +1661,15 @@ int odp_plan_finish(odp_plan *p, odp_result *results)
  * the kernels that its shapes take without lockstep (a plan of its own, made the
  * first time).  Measured on GB300, us, n = 4096, d = 24 through ODP_Set_aspl,
  * lockstep against this, beside chains of n = 8192: 966 / 395; 16384: 2618 / 155;
- * 32768: 7262 / 163; 90 x 90 grids: 6678 / 142; alone 33 / 76. */
+ * 32768: 7262 / 163; 90 x 90 grids: 6678 / 142; alone 33 / 76.  Behind team
+ * batches, which leave less room to other kernels, a call of more than 200 us
+ * waits: beside chains of n = 8192, n = 9999 (110 us by the estimate) 1035 / 547, 40
+ * graphs of n = 300 to 2000 1556 / 735, but n = 20000 (230) 1278 / 1329, 97 x 103 grid
+ * (300) 1077 / 2270. */
 static odp_plan *plan_for_call(odp_plan *p)
 {
-  if(!p->shapes || !odp_serving()) return p;
+  const int held = p->shapes ? odp_serving() : 0;
+  if(!held || (held == 1 && p->estimate > 200.0)) return p;
   if(!p->beside){
     odp_tuning t = p->tuning;
     t.sweep = 0;

@@ -104,6 +104,7 @@ typedef struct odp_plan {
   void *d_sync;                /* its counters */
   unsigned int *h_abort;       /* pinned: set when one of its waits ran out */
   odp_shape *shapes;           /* lockstep plans: the shapes, with degree tables of their own */
+  double estimate;             /* us of a call in lockstep, alone */
   struct odp_plan *beside;     /* the same shapes without lockstep, for calls beside a busy server */
   struct odp_plan *ran;        /* the plan that the last call ran, this one or `beside` */
 } odp_plan;
@@ -130,7 +131,7 @@ void odp_tuning_defaults(odp_tuning *t, int batch);
 /* The defaults for `count` graphs with the ODPX_Set_tuning overrides applied. */
 void odp_tuning_for(int count, odp_tuning *t);
 /* Batches in flight, of all servers of the process, that hold their part of
- * the GPU for long. */
+ * the GPU for long: 2 if there are any of the engine, 1 of the team kernel, or 0. */
 int  odp_serving(void);
 /* Returns 0 on success, else an ODPX_ERR_* code (include/odp_gb300.h). */
 int  odp_plan_create(const odp_shape *shapes, int count, const odp_tuning *tuning, odp_plan **out);

@@ -84,7 +84,7 @@ typedef struct {
   long long *members;          /* request ids of the running batch */
   int *b_first, *b_count;      /* a team batch's members' writes */
   int nmembers;
-  int holds;                   /* the batch counts among those of odp_serving */
+  int holds;                   /* the batch counts among those of odp_serving: 1, 2 (0: it does not) */
   /* the batch formed and not yet issued */
   int b_nw, b_njobs, b_nslots;
   size_t b_slots_off, b_jobs_off, b_outcomes_off, b_acc_bytes;
@@ -248,14 +248,19 @@ static int delta_writes(serve_graph *g, const ODPX_Delta *dl, gbx_write *w)
  * 491 / 853; beside 32 of n = 8192 (1000): 966 / 395, 1278 / 1280, 1077 / 2096, 40
  * graphs of n = 300 to 2000 1556 / 861. */
 #define HOLD_US 300.0
-static int g_serving = 0;
+static int g_serving[2] = {0, 0};     /* of the team kernel, of the engine */
 
-int odp_serving(void) { return __atomic_load_n(&g_serving, __ATOMIC_RELAXED); }
-
-static void hold(serve_lane *l, int on)
+int odp_serving(void)
 {
-  if(l->holds != on) __atomic_add_fetch(&g_serving, on - l->holds, __ATOMIC_RELAXED);
-  l->holds = on;
+  return __atomic_load_n(&g_serving[1], __ATOMIC_RELAXED) ? 2 : __atomic_load_n(&g_serving[0], __ATOMIC_RELAXED) ? 1 : 0;
+}
+
+/* kind: 0 the lane's batch does not hold the GPU, 1 of the team kernel, 2 of the engine */
+static void hold(serve_lane *l, int kind)
+{
+  if(l->holds) __atomic_sub_fetch(&g_serving[l->holds - 1], 1, __ATOMIC_RELAXED);
+  if(kind) __atomic_add_fetch(&g_serving[kind - 1], 1, __ATOMIC_RELAXED);
+  l->holds = kind;
 }
 
 /* Whether all records of lane l's team batch have arrived. */
@@ -441,7 +446,7 @@ static int form_batch(odp_server *s, serve_lane *l, double max_seed_cost)
     form_team(s, l, nreq);
     return nreq;
   }
-  hold(l, 1);
+  hold(l, 2);
 
   /* Active slots: as many leading jobs as fit the lane's share of L2 (at
    * least one).  Lanes run at the same time, so their bitsets together must

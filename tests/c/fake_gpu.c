@@ -15,6 +15,7 @@ int fake_abort_at;             /* that launch (from 1): a wait runs out, no reco
 int fake_late_at;              /* that launch: complete, and then a wait runs out all the same */
 const int *fake_adjacency;     /* of the last lockstep launch */
 int fake_pending;              /* events are not complete while set */
+int fake_pending_from;         /* nor from that launch on */
 
 static int next(int kind)
 {
@@ -49,7 +50,12 @@ int gbx_scatter(const gbx_write *w, int n, void *s)
 int gbx_event_create(void **e){ *e = malloc(1); return 0; }
 int gbx_event_destroy(void *e){ free(e); return 0; }
 int gbx_event_record(void *e, void *s){ (void)e; (void)s; return 0; }
-int gbx_event_query(void *e){ (void)e; return __atomic_load_n(&fake_pending, __ATOMIC_ACQUIRE); }
+int gbx_event_query(void *e)
+{
+  (void)e;
+  const int from = __atomic_load_n(&fake_pending_from, __ATOMIC_ACQUIRE);
+  return __atomic_load_n(&fake_pending, __ATOMIC_ACQUIRE) || (from && fake_total >= from);
+}
 int gbx_event_elapsed_ms(void *a, void *b, float *ms){ (void)a; (void)b; *ms = 1.0f; return 0; }
 int gbx_capture_begin(void *s){ (void)s; return 1; }       /* plans are created with use_graph off */
 int gbx_capture_end(void *s, void **g){ (void)s; *g = NULL; return 1; }

@@ -52,7 +52,7 @@ def fake(library, monkeypatch):
     monkeypatch.setenv("ODP_GB300_GRAPH", "0")
     f = Fake(og.load())
     yield f
-    f.abort_at = f.late_at = f.pending = 0
+    f.abort_at = f.late_at = f.pending = f.pending_from = 0
 
 
 def ring(n, d=4):
@@ -267,3 +267,35 @@ def test_served_graphs_of_many_rows_a_source_stay_on_the_engine(fake, n, s, kern
     served(srv, [og.GraphSpec(np.zeros((n // s, 8), np.int32), nodes=n, symmetries=s)])
     assert set(fake.counts) == {kernel}
     srv.close()
+
+
+def test_long_calls_wait_for_team_batches(fake):
+    """Behind long team batches a short call goes to the other kernels, a long one
+    stays in lockstep."""
+    plans = [og.Batch([g]) for g in (og.GraphSpec(ring(4096, 24), nodes=4096), og.GraphSpec(ring(97 * 103, 6), grid=True, width=97, height=103),
+                                     og.GraphSpec(ring(30000, 4), nodes=30000))]
+    srv = og.Server(lanes=1, max_nodes=8192, memory_mb=512)
+    handles = [srv.register(og.GraphSpec(ring(8192, 8), nodes=8192)) for _ in range(17)]
+    fake.pending = 1
+    fake.abort_at = fake.total + 1                       # a batch of one, in flight without records
+    ids = [srv.submit(handles[0], [])]
+    launched(fake, "team")
+    ids += [srv.submit(h, []) for h in handles[1:]]      # these wait for the lane, and then make one batch
+    for b in plans:
+        b.run()
+    assert [b.path() for b in plans] == ["lockstep"] * 3
+    fake.counts = 0
+    fake.abort_at = fake.pending_from = fake.total + 1   # which stays in flight as well
+    fake.pending = 0
+    launched(fake, "team")
+    for b in plans:
+        b.run()
+    assert [b.path() for b in plans] == ["engine", "lockstep", "lockstep"]
+    fake.pending_from = 0
+    for r in ids:
+        assert timed_out(lambda: srv.wait(r))
+    srv.close()
+    for b in plans:
+        b.run()
+        assert b.path() == "lockstep"
+        b.close()
